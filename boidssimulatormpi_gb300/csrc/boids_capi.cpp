@@ -745,6 +745,7 @@ static int step_once(boids_sim *s, bool rec)
         {
             PhaseTimer pt(s, 0);
             CK(boidsgpu::launch_grid_scan(s->k, s->b, s->stream, &s->launches));
+            CK(boidsgpu::launch_grid_classify(s->k, s->b, s->stream, &s->launches));
             CK(boidsgpu::launch_grid_scatter(s->k, s->b, s->cur, true, s->stream, &s->launches));
             s->acc.bin_launches += 2;
         }
@@ -1066,6 +1067,7 @@ int boids_get_neighbor_sets(boids_sim *s, int32_t *count3n, uint64_t *hash3n)
     if (!s->b.dhash && (rc = dalloc(&s->b.dhash, 3 * cap))) return rc;
     if (s->engine == 1) {
         CK(boidsgpu::launch_grid_scan(s->k, s->b, s->stream, &s->launches));
+        CK(boidsgpu::launch_grid_classify(s->k, s->b, s->stream, &s->launches));
         CK(boidsgpu::launch_grid_scatter(s->k, s->b, s->cur, false, s->stream, &s->launches));
         CK(boidsgpu::launch_grid_force(s->k, s->b, 1 - s->cur, true, false, s->stream, &s->launches));
     } else {

@@ -162,16 +162,17 @@ constexpr int kTuneCount = sizeof(kTuneCand) / sizeof(kTuneCand[0]);
 // The dense kernel's work items are (full-size cell, first boid) pairs, one
 // per kDenseRound boids of a dense cell, so that the boids of one crowded
 // cell spread over several CTAs.  Words the work list can need in one step:
-// at most one item per non-empty cell plus one per kDenseRound boids, two
-// words per item.
-constexpr int kDenseRound = 128;
+// at most one item per non-empty cell plus one per kDenseRound boids, and
+// never more than one per boid, two words per item.
+constexpr int kDenseRound = 32;
 inline size_t dense_list_capacity(size_t ncell, size_t n)
 {
     const size_t by_cells = ncell / 4;
-    return 2 * ((by_cells < n ? by_cells : n) + n / kDenseRound + 1);
+    const size_t items = (by_cells < n ? by_cells : n) + n / kDenseRound + 1;
+    return 2 * (items < n ? items : n);
 }
 constexpr int kDenseCap = 512;        // candidates of a dense cell held in shared memory
-constexpr int kDenseCtasPerSm = 7;   // resident CTAs of the dense-cell kernel per SM (its launch bounds)
+constexpr int kDenseCtasPerSm = 8;   // resident CTAs of the dense-cell kernel per SM (its launch bounds)
 constexpr int kApCap = 256;           // all-pairs engine: neighbours kept per boid (more: an O(N) scan)
 constexpr uint32_t kMaxBoids = 1u << 29;  // slot index packs into 29 bits
 constexpr int kMaxGridAxis = 812;          // device cells per axis: 4 G^3 < 2^31
@@ -202,10 +203,13 @@ cudaError_t launch_frame(const float4 *pos4, const float4 *vel4, const float *fo
 cudaError_t launch_grid_keys(const StepConst &k, const float4 *pos, uint32_t *key, uint32_t *rank,
                              uint32_t *count, cudaStream_t s, uint64_t *launches,
                              const FlockTable *ft = nullptr);
-// Scan of the cell counts, then the dense-cell classification (flags and
-// work list) of every full-size cell.
+// Scan of the cell counts; clears the step's work counters.
 cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream_t s, uint64_t *launches,
                              const FlockTable *ft = nullptr);
+// After the scan: the dense-cell classification (flags and work list) of
+// every full-size cell.
+cudaError_t launch_grid_classify(const StepConst &k, const DevBuffers &b, cudaStream_t s, uint64_t *launches,
+                                 const FlockTable *ft = nullptr);
 cudaError_t launch_grid_scatter(const StepConst &k, const DevBuffers &b, int from, bool zero_counts,
                                 cudaStream_t s, uint64_t *launches, const FlockTable *ft = nullptr);
 // Rules + integration over the sorted state b.pos[from]; writes the new state

@@ -135,6 +135,7 @@ int step_once(boids_ensemble *e)
 {
     if (!e->binned) {
         CK(boidsgpu::launch_grid_scan(e->ks[0], e->b, e->stream, &e->launches, &e->ft));
+    CK(boidsgpu::launch_grid_classify(e->ks[0], e->b, e->stream, &e->launches, &e->ft));
         CK(boidsgpu::launch_grid_scatter(e->ks[0], e->b, e->cur, true, e->stream, &e->launches, &e->ft));
         e->cur = 1 - e->cur;
     }
@@ -149,6 +150,7 @@ int bin_now(boids_ensemble *e)
 {
     if (e->binned) return 0;
     CK(boidsgpu::launch_grid_scan(e->ks[0], e->b, e->stream, &e->launches, &e->ft));
+    CK(boidsgpu::launch_grid_classify(e->ks[0], e->b, e->stream, &e->launches, &e->ft));
     CK(boidsgpu::launch_grid_scatter(e->ks[0], e->b, e->cur, true, e->stream, &e->launches, &e->ft));
     e->cur = 1 - e->cur;
     e->binned = true;

@@ -1227,22 +1227,15 @@ constexpr int kDenseKT = kDenseCap / kDT;      // candidates per thread when the
 
 constexpr int kMaxCuts = 32;                   // id windows of a huge cell planned at once
 
-// Accepted neighbours are marked in three bit masks per boid (cohesion,
-// separation, alignment) over the id-ordered candidate list; the ordered sums
-// then walk the masks.  kMaskWords words hold the masks of one round of
-// boids, so a round takes at most kMaskWords / (3 * words) boids.
-constexpr int kMaskWords = kDenseCap + kRadixWords(kDT);
-// At most kSumsMax boids per round: the per-boid table of the exact tests and
-// the per-boid results of the ordered sums hold that many.
-constexpr int kSumsMax = 72;
-// Filter hits queued per warp for the exact tests: a filter iteration adds at
-// most two per lane, so the queue is flushed once it holds kQueue - 64.
-constexpr int kQueue = 192;
+// A warp's ring of filter hits: an iteration adds at most 64 to fewer than 32.
+constexpr int kHitRing = 128;
+// Columns of a warp's staged summands, padded so that the nine rows' 16-byte
+// reads fall into different banks.
+constexpr int kSumCols = 36;
 
 // Shared memory of k_grid_dense.  Regions whose lifetimes do not overlap
-// share storage: the sort keys become the id-ordered candidate array, the
-// gather slots and radix histogram become the rule masks, and the filter-hit
-// buffers become the per-boid sums.
+// share storage: the sort keys become the id-ordered candidate array, and the
+// gather slots and sort counters become the warps' staged summands.
 struct DenseSmem {
     union {
         uint64_t keys[2][kDenseCap];  // (id << 16) | (segment << 11) | gather index
@@ -1253,15 +1246,10 @@ struct DenseSmem {
             uint32_t gslot[kDenseCap];      // state slot, by gather index
             uint32_t hist[kRadixWords(kDT)];  // sort counters (block_bucket_sort, block_radix_sort)
         } s;
-        uint32_t masks[kMaskWords];         // rule r of round boid i: words (r * nbr + i) * wstride ...
+        __align__(16) float st[kDT / 32][9][kSumCols];  // per warp: a round's summands, by component
     } v;
-    union {
-        struct {
-            uint32_t queue[kDT / 32][kQueue];  // per warp: filter hits, round boid << 11 | candidate
-            float4 obs[2][kSumsMax];           // per round boid: (position, |v|), (velocity, 1/|v|)
-        } a;
-        Acc sums[kSumsMax];                    // the ordered sums of each boid of the round
-    } w;
+    uint16_t hits[kDT / 32][kHitRing];     // per warp: filter hits (candidates), a ring
+    uint32_t res[12][kDenseRound + 1];     // the item's sums and counts, by boid
     uint32_t seg_j0[18], seg_k0[19];
     float seg_s[18][3];
     uint32_t work, flock;
@@ -1288,109 +1276,6 @@ static_assert(kDenseCap <= 2048, "gather index must fit 11 bits");
 // |xj - xi| > F/2 holds (|xj - xi| > F - R) and inside the field it fails
 // (|xj - xi| < R).  Where the reference images a candidate otherwise, it is
 // farther than R from the boid in both placements and no rule accepts it.
-
-// The ordered sums of a round's boids run as jobs, each a (job, boid) pair
-// taken by one lane, job-major so that the lanes of a warp run the same code:
-// jobs 0-5 are the cohesion sum's x, y, z and the alignment sum's x, y, z
-// (jobs 0 and 3 also count), job 6 the separation sum (all three components,
-// from the normalised offsets), job 7 the neighbour-set id hashes
-// (diagnostics only).  Each walks its rule's mask word by word from candidate
-// 0 up: ascending id, the reference's order of accumulation, so every float
-// sum is the reference's sequence of additions.  A job's running value starts
-// from the earlier id windows' partial sums (carry) or zero, and ends in out.
-__device__ __forceinline__ void dense_sum_job(const DenseSmem &sm, const uint32_t *m, uint32_t words, uint32_t job,
-                                              const Acc *carry, Acc &out)
-{
-    const bool coh = job < 3;
-    const uint32_t c = job % 3;
-    // the summands: the candidates' imaged positions, or their velocities
-    const float *base = coh ? reinterpret_cast<const float *>(sm.u.spos) + c
-                            : (c == 0 ? sm.svx : (c == 1 ? sm.svy : sm.svz));
-    const uint32_t sh = coh ? 2u : 0u;  // element q at base[q << sh]
-    float *dst = reinterpret_cast<float *>(&out) + (coh ? 0 : 6) + c;
-    float acc = carry ? reinterpret_cast<const float *>(carry)[(coh ? 0 : 6) + c] : 0.f;
-    int cnt = 0;
-    uint32_t next = words > 0 ? m[0] : 0u;  // each mask word is read one word ahead
-    for (uint32_t w = 0; w < words; ++w) {
-        uint32_t bits = next;
-        if (w + 1 < words) next = m[w + 1];
-        cnt += __popc(bits);
-        const uint32_t q0 = w * 32;
-        // four entries per iteration: their loads in flight together, their
-        // additions in order
-        while (bits) {
-            const uint32_t b0 = (uint32_t)__ffs(bits) - 1;
-            bits &= bits - 1;
-            const bool h1 = bits != 0;
-            const uint32_t b1 = h1 ? (uint32_t)__ffs(bits) - 1 : b0;
-            bits &= bits - 1;
-            const bool h2 = bits != 0;
-            const uint32_t b2 = h2 ? (uint32_t)__ffs(bits) - 1 : b0;
-            bits &= bits - 1;
-            const bool h3 = bits != 0;
-            const uint32_t b3 = h3 ? (uint32_t)__ffs(bits) - 1 : b0;
-            bits &= bits - 1;
-            const float v0 = base[(q0 + b0) << sh], v1 = base[(q0 + b1) << sh];
-            const float v2 = base[(q0 + b2) << sh], v3 = base[(q0 + b3) << sh];
-            acc = __fadd_rn(acc, v0);
-            if (h1) acc = __fadd_rn(acc, v1);
-            if (h2) acc = __fadd_rn(acc, v2);
-            if (h3) acc = __fadd_rn(acc, v3);
-        }
-    }
-    *dst = acc;
-    if (c == 0) {
-        int *n = coh ? &out.ncoh : &out.nali;
-        *n = cnt + (carry ? (coh ? carry->ncoh : carry->nali) : 0);
-    }
-}
-
-// Job 6: the separation sum (Vector3D::normalized of pi - t, as acc_add).
-__device__ __forceinline__ void dense_sep_job(const DenseSmem &sm, const uint32_t *m, uint32_t words, float3 pi,
-                                              const Acc *carry, Acc &out)
-{
-    float3 sep = carry ? carry->sep : make_float3(0.f, 0.f, 0.f);
-    int cnt = carry ? carry->nsep : 0;
-    uint32_t next = words > 0 ? m[0] : 0u;
-    for (uint32_t w = 0; w < words; ++w) {
-        uint32_t bits = next;
-        if (w + 1 < words) next = m[w + 1];
-        cnt += __popc(bits);
-        while (bits) {
-            const uint32_t q = w * 32 + (uint32_t)(__ffs(bits) - 1);
-            bits &= bits - 1;
-            const float4 t = sm.u.spos[q];
-            const float dx = __fsub_rn(pi.x, t.x), dy = __fsub_rn(pi.y, t.y), dz = __fsub_rn(pi.z, t.z);
-            const float n = nrm3(dx, dy, dz);
-            sep.x = __fadd_rn(sep.x, __fdiv_rn(dx, n));
-            sep.y = __fadd_rn(sep.y, __fdiv_rn(dy, n));
-            sep.z = __fadd_rn(sep.z, __fdiv_rn(dz, n));
-        }
-    }
-    out.sep = sep;
-    out.nsep = cnt;
-}
-
-// Job 7 (diagnostics): the order-free id fingerprints of the three sets.
-__device__ __forceinline__ void dense_hash_job(const DenseSmem &sm, const uint32_t *m0, uint32_t rstride,
-                                               uint32_t words, const Acc *carry, Acc &out,
-                                               const float4 *__restrict__ pos)
-{
-    for (uint32_t r = 0; r < 3; ++r) {
-        const uint32_t *m = m0 + r * rstride;
-        uint64_t h = carry ? carry->h[r] : 0;
-        for (uint32_t w = 0; w < words; ++w) {
-            uint32_t bits = m[w];
-            while (bits) {
-                const uint32_t q = w * 32 + (uint32_t)(__ffs(bits) - 1);
-                bits &= bits - 1;
-                const uint32_t j = __float_as_uint(sm.u.spos[q].w);
-                h += id_hash(__float_as_uint(__ldg(&pos[j].w)));
-            }
-        }
-        out.h[r] = h;
-    }
-}
 
 // Id window of a huge cell (more than kDenseCap candidates): the largest hi
 // such that the candidates with ids in [lo, hi) fit the shared list.  A
@@ -1522,18 +1407,27 @@ __device__ void dense_window_plan(DenseSmem &sm, const GridIn &g, int ns, uint32
 }
 
 // One CTA takes one work item at a time (dynamic queue): a crowded cell and
-// up to 128 of its boids (a cell with more boids is several items, taken by
-// several CTAs).  The cell's 27-cell candidates are radix-sorted by id once
-// per item.  The item's boids go in rounds; the round's nbr boids x the
-// candidate list is split over all threads: each boid gets L = 128/nbr
-// lanes, lane l walks chunk l of the id-ordered list with the
-// half-precision filter and exact tests, and marks the accepted neighbours
-// in the boid's three rule masks (bit q = candidate q).  The ordered sums
-// then run as jobs, one float sum (or the separation sum) per lane of the
-// boid, each walking its mask from candidate 0 up: ascending id, as the
-// reference accumulates.  A cell with more than kDenseCap candidates is done
-// in ascending id windows that each fit the list; the sums are carried from
-// window to window through o.carry.
+// up to kDenseRound of its boids (a cell with more boids is several items,
+// taken by several CTAs).  The cell's 27-cell candidates are sorted by id once
+// per item.  Then each warp takes a boid at a time: its lanes filter the list
+// in half precision, 64 candidates an iteration, the hits are compacted into
+// the warp's queue, 32 of them at a time take the exact tests, and the
+// accepted, compacted again, are added up by nine lanes, one component of the
+// three rules' sums each.  The list is in id order and every compaction keeps
+// it, so the sums are in ascending id, as the reference accumulates.  A cell
+// with more than kDenseCap candidates is done in ascending id windows that
+// each fit the list; the sums are carried from window to window through
+// o.carry.
+//
+// Bound by instruction issue (74 % of the slots at 8 CTAs per SM, N = 2^20
+// after 1000 updates).  A warp per boid replaced a lane per (boid, chunk of
+// candidates) with rule masks and a lane per sum: that form needed a round of
+// up to 72 boids to fill its lanes, so items held up to 128 boids and a small
+// flock's few items left most SMs idle.  Items of 32 boids and no barrier
+// between a boid's filter and its sums took a step of 1000 boids of test.ini
+// from 209 to 108 us, of gathered flocks of 16 384 boids from 250 to 188 us,
+// of 65 537 from 376 to 264, of 262 143 from 697 to 603 and of 2^20 from 2350
+// to 2228 (alternating runs of both builds on one GB300).
 template <bool DIAG, bool MULTI>
 __global__ void __launch_bounds__(kDT, kDenseCtasPerSm)
 k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint32_t *__restrict__ dense_n,
@@ -1694,146 +1588,169 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
             __syncthreads();
             const bool first = lo == 0, last = hi >= k.n;
 
-            // The item's boids go in rounds of nbr (as many as the rule masks
-            // and the per-boid sums hold); each boid of a round gets L lanes.
-            const uint32_t words = (nw + 31) / 32, wstride = words | 1u;  // odd: boids' words in other banks
-            const uint32_t pool_nbr = (uint32_t)kMaskWords / (3u * wstride);
+            // A warp per boid of the item.  The candidates are in id order, so the
+            // filter's hits, the accepted among them and their summands are too.
             const uint32_t rend = min(b, rbeg + (uint32_t)kDenseRound);
-            const uint32_t njobs = DIAG ? 8u : 7u;
-            for (uint32_t r0 = rbeg; r0 < rend;) {
-                const uint32_t nbr = min(min(rend - r0, (uint32_t)kDT), min((uint32_t)kSumsMax, pool_nbr));
-                const uint32_t L = (uint32_t)kDT / nbr;               // lanes per boid
-                const uint32_t csz = ((nw + L - 1) / L + 1) & ~1u;    // chunk length (even: whole pairs)
-                const bool act = (uint32_t)t < nbr * L;
-                const uint32_t bi = act ? (uint32_t)t % nbr : 0, l = act ? (uint32_t)t / nbr : 0;
-                const uint32_t k0 = act ? min(nw, l * csz) : 0, k1 = act ? min(nw, k0 + csz) : 0;
-                uint32_t *masks = sm.v.masks;
-                for (uint32_t i = (uint32_t)t; i < 3 * nbr * wstride; i += kDT) masks[i] = 0;
-                // the round's boids, for the filter constants and the exact tests
-                for (uint32_t i = (uint32_t)t; i < nbr; i += kDT) {
-                    const float4 pp = g.pos[own0 + r0 + i], vv = g.vel[own0 + r0 + i];
-                    const Sight sg = make_sight(xyz(vv));
-                    sm.w.a.obs[0][i] = make_float4(pp.x, pp.y, pp.z, sg.nv);
-                    sm.w.a.obs[1][i] = make_float4(vv.x, vv.y, vv.z, sg.inv_nv);
+            const uint32_t npairs = (nw + 1) / 2;
+            const int lane = t & 31, wid = t >> 5;
+            const unsigned below = (1u << lane) - 1u;
+            uint16_t *hits = sm.hits[wid];
+            float(&st)[9][kSumCols] = sm.v.st[wid];
+            for (uint32_t i = rbeg + wid; i < rend; i += kDT / 32) {
+                const uint32_t s = own0 + i;
+                const float3 pi = xyz(__ldg(g.pos + s));
+                const Sight si = make_sight(xyz(__ldg(g.vel + s)));
+                // lane c < 9: component c of (cohesion, separation, alignment)
+                float acc = 0.f;
+                int ncoh = 0, nsep = 0, nali = 0;
+                uint64_t h0 = 0, h1 = 0, h2 = 0;
+                if (!first) {  // the earlier id windows' sums
+                    const Acc *cin = o.carry + s;
+                    if (lane < 9) acc = reinterpret_cast<const float *>(cin)[lane];
+                    ncoh = cin->ncoh;
+                    nsep = cin->nsep;
+                    nali = cin->nali;
                 }
-                __syncthreads();  // the masks are clear, the table is written
-                {
-                    const float4 o0 = sm.w.a.obs[0][bi], o1 = sm.w.a.obs[1][bi];
-                    const float3 pi = xyz(o0), vi = xyz(o1);
-                    // The filter in half precision, two candidates per instruction:
-                    // it keeps every pair within the filter radius and drops only
-                    // pairs whose exact v . r is negative (the bounds are in hfilt,
-                    // hdot0 and hdot1); the exact tests decide the rest.
-                    const __half2 bx = __float2half2_rn((pi.x - cen.x) * k.hsc);
-                    const __half2 by = __float2half2_rn((pi.y - cen.y) * k.hsc);
-                    const __half2 bz = __float2half2_rn((pi.z - cen.z) * k.hsc);
-                    const float vt = o0.w * k.hvsc;
-                    const bool pre = k.cone_pre && vt <= 1.0f;
-                    const __half2 hvx = __float2half2_rn(pre ? vi.x * k.hvsc : 0.f);
-                    const __half2 hvy = __float2half2_rn(pre ? vi.y * k.hvsc : 0.f);
-                    const __half2 hvz = __float2half2_rn(pre ? vi.z * k.hvsc : 0.f);
-                    const __half2 hf2 = __half2half2(__float2half_ru(k.hfilt));
-                    const __half2 hd2 = __half2half2(pre ? __float2half_rd(-(k.hdot0 + k.hdot1 * vt))
-                                                         : __ushort_as_half((unsigned short)0xfc00u));  // -inf
-                    const uint32_t p0 = k0 >> 1, plen = k1 > k0 ? ((k1 + 1) >> 1) - p0 : 0;  // pairs
-                    const uint32_t maxlen = __reduce_max_sync(0xffffffffu, plen);
-                    const int lane = t & 31;
-                    uint32_t *queue = sm.w.a.queue[t >> 5];
-                    uint32_t qlen = 0;  // the same in every lane of the warp
-                    // exact tests of the queued hits, every lane of the warp
-                    // busy; accepted neighbours are marked in the boid's masks
-                    auto flush = [&]() {
+                // The filter in half precision, two candidates per instruction:
+                // it keeps every pair within the filter radius and drops only
+                // pairs whose exact v . r is negative (the bounds are in hfilt,
+                // hdot0 and hdot1); the exact tests decide the rest.
+                const __half2 bx = __float2half2_rn((pi.x - cen.x) * k.hsc);
+                const __half2 by = __float2half2_rn((pi.y - cen.y) * k.hsc);
+                const __half2 bz = __float2half2_rn((pi.z - cen.z) * k.hsc);
+                const float vt = si.nv * k.hvsc;
+                const bool pre = k.cone_pre && vt <= 1.0f;
+                const __half2 hvx = __float2half2_rn(pre ? si.v.x * k.hvsc : 0.f);
+                const __half2 hvy = __float2half2_rn(pre ? si.v.y * k.hvsc : 0.f);
+                const __half2 hvz = __float2half2_rn(pre ? si.v.z * k.hvsc : 0.f);
+                const __half2 hf2 = __half2half2(__float2half_ru(k.hfilt));
+                const __half2 hd2 = __half2half2(pre ? __float2half_rd(-(k.hdot0 + k.hdot1 * vt))
+                                                     : __ushort_as_half((unsigned short)0xfc00u));  // -inf
+                uint32_t qh = 0, nq = 0;  // the ring's head and length, the same in every lane
+                for (uint32_t p0 = 0; p0 < npairs; p0 += 32) {
+                    const uint32_t pp = p0 + lane;
+                    unsigned keep = 0;
+                    if (pp < npairs) {
+                        const __half2 dx = __hsub2(sm.hx[pp], bx), dy = __hsub2(sm.hy[pp], by),
+                                      dz = __hsub2(sm.hz[pp], bz);
+                        const __half2 d2 = __hfma2(dz, dz, __hfma2(dy, dy, __hmul2(dx, dx)));
+                        const __half2 dv = __hfma2(hvz, dz, __hfma2(hvy, dy, __hmul2(hvx, dx)));
+                        keep = __hlt2_mask(d2, hf2) & __hge2_mask(dv, hd2);
+                    }
+                    const bool e0 = keep & 1u, e1 = keep >> 16;
+                    const unsigned m0 = __ballot_sync(0xffffffffu, e0), m1 = __ballot_sync(0xffffffffu, e1);
+                    uint32_t at = qh + nq + __popc(m0 & below) + __popc(m1 & below);
+                    if (e0) hits[at++ & (kHitRing - 1)] = (uint16_t)(2 * pp);
+                    if (e1) hits[at & (kHitRing - 1)] = (uint16_t)(2 * pp + 1);
+                    nq += __popc(m0) + __popc(m1);
+                    // exact tests of 32 hits at a time, and the sums of those accepted;
+                    // the last pairs' hits whatever their number
+                    const uint32_t enough = p0 + 32 < npairs ? 32u : 1u;
+                    while (nq >= enough) {
                         __syncwarp();
-                        for (uint32_t e = (uint32_t)lane; e < qlen; e += 32) {
-                            const uint32_t en = queue[e];
-                            const uint32_t eb = en >> 11, q = en & 0x7ffu;
-                            const float4 cq = sm.u.spos[q];
-                            if (__float_as_uint(cq.w) == own0 + r0 + eb) continue;
-                            const float4 a0 = sm.w.a.obs[0][eb], a1 = sm.w.a.obs[1][eb];
-                            Sight sg;
-                            sg.v = xyz(a1);
-                            sg.nv = a0.w;
-                            sg.inv_nv = a1.w;
-                            const int f = pair_flags(xyz(a0), sg, xyz(cq), k);
-                            if (!f) continue;
-                            uint32_t *mb = masks + eb * wstride + (q >> 5);
-                            const uint32_t bit = 1u << (q & 31);
-                            if (f & 1) atomicOr(mb, bit);
-                            if (f & 2) atomicOr(mb + nbr * wstride, bit);
-                            if (f & 4) atomicOr(mb + 2 * nbr * wstride, bit);
+                        int f = 0;
+                        float4 cq = make_float4(0.f, 0.f, 0.f, 0.f);
+                        uint32_t q = 0;
+                        if ((uint32_t)lane < nq) {
+                            q = hits[(qh + lane) & (kHitRing - 1)];
+                            cq = sm.u.spos[q];
+                            if (__float_as_uint(cq.w) != s) f = pair_flags(pi, si, xyz(cq), k);
+                        }
+                        const uint32_t done = min(nq, 32u);
+                        qh += done;
+                        nq -= done;
+                        const unsigned am = __ballot_sync(0xffffffffu, f != 0);
+                        if (!am) continue;
+                        const int m = __popc(am);
+                        const bool co = f & 1, se = f & 2, al = f & 4;
+                        const unsigned cm = __ballot_sync(0xffffffffu, co), em = __ballot_sync(0xffffffffu, se),
+                                       lm = __ballot_sync(0xffffffffu, al);
+                        ncoh += __popc(cm);
+                        nsep += __popc(em);
+                        nali += __popc(lm);
+                        // Column by column, lanes 0-8 add the accepted up, a component
+                        // each.  A rule that did not accept a neighbour adds +0, which
+                        // leaves a float sum that started at +0 unchanged (it is never
+                        // -0): every sum is the reference's sequence of additions.
+                        if (f) {
+                            const int c = __popc(am & below);
+                            st[0][c] = co ? cq.x : 0.f;
+                            st[1][c] = co ? cq.y : 0.f;
+                            st[2][c] = co ? cq.z : 0.f;
+                            st[6][c] = al ? sm.svx[q] : 0.f;
+                            st[7][c] = al ? sm.svy[q] : 0.f;
+                            st[8][c] = al ? sm.svz[q] : 0.f;
+                            if (em) {
+                                float3 u = make_float3(0.f, 0.f, 0.f);
+                                if (se) {  // Vector3D::normalized of pi - t
+                                    const float dx = __fsub_rn(pi.x, cq.x), dy = __fsub_rn(pi.y, cq.y),
+                                                dz = __fsub_rn(pi.z, cq.z);
+                                    const float n = nrm3(dx, dy, dz);
+                                    u = make_float3(__fdiv_rn(dx, n), __fdiv_rn(dy, n), __fdiv_rn(dz, n));
+                                }
+                                st[3][c] = u.x;
+                                st[4][c] = u.y;
+                                st[5][c] = u.z;
+                            }
+                            if (DIAG) {
+                                const uint64_t h = id_hash(__float_as_uint(__ldg(&g.pos[__float_as_uint(cq.w)].w)));
+                                if (co) h0 += h;
+                                if (se) h1 += h;
+                                if (al) h2 += h;
+                            }
+                        }
+                        // columns m .. up to a multiple of four: +0
+                        const int pad = (4 - m) & 3;
+                        if (lane < 9 * 4 && (lane & 3) < pad) st[lane >> 2][m + (lane & 3)] = 0.f;
+                        if (lane < pad) st[8][m + lane] = 0.f;
+                        __syncwarp();
+                        if (lane < 9 && (em || lane < 3 || lane >= 6)) {
+                            const float *row = st[lane];
+                            for (int c = 0; c < m; c += 4) {
+                                const float4 x = *reinterpret_cast<const float4 *>(row + c);
+                                acc = __fadd_rn(acc, x.x);
+                                acc = __fadd_rn(acc, x.y);
+                                acc = __fadd_rn(acc, x.z);
+                                acc = __fadd_rn(acc, x.w);
+                            }
                         }
                         __syncwarp();
-                        qlen = 0;
-                    };
-                    // A lane's hits of kHitGroup iterations (two candidates
-                    // each) collect in a register, then go to the warp's queue
-                    // together (one scan of the lanes' counts); the queue is
-                    // tested first when they would not fit.
-                    constexpr uint32_t kHitGroup = kQueue / 64;
-                    uint32_t hm = 0;
-                    for (uint32_t it = 0; it < maxlen; ++it) {
-                        const uint32_t gi = it % kHitGroup;
-                        if (it < plen) {
-                            const uint32_t pp = p0 + it;
-                            const __half2 dx = __hsub2(sm.hx[pp], bx), dy = __hsub2(sm.hy[pp], by),
-                                          dz = __hsub2(sm.hz[pp], bz);
-                            const __half2 d2 = __hfma2(dz, dz, __hfma2(dy, dy, __hmul2(dx, dx)));
-                            const __half2 dv = __hfma2(hvz, dz, __hfma2(hvy, dy, __hmul2(hvx, dx)));
-                            const unsigned keep = __hlt2_mask(d2, hf2) & __hge2_mask(dv, hd2);
-                            hm |= ((keep & 1u) | ((keep >> 15) & 2u)) << (2 * gi);
-                        }
-                        const bool end = it + 1 == maxlen;
-                        if (gi == kHitGroup - 1 || end) {
-                            const uint32_t cnt = __popc(hm);
-                            uint32_t incl = cnt;
+                    }
+                }
+                const uint32_t word = lane < 9 ? __float_as_uint(acc)
+                                               : (uint32_t)(lane == 9 ? ncoh : (lane == 10 ? nsep : nali));
+                if (DIAG) {
 #pragma unroll
-                            for (int o = 1; o < 32; o <<= 1) {
-                                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                                if (lane >= o) incl += y;
-                            }
-                            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-                            if (qlen + total > (uint32_t)kQueue) flush();
-                            uint32_t at = qlen + incl - cnt;
-                            const uint32_t q0 = 2 * (p0 + it - gi);  // the candidate of bit 0
-                            while (hm) {
-                                const uint32_t bb = (uint32_t)__ffs(hm) - 1;
-                                hm &= hm - 1;
-                                queue[at++] = (bi << 11) | (q0 + bb);
-                            }
-                            qlen += total;
-                            if (end || qlen > (uint32_t)kQueue - 64) flush();
-                        }
+                    for (int q = 16; q > 0; q >>= 1) {
+                        h0 += __shfl_xor_sync(0xffffffffu, h0, q);
+                        h1 += __shfl_xor_sync(0xffffffffu, h1, q);
+                        h2 += __shfl_xor_sync(0xffffffffu, h2, q);
                     }
-                }
-                // the separation job's boid (at most one per thread): its
-                // position from the round's table, which the sums overwrite
-                float3 sep_pi = make_float3(0.f, 0.f, 0.f);
-                for (uint32_t pj = (uint32_t)t; pj < 7 * nbr; pj += kDT)
-                    if (pj >= 6 * nbr) sep_pi = xyz(sm.w.a.obs[0][pj - 6 * nbr]);
-                __syncthreads();  // the masks are complete; the hit buffers are dead
-                for (uint32_t pj = (uint32_t)t; pj < njobs * nbr; pj += kDT) {
-                    const uint32_t job = pj / nbr, jb = pj - job * nbr;
-                    const uint32_t js = own0 + r0 + jb;
-                    const Acc *cin = first ? nullptr : o.carry + js;
-                    Acc &out = sm.w.sums[jb];
-                    if (job < 6) {
-                        dense_sum_job(sm, masks + ((job < 3 ? 0u : 2u) * nbr + jb) * wstride, words, job, cin, out);
-                    } else if (job == 6) {
-                        dense_sep_job(sm, masks + (nbr + jb) * wstride, words, sep_pi, cin, out);
-                    } else if (DIAG) {
-                        dense_hash_job(sm, masks + jb * wstride, nbr * wstride, words, cin, out, g.pos);
+                    if (lane == 0) {
+                        uint64_t *hs = last ? o.dhash + 3 * (size_t)(__float_as_uint(g.pos[s].w) + (k.slot_base - k.slot_off))
+                                            : o.carry[s].h;
+                        const uint64_t *hc = first ? nullptr : o.carry[s].h;
+                        hs[0] = h0 + (hc ? hc[0] : 0);
+                        hs[1] = h1 + (hc ? hc[1] : 0);
+                        hs[2] = h2 + (hc ? hc[2] : 0);
                     }
+                    if (last && lane >= 9 && lane < 12)
+                        o.dcnt[3 * (size_t)(__float_as_uint(g.pos[s].w) + (k.slot_base - k.slot_off)) + lane - 9] =
+                            (int)word;
                 }
-                __syncthreads();
-                if (act && l == 0) {
-                    const uint32_t s = own0 + r0 + bi;
-                    Acc a = sm.w.sums[bi];
-                    if (!DIAG) a.h[0] = a.h[1] = a.h[2] = 0;
-                    if (last) finish_boid<DIAG>(a, g.pos[s], xyz(g.vel[s]), s, o, k);
-                    else o.carry[s] = a;
+                if (lane < 12) {
+                    if (!last) reinterpret_cast<uint32_t *>(o.carry + s)[lane] = word;
+                    else if (!DIAG) sm.res[lane][i - rbeg] = word;
                 }
-                __syncthreads();  // masks and sums are reused by the next round
-                r0 += nbr;
+            }
+            __syncthreads();  // the list is free, the results are written
+            if (!DIAG && last && (uint32_t)t < rend - rbeg) {
+                const uint32_t s = own0 + rbeg + t;
+                Acc a;
+                uint32_t *aw = reinterpret_cast<uint32_t *>(&a);
+#pragma unroll
+                for (int c = 0; c < 12; ++c) aw[c] = sm.res[c][t];
+                finish_boid<DIAG>(a, g.pos[s], xyz(g.vel[s]), s, o, k);
             }
             if (last) break;
             lo = hi;
@@ -2066,10 +1983,18 @@ cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream
     if (ft && b.defer_cnt && (e = cudaMemsetAsync(b.defer_cnt, 0, sizeof(uint32_t) * ft->count, st)) != cudaSuccess)
         return e;  // an ensemble's per-flock deferred counts
     k_grid_scan<<<b.nscan_blocks, kScanThreads, 0, st>>>(b.count, b.lstart, b.bsum, b.ticket, b.nscan_blocks);
+    *launches += 1;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_grid_classify(const StepConst &k, const DevBuffers &b, cudaStream_t st, uint64_t *launches,
+                                 const FlockTable *ft)
+{
+    cudaError_t e;
     const uint32_t nfull = b.ncell / 4;
     const int windows = b.carry != nullptr;
-    // with a side stream the classification runs beside the scatter, which
-    // the caller queues next; launch_grid_force waits for it
+    // with a side stream the classification runs beside what the caller
+    // queues next (the scatter); launch_grid_force waits for it
     cudaStream_t cs = st;
     if (b.aux) {
         if ((e = cudaEventRecord(b.fork, st)) != cudaSuccess) return e;
@@ -2084,7 +2009,7 @@ cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream
                                                                         b.dense_list, b.dense_n, nfull, windows, k,
                                                                         FlockTable{});
     if (b.aux && (e = cudaEventRecord(b.cjoin, b.aux)) != cudaSuccess) return e;
-    *launches += 2;
+    *launches += 1;
     return cudaGetLastError();
 }
 

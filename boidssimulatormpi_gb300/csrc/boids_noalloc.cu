@@ -143,7 +143,6 @@ size_t layout(const boidsgpu::StepConst &k, unsigned char *base, boidsgpu::DevBu
     b->ncell = (uint32_t)k.Gx * k.G * k.G;
     b->ncell_pad = (b->ncell + 1 + boidsgpu::kScanTile - 1) / boidsgpu::kScanTile * boidsgpu::kScanTile;
     b->nscan_blocks = b->ncell_pad / boidsgpu::kScanTile;
-    const size_t ndense = boidsgpu::dense_list_capacity(b->ncell, n);
     size_t off = 0;
     auto take = [&](size_t bytes) {
         unsigned char *p = base ? base + off : nullptr;
@@ -154,13 +153,16 @@ size_t layout(const boidsgpu::StepConst &k, unsigned char *base, boidsgpu::DevBu
         b->pos[i] = reinterpret_cast<float4 *>(take(16 * n));
         b->vel[i] = reinterpret_cast<float4 *>(take(16 * n));
     }
-    b->key = reinterpret_cast<uint32_t *>(take(4 * n));
-    b->rank = reinterpret_cast<uint32_t *>(take(4 * n));
+    // the keys and ranks are dead once the scatter has read them: the dense
+    // kernel's work list (at most two words per boid) takes their place
+    unsigned char *keys = take(8 * n);
+    b->key = reinterpret_cast<uint32_t *>(keys);
+    b->rank = keys ? b->key + n : nullptr;
+    b->dense_list = b->key;
     b->count = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad));
     b->lstart = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad));
     b->bsum = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->nscan_blocks));
     b->ticket = reinterpret_cast<uint32_t *>(take(4));
-    b->dense_list = reinterpret_cast<uint32_t *>(take(4 * ndense));
     b->dense_n = reinterpret_cast<uint32_t *>(take(12));
     b->dflag = take(b->ncell / 4);
     b->carry = nullptr;  // no id windows: cells over the dense list's capacity stay per-boid
@@ -203,14 +205,17 @@ extern "C" int boids_step_noalloc(const boids_params *params, const float *pos3n
     b.dense_grid = (uint32_t)(nsm > 0 ? nsm : 1) * boidsgpu::kDenseCtasPerSm;
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     uint64_t launches = 0;
+    boidsgpu::DevBuffers rules = b;  // the rule kernels bin nothing for a next step
+    rules.key = rules.rank = nullptr;
     // the array keeps the previous call's contents: clear what must start at zero
     if ((e = cudaMemsetAsync(b.count, 0, 4 * (size_t)b.ncell_pad, st)) == cudaSuccess &&
         (e = cudaMemsetAsync(b.ticket, 0, 4, st)) == cudaSuccess &&
         (e = boidsgpu::launch_pack(pos3n_in, vel3n_in, b.pos[0], b.vel[0], 0, n, nullptr, 0.f, &k, b.key, b.rank,
                                    b.count, st, &launches)) == cudaSuccess &&
         (e = boidsgpu::launch_grid_scan(k, b, st, &launches)) == cudaSuccess &&
-        (e = boidsgpu::launch_grid_scatter(k, b, 0, true, st, &launches)) == cudaSuccess &&
-        (e = boidsgpu::launch_grid_force(k, b, 1, false, false, st, &launches)) == cudaSuccess &&
+        (e = boidsgpu::launch_grid_scatter(k, b, 0, false, st, &launches)) == cudaSuccess &&
+        (e = boidsgpu::launch_grid_classify(k, b, st, &launches)) == cudaSuccess &&
+        (e = boidsgpu::launch_grid_force(k, rules, 1, false, false, st, &launches)) == cudaSuccess &&
         // the sorted copy in b.pos[1] is dead once the rules have run: it
         // holds the id -> slot table of the unpacking
         (e = boidsgpu::launch_unpack(b.pos[0], b.vel[0], reinterpret_cast<uint32_t *>(b.pos[1]), pos3n_out,

@@ -1,0 +1,52 @@
+"""The grid engine's rule kernels at the edges of their tiles: crowds of one
+boid, of a warp's 32 and an item's 32 plus or minus one, of the shared list's
+512 candidates plus or minus one and beyond, in one cell and across the
+periodic corner, each bit for bit against the oracle (one update, its rule
+forces, and the neighbour sets)."""
+import numpy as np
+import pytest
+
+from conftest import assert_bits_equal, make_params, make_sim
+
+pytestmark = pytest.mark.gpu
+
+FIELD = 0.7  # 13 device cells per axis with marun2019's radii
+
+
+def crowd_state(m, others, centre, seed):
+    """m boids in a ball of radius 0.018 around the centre (periodic), the
+    others uniform; ids shuffled, so that the crowd's are spread."""
+    rng = np.random.default_rng(seed)
+    d = rng.normal(size=(m, 3))
+    d *= 0.018 * rng.uniform(0, 1, (m, 1)) ** (1 / 3) / np.linalg.norm(d, axis=1, keepdims=True)
+    pos = np.concatenate([np.mod(centre + d, FIELD), rng.uniform(0, FIELD, (others, 3))])
+    v = rng.normal(size=pos.shape)
+    v *= rng.uniform(0.001, 0.005, (len(v), 1)) / np.linalg.norm(v, axis=1, keepdims=True)
+    perm = rng.permutation(len(pos))
+    return pos[perm].astype(np.float32).reshape(-1), v[perm].astype(np.float32).reshape(-1)
+
+
+@pytest.mark.parametrize("corner", [False, True])
+@pytest.mark.parametrize("tuning", [None, (1, 1, 0, 0), (1 << 30,) * 4])
+@pytest.mark.parametrize("m", [1, 31, 32, 33, 64, 129, 256, 511, 512, 513, 1100])
+def test_crowds_at_tile_edges(boids_lib, oracle_mod, m, tuning, corner):
+    O, prm = oracle_mod, oracle_mod.MARUN2019
+    centre = 0.0 if corner else 6.5 * FIELD / 13
+    pos, vel = crowd_state(m, 40, centre, 1000 + m)
+    n = len(pos) // 3
+    p = make_params(O, n, FIELD, prm)
+    op, ov = pos.copy(), vel.copy()
+    of = O.GridPort(p, op).step(op, ov, 1, forces=True)
+    sim = make_sim(boids_lib, "grid", n, FIELD, prm)
+    if tuning:
+        sim.set_tuning(*tuning)
+    sim.set_state(pos, vel)
+    c, h = sim.neighbor_sets()
+    oc, oh = O.neighbor_sets(p, pos, vel)
+    assert np.array_equal(c, oc) and np.array_equal(h, oh)
+    sim.update(1)
+    gp, gv = sim.state()
+    assert_bits_equal(gp, op, "positions")
+    assert_bits_equal(gv, ov, "velocities")
+    assert_bits_equal(sim.forces(), of, "forces")
+    sim.close()
