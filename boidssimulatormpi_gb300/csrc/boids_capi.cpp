@@ -184,7 +184,7 @@ void free_buffers(DevBuffers &b)
 {
     void *ptrs[] = {b.pos[0], b.pos[1], b.vel[0], b.vel[1], b.key, b.rank, b.count, b.lstart,
                     b.bsum, b.ticket, b.ap_cnt, b.ap_list, b.forces, b.stage, b.cells8, b.dcnt, b.dhash,
-                    b.dense_list, b.dense_n, b.flag, b.dflag, b.carry, b.defer, b.ovf, b.ovf_n, b.wscratch};
+                    b.dense_list, b.dense_n, b.flag, b.slot_of, b.dflag, b.carry, b.defer, b.ovf, b.ovf_n, b.wscratch};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (b.aux) cudaStreamDestroy(b.aux);
@@ -513,6 +513,7 @@ int boids_create(const boids_params *params, boids_sim **out)
         ALLOC(&b.ticket, 1, true);
         const size_t ndense = boidsgpu::dense_list_capacity(b.ncell, n);
         ALLOC(&b.dense_list, ndense);
+        ALLOC(&b.slot_of, std::min<size_t>(n, boidsgpu::kWarpBoids));
         ALLOC(&b.dflag, b.ncell / 4);
         {
             unsigned char *carry = nullptr;
@@ -910,6 +911,7 @@ int boids_set_tuning(boids_sim *s, const int32_t *t)
     s->k.defer_min = (uint32_t)t[1];
     s->k.cand_defer = (uint32_t)t[2];
     s->k.lone_cand = (uint32_t)t[3];
+    s->k.tuned = 1;
     return BOIDS_OK;
 }
 
@@ -958,6 +960,7 @@ int boids_autotune(boids_sim *s, int32_t steps_per_trial)
         s->k.defer_min = boidsgpu::kTuneCand[c][1];
         s->k.cand_defer = boidsgpu::kTuneCand[c][2];
         s->k.lone_cand = boidsgpu::kTuneCand[c][3];
+        s->k.tuned = c > 0;  // the first is the default, with the default's choice of kernels
         if ((rc = restore()) || (rc = boids_step(s, 1))) break;  // one warm-up update
         float ms = 0.f;
         if (cudaEventRecord(t0, s->stream) != cudaSuccess || (rc = boids_step(s, steps_per_trial)) ||
@@ -977,6 +980,7 @@ int boids_autotune(boids_sim *s, int32_t steps_per_trial)
         s->k.defer_min = boidsgpu::kTuneCand[best_i][1];
         s->k.cand_defer = boidsgpu::kTuneCand[best_i][2];
         s->k.lone_cand = boidsgpu::kTuneCand[best_i][3];
+        s->k.tuned = best_i > 0;
     }
     int rc2 = restore();
     if (!rc2 && cudaStreamSynchronize(s->stream) != cudaSuccess) rc2 = cuda_fail(cudaGetLastError(), "boids_autotune");

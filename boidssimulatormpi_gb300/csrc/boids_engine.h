@@ -82,6 +82,7 @@ struct StepConst {
     // defer_min or more whose 27-cell neighbourhood holds over cand_defer
     // boids, and any non-empty cell whose neighbourhood holds over lone_cand.
     uint32_t dense_min, defer_min, cand_defer, lone_cand;
+    uint32_t tuned;  // those were set (boids_set_tuning, an autotuner): the split applies whatever the size
 };
 
 // A batched ensemble's flock table, in device memory.  Every block of
@@ -124,6 +125,8 @@ struct DevBuffers {
     // forked from and joined back to the engine's stream (null: in order).
     cudaStream_t aux;
     cudaEvent_t fork, join, cjoin;  // cjoin: the classification's end (it runs beside the scatter)
+    uint32_t *slot_of;         // slot of each id after the scatter (from its flock's slot_base), kept where
+                               // k_grid_warp takes every boid (null: it never does)
     uint8_t *dflag;            // per full-size cell: 1 when the dense kernel takes it
     void *carry;               // per slot, kCarryBytes: partial sums between id windows (null: no windows)
     uint32_t *flag;            // set_state range check (1 word)
@@ -171,6 +174,12 @@ inline size_t dense_list_capacity(size_t ncell, size_t n)
     const size_t items = (by_cells < n ? by_cells : n) + n / kDenseRound + 1;
     return 2 * (items < n ? items : n);
 }
+// Flocks of up to this many boids (all flocks of an ensemble together) are
+// updated a warp per boid (k_grid_warp), the others by the cells' split.  A
+// step with either, us: 32 768 boids uniform 58 / 74, gathered 90 / 215;
+// 49 152 uniform 75 / 71, gathered 124 / 251; 65 537 uniform 95 / 73.  The
+// line lies where a uniform flock takes the same time with both.
+constexpr uint32_t kWarpBoids = 40960;
 constexpr int kDenseCap = 512;        // candidates of a dense cell held in shared memory
 constexpr int kDenseCtasPerSm = 8;   // resident CTAs of the dense-cell kernel per SM (its launch bounds)
 constexpr int kApCap = 256;           // all-pairs engine: neighbours kept per boid (more: an O(N) scan)

@@ -69,11 +69,13 @@ struct boids_ensemble {
     cudaStream_t stream = nullptr;
     int cur = 0;           // buffer holding the state
     bool binned = false;   // b.pos[cur] is freshly binned (the next step skips the counting sort)
+    bool binned_tuned = false;  // tuned when it was binned: the rules run on what was classified then
     bool keys_stale = false;  // set_state changed b.pos[cur]: recompute every key before the next scan
     bool has_state = false;
     cudaGraphExec_t graph = nullptr;
     uint64_t graph_launches = 0;  // kernel launches per replay
     uint64_t launches = 0;
+    bool tuned = false;       // tune was set or chosen by the autotuner
     uint32_t tune[4] = {boidsgpu::kDenseMin, boidsgpu::kDeferMin, boidsgpu::kCandDefer, boidsgpu::kLoneCand};
 };
 
@@ -85,7 +87,7 @@ void release(boids_ensemble *e)
     DevBuffers &b = e->b;
     if (e->stream) cudaStreamSynchronize(e->stream);
     void *ptrs[] = {b.pos[0], b.pos[1], b.vel[0], b.vel[1], b.key, b.rank, b.count, b.lstart, b.bsum, b.ticket,
-                    b.dense_list, b.dense_n, b.dflag, b.carry, b.defer, b.defer_cnt, b.wscratch, e->d_ks, e->d_blk,
+                    b.dense_list, b.dense_n, b.slot_of, b.dflag, b.carry, b.defer, b.defer_cnt, b.wscratch, e->d_ks, e->d_blk,
                     e->d_cell4,
                     e->d_link, e->d_acc, e->d_com, e->d_largest, e->d_err};
     for (void *p : ptrs)
@@ -139,7 +141,9 @@ int step_once(boids_ensemble *e)
         CK(boidsgpu::launch_grid_scatter(e->ks[0], e->b, e->cur, true, e->stream, &e->launches, &e->ft));
         e->cur = 1 - e->cur;
     }
-    CK(boidsgpu::launch_grid_force(e->ks[0], e->b, e->cur, false, false, e->stream, &e->launches, &e->ft));
+    StepConst k = e->ks[0];
+    if (e->binned) k.tuned = e->binned_tuned;
+    CK(boidsgpu::launch_grid_force(k, e->b, e->cur, false, false, e->stream, &e->launches, &e->ft));
     e->cur = 1 - e->cur;
     e->binned = false;
     return 0;
@@ -154,6 +158,7 @@ int bin_now(boids_ensemble *e)
     CK(boidsgpu::launch_grid_scatter(e->ks[0], e->b, e->cur, true, e->stream, &e->launches, &e->ft));
     e->cur = 1 - e->cur;
     e->binned = true;
+    e->binned_tuned = e->tuned;
     return 0;
 }
 
@@ -200,6 +205,7 @@ int upload_table(boids_ensemble *e)
         k.defer_min = e->tune[1];
         k.cand_defer = e->tune[2];
         k.lone_cand = e->tune[3];
+        k.tuned = e->tuned;
     }
     CK(cudaMemcpyAsync(e->d_ks, e->ks.data(), sizeof(StepConst) * e->ks.size(), cudaMemcpyHostToDevice, e->stream));
     if (e->graph) {  // re-captured on the next step
@@ -279,6 +285,7 @@ int boids_ensemble_create(const boids_flock_desc *flocks, uint32_t count, boids_
     ALLOC(&b.ticket, 1);
     ALLOC(&b.dense_list, boidsgpu::dense_list_capacity(b.ncell, e->total_boids));
     ALLOC(&b.dense_n, 3);
+    if (ns <= boidsgpu::kWarpBoids) ALLOC(&b.slot_of, ns);
     ALLOC(&b.dflag, b.ncell / 4);
     {
         unsigned char *carry = nullptr;
@@ -519,8 +526,10 @@ int boids_ensemble_autotune(boids_ensemble *e, int32_t steps_per_trial)
         rc = cuda_fail(cudaGetLastError(), "boids_ensemble_autotune");
     uint32_t keep[4];
     std::memcpy(keep, e->tune, sizeof keep);
+    const bool keep_tuned = e->tuned;
     for (int c = 0; !rc && c < boidsgpu::kTuneCount; ++c) {
         std::memcpy(e->tune, boidsgpu::kTuneCand[c], sizeof e->tune);
+        e->tuned = c > 0;  // the first is the default, with the default's choice of kernels
         if ((rc = upload_table(e)) || (rc = restore()) || (rc = step_once(e))) break;  // one warm-up step
         if (cudaEventRecord(t0, e->stream) != cudaSuccess) { rc = cuda_fail(cudaGetLastError(), "cudaEventRecord"); break; }
         for (int t = 0; t < steps_per_trial && !rc; ++t) rc = step_once(e);
@@ -538,6 +547,7 @@ int boids_ensemble_autotune(boids_ensemble *e, int32_t steps_per_trial)
     }
     if (!rc) std::memcpy(e->tune, boidsgpu::kTuneCand[best_i], sizeof e->tune);
     else std::memcpy(e->tune, keep, sizeof e->tune);
+    e->tuned = rc ? keep_tuned : best_i > 0;
     int rc2 = upload_table(e);
     if (!rc2) rc2 = restore();
     if (!rc2 && cudaStreamSynchronize(e->stream) != cudaSuccess) rc2 = cuda_fail(cudaGetLastError(), "autotune");
@@ -563,6 +573,7 @@ int boids_ensemble_set_tuning(boids_ensemble *e, const int32_t *t)
     int rc = use_device(e);
     if (rc) return rc;
     for (int i = 0; i < 4; ++i) e->tune[i] = (uint32_t)t[i];
+    e->tuned = true;
     return upload_table(e);
 }
 

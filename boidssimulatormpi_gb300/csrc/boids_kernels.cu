@@ -525,22 +525,26 @@ __global__ void k_grid_scatter(const float4 *__restrict__ pin, const float4 *__r
                                const uint32_t *__restrict__ key, const uint32_t *__restrict__ rank,
                                const uint32_t *__restrict__ lstart, const uint32_t *__restrict__ bsum,
                                float4 *__restrict__ pout, float4 *__restrict__ vout,
-                               uint32_t *__restrict__ count_to_zero, uint32_t n, FlockTable ft)
+                               uint32_t *__restrict__ count_to_zero, uint32_t *__restrict__ slot_of, uint32_t n,
+                               FlockTable ft)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t off = 0;
+    uint32_t off = 0, first = 0;  // the flock's padding and first slot
     if (MULTI) {
         if (s >= ft.nslots) return;
         const StepConst &k = ft.ks[ft.blk_flock[s / kSlotAlign]];
         if (s - k.slot_base >= k.n) return;
         off = k.slot_off;
+        first = k.slot_base;
     } else if (s >= n) {
         return;
     }
     const uint32_t c = key[s];
     const uint32_t d = cell_start(lstart, bsum, c) + rank[s] + off;
-    pout[d] = pin[s];
+    const float4 p = pin[s];
+    pout[d] = p;
     vout[d] = vin[s];
+    if (slot_of) slot_of[first + __float_as_uint(p.w)] = d;
     if (count_to_zero) count_to_zero[c] = 0;  // every binned cell, for the next step's keys
 }
 
@@ -668,6 +672,7 @@ struct GridIn {
     const uint32_t *__restrict__ lstart;
     const uint32_t *__restrict__ bsum;
     const uint8_t *__restrict__ dflag;  // per full-size cell: taken by k_grid_dense
+    const uint32_t *__restrict__ slot_of;  // k_grid_warp: slot of each id, from its flock's slot_base
 };
 
 struct SparseSmem {
@@ -1080,6 +1085,487 @@ k_grid_sparse_more(GridIn g, GridOut o, StepConst kp, FlockTable ft)
         while (__any_sync(0xffffffffu, need))
             sparse_pass<DIAG>(sm, t, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n);
         if (act) finish_boid<DIAG>(a, p4, sight.v, s, o, k);
+    }
+}
+
+// ------------------------------------------------------------------ a warp per boid
+
+// k_grid_warp: the 32 lanes of a warp update one boid together, straight from
+// the cell table: the flocks too small to fill the GPU with a thread per boid
+// or a CTA per cell.
+//
+//   1. lane r takes row r of the boid's nine neighbour rows: the x cells its
+//      sphere reaches, as runs of slots (sparse_segments' rule, a row a lane);
+//   2. the runs are walked with 8, 16 or 32 lanes each, four, two or one at a
+//      time, by the longest run, so that short rows share an iteration and no
+//      lane searches for its run; candidates passing the float filter are
+//      compacted into a queue, and every 32 of them take the exact tests;
+//   3. accepted neighbours (at most kWarpList at a time) are put in id order:
+//      by counting smaller ids up to 32 of them, by one bucket pass over their
+//      id range beyond;
+//   4. 32 at a time in id order, each lane prepares one neighbour's summands
+//      (image, velocity, normalised offset), and nine lanes add them up, one
+//      component each.  A neighbour a rule does not accept contributes +0,
+//      which leaves a float sum that started at +0 unchanged (such a sum is
+//      never -0), so every sum is the reference's sequence of additions;
+//   5. the boid is finished by nine lanes, a component each.
+//
+// A boid that accepts more than kWarpList neighbours starts over in warp_many,
+// which needs no sort: the filter's hits are marked in a bit map over ids.
+//
+// Bound by instruction issue once every SM has its 32 warps, by the length of
+// one boid's chain of loads, tests and sums below that (about 15 us).  A step
+// of 1000 boids of test.ini takes 28 us where the split of cells over
+// k_grid_sparse and k_grid_dense took 109 (their few CTAs leave most SMs
+// idle), gathered flocks of 16 384 boids 54 us (188), of 32 768 boids 90 us
+// (215), uniform ones 36 us (65) and 58 us (74), all with the counting sort.
+// Per-boid work is about five times k_grid_sparse's on a uniform flock
+// (1240 warp instructions against 190 a boid), hence kWarpBoids.
+constexpr int kWarpWarps = 4;    // warps of a CTA
+constexpr int kWarpCtas = 8;     // CTAs per SM
+constexpr int kWarpList = 256;   // accepted neighbours kept
+constexpr int kWarpBuckets = 128;
+constexpr int kWarpIds = 8192;   // ids of a window of warp_many
+
+struct WarpSmem {  // of one warp
+    uint32_t lid[kWarpList], lsl[kWarpList];  // accepted: id; slot | rules << 29
+    uint8_t ord[kWarpList];                   // the list's entries in id order
+    union {
+        float st[9][32 + 4];                  // summands of 32 neighbours, by component
+        struct {
+            uint32_t cnt[kWarpBuckets + 4];   // the ordering's bucket counters
+            uint8_t at[kWarpList];            // an entry's arrival in its bucket
+            uint8_t ent[kWarpList];           // entries by bucket
+        } b;
+    } u;
+    float4 shift[18];                         // run: image shift
+    uint2 run[18];                            // run: first slot | wrapped << 31, length
+    uint32_t queue[64];                       // filter hits, a ring: slot | wrapped << 31
+};
+static_assert(kWarpList <= 256, "entries are named in a byte");
+
+// The warp's n list entries in id order into sm.ord.
+__device__ __forceinline__ void warp_order(WarpSmem &sm, int lane, int n)
+{
+    uint32_t *lid = sm.lid;
+    if (n <= 32) {
+        const uint32_t id = lane < n ? lid[lane] : 0xffffffffu;
+        if (lane >= n) lid[lane] = 0xffffffffu;
+        else sm.ord[lane] = (uint8_t)lane;  // equal ids (a state no update makes) leave no stale entry
+        __syncwarp();
+        int rank = 0;
+        for (int j = 0; j < n; j += 4) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(lid + j);
+            rank += (w.x < id) + (w.y < id) + (w.z < id) + (w.w < id);
+        }
+        if (lane < n) sm.ord[rank] = (uint8_t)lane;
+        __syncwarp();
+        return;
+    }
+    // one bucket pass over the ids' range, then each entry's place inside its
+    // bucket by counting the smaller ids there
+    uint32_t *cnt = sm.u.b.cnt;
+    *reinterpret_cast<uint4 *>(cnt + 4 * lane) = make_uint4(0, 0, 0, 0);
+    uint32_t mn = 0xffffffffu, mx = 0;
+    for (int i = lane; i < n; i += 32) {
+        const uint32_t id = lid[i];
+        mn = min(mn, id);
+        mx = max(mx, id);
+        sm.ord[i] = (uint8_t)i;
+    }
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    static_assert(kWarpBuckets == 128, "four buckets a lane, 2^7 of them");
+    const uint32_t range = mx - mn;
+    const int shift = range >> 7 ? 32 - __clz(range) - 7 : 0;
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) sm.u.b.at[i] = (uint8_t)atomicAdd(cnt + ((lid[i] - mn) >> shift), 1u);
+    __syncwarp();
+    const uint4 c = *reinterpret_cast<const uint4 *>(cnt + 4 * lane);
+    const uint32_t sum = c.x + c.y + c.z + c.w;
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const uint32_t ex = incl - sum;
+    *reinterpret_cast<uint4 *>(cnt + 4 * lane) = make_uint4(ex, ex + c.x, ex + c.x + c.y, ex + c.x + c.y + c.z);
+    if (lane == 31) cnt[kWarpBuckets] = incl;
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) sm.u.b.ent[cnt[(lid[i] - mn) >> shift] + sm.u.b.at[i]] = (uint8_t)i;
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+        const uint32_t id = lid[i], b = (id - mn) >> shift, b0 = cnt[b], b1 = cnt[b + 1];
+        uint32_t rank = b0;
+        if (b1 - b0 > 1)
+            for (uint32_t j = b0; j < b1; ++j) rank += lid[sm.u.b.ent[j]] < id;
+        sm.ord[rank] = (uint8_t)i;
+    }
+    __syncwarp();
+}
+
+// One boid's sums: lane c < 9 holds component c of (cohesion, separation,
+// alignment) in acc; the counts (and the diagnostics' id hashes, each lane's
+// own part) are beside it.
+struct WarpSums {
+    float acc;
+    int ncoh, nsep, nali;
+    uint64_t h[3];
+};
+
+// Adds up to 32 neighbours, a lane each in ascending id, accepted by rules f
+// (0: none): image t, velocity vj.  The accepted are compacted into the
+// columns of sm.u.st, and lanes 0-8 add those up.
+template <bool DIAG>
+__device__ __forceinline__ void warp_add(WarpSmem &sm, int lane, int f, float3 t, float4 vj, uint32_t id, float3 pi,
+                                         WarpSums &a)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const unsigned am = __ballot_sync(kAll, f != 0);
+    if (!am) return;
+    const int m = __popc(am);
+    const bool co = f & 1, se = f & 2, al = f & 4;
+    const unsigned em = __ballot_sync(kAll, se);
+    a.ncoh += __popc(__ballot_sync(kAll, co));
+    a.nsep += __popc(em);
+    a.nali += __popc(__ballot_sync(kAll, al));
+    float(&st)[9][36] = sm.u.st;
+    if (f) {
+        const int c = __popc(am & ((1u << lane) - 1u));
+        st[0][c] = co ? t.x : 0.f;
+        st[1][c] = co ? t.y : 0.f;
+        st[2][c] = co ? t.z : 0.f;
+        st[6][c] = al ? vj.x : 0.f;
+        st[7][c] = al ? vj.y : 0.f;
+        st[8][c] = al ? vj.z : 0.f;
+        if (em) {
+            float3 u = make_float3(0.f, 0.f, 0.f);
+            if (se) {  // Vector3D::normalized of pi - t
+                const float dx = __fsub_rn(pi.x, t.x), dy = __fsub_rn(pi.y, t.y), dz = __fsub_rn(pi.z, t.z);
+                const float n = nrm3(dx, dy, dz);
+                u = make_float3(__fdiv_rn(dx, n), __fdiv_rn(dy, n), __fdiv_rn(dz, n));
+            }
+            st[3][c] = u.x;
+            st[4][c] = u.y;
+            st[5][c] = u.z;
+        }
+        if (DIAG) {
+            const uint64_t h = id_hash(id);
+            if (co) a.h[0] += h;
+            if (se) a.h[1] += h;
+            if (al) a.h[2] += h;
+        }
+    }
+    // columns m .. up to a multiple of four: +0
+    const int pad = (4 - m) & 3;
+    if ((lane & 3) < pad) st[lane >> 2][m + (lane & 3)] = 0.f;
+    if (lane < pad) st[8][m + lane] = 0.f;
+    __syncwarp();
+    if (lane < 9 && (em || lane < 3 || lane >= 6)) {
+        const float *row = st[lane];
+        for (int c = 0; c < m; c += 4) {
+            const float4 x = *reinterpret_cast<const float4 *>(row + c);
+            a.acc = __fadd_rn(a.acc, x.x);
+            a.acc = __fadd_rn(a.acc, x.y);
+            a.acc = __fadd_rn(a.acc, x.z);
+            a.acc = __fadd_rn(a.acc, x.w);
+        }
+    }
+    __syncwarp();
+}
+
+// The search of a boid that accepts more than kWarpList neighbours: for
+// windows of kWarpIds ids in ascending order, the filter's hits are marked in
+// a bit map of the window, its bits are expanded in id order, and the hits
+// found through the id -> slot table take the exact tests and are added up,
+// 32 at a time.  Out of line: it is rare.
+template <bool DIAG>
+__device__ __noinline__ void warp_many(WarpSmem *smp, const GridIn &g, const StepConst &k, uint32_t s, float3 pi,
+                                       const Sight &si, float dot_lim, int nr, bool shifted, WarpSums &a)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    WarpSmem &sm = *smp;
+    const int lane = threadIdx.x & 31;
+    uint32_t *map = sm.lid;                                   // kWarpIds bits
+    uint16_t *hits = reinterpret_cast<uint16_t *>(sm.lsl);    // lsl and ord: a group's hits and the rest before it
+    constexpr int kGroup = 16;                                // map words expanded at a time
+    static_assert(kWarpIds == 32 * kWarpList, "the map takes the list's ids");
+    static_assert(2 * (32 * kGroup + 32) <= sizeof(sm.lsl) + sizeof(sm.ord), "a group's hits fit");
+    a = WarpSums{};
+    for (uint32_t w0 = 0; w0 < k.n; w0 += kWarpIds) {
+        for (int i = lane; i < kWarpList; i += 32) map[i] = 0;
+        __syncwarp();
+        for (int r = 0; r < nr; ++r) {
+            const uint2 rn = sm.run[r];
+            const float4 sh = sm.shift[r];
+            const float3 q = make_float3(pi.x - sh.x, pi.y - sh.y, pi.z - sh.z);
+            for (uint32_t off = lane; off < rn.y; off += 32) {
+                const uint32_t slot = (rn.x & 0x7fffffffu) + off;
+                const float4 pj = __ldg(g.pos + slot);
+                const float dx = pj.x - q.x, dy = pj.y - q.y, dz = pj.z - q.z;
+                const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+                const float dv = __fmaf_rn(si.v.z, dz, __fmaf_rn(si.v.y, dy, __fmul_rn(si.v.x, dx)));
+                const uint32_t id = __float_as_uint(pj.w) - w0;
+                if (d2 < k.filt_r2 && dv >= dot_lim && slot != s && id < (uint32_t)kWarpIds)
+                    atomicOr(map + (id >> 5), 1u << (id & 31));
+            }
+        }
+        __syncwarp();
+        int nh = 0;  // hits waiting
+        for (int g0 = 0; g0 < kWarpList; g0 += kGroup) {
+            uint32_t bits = lane < kGroup ? map[g0 + lane] : 0u;
+            int incl = __popc(bits);
+#pragma unroll
+            for (int o = 1; o < kGroup; o <<= 1) {
+                const int y = __shfl_up_sync(kAll, incl, o);
+                if (lane >= o) incl += y;
+            }
+            int at = nh + incl - __popc(bits);
+            nh += __shfl_sync(kAll, incl, kGroup - 1);
+            while (bits) {
+                hits[at++] = (uint16_t)(((g0 + lane) << 5) + __ffs(bits) - 1);
+                bits &= bits - 1;
+            }
+            __syncwarp();
+            int h0 = 0;
+            const int enough = g0 + kGroup < kWarpList ? 32 : 1;
+            while (nh >= enough) {
+                int f = 0;
+                uint32_t id = 0;
+                float3 t = make_float3(0.f, 0.f, 0.f);
+                float4 vj = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (lane < nh) {
+                    id = w0 + hits[h0 + lane];
+                    const uint32_t slot = __ldg(g.slot_of + k.slot_base + id);
+                    const float4 pj = __ldg(g.pos + slot);
+                    t = shifted ? image3(xyz(pj), pi, k) : xyz(pj);
+                    f = pair_flags(pi, si, t, k);
+                    if (f) vj = __ldg(g.vel + slot);
+                }
+                warp_add<DIAG>(sm, lane, f, t, vj, id, pi, a);
+                const int done = min(nh, 32);
+                h0 += done;
+                nh -= done;
+            }
+            // the rest to the front
+            const uint16_t rest = lane < nh ? hits[h0 + lane] : 0;
+            __syncwarp();
+            if (lane < nh) hits[lane] = rest;
+            __syncwarp();
+        }
+    }
+}
+
+// finish_boid by the lanes of a warp: lane 3 r + c holds component c of rule
+// r's sum (cohesion, separation, alignment) in acc.
+__device__ __forceinline__ void warp_finish(float acc, int ncoh, int nali, float4 p4, float3 vi, uint32_t s, int lane,
+                                            const GridOut &o, const StepConst &k)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const int r = lane / 3, c = lane - 3 * r;
+    const float pc = c == 0 ? p4.x : (c == 1 ? p4.y : p4.z), vc = c == 0 ? vi.x : (c == 1 ? vi.y : vi.z);
+    float f = acc;
+    const int q = r == 0 ? ncoh : nali;
+    if (r != 1 && q != 0) f = __fsub_rn(__fdiv_rn(acc, __int2float_rn(q)), r == 0 ? pc : vc);
+    f = __fmul_rn(f, r == 0 ? k.cc : (r == 1 ? k.cs : k.ca));
+    const float fs = __shfl_sync(kAll, f, c + 3), fa = __shfl_sync(kAll, f, c + 6);
+    // lanes 0-2: a component each (the others' values are not used)
+    float v = __fadd_rn(vc, __fadd_rn(__fadd_rn(f, fs), fa));
+    const float n = nrm3(__shfl_sync(kAll, v, 0), __shfl_sync(kAll, v, 1), __shfl_sync(kAll, v, 2));
+    if (n > 0.0f && n > k.vmax_dn) v = __fmul_rn(__fdiv_rn(v, n), k.vmax_f);
+    else if (n > 0.0f && n < k.vmin_up) v = __fmul_rn(__fdiv_rn(v, n), k.vmin_f);
+    const float x = lane < 3 ? wrap1(__fadd_rn(pc, v), k) : p4.w;
+    const float x0 = __shfl_sync(kAll, x, 0), x1 = __shfl_sync(kAll, x, 1), x2 = __shfl_sync(kAll, x, 2);
+    if (lane < 4) {
+        reinterpret_cast<float *>(o.pos_out + s)[lane] = x;
+        reinterpret_cast<float *>(o.vel_out + s)[lane] = lane < 3 ? v : 0.f;
+    }
+    if (o.key_out && lane == 0) {  // binning for the next step
+        const uint32_t cell = k.cell_base + cell_key(make_float3(x0, x1, x2), k);
+        o.key_out[s] = cell;
+        o.rank_out[s] = atomicAdd(o.count + cell, 1u);
+    }
+    if (o.forces && lane < 9)
+        o.forces[(size_t)9 * (__float_as_uint(p4.w) + (k.slot_base - k.slot_off)) + lane] = f;
+}
+
+template <bool DIAG, bool MULTI>
+__global__ void __launch_bounds__(kWarpWarps * 32, kWarpCtas)
+k_grid_warp(GridIn g, GridOut o, StepConst kp, FlockTable ft)
+{
+    __shared__ WarpSmem sms[kWarpWarps];
+    __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
+    StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
+    if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * kWarpWarps / kSlotAlign]);
+    const StepConst &k = MULTI ? kf : kp;
+    const uint32_t s = blockIdx.x * kWarpWarps + (threadIdx.x >> 5);
+    if (s - k.slot_base >= k.n) return;
+    WarpSmem &sm = sms[threadIdx.x >> 5];
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 p4 = __ldg(g.pos + s);
+    const float3 pi = xyz(p4);
+    const Sight si = make_sight(xyz(__ldg(g.vel + s)));
+    const float dot_lim = k.cone_pre ? -(si.nv * k.dot_eps) : -INFINITY;
+
+    // ---- the boid's runs of candidates, a row per lane
+    const int G = k.G, Gx = k.Gx;
+    uint32_t ja = 0, la = 0, jb = 0, lb = 0;
+    float sx0 = 0.f, sx1 = 0.f, sy = 0.f, sz = 0.f;
+    if (lane < 9) {
+        const int cy = cell1(pi.y, k), cz = cell1(pi.z, k);
+        const int dz = lane / 3 - 1, dy = lane - 3 * (lane / 3) - 1;
+        const float eps = k.side * 1e-5f;
+        const float ddy = dy == 0 ? 0.f : fmaxf(0.f, dy < 0 ? pi.y - (float)cy * k.side - eps
+                                                          : (float)(cy + 1) * k.side - pi.y - eps);
+        const float ddz = dz == 0 ? 0.f : fmaxf(0.f, dz < 0 ? pi.z - (float)cz * k.side - eps
+                                                          : (float)(cz + 1) * k.side - pi.z - eps);
+        const float rem = k.trim_r2 - ddy * ddy - ddz * ddz;
+        if (rem > 0.f) {
+            const float rx = rem * rsqrtf(rem);  // trim_r2's margin covers its rounding
+            // clamped as in sparse_segments: a state outside the field stays within the cell tables
+            const int lo = max(__float2int_rd((pi.x - rx) * k.inv_subx), 1 - Gx);
+            const int hi = min(__float2int_rd((pi.x + rx) * k.inv_subx), 2 * Gx - 2);
+            int a0 = lo, a1 = hi + 1, c0 = 0, c1 = 0;
+            if (lo < 0) { a0 = lo + Gx; a1 = Gx; sx0 = -k.Ff; c1 = min(hi + 1, Gx); }
+            else if (hi >= Gx) { a1 = Gx; c1 = hi + 1 - Gx; sx1 = k.Ff; }
+            int zz = cz + dz, yy = cy + dy;
+            if (zz < 0) { zz += G; sz = -k.Ff; } else if (zz >= G) { zz -= G; sz = k.Ff; }
+            if (yy < 0) { yy += G; sy = -k.Ff; } else if (yy >= G) { yy -= G; sy = k.Ff; }
+            const uint32_t rb = k.cell_base + (uint32_t)(zz * G + yy) * (uint32_t)Gx;
+            if (a1 > a0) {
+                ja = slot_start(g.lstart, g.bsum, rb + a0, k);
+                la = slot_start(g.lstart, g.bsum, rb + a1, k) - ja;
+            }
+            if (c1 > c0) {
+                jb = slot_start(g.lstart, g.bsum, rb + c0, k);
+                lb = slot_start(g.lstart, g.bsum, rb + c1, k) - jb;
+            }
+        }
+    }
+    const bool wa = sx0 != 0.f || sy != 0.f || sz != 0.f, wb = sx1 != 0.f || sy != 0.f || sz != 0.f;
+    const unsigned ba = __ballot_sync(kAll, la != 0), bb = __ballot_sync(kAll, lb != 0);
+    const bool shifted = __any_sync(kAll, (la && wa) || (lb && wb));
+    const int na = __popc(ba), nr = na + __popc(bb);  // non-empty runs
+    if (la) {
+        const int q = __popc(ba & below);
+        sm.run[q] = make_uint2(ja | (wa ? 0x80000000u : 0u), la);
+        sm.shift[q] = make_float4(sx0, sy, sz, 0.f);
+    }
+    if (lb) {
+        const int q = na + __popc(bb & below);
+        sm.run[q] = make_uint2(jb | (wb ? 0x80000000u : 0u), lb);
+        sm.shift[q] = make_float4(sx1, sy, sz, 0.f);
+    }
+    // lanes per run: 8 or 16 where every run fits, else 32
+    const uint32_t longest = __reduce_max_sync(kAll, max(la, lb));
+    const int wsh = longest <= 8 ? 3 : (longest <= 16 ? 4 : 5);
+    const int rstep = 32 >> wsh, rsub = lane >> wsh;
+    const uint32_t off0 = lane & ((1 << wsh) - 1);
+    __syncwarp();
+
+    WarpSums a{};
+    int nl = 0, nq = 0;  // accepted; filter hits waiting in the ring
+    uint32_t qh = 0;     // the ring's head
+    for (int r = 0; r < nr; r += rstep) {
+        const int ri = r + rsub;
+        const uint2 rn = ri < nr ? sm.run[ri] : make_uint2(0u, 0u);
+        float3 q = pi;  // the query point: the candidate's image is pj + shift
+        if (shifted && ri < nr) {
+            const float4 sh = sm.shift[ri];
+            q = make_float3(pi.x - sh.x, pi.y - sh.y, pi.z - sh.z);
+        }
+        // (a run longer than its lanes is walked by the whole warp: its length
+        // is the same in every lane)
+        uint32_t base = 0;
+        do {
+            const uint32_t off = base + off0;
+            bool hit = false;
+            const uint32_t w = rn.x + off, slot = w & 0x7fffffffu;
+            if (off < rn.y) {
+                const float4 pj = __ldg(g.pos + slot);
+                const float dx = pj.x - q.x, dy = pj.y - q.y, dz = pj.z - q.z;
+                const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+                const float dv = __fmaf_rn(si.v.z, dz, __fmaf_rn(si.v.y, dy, __fmul_rn(si.v.x, dx)));
+                hit = d2 < k.filt_r2 && dv >= dot_lim && slot != s;
+            }
+            const unsigned hm = __ballot_sync(kAll, hit);
+            if (hit) sm.queue[(qh + nq + __popc(hm & below)) & 63] = w;
+            nq += __popc(hm);
+            // exact tests of the hits, 32 at a time; the last candidates' hits
+            // whatever their number
+            base += 32;
+            const int enough = r + rstep < nr || base < rn.y ? 32 : 1;
+            while (nq >= enough) {
+                __syncwarp();
+                int f = 0;
+                uint32_t id = 0, js = 0;
+                if (lane < nq) {
+                    const uint32_t e = sm.queue[(qh + lane) & 63];
+                    js = e & 0x7fffffffu;
+                    const float4 pj = __ldg(g.pos + js);
+                    id = __float_as_uint(pj.w);
+                    // a hit from a run without periodic shift is its own minimum image
+                    const float3 t = (e >> 31) ? image3(xyz(pj), pi, k) : xyz(pj);
+                    f = pair_flags(pi, si, t, k);
+                }
+                const int done = min(nq, 32);
+                qh += done;
+                nq -= done;
+                const unsigned am = __ballot_sync(kAll, f != 0);
+                const int at = nl + __popc(am & below);
+                if (f && at < kWarpList) {
+                    sm.lid[at] = id;
+                    sm.lsl[at] = js | ((uint32_t)f << 29);
+                }
+                nl += __popc(am);
+            }
+        } while (base < rn.y);
+        if (nl > kWarpList) break;
+    }
+    __syncwarp();
+    if (nl > kWarpList) {
+        warp_many<DIAG>(&sm, g, k, s, pi, si, dot_lim, nr, shifted, a);
+    } else if (nl > 0) {
+        // the accepted neighbours in id order, the next 32 neighbours' loads in
+        // flight under each 32's sums
+        warp_order(sm, lane, nl);
+        uint32_t e = 0;
+        float4 pj = zero4, vj = zero4;
+        auto load = [&](int i) {
+            e = 0;
+            if (i < nl) {
+                e = sm.lsl[sm.ord[i]];
+                pj = __ldg(g.pos + (e & 0x1fffffffu));
+                vj = __ldg(g.vel + (e & 0x1fffffffu));
+            }
+        };
+        load(lane);
+        for (int c0 = 0; c0 < nl; c0 += 32) {
+            const int f = (int)(e >> 29);
+            const float3 t = shifted ? image3(xyz(pj), pi, k) : xyz(pj);
+            const float4 v = vj;
+            const uint32_t id = __float_as_uint(pj.w);
+            load(c0 + 32 + lane);
+            warp_add<DIAG>(sm, lane, f, t, v, id, pi, a);
+        }
+    }
+    if (DIAG) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+#pragma unroll
+            for (int q = 16; q > 0; q >>= 1) a.h[r] += __shfl_xor_sync(kAll, a.h[r], q);
+        }
+        if (lane == 0) {
+            const uint32_t id = __float_as_uint(p4.w) + (k.slot_base - k.slot_off);
+            o.dcnt[3 * id + 0] = a.ncoh; o.dcnt[3 * id + 1] = a.nsep; o.dcnt[3 * id + 2] = a.nali;
+            o.dhash[3 * id + 0] = a.h[0]; o.dhash[3 * id + 1] = a.h[1]; o.dhash[3 * id + 2] = a.h[2];
+        }
+    } else {
+        warp_finish(a.acc, a.ncoh, a.nali, p4, si.v, s, lane, o, k);
     }
 }
 
@@ -1916,6 +2402,13 @@ __global__ void k_ref_cells(const float4 *__restrict__ pos, int32_t *__restrict_
 
 static inline unsigned blocks_for(uint32_t n, unsigned t) { return (n + t - 1) / t; }
 
+// Whether every boid goes to k_grid_warp: flocks (or ensembles) of at most
+// kWarpBoids slots, unless the cells' split was set by hand.
+static inline bool grid_by_warp(const StepConst &k, const DevBuffers &b, const FlockTable *ft)
+{
+    return b.slot_of && !k.tuned && (ft ? ft->nslots : k.n) <= kWarpBoids;
+}
+
 cudaError_t launch_pack(const float *pos3, const float *vel3, float4 *pos4, float4 *vel4, uint32_t i0, uint32_t i1,
                         uint32_t *bad, float hi, const StepConst *bin, uint32_t *key, uint32_t *rank,
                         uint32_t *count, cudaStream_t st, uint64_t *launches)
@@ -1978,9 +2471,11 @@ cudaError_t launch_grid_keys(const StepConst &k, const float4 *pos, uint32_t *ke
 cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream_t st, uint64_t *launches,
                              const FlockTable *ft)
 {
-    cudaError_t e = cudaMemsetAsync(b.dense_n, 0, 3 * sizeof(uint32_t), st);  // items, work queue, deferred
-    if (e != cudaSuccess) return e;
-    if (ft && b.defer_cnt && (e = cudaMemsetAsync(b.defer_cnt, 0, sizeof(uint32_t) * ft->count, st)) != cudaSuccess)
+    cudaError_t e = cudaSuccess;
+    const bool by_cells = !grid_by_warp(k, b, ft);
+    if (by_cells && (e = cudaMemsetAsync(b.dense_n, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess)
+        return e;  // items, work queue, deferred
+    if (by_cells && ft && b.defer_cnt && (e = cudaMemsetAsync(b.defer_cnt, 0, sizeof(uint32_t) * ft->count, st)) != cudaSuccess)
         return e;  // an ensemble's per-flock deferred counts
     k_grid_scan<<<b.nscan_blocks, kScanThreads, 0, st>>>(b.count, b.lstart, b.bsum, b.ticket, b.nscan_blocks);
     *launches += 1;
@@ -1990,6 +2485,7 @@ cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream
 cudaError_t launch_grid_classify(const StepConst &k, const DevBuffers &b, cudaStream_t st, uint64_t *launches,
                                  const FlockTable *ft)
 {
+    if (grid_by_warp(k, b, ft)) return cudaSuccess;
     cudaError_t e;
     const uint32_t nfull = b.ncell / 4;
     const int windows = b.carry != nullptr;
@@ -2019,12 +2515,13 @@ cudaError_t launch_grid_scatter(const StepConst &k, const DevBuffers &b, int fro
     const uint32_t n = ft ? ft->nslots : k.n;
     if (n == 0) return cudaSuccess;
     uint32_t *cz = zero_counts ? b.count : nullptr;
+    uint32_t *so = grid_by_warp(k, b, ft) ? b.slot_of : nullptr;
     if (ft)
         k_grid_scatter<true><<<blocks_for(n, 256), 256, 0, st>>>(b.pos[from], b.vel[from], b.key, b.rank, b.lstart,
-                                                                 b.bsum, b.pos[1 - from], b.vel[1 - from], cz, n, *ft);
+                                                                 b.bsum, b.pos[1 - from], b.vel[1 - from], cz, so, n, *ft);
     else
         k_grid_scatter<false><<<blocks_for(n, 256), 256, 0, st>>>(b.pos[from], b.vel[from], b.key, b.rank, b.lstart,
-                                                                  b.bsum, b.pos[1 - from], b.vel[1 - from], cz, n,
+                                                                  b.bsum, b.pos[1 - from], b.vel[1 - from], cz, so, n,
                                                                   FlockTable{});
     ++*launches;
     return cudaGetLastError();
@@ -2053,6 +2550,11 @@ template <bool DIAG, bool MULTI>
 cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, const DevBuffers &b, unsigned nsp,
                        const FlockTable &ft, cudaStream_t st)
 {
+    if (grid_by_warp(k, b, MULTI ? &ft : nullptr)) {
+        k_grid_warp<DIAG, MULTI><<<blocks_for(MULTI ? ft.nslots : k.n, kWarpWarps), kWarpWarps * 32, 0, st>>>(g, o, k,
+                                                                                                          ft);
+        return cudaGetLastError();
+    }
     cudaError_t e = dense_smem_opt_in<DIAG, MULTI>();
     if (e != cudaSuccess) return e;
     if (b.aux && (e = cudaStreamWaitEvent(st, b.cjoin, 0)) != cudaSuccess) return e;  // the classification
@@ -2080,7 +2582,7 @@ cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from,
 {
     const uint32_t n = ft ? ft->nslots : k.n;
     if (n == 0) return cudaSuccess;
-    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, b.dflag};
+    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, b.dflag, b.slot_of};
     GridOut o{};
     o.carry = static_cast<Acc *>(b.carry);
     o.wscratch = b.carry ? b.wscratch : nullptr;
@@ -2109,7 +2611,7 @@ cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from,
     cudaError_t e;
     if (ft) e = diag ? grid_force<true, true>(k, g, o, b, nsp, *ft, st) : grid_force<false, true>(k, g, o, b, nsp, *ft, st);
     else e = diag ? grid_force<true, false>(k, g, o, b, nsp, none, st) : grid_force<false, false>(k, g, o, b, nsp, none, st);
-    if (e == cudaSuccess) *launches += o.defer ? 3 : 2;
+    if (e == cudaSuccess) *launches += grid_by_warp(k, b, ft) ? 1 : (o.defer ? 3 : 2);
     return e;
 }
 
@@ -2346,7 +2848,7 @@ cudaError_t launch_ensemble_stats(const DevBuffers &b, int from, const FlockTabl
     if ((e = cudaMemsetAsync(err, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
     k_stat_moments<<<nb, kStatThreads, 0, st>>>(b.pos[from], b.vel[from], ft, acc, parent);
     k_stat_com<<<blocks_for(ft.count, 128), 128, 0, st>>>(acc, ft.ks, ft.count, com);
-    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, nullptr};  // k_stat_pairs reads no dense flags
+    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, nullptr, nullptr};  // k_stat_pairs reads only cells
     k_stat_pairs<<<nb, kStatThreads, 0, st>>>(g, ft, com, link, acc, parent, err);
     k_stat_roots<<<blocks_for(ft.nslots, 256), 256, 0, st>>>(ft, parent, size, err);
     k_stat_largest<<<blocks_for(ft.nslots, 256), 256, 0, st>>>(ft, parent, size, largest);

@@ -165,6 +165,10 @@ size_t layout(const boidsgpu::StepConst &k, unsigned char *base, boidsgpu::DevBu
     b->ticket = reinterpret_cast<uint32_t *>(take(4));
     b->dense_n = reinterpret_cast<uint32_t *>(take(12));
     b->dflag = take(b->ncell / 4);
+    // the counts are dead after the scan: the id -> slot table of a small
+    // flock takes their place where it fits, so that it costs no scratch there
+    if (k.n <= boidsgpu::kWarpBoids)
+        b->slot_of = n <= b->ncell_pad ? b->count : reinterpret_cast<uint32_t *>(take(4 * n));
     b->carry = nullptr;  // no id windows: cells over the dense list's capacity stay per-boid
     b->defer = nullptr;  // and the thread-per-boid kernel takes all of its boids' passes
     return off;

@@ -26,18 +26,12 @@ def crowd_state(m, others, centre, seed):
     return pos[perm].astype(np.float32).reshape(-1), v[perm].astype(np.float32).reshape(-1)
 
 
-@pytest.mark.parametrize("corner", [False, True])
-@pytest.mark.parametrize("tuning", [None, (1, 1, 0, 0), (1 << 30,) * 4])
-@pytest.mark.parametrize("m", [1, 31, 32, 33, 64, 129, 256, 511, 512, 513, 1100])
-def test_crowds_at_tile_edges(boids_lib, oracle_mod, m, tuning, corner):
-    O, prm = oracle_mod, oracle_mod.MARUN2019
-    centre = 0.0 if corner else 6.5 * FIELD / 13
-    pos, vel = crowd_state(m, 40, centre, 1000 + m)
-    n = len(pos) // 3
+def check(B, O, pos, vel, tuning):
+    prm, n = O.MARUN2019, len(pos) // 3
     p = make_params(O, n, FIELD, prm)
     op, ov = pos.copy(), vel.copy()
     of = O.GridPort(p, op).step(op, ov, 1, forces=True)
-    sim = make_sim(boids_lib, "grid", n, FIELD, prm)
+    sim = make_sim(B, "grid", n, FIELD, prm)
     if tuning:
         sim.set_tuning(*tuning)
     sim.set_state(pos, vel)
@@ -50,3 +44,44 @@ def test_crowds_at_tile_edges(boids_lib, oracle_mod, m, tuning, corner):
     assert_bits_equal(gv, ov, "velocities")
     assert_bits_equal(sim.forces(), of, "forces")
     sim.close()
+    return c
+
+
+@pytest.mark.parametrize("corner", [False, True])
+@pytest.mark.parametrize("tuning", [None, (1, 1, 0, 0), (1 << 30,) * 4])
+@pytest.mark.parametrize("m", [1, 31, 32, 33, 64, 129, 256, 511, 512, 513, 1100])
+def test_crowds_at_tile_edges(boids_lib, oracle_mod, m, tuning, corner):
+    pos, vel = crowd_state(m, 40, 0.0 if corner else 6.5 * FIELD / 13, 1000 + m)
+    check(boids_lib, oracle_mod, pos, vel, tuning)
+
+
+@pytest.mark.parametrize("others", [8192 - 700, 8193 - 700, 17000])
+def test_crowds_over_the_list_across_id_windows(boids_lib, oracle_mod, others):
+    """More accepted neighbours than a warp's list holds, with ids over one,
+    just over one and three windows of its bit map."""
+    pos, vel = crowd_state(700, others, 0.0, others)
+    c = check(boids_lib, oracle_mod, pos, vel, None)
+    assert c.max() > 256
+
+
+def test_ensemble_tuned_between_statistics_and_step(boids_lib):
+    """Thresholds set while the statistics' binning waits for its step: that
+    step runs on what was classified, the later ones by the thresholds."""
+    B = boids_lib
+    m = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008))
+    flocks = [(B.flock_params(n, (n / 16384) ** (1 / 3), m["sep"], m["ali"], m["coh"], 0.005, 0.001),
+               B.INIT_RANDOM_UNIFORM, 5 + n) for n in (1000, 3000)]
+    a, b = B.Ensemble(flocks), B.Ensemble(flocks)
+    for e in (a, b):
+        e.init()
+        e.step(60)
+    a.stats()
+    a.set_tuning(4, 2, 64, 32)
+    for e in (a, b):
+        e.step(3)
+    for f in range(len(flocks)):
+        for x, y in zip(a.state(f), b.state(f)):
+            assert_bits_equal(x, y, "flock %d" % f)
+        assert a.tuning() == (4, 2, 64, 32)
+    a.close()
+    b.close()
