@@ -183,7 +183,7 @@ namespace {
 void free_buffers(DevBuffers &b)
 {
     void *ptrs[] = {b.pos[0], b.pos[1], b.vel[0], b.vel[1], b.key, b.rank, b.count, b.lstart,
-                    b.bsum, b.ticket, b.ap_cnt, b.ap_list, b.forces, b.stage, b.cells8, b.dcnt, b.dhash,
+                    b.bsum, b.ticket, b.ap_cnt, b.ap_list, b.ap_emb, b.forces, b.stage, b.cells8, b.dcnt, b.dhash,
                     b.dense_list, b.dense_n, b.flag, b.slot_of, b.dflag, b.carry, b.defer, b.ovf, b.ovf_n, b.wscratch};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -384,6 +384,18 @@ int make_constants(const boids_params &p, StepConst &k, bool *ref_ok)
     const double rf = (double)rmax * (1.0 + 1e-4) + 8.0 * ulpF;
     k.filt_r2 = (float)(rf * rf);
     k.box_lim = (float)(p.field_size / 2 - rf * (1.0 + 1e-4) - 8.0 * ulpF);
+    {
+        // The all-pairs product filter sums cos(2 pi dx / F) over the axes, for
+        // a pair within rf at least 3 - (2 pi rf / F)^2 / 2 (cos a >= 1 - a^2 / 2).
+        // Rounding cosines and sines (at most 1) to half precision moves each
+        // by at most 2^-12, an axis's sum by 2 sqrt(2) 2^-12 + 2^-23: 2.08e-3
+        // over the axes; the angles of coordinates up to 4 F (2^-23 relative),
+        // sincospif, the FP32 sum of eight products and ap_min's own split into
+        // two half-precision terms add less than 1e-4.
+        const double r = 2.0 * M_PI * (rf * (1.0 + 1e-4) + 8.0 * ulpF) / p.field_size;
+        k.ap_turn = (float)(2.0 / p.field_size);
+        k.ap_min = f_dn(3.0 - r * r / 2.0 - 2.3e-3);
+    }
     // The filters' relative vector differs from the exact imaged one by a
     // few ulps of the coordinates (at most 2F in magnitude), each dot
     // product by those times |v|_1 <= sqrt(3)|v| plus three roundings of
@@ -558,6 +570,7 @@ int boids_create(const boids_params *params, boids_sim **out)
         b.ap_cap = boidsgpu::kApCap;
         ALLOC(&b.ap_cnt, n, true);
         ALLOC(&b.ap_list, n * b.ap_cap);
+        ALLOC(&b.ap_emb, n);
     }
     if (p.flags & BOIDS_FLAG_RECORD_FORCES) ALLOC(&b.forces, 9 * n);
 #undef ALLOC

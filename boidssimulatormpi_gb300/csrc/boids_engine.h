@@ -44,6 +44,7 @@ struct StepConst {
     float filt_r2;       // squared radius of the conservative fast filter
     float box_lim;       // all-pairs box filter: ||dx| - F/2| > box_lim
     float halfFf;        // (float)(F/2) for the box filter
+    float ap_turn, ap_min;  // all-pairs product filter: 2 / F, least sum of the axes' cosines of a pair in reach
     float cc, cs, ca;    // (float) force coefficients: cohesion, separation, alignment
     float vmax_dn, vmin_up;  // speed clamp tests
     float vmax_f, vmin_f;    // speed clamp scale factors (float)vmax, (float)vmin
@@ -106,6 +107,7 @@ struct DevBuffers {
     uint32_t *bsum;            // per scan tile: offset of the tile
     uint32_t *ticket;          // scan completion counter (1 word)
     uint32_t *ap_cnt, *ap_list;  // all-pairs: per boid neighbour count and list
+    uint4 *ap_emb;             // all-pairs: per boid filter vector
     float *forces;             // 9 per boid (id order), optional
     float *stage;              // 6 per boid, host<->device staging
     int32_t *cells8;           // 8 per boid (id order)

@@ -186,20 +186,6 @@ __device__ __forceinline__ void acc_add(Acc &a, float3 pi, float3 t, float3 vj, 
     }
 }
 
-// Exact test of candidate j (state slot) and, if accepted, accumulation.
-template <bool DIAG>
-__device__ __forceinline__ void visit(Acc &a, float3 pi, const Sight &s, const float4 *__restrict__ pos,
-                                      const float4 *__restrict__ vel, uint32_t j, const StepConst &k)
-{
-    const float4 pj = __ldg(pos + j);
-    const float3 t = image3(xyz(pj), pi, k);
-    const int f = pair_flags(pi, s, t, k);
-    if (f) {
-        const float3 vj = (f & 4) ? xyz(__ldg(vel + j)) : make_float3(0.f, 0.f, 0.f);
-        acc_add<DIAG>(a, pi, t, vj, f, __float_as_uint(pj.w));
-    }
-}
-
 // Rule finalisation (src/boid_simulation_grid.cpp:243-252): returns the three
 // scaled rule forces, which are also get_force's values (:319-334).
 __device__ __forceinline__ void acc_finish(const Acc &a, float3 pi, float3 vi, const StepConst &k,
@@ -1357,17 +1343,30 @@ __device__ __noinline__ void warp_many(WarpSmem *smp, const GridIn &g, const Ste
     }
 }
 
-// finish_boid by the lanes of a warp: lane 3 r + c holds component c of rule
-// r's sum (cohesion, separation, alignment) in acc.
-__device__ __forceinline__ void warp_finish(float acc, int ncoh, int nali, float4 p4, float3 vi, uint32_t s, int lane,
-                                            const GridOut &o, const StepConst &k)
+// finish_boid by the lanes of a warp.
+template <bool DIAG>
+__device__ __forceinline__ void warp_finish(WarpSums &a, float4 p4, float3 vi, uint32_t s, int lane, const GridOut &o,
+                                            const StepConst &k)
 {
     constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t out = __float_as_uint(p4.w) + (k.slot_base - k.slot_off);  // the boid's output row
+    if (DIAG) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+#pragma unroll
+            for (int q = 16; q > 0; q >>= 1) a.h[r] += __shfl_xor_sync(kAll, a.h[r], q);
+        }
+        if (lane == 0) {
+            o.dcnt[3 * out + 0] = a.ncoh; o.dcnt[3 * out + 1] = a.nsep; o.dcnt[3 * out + 2] = a.nali;
+            o.dhash[3 * out + 0] = a.h[0]; o.dhash[3 * out + 1] = a.h[1]; o.dhash[3 * out + 2] = a.h[2];
+        }
+        return;
+    }
     const int r = lane / 3, c = lane - 3 * r;
     const float pc = c == 0 ? p4.x : (c == 1 ? p4.y : p4.z), vc = c == 0 ? vi.x : (c == 1 ? vi.y : vi.z);
-    float f = acc;
-    const int q = r == 0 ? ncoh : nali;
-    if (r != 1 && q != 0) f = __fsub_rn(__fdiv_rn(acc, __int2float_rn(q)), r == 0 ? pc : vc);
+    float f = a.acc;
+    const int q = r == 0 ? a.ncoh : a.nali;
+    if (r != 1 && q != 0) f = __fsub_rn(__fdiv_rn(a.acc, __int2float_rn(q)), r == 0 ? pc : vc);
     f = __fmul_rn(f, r == 0 ? k.cc : (r == 1 ? k.cs : k.ca));
     const float fs = __shfl_sync(kAll, f, c + 3), fa = __shfl_sync(kAll, f, c + 6);
     // lanes 0-2: a component each (the others' values are not used)
@@ -1387,7 +1386,7 @@ __device__ __forceinline__ void warp_finish(float acc, int ncoh, int nali, float
         o.rank_out[s] = atomicAdd(o.count + cell, 1u);
     }
     if (o.forces && lane < 9)
-        o.forces[(size_t)9 * (__float_as_uint(p4.w) + (k.slot_base - k.slot_off)) + lane] = f;
+        o.forces[(size_t)9 * out + lane] = f;
 }
 
 template <bool DIAG, bool MULTI>
@@ -1553,20 +1552,7 @@ k_grid_warp(GridIn g, GridOut o, StepConst kp, FlockTable ft)
             warp_add<DIAG>(sm, lane, f, t, v, id, pi, a);
         }
     }
-    if (DIAG) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-#pragma unroll
-            for (int q = 16; q > 0; q >>= 1) a.h[r] += __shfl_xor_sync(kAll, a.h[r], q);
-        }
-        if (lane == 0) {
-            const uint32_t id = __float_as_uint(p4.w) + (k.slot_base - k.slot_off);
-            o.dcnt[3 * id + 0] = a.ncoh; o.dcnt[3 * id + 1] = a.nsep; o.dcnt[3 * id + 2] = a.nali;
-            o.dhash[3 * id + 0] = a.h[0]; o.dhash[3 * id + 1] = a.h[1]; o.dhash[3 * id + 2] = a.h[2];
-        }
-    } else {
-        warp_finish(a.acc, a.ncoh, a.nali, p4, si.v, s, lane, o, k);
-    }
+    warp_finish<DIAG>(a, p4, si.v, s, lane, o, k);
 }
 
 // ------------------------------------------------------------------ dense cells: CTA per cell
@@ -2246,114 +2232,253 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
 
 // ------------------------------------------------------------------ all-pairs engine
 
-// Phase 1: a 2-D grid of (i-tile, j-tile) blocks tests every ordered pair.
-// A box filter on the minimum-image offset (||dx| - F/2| > F/2 - R per axis)
-// rejects almost all pairs; survivors get the exact tests and accepted
-// neighbours are appended to the boid's list (unordered).  A thread's box
-// hits are buffered and the whole warp runs their exact tests together once a
-// buffer is nearly full (and at the end of the tile), so the rare hits do not
-// stall the filter loop of the other 31 lanes, as they would inline.
+// Every ordered pair is tested by a filter that is a matrix product.  A boid's
+// coordinates become the cosines and sines of 2 pi x / F, 2 pi y / F and
+// 2 pi z / F: six half-precision values whose inner product with another
+// boid's is the sum over the axes of cos(2 pi (xi - xj) / F), which is periodic
+// by itself, with no minimum image to take.  A pair within the radius r has a
+// sum of at least 3 - (2 pi r / F)^2 / 2; StepConst::ap_min is that less the
+// rounding's bound, so the filter drops no pair the exact tests accept (it
+// keeps a ball of about 1.05 r at r = F / 32).  Two further terms, w_i * 1 and
+// 1 * u_j, subtract ap_min (w + u = -ap_min, u the rounding of w), and pass
+// every pair of a boid so far outside the field (over 4 F) that its angles are
+// not exact enough.
+//
+// 64 boids a warp against 8 at a time: four mma.m16n8k8, and an AND over their
+// 16 results a lane, whose sign says whether any pair passed.  Survivors are queued per warp and take the exact
+// tests 32 at a time; accepted neighbours are appended to the boid's list
+// (unordered).
+//
+// Bound by instruction issue (62 % of the slots, the tensor pipe 57 % active):
+// 1024 pairs take 67 warp instructions, half of them in the 40 % of the steps
+// in which some pair passes, where a box filter on the FP32 offsets took 15.7
+// per pair and thread.  N = 65 536, F = 1.6: 0.39 ms a launch (1.79 before),
+// 1.1e13 pairs/s.  One code path tests the queue: inlined at each of the 32
+// results it cost 0.1 ms in instruction fetches.  mma.sync serves better than
+// tcgen05 here: the product is eight deep and every one of its N^2 results has
+// to come back through registers to be compared, so the tensor rate is not
+// what counts.
 constexpr int kApThreads = 128;
-constexpr int kApKI = 8;                        // i per thread
-constexpr int kApTileI = kApThreads * kApKI;    // 1024
-constexpr int kApTileJ = 1024;
-constexpr int kApHits = 24;                     // box hits buffered per thread
-static_assert(kApHits > kApKI, "a j step's hits fit the buffer");
+constexpr int kApTilesM = 4;                                  // 16-boid tiles of a warp
+constexpr int kApWarpI = 16 * kApTilesM;                      // its boids i
+constexpr int kApTileI = kApWarpI * (kApThreads / 32);        // 256
+constexpr int kApTileJ = 1024;                                // most boids j of a CTA
+static_assert(kApCap <= kWarpList, "k_ap_accumulate orders a boid's list in shared memory");
 
-__global__ void __launch_bounds__(kApThreads)
-k_ap_pairs(const float4 *__restrict__ pos, const float4 *__restrict__ vel, uint32_t *__restrict__ cnt,
-           uint32_t *__restrict__ list, uint32_t cap, StepConst k)
+// A boid's filter vector: per axis (cos, sin), then (w, u).
+__global__ void k_ap_embed(const float4 *__restrict__ pos, uint4 *__restrict__ emb, uint32_t n, StepConst k)
 {
-    __shared__ float4 sp[kApTileJ];
-    __shared__ uint16_t hits[kApHits][kApThreads];  // r << 10 | tile j
-    const uint32_t n = k.n;
-    const uint32_t j0 = blockIdx.y * kApTileJ;
-    const uint32_t jn = min((uint32_t)kApTileJ, n - j0);
-    const uint32_t ibase = blockIdx.x * kApTileI + threadIdx.x;
-    for (uint32_t t = threadIdx.x; t < jn; t += kApThreads) sp[t] = pos[j0 + t];
-    float3 pi[kApKI];
-    const float nanf_ = __uint_as_float(0x7fffffffu);  // fails every filter test
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 p = pos[i];
+    const float far = fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z));
+    const float c[3] = {p.x, p.y, p.z};
+    __half2 h[4];
 #pragma unroll
-    for (int r = 0; r < kApKI; ++r) {
-        const uint32_t i = ibase + r * kApThreads;
-        pi[r] = i < n ? xyz(pos[i]) : make_float3(nanf_, nanf_, nanf_);
+    for (int d = 0; d < 3; ++d) {
+        float sn = 0.f, cs = 0.f;
+        if (fabsf(c[d]) <= 4.f * k.Ff) sincospif(c[d] * k.ap_turn, &sn, &cs);
+        h[d] = __floats2half2_rn(cs, sn);
     }
-    __syncthreads();
-    int nh = 0;
-    // the exact tests of this thread's buffered hits (all lanes call it)
-    auto flush = [&]() {
-        for (int e = 0; e < nh; ++e) {
-            const uint32_t en = hits[e][threadIdx.x];
-            const uint32_t i = ibase + (en >> 10) * kApThreads, tj = en & 1023u, j = j0 + tj;
-            if (i == j) continue;
-            const float3 p = xyz(pos[i]);
-            const Sight s = make_sight(xyz(vel[i]));
-            const int f = pair_flags(p, s, image3(xyz(sp[tj]), p, k), k);
-            if (f) {
-                const uint32_t q = atomicAdd(cnt + i, 1u);
-                if (q < cap) list[(size_t)i * cap + q] = j | ((uint32_t)f << 29);
-            }
-        }
-        nh = 0;
-    };
-    const float h = k.halfFf, lim = k.box_lim;
-    for (uint32_t t = 0; t < jn; ++t) {
-        const float4 pj = sp[t];
-#pragma unroll
-        for (int r = 0; r < kApKI; ++r) {
-            const bool nx = fabsf(fabsf(pj.x - pi[r].x) - h) > lim;
-            const bool ny = fabsf(fabsf(pj.y - pi[r].y) - h) > lim;
-            const bool nz = fabsf(fabsf(pj.z - pi[r].z) - h) > lim;
-            if (nx && ny && nz) hits[nh++][threadIdx.x] = (uint16_t)((r << 10) | t);
-        }
-        if (__any_sync(0xffffffffu, nh > kApHits - kApKI)) flush();
-    }
-    flush();
+    // (a NaN coordinate, which no rule accepts, leaves its cosine and sine zero)
+    const __half w = __float2half_rn(-k.ap_min);
+    const float pass = far > 4.f * k.Ff ? 8.f : 0.f, u = -k.ap_min - __half2float(w);
+    h[3] = __floats2half2_rn(__half2float(w) + pass, u + pass);
+    emb[i] = *reinterpret_cast<const uint4 *>(h);
 }
 
-// Phase 2: per boid, sort its neighbours by id and accumulate in that order,
-// then finish and integrate.  A boid with more than `cap` neighbours scans
-// all boids in order instead.
+__global__ void __launch_bounds__(kApThreads)
+k_ap_pairs(const float4 *__restrict__ pos, const float4 *__restrict__ vel, const uint4 *__restrict__ emb,
+           uint32_t *__restrict__ cnt, uint32_t *__restrict__ list, uint32_t cap, uint32_t tile_j, StepConst k)
+{
+    __shared__ uint4 sj[kApTileJ];                     // the j's vectors, (1, u) last
+    __shared__ uint32_t queue[kApThreads / 32][64];    // per warp: surviving pairs, i << 10 | j in their tiles
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t n = k.n;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t j0 = blockIdx.y * tile_j, jn = min(tile_j, n - j0), jpad = (jn + 15) & ~15u;
+    const uint32_t i0 = blockIdx.x * kApTileI + wid * kApWarpI;
+    for (uint32_t q = threadIdx.x; q < jpad; q += kApThreads) {
+        uint4 e = make_uint4(0, 0, 0, 0xc8000000u);  // past the end: no angles, u = -8
+        if (q < jn) e = emb[j0 + q];
+        e.w = (e.w & 0xffff0000u) | 0x3c00u;
+        sj[q] = e;
+    }
+    uint32_t a[kApTilesM][2];  // rows g and g + 8 of each tile, terms 2t and 2t + 1
+    const uint32_t *ew = reinterpret_cast<const uint32_t *>(emb);
+#pragma unroll
+    for (int m = 0; m < kApTilesM; ++m)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t i = i0 + 16 * m + 8 * r + g;
+            a[m][r] = i < n ? ew[4 * (size_t)i + t] : 0u;
+            if (t == 3) a[m][r] = (a[m][r] & 0xffffu) | 0x3c000000u;  // (w, 1)
+        }
+    __syncthreads();
+    if (i0 >= n) return;
+    uint32_t *q = queue[wid];
+    int nq = 0;
+    auto test = [&](int from, int count) {  // the exact tests of queue entries [from, from + count)
+        __syncwarp();
+        if (lane < count) {
+            const uint32_t e = q[from + lane];
+            const uint32_t i = i0 + (e >> 10), tj = e & 1023u, j = j0 + tj;
+            if (i != j && i < n && tj < jn) {
+                const float3 p = xyz(pos[i]);
+                const Sight s = make_sight(xyz(vel[i]));
+                const int f = pair_flags(p, s, image3(xyz(pos[j]), p, k), k);
+                if (f) {
+                    const uint32_t at = atomicAdd(cnt + i, 1u);
+                    if (at < cap) list[(size_t)i * cap + at] = j | ((uint32_t)f << 29);
+                }
+            }
+        }
+        __syncwarp();
+    };
+    const uint32_t *bw = reinterpret_cast<const uint32_t *>(sj) + 4 * g + t;
+    for (uint32_t jt = 0; jt < jpad; jt += 16) {  // two tiles of 8 j
+        float d[2][kApTilesM][4];
+        int all = -1;  // sign set: no pair passed
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t b = bw[4 * (jt + 8 * h)];
+#pragma unroll
+            for (int m = 0; m < kApTilesM; ++m) {
+                float(&x)[4] = d[h][m];
+                asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+                    "{%7, %7, %7, %7};"
+                    : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+                    : "r"(a[m][0]), "r"(a[m][1]), "r"(b), "f"(0.f));
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int m = 0; m < kApTilesM; ++m)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) all &= __float_as_int(d[h][m][r]);
+        if (!__any_sync(kAll, all >= 0)) continue;
+        // a bit per result, the first one highest: 0 for a pair that passed
+        uint32_t miss = 0;
+        static_assert(2 * kApTilesM * 4 == 32, "a lane's results fill a word");
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int m = 0; m < kApTilesM; ++m)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) miss = __funnelshift_l(__float_as_uint(d[h][m][r]), miss, 1);
+        for (;;) {  // each lane's next passing pair
+            const unsigned hm = __ballot_sync(kAll, ~miss != 0);
+            if (!hm) break;
+            if (~miss != 0) {
+                const int x = __clz(~miss), r = x & 3, m = (x >> 2) & 3, h = x >> 4;
+                miss |= 0x80000000u >> x;
+                q[nq + __popc(hm & below)] =
+                    ((uint32_t)(16 * m + (r >> 1) * 8 + g) << 10) | (jt + 8 * h + 2 * t + (r & 1));
+            }
+            nq += __popc(hm);
+            if (nq >= 32) {
+                nq -= 32;
+                test(nq, 32);
+            }
+        }
+    }
+    test(0, nq);
+}
+
+// Then a warp per boid: its neighbours in id order, added up and the boid
+// finished as in k_grid_warp.  A boid with more than `cap` neighbours takes
+// all boids in order instead, 32 at a time.  The lists are scattered 4-byte
+// stores of the pass before, whose sectors the first read fills from DRAM: a
+// warp loads its next boid's record, count and first 32 entries before it
+// works on the present one's (67 us at N = 65 536; 189 us with a CTA per four
+// boids that waits for them).
 template <bool DIAG>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kWarpWarps * 32, kWarpCtas)
 k_ap_accumulate(const float4 *__restrict__ pos, const float4 *__restrict__ vel, uint32_t *__restrict__ cnt,
                 const uint32_t *__restrict__ list, uint32_t cap, GridOut o, StepConst k)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ WarpSmem sms[kWarpWarps];
+    WarpSmem &sm = sms[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t step = gridDim.x * kWarpWarps;
+    uint32_t i = blockIdx.x * kWarpWarps + (threadIdx.x >> 5);
     if (i >= k.n) return;
-    const float4 p4 = pos[i], v4 = vel[i];
-    const float3 pi = xyz(p4), vi = xyz(v4);
-    const uint32_t m = cnt[i];
-    cnt[i] = 0;  // ready for the next step
-    Acc a;
-    acc_zero(a);
-    if (m <= cap) {
-        uint32_t lst[kApCap];
-        for (uint32_t q = 0; q < m; ++q) {
-            const uint32_t e = list[(size_t)i * cap + q];
-            uint32_t w = q;
-            while (w > 0 && (lst[w - 1] & 0x1fffffffu) > (e & 0x1fffffffu)) { lst[w] = lst[w - 1]; --w; }
-            lst[w] = e;
+    float4 p4 = __ldg(pos + i), v4 = __ldg(vel + i);
+    uint32_t m = cnt[i], e0 = list[(size_t)i * cap + lane];  // (entries past the count are not used)
+    for (;;) {
+        const uint32_t nx = i + step;
+        float4 p_next = zero4, v_next = zero4;
+        uint32_t m_next = 0, e_next = 0;
+        if (nx < k.n) {
+            p_next = __ldg(pos + nx);
+            v_next = __ldg(vel + nx);
+            m_next = cnt[nx];
+            e_next = list[(size_t)nx * cap + lane];
         }
-        for (uint32_t q = 0; q < m; ++q) {
-            const uint32_t j = lst[q] & 0x1fffffffu;
-            const int f = (int)(lst[q] >> 29);
-            const float3 t = image3(xyz(pos[j]), pi, k);
-            const float3 vj = (f & 4) ? xyz(vel[j]) : make_float3(0.f, 0.f, 0.f);
-            acc_add<DIAG>(a, pi, t, vj, f, j);
+        const uint32_t *mine = list + (size_t)i * cap;
+        const float3 pi = xyz(p4);
+        const Sight si = make_sight(xyz(v4));
+        if (lane == 0) cnt[i] = 0;  // ready for the next step
+        WarpSums a{};
+        if (m <= cap) {
+            for (uint32_t q = lane; q < m; q += 32) {
+                const uint32_t e = q < 32 ? e0 : mine[q];
+                sm.lid[q] = e & 0x1fffffffu;
+                sm.lsl[q] = e;
+            }
+            __syncwarp();
+            if (m > 0) warp_order(sm, lane, (int)m);
+            uint32_t e = 0;
+            float4 pj = zero4, vj = zero4;
+            auto load = [&](uint32_t q) {
+                e = 0;
+                if (q < m) {
+                    e = sm.lsl[sm.ord[q]];
+                    pj = __ldg(pos + (e & 0x1fffffffu));
+                    vj = __ldg(vel + (e & 0x1fffffffu));
+                }
+            };
+            load(lane);
+            for (uint32_t q0 = 0; q0 < m; q0 += 32) {
+                const int f = (int)(e >> 29);
+                const uint32_t j = e & 0x1fffffffu;
+                const float3 t = image3(xyz(pj), pi, k);
+                const float4 v = vj;
+                load(q0 + 32 + lane);
+                warp_add<DIAG>(sm, lane, f, t, v, j, pi, a);
+            }
+        } else {
+            for (uint32_t j0 = 0; j0 < k.n; j0 += 32) {
+                const uint32_t j = j0 + lane;
+                int f = 0;
+                float3 t = make_float3(0.f, 0.f, 0.f);
+                float4 vj = zero4;
+                if (j < k.n && j != i) {
+                    const float4 pj = pos[j];
+                    const bool nx = fabsf(fabsf(pj.x - pi.x) - k.halfFf) > k.box_lim;
+                    const bool ny = fabsf(fabsf(pj.y - pi.y) - k.halfFf) > k.box_lim;
+                    const bool nz = fabsf(fabsf(pj.z - pi.z) - k.halfFf) > k.box_lim;
+                    if (nx && ny && nz) {
+                        t = image3(xyz(pj), pi, k);
+                        f = pair_flags(pi, si, t, k);
+                        if (f) vj = vel[j];
+                    }
+                }
+                warp_add<DIAG>(sm, lane, f, t, vj, j, pi, a);
+            }
         }
-    } else {
-        const Sight s = make_sight(vi);
-        for (uint32_t j = 0; j < k.n; ++j) {
-            if (j == i) continue;
-            const float4 pj = pos[j];
-            const bool nx = fabsf(fabsf(pj.x - pi.x) - k.halfFf) > k.box_lim;
-            const bool ny = fabsf(fabsf(pj.y - pi.y) - k.halfFf) > k.box_lim;
-            const bool nz = fabsf(fabsf(pj.z - pi.z) - k.halfFf) > k.box_lim;
-            if (nx && ny && nz) visit<DIAG>(a, pi, s, pos, vel, j, k);
-        }
+        warp_finish<DIAG>(a, p4, si.v, i, lane, o, k);
+        if (nx >= k.n) break;
+        i = nx;
+        p4 = p_next;
+        v4 = v_next;
+        m = m_next;
+        e0 = e_next;
+        __syncwarp();  // the list is rewritten
     }
-    finish_boid<DIAG>(a, p4, vi, i, o, k);
 }
 
 // ------------------------------------------------------------------ reference cell indices
@@ -2619,8 +2744,15 @@ cudaError_t launch_allpairs(const StepConst &k, const DevBuffers &b, int from, b
                             cudaStream_t st, uint64_t *launches)
 {
     if (k.n == 0) return cudaSuccess;
-    dim3 grid(blocks_for(k.n, kApTileI), blocks_for(k.n, kApTileJ));
-    k_ap_pairs<<<grid, kApThreads, 0, st>>>(b.pos[from], b.vel[from], b.ap_cnt, b.ap_list, b.ap_cap, k);
+    k_ap_embed<<<blocks_for(k.n, 128), 128, 0, st>>>(b.pos[from], b.ap_emb, k.n, k);
+    // the j tiles shrink until the GPU has a few CTAs per SM: where every pair
+    // passes the filter (a small field), the exact tests are the work
+    uint32_t tile_j = kApTileJ;
+    while (tile_j > 16 && (uint64_t)blocks_for(k.n, kApTileI) * blocks_for(k.n, tile_j) < 4 * 152) tile_j /= 2;
+    dim3 grid(blocks_for(k.n, kApTileI), blocks_for(k.n, tile_j));
+    k_ap_pairs<<<grid, kApThreads, 0, st>>>(b.pos[from], b.vel[from], b.ap_emb, b.ap_cnt, b.ap_list, b.ap_cap, tile_j,
+                                            k);
+    *launches += 1;
     cudaError_t e = cudaGetLastError();
     ++*launches;
     if (e != cudaSuccess) return e;
@@ -2633,11 +2765,11 @@ cudaError_t launch_allpairs(const StepConst &k, const DevBuffers &b, int from, b
         o.vel_out = b.vel[1 - from];
         o.forces = record_forces ? b.forces : nullptr;
     }
-    const unsigned nb = blocks_for(k.n, 128);
+    const unsigned nb = min(blocks_for(k.n, kWarpWarps), 152u * kWarpCtas), nt = kWarpWarps * 32;
     if (diag) {
-        k_ap_accumulate<true><<<nb, 128, 0, st>>>(b.pos[from], b.vel[from], b.ap_cnt, b.ap_list, b.ap_cap, o, k);
+        k_ap_accumulate<true><<<nb, nt, 0, st>>>(b.pos[from], b.vel[from], b.ap_cnt, b.ap_list, b.ap_cap, o, k);
     } else {
-        k_ap_accumulate<false><<<nb, 128, 0, st>>>(b.pos[from], b.vel[from], b.ap_cnt, b.ap_list, b.ap_cap, o, k);
+        k_ap_accumulate<false><<<nb, nt, 0, st>>>(b.pos[from], b.vel[from], b.ap_cnt, b.ap_list, b.ap_cap, o, k);
     }
     ++*launches;
     return cudaGetLastError();

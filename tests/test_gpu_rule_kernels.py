@@ -85,3 +85,30 @@ def test_ensemble_tuned_between_statistics_and_step(boids_lib):
         assert a.tuning() == (4, 2, 64, 32)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("field", [0.7, 0.13])  # 0.13: every pair is near the radius, no device cells
+@pytest.mark.parametrize("n", [1, 2, 15, 17, 63, 64, 65, 255, 257, 1023, 1025, 1041])
+def test_all_pairs_at_tile_edges(boids_lib, oracle_mod, n, field):
+    """The N^2 kernels at the edges of their 8, 16, 64, 256 and 1024 boid
+    tiles, some boids outside the field and beyond the distance up to which
+    the filter's angles are used."""
+    O, prm = oracle_mod, oracle_mod.MARUN2019
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(0, field, (n, 3))
+    out = rng.random(n) < 0.2
+    pos[out] += field * rng.integers(-6, 7, (out.sum(), 3))
+    v = rng.normal(size=(n, 3))
+    v *= rng.uniform(0.001, 0.005, (n, 1)) / np.linalg.norm(v, axis=1, keepdims=True)
+    pos, vel = pos.astype(np.float32).reshape(-1), v.astype(np.float32).reshape(-1)
+    p = make_params(O, n, field, prm)
+    op, ov = pos.copy(), vel.copy()
+    of = O.step_allpairs(p, op, ov, 2, forces=True)
+    sim = make_sim(boids_lib, "pairs", n, field, prm)
+    sim.set_state(pos, vel)
+    sim.update(2)
+    gp, gv = sim.state()
+    assert_bits_equal(gp, op, "positions")
+    assert_bits_equal(gv, ov, "velocities")
+    assert_bits_equal(sim.forces(), of, "forces")
+    sim.close()
