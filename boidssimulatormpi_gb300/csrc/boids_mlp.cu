@@ -120,6 +120,7 @@ constexpr int kTcThreads = 128;
 constexpr uint32_t kTcABytes = kTcM * kTcK * 2;   // 64 KB
 constexpr uint32_t kTcBBytes = kTcN * kTcK * 2;   // 128 KB
 constexpr size_t kTcSmem = kTcABytes + kTcBBytes + 1024 + 64;
+constexpr size_t kTcSplitSmem = kTcABytes + 64 * kTcK * 2 + 1024 + 64;  // 64 of the columns
 constexpr uint32_t kTcSpinLimit = 1u << 22;      // bounded wait on the accumulator
 
 __device__ uint32_t g_mlp_tc_error;  // set when a tile's wait gave up (the host reports it)
@@ -158,17 +159,26 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
 
-// One CTA per SM walks 128-row tiles: the weight image is loaded once, and
-// the next tile's activations are copied in (cp.async) while the current
-// tile's accumulator is read out.
+// A CTA takes kN of the 256 columns of its 128-row tiles (kN = 256: one CTA
+// per SM walks the tiles, the weight image is loaded once, and the next tile's
+// activations are copied in (cp.async) while the current tile's accumulator is
+// read out; kN = 64: a batch of few tiles is spread over four times as many
+// CTAs, 9 against 18 us for the 256 rows of a training batch).
+constexpr int kTcSplit = 64;
+static_assert(kTcSplitSmem == kTcABytes + kTcSplit * kTcK * 2 + 1024 + 64, "kTcSplit columns of weights");
+template <int kN>
 __global__ void __launch_bounds__(kTcThreads, 1)
 k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat16 *__restrict__ wimg,
                 const float *__restrict__ bias, float *__restrict__ pre, __nv_bfloat16 *__restrict__ h)
 {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
+    constexpr uint32_t kB = kN * kTcK * 2;  // its part of the weight image
     unsigned char *sa = tc_smem, *sb = tc_smem + kTcABytes;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(tc_smem + kTcABytes + kTcBBytes);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tc_smem + kTcABytes + kTcBBytes + 8);
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(tc_smem + kTcABytes + kB);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tc_smem + kTcABytes + kB + 8);
+    const int parts = kTcN / kN, tile0 = blockIdx.x / parts, tstep = gridDim.x / parts;
+    const int n0 = (blockIdx.x % parts) * kN;
+    wimg += (size_t)n0 * kTcK;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int ntiles = (rows + kTcM - 1) / kTcM;
     const uint32_t sa_s = (uint32_t)__cvta_generic_to_shared(sa), sb_s = (uint32_t)__cvta_generic_to_shared(sb);
@@ -181,16 +191,16 @@ k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat
             cp_async16(sa_s + core_off(r, k0), a + (size_t)(in ? m0 + r : 0) * kTcK + k0, in ? 16u : 0u);
         }
     };
-    for (uint32_t i = t; i < kTcBBytes / 16; i += kTcThreads) cp_async16(sb_s + 16 * i, wimg + 8 * i, 16u);
-    if ((int)blockIdx.x < ntiles) load_a(blockIdx.x);
+    for (uint32_t i = t; i < kB / 16; i += kTcThreads) cp_async16(sb_s + 16 * i, wimg + 8 * i, 16u);
+    if (tile0 < ntiles) load_a(tile0);
     const uint32_t mbar_a = (uint32_t)__cvta_generic_to_shared(mbar);
     if (t == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_a));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {  // the accumulator: 256 columns of tensor memory
+    if (warp == 0) {  // the accumulator: kN columns of tensor memory
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::
-                         "r"((uint32_t)__cvta_generic_to_shared(tmem_slot)), "r"((uint32_t)kTcN));
+                         "r"((uint32_t)__cvta_generic_to_shared(tmem_slot)), "r"((uint32_t)kN));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
@@ -203,10 +213,10 @@ k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat
     // kind::f16: FP32 D (bit 4), BF16 A and B (bits 7, 10), both K-major,
     // N / 8 at bit 17, M / 16 at bit 24
     const uint32_t idesc =
-        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTcN >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
+        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
     uint32_t phase = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    for (int tile = tile0; tile < ntiles; tile += tstep) {
         if (t == 0) {
 #pragma unroll 1
             for (int kk = 0; kk < kTcK / 16; ++kk) {
@@ -237,13 +247,13 @@ k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat
             break;
         }
         // the activations' buffer is free: the next tile's copy runs under the epilogue
-        const int nxt = tile + gridDim.x;
+        const int nxt = tile + tstep;
         if (nxt < ntiles) load_a(nxt);
         // epilogue: warp w reads tensor-memory lanes 32w.. (its rows), 32 columns at a time
         const int r = tile * kTcM + warp * 32 + lane;
         const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
-        for (int c = 0; c < kTcN; c += 32) {
+        for (int c = 0; c < kN; c += 32) {
             uint32_t v[32];
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -262,15 +272,15 @@ k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat
                     __align__(16) __nv_bfloat16 hb[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
-                        f[e] = __uint_as_float(v[q + e]) + __ldg(bias + c + q + e);
+                        f[e] = __uint_as_float(v[q + e]) + __ldg(bias + n0 + c + q + e);
                         hb[e] = __float2bfloat16_rn(fmaxf(f[e], 0.f));
                     }
                     if (pre) {
-                        float4 *po = reinterpret_cast<float4 *>(pre + (size_t)r * kTcN + c + q);
+                        float4 *po = reinterpret_cast<float4 *>(pre + (size_t)r * kTcN + n0 + c + q);
                         po[0] = make_float4(f[0], f[1], f[2], f[3]);
                         po[1] = make_float4(f[4], f[5], f[6], f[7]);
                     }
-                    *reinterpret_cast<uint4 *>(h + (size_t)r * kTcN + c + q) = *reinterpret_cast<const uint4 *>(hb);
+                    *reinterpret_cast<uint4 *>(h + (size_t)r * kTcN + n0 + c + q) = *reinterpret_cast<const uint4 *>(hb);
                 }
             }
         }
@@ -286,7 +296,7 @@ k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTcN));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kN));
     }
 }
 
@@ -556,6 +566,414 @@ __global__ void k_gather_rows(const float *__restrict__ src, const int *__restri
     dst[i] = src[(long long)idx[r] * cols + c];
 }
 
+// ------------------------------------------------------------------ a training batch in five kernels
+//
+// The 8 -> 256 -> 256 -> 4 network's forward and backward pass and its Adam
+// step, for one batch: k_mlp_first (gather, first layer, weight image),
+// k_mlp_hidden_tc, k_mlp_out (output layer, loss, gradient of the hidden
+// layer's outputs), k_mlp_back2 (everything that needs those), k_mlp_back1
+// (first layer's gradients, the update).  Every product is the same sequence
+// of mma.m16n8k16 over ascending K as k_mlp_gemm's, and every column sum the
+// same order as k_mlp_colsum's, so the results are the same bits.
+//
+// Bound by the chain of launches and of loads inside each (a batch is
+// 0.1 GFLOP).  A batch of 256 rows took 17 launches and 174 us, most of it in
+// k_mlp_gemm's 2-byte strided loads on few CTAs; the operands are now staged
+// through shared memory with 16-byte copies and read with ldmatrix.
+constexpr int kFH = 256, kFIn = 8, kFOut = 4, kFThreads = 256;
+
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+        "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <bool kTrans>
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16 *p)
+{
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    if (kTrans)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+
+// rows x cols (cols a multiple of 8) of a row-major matrix of row length ld
+// into shared memory with row length cols + 8; rows past `have` are zero.
+__device__ __forceinline__ void stage_rows(__nv_bfloat16 *dst, const __nv_bfloat16 *src, int ld, int rows, int cols,
+                                           int have)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int per = cols / 8;
+    for (int i = threadIdx.x; i < rows * per; i += kFThreads) {
+        const int r = i / per, c = (i - r * per) * 8;
+        const bool in = r < have;
+        cp_async16(d + 2 * (r * (cols + 8) + c), src + (size_t)(in ? r : 0) * ld + c, in ? 16u : 0u);
+    }
+}
+
+struct AdamArgs {
+    float *m, *v;
+    float lr, b1, b2, c1, c2, eps;
+};
+
+// One parameter's update (null m: the gradient is stored instead).
+__device__ __forceinline__ void adam_or_store(const AdamArgs &ad, float *p, __nv_bfloat16 *p16, float *grad,
+                                              long long i, float gi)
+{
+    if (!ad.m) {
+        grad[i] = gi;
+        return;
+    }
+    const float mi = ad.b1 * ad.m[i] + (1.f - ad.b1) * gi;
+    const float vi = ad.b2 * ad.v[i] + (1.f - ad.b2) * gi * gi;
+    ad.m[i] = mi;
+    ad.v[i] = vi;
+    const float q = p[i] - ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + ad.eps);
+    p[i] = q;
+    p16[i] = __float2bfloat16_rn(q);
+}
+
+// 16 rows a CTA: x[idx] rounded to BF16, and the first layer; further CTAs
+// lay the hidden weights out for the tensor cores.
+__global__ void __launch_bounds__(kFThreads)
+k_mlp_first(const float *__restrict__ x, const int *__restrict__ idx, int rows, const __nv_bfloat16 *__restrict__ w1,
+            const float *__restrict__ b1, const __nv_bfloat16 *__restrict__ w2, __nv_bfloat16 *__restrict__ img,
+            __nv_bfloat16 *__restrict__ x16, float *__restrict__ pre1, __nv_bfloat16 *__restrict__ h1, int row_ctas)
+{
+    if ((int)blockIdx.x >= row_ctas) {  // as k_mlp_tile_w
+        const uint32_t i = (blockIdx.x - row_ctas) * kFThreads + threadIdx.x;
+        const uint32_t n = i % kTcN, k0 = i / kTcN * 8;
+        __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = w2[(size_t)(k0 + e) * kTcN + n];
+        *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(img) + core_off(n, k0)) =
+            *reinterpret_cast<const uint4 *>(v);
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+    const int r0 = blockIdx.x * 16;
+    uint32_t a[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int r = r0 + g + 8 * q;
+        if (r >= rows) continue;
+        const float2 v = *reinterpret_cast<const float2 *>(x + (size_t)(idx ? idx[r] : r) * kFIn + 2 * t4);
+        a[q] = pack2(__float2bfloat16_rn(v.x), __float2bfloat16_rn(v.y));
+        if (warp == 0) *reinterpret_cast<uint32_t *>(x16 + (size_t)r * kFIn + 2 * t4) = a[q];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int nn = warp * 32 + 8 * j, n = nn + g;
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        mma16816(d, a, pack2(w1[2 * t4 * kFH + n], w1[(2 * t4 + 1) * kFH + n]), 0u);
+        const int c = nn + 2 * t4;
+        const float2 bb = *reinterpret_cast<const float2 *>(b1 + c);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = r0 + g + 8 * q;
+            if (r >= rows) continue;
+            const float v0 = d[2 * q] + bb.x, v1 = d[2 * q + 1] + bb.y;
+            *reinterpret_cast<float2 *>(pre1 + (size_t)r * kFH + c) = make_float2(v0, v1);
+            *reinterpret_cast<uint32_t *>(h1 + (size_t)r * kFH + c) =
+                pack2(__float2bfloat16_rn(fmaxf(v0, 0.f)), __float2bfloat16_rn(fmaxf(v1, 0.f)));
+        }
+    }
+}
+
+// 16 rows a CTA: y = h2 W3 + b3 (warp 0), the loss and dy, and
+// d2 = (dy W3^T) * (pre2 > 0) (all warps, 32 columns each).
+__global__ void __launch_bounds__(kFThreads)
+k_mlp_out(const __nv_bfloat16 *__restrict__ h2, const float *__restrict__ pre2, const float *__restrict__ tgt,
+          const int *__restrict__ idx, int rows, const __nv_bfloat16 *__restrict__ w3, const float *__restrict__ b3,
+          float scale, float *__restrict__ dy, __nv_bfloat16 *__restrict__ dy16, float *__restrict__ d2,
+          __nv_bfloat16 *__restrict__ d2_16, double *loss)
+{
+    __shared__ __align__(16) __nv_bfloat16 sh[16 * (kFH + 8)];
+    __shared__ __align__(16) __nv_bfloat16 sw[kFH * kFOut];
+    __shared__ __align__(4) __nv_bfloat16 sdy[16 * kFOut];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+    const int r0 = blockIdx.x * 16;
+    stage_rows(sh, h2 + (size_t)r0 * kFH, kFH, 16, kFH, rows - r0);
+    if (threadIdx.x < kFH * kFOut / 8)
+        cp_async16((uint32_t)__cvta_generic_to_shared(sw) + 16 * threadIdx.x, w3 + 8 * threadIdx.x, 16u);
+    // this thread's pre-activations, in flight meanwhile
+    float2 pm[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = r0 + g + 8 * q;
+            pm[j][q] = r < rows ? *reinterpret_cast<const float2 *>(pre2 + (size_t)r * kFH + warp * 32 + 8 * j + 2 * t4)
+                                : make_float2(0.f, 0.f);
+        }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        const __nv_bfloat16 zero = __ushort_as_bfloat16(0);
+#pragma unroll
+        for (int kk = 0; kk < kFH; kk += 16) {
+            uint32_t a[4];
+            ldsm4<false>(a, sh + (lane & 15) * (kFH + 8) + kk + (lane >> 4) * 8);
+            const int ka = kk + 2 * t4;
+            const bool in = g < kFOut;
+            mma16816(d, a, in ? pack2(sw[ka * kFOut + g], sw[(ka + 1) * kFOut + g]) : pack2(zero, zero),
+                     in ? pack2(sw[(ka + 8) * kFOut + g], sw[(ka + 9) * kFOut + g]) : pack2(zero, zero));
+        }
+        double e2 = 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int rl = g + (q >= 2 ? 8 : 0), r = r0 + rl, c = 2 * t4 + (q & 1);
+            if (c >= kFOut) continue;
+            float gr = 0.f;
+            if (r < rows) {
+                const float e = (d[q] + b3[c]) - tgt[(size_t)(idx ? idx[r] : r) * kFOut + c];
+                e2 += (double)e * e;
+                gr = 2.f * e * scale;
+                dy[(size_t)r * kFOut + c] = gr;
+                dy16[(size_t)r * kFOut + c] = __float2bfloat16_rn(gr);
+            }
+            sdy[rl * kFOut + c] = __float2bfloat16_rn(gr);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) e2 += __shfl_down_sync(0xffffffffu, e2, o);
+        if (lane == 0) atomicAdd(loss, e2 * scale);
+    }
+    __syncthreads();
+    uint32_t a[4] = {0u, 0u, 0u, 0u};
+    if (t4 < 2) {
+        a[0] = *reinterpret_cast<const uint32_t *>(sdy + g * kFOut + 2 * t4);
+        a[1] = *reinterpret_cast<const uint32_t *>(sdy + (g + 8) * kFOut + 2 * t4);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int nn = warp * 32 + 8 * j, c = nn + 2 * t4;
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        mma16816(d, a, t4 < 2 ? *reinterpret_cast<const uint32_t *>(sw + (nn + g) * kFOut + 2 * t4) : 0u, 0u);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = r0 + g + 8 * q;
+            if (r >= rows) continue;
+            const float v0 = pm[j][q].x > 0.f ? d[2 * q] : 0.f, v1 = pm[j][q].y > 0.f ? d[2 * q + 1] : 0.f;
+            *reinterpret_cast<float2 *>(d2 + (size_t)r * kFH + c) = make_float2(v0, v1);
+            *reinterpret_cast<uint32_t *>(d2_16 + (size_t)r * kFH + c) =
+                pack2(__float2bfloat16_rn(v0), __float2bfloat16_rn(v1));
+        }
+    }
+}
+
+// Sums of columns c0 .. c0 + kC - 1 (kC 4 or 8) of d (row length cols), in
+// k_mlp_colsum's order; thread j < kC returns column c0 + j's.
+template <int kC>
+__device__ __forceinline__ float colsums(const float *__restrict__ d, int rows, int cols, int c0, float *part)
+{
+    float s[kC] = {};
+    for (int r = threadIdx.x; r < rows; r += kFThreads) {
+#pragma unroll
+        for (int j = 0; j < kC; j += 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(d + (size_t)r * cols + c0 + j);
+            s[j] += v.x;
+            s[j + 1] += v.y;
+            s[j + 2] += v.z;
+            s[j + 3] += v.w;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kC; ++j) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_down_sync(0xffffffffu, s[j], o);
+        if ((threadIdx.x & 31) == 0) part[(threadIdx.x >> 5) * kC + j] = s[j];
+    }
+    __syncthreads();
+    float t = 0.f;
+    if (threadIdx.x < kC)
+        for (int w = 0; w < kFThreads / 32; ++w) t += part[w * kC + threadIdx.x];
+    return t;
+}
+
+// Everything that needs dy and d2, by ranges of CTAs:
+//   32            dW2 = h1^T d2, 32 x 64 outputs each
+//   8             dW3 = h2^T dy, 32 rows each
+//   4 ceil(rows / 16)  d1 = (d2 W2^T) * (pre1 > 0), 16 x 64 outputs each
+//   32, 1         db2, db3
+constexpr int kBackK = 256;  // rows of a K pass
+constexpr size_t kBackSmem = 2 * (size_t)(kBackK * (32 + 8) + kBackK * (64 + 8));
+static_assert(kBackSmem >= 2 * (size_t)(16 + 64) * (kFH + 8), "d1's operands fit");
+
+__global__ void __launch_bounds__(kFThreads)
+k_mlp_back2(const __nv_bfloat16 *__restrict__ h1, const __nv_bfloat16 *__restrict__ h2,
+            const float *__restrict__ pre1, const float *__restrict__ dy, const __nv_bfloat16 *__restrict__ dy16,
+            const float *__restrict__ d2, const __nv_bfloat16 *__restrict__ d2_16, int rows,
+            const __nv_bfloat16 *__restrict__ w2, float *__restrict__ gw2, float *__restrict__ gb2,
+            float *__restrict__ gw3, float *__restrict__ gb3, float *__restrict__ d1,
+            __nv_bfloat16 *__restrict__ d1_16)
+{
+    extern __shared__ __align__(16) unsigned char back_smem[];
+    __shared__ float part[64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3, mat = lane >> 3;
+    int blk = blockIdx.x;
+    if (blk < 32 + 8) {
+        // A = h^T of 32 columns m0.., staged as K rows of h1 (dW2) or h2 (dW3)
+        const bool w2part = blk < 32;
+        const int m0 = w2part ? (blk >> 2) * 32 : (blk - 32) * 32, n0 = w2part ? (blk & 3) * 64 : 0;
+        constexpr int la = 32 + 8, lb = 64 + 8;
+        __nv_bfloat16 *sa = reinterpret_cast<__nv_bfloat16 *>(back_smem), *sb = sa + kBackK * la;
+        const int mw = (warp & 1) * 16, nw = (warp >> 1) * 16;  // the warp's 16 x 16 outputs
+        float d[2][4] = {};
+        for (int k0 = 0; k0 < rows; k0 += kBackK) {
+            const int have = min(kBackK, rows - k0), kr = (have + 15) & ~15;
+            stage_rows(sa, (w2part ? h1 : h2) + (size_t)k0 * kFH + m0, kFH, kr, 32, have);
+            if (w2part) stage_rows(sb, d2_16 + (size_t)k0 * kFH + n0, kFH, kr, 64, have);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            if (w2part) {
+                for (int kk = 0; kk < kr; kk += 16) {
+                    uint32_t a[4], b[4];
+                    ldsm4<true>(a, sa + (kk + (lane & 7) + (mat >> 1) * 8) * la + mw + (mat & 1) * 8);
+                    ldsm4<true>(b, sb + (kk + (lane & 7) + (mat & 1) * 8) * lb + nw + (mat >> 1) * 8);
+                    mma16816(d[0], a, b[0], b[1]);
+                    mma16816(d[1], a, b[2], b[3]);
+                }
+            } else if (warp < 2) {
+                const __nv_bfloat16 zero = __ushort_as_bfloat16(0);
+                auto el = [&](int k) { return g < kFOut && k < rows ? dy16[(size_t)k * kFOut + g] : zero; };
+                for (int kk = 0; kk < kr; kk += 16) {
+                    uint32_t a[4];
+                    ldsm4<true>(a, sa + (kk + (lane & 7) + (mat >> 1) * 8) * la + mw + (mat & 1) * 8);
+                    const int k = k0 + kk + 2 * t4;
+                    mma16816(d[0], a, pack2(el(k), el(k + 1)), pack2(el(k + 8), el(k + 9)));
+                }
+            }
+            __syncthreads();
+        }
+        if (w2part) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    *reinterpret_cast<float2 *>(gw2 + (size_t)(m0 + mw + g + 8 * q) * kFH + n0 + nw + 8 * j + 2 * t4) =
+                        make_float2(d[j][2 * q], d[j][2 * q + 1]);
+        } else if (warp < 2 && t4 < 2) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                gw3[(size_t)(m0 + mw + g + 8 * q) * kFOut + 2 * t4] = d[0][2 * q];
+                gw3[(size_t)(m0 + mw + g + 8 * q) * kFOut + 2 * t4 + 1] = d[0][2 * q + 1];
+            }
+        }
+        return;
+    }
+    blk -= 32 + 8;
+    const int d1_ctas = 4 * ((rows + 15) / 16);
+    if (blk < d1_ctas) {
+        const int r0 = (blk >> 2) * 16, n0 = (blk & 3) * 64;
+        constexpr int ld = kFH + 8;
+        __nv_bfloat16 *sa = reinterpret_cast<__nv_bfloat16 *>(back_smem), *sb = sa + 16 * ld;
+        stage_rows(sa, d2_16 + (size_t)r0 * kFH, kFH, 16, kFH, rows - r0);
+        stage_rows(sb, w2 + (size_t)n0 * kFH, kFH, 64, kFH, 64);
+        const int c = n0 + warp * 8 + 2 * t4;
+        float2 pm[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = r0 + g + 8 * q;
+            pm[q] = r < rows ? *reinterpret_cast<const float2 *>(pre1 + (size_t)r * kFH + c) : make_float2(0.f, 0.f);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int kk = 0; kk < kFH; kk += 32) {
+            uint32_t a0[4], a1[4], b[4];
+            ldsm4<false>(a0, sa + (lane & 15) * ld + kk + (lane >> 4) * 8);
+            ldsm4<false>(a1, sa + (lane & 15) * ld + kk + 16 + (lane >> 4) * 8);
+            ldsm4<false>(b, sb + (warp * 8 + (lane & 7)) * ld + kk + mat * 8);
+            mma16816(d, a0, b[0], b[1]);
+            mma16816(d, a1, b[2], b[3]);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = r0 + g + 8 * q;
+            if (r >= rows) continue;
+            const float v0 = pm[q].x > 0.f ? d[2 * q] : 0.f, v1 = pm[q].y > 0.f ? d[2 * q + 1] : 0.f;
+            *reinterpret_cast<float2 *>(d1 + (size_t)r * kFH + c) = make_float2(v0, v1);
+            *reinterpret_cast<uint32_t *>(d1_16 + (size_t)r * kFH + c) =
+                pack2(__float2bfloat16_rn(v0), __float2bfloat16_rn(v1));
+        }
+        return;
+    }
+    blk -= d1_ctas;
+    if (blk < 32) {
+        const float v = colsums<8>(d2, rows, kFH, 8 * blk, part);
+        if (threadIdx.x < 8) gb2[8 * blk + threadIdx.x] = v;
+    } else {
+        const float v = colsums<4>(dy, rows, kFOut, 0, part);
+        if (threadIdx.x < kFOut) gb3[threadIdx.x] = v;
+    }
+}
+
+// The first layer's gradients and the update, by ranges of CTAs:
+//   16        dW1 = x^T d1, two warps of 8 columns each
+//   32        db1
+//   the rest  Adam on the other parameters, 4 a thread (training only)
+__global__ void __launch_bounds__(kFThreads)
+k_mlp_back1(const __nv_bfloat16 *__restrict__ x16, const float *__restrict__ d1,
+            const __nv_bfloat16 *__restrict__ d1_16, int rows, float *__restrict__ p, __nv_bfloat16 *__restrict__ p16,
+            float *__restrict__ grad, long long np, AdamArgs ad)
+{
+    __shared__ __align__(16) __nv_bfloat16 sx[kBackK * kFIn], sd[kBackK * 16];
+    __shared__ float part[64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+    int blk = blockIdx.x;
+    constexpr int kW1 = kFIn * kFH;
+    if (blk < 16) {  // columns 16 blk .. 16 blk + 15, two warps
+        const int n0 = 16 * blk;
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k0 = 0; k0 < rows; k0 += kBackK) {
+            const int have = min(kBackK, rows - k0), kr = (have + 15) & ~15;
+            const uint32_t sxa = (uint32_t)__cvta_generic_to_shared(sx), sda = (uint32_t)__cvta_generic_to_shared(sd);
+            for (int i = threadIdx.x; i < kr; i += kFThreads)
+                cp_async16(sxa + 16 * i, x16 + (size_t)(i < have ? k0 + i : 0) * kFIn, i < have ? 16u : 0u);
+            for (int i = threadIdx.x; i < 2 * kr; i += kFThreads)
+                cp_async16(sda + 16 * i, d1_16 + (size_t)((i >> 1) < have ? k0 + (i >> 1) : 0) * kFH + n0 + 8 * (i & 1),
+                           (i >> 1) < have ? 16u : 0u);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            if (warp < 2) {
+                const int n = 8 * warp + g;
+                for (int kk = 0; kk < kr; kk += 16) {
+                    const int k = kk + 2 * t4;
+                    const uint32_t a[4] = {pack2(sx[k * kFIn + g], sx[(k + 1) * kFIn + g]), 0u,
+                                           pack2(sx[(k + 8) * kFIn + g], sx[(k + 9) * kFIn + g]), 0u};
+                    mma16816(d, a, pack2(sd[k * 16 + n], sd[(k + 1) * 16 + n]),
+                             pack2(sd[(k + 8) * 16 + n], sd[(k + 9) * 16 + n]));
+                }
+            }
+            __syncthreads();
+        }
+        if (warp < 2) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                adam_or_store(ad, p, p16, grad, (long long)g * kFH + n0 + 8 * warp + 2 * t4 + q, d[q]);
+        }
+        return;
+    }
+    blk -= 16;
+    if (blk < 32) {
+        const float v = colsums<8>(d1, rows, kFH, 8 * blk, part);
+        if (threadIdx.x < 8) adam_or_store(ad, p, p16, grad, kW1 + 8 * blk + threadIdx.x, v);
+        return;
+    }
+    const long long i = kW1 + kFH + 4 * ((long long)(blk - 32) * kFThreads + threadIdx.x);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (i + q < np) adam_or_store(ad, p, p16, grad, i + q, grad[i + q]);
+}
+
 unsigned nb(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 int fail(int code, const std::string &m) { return boidsgpu::set_last_error(code, m.c_str()); }
@@ -632,6 +1050,42 @@ MatB transposed(const __nv_bfloat16 *p, int rows, int cols)  // the transpose of
     return MatB{p, 1, rows == 0 ? 0 : cols, cols, rows};
 }
 
+// The hidden product of `rows` rows in m->h1: a few tiles are split by columns
+// so that more SMs take part (up to a quarter of them have a tile).
+void hidden_tc(boids_mlp *m, int rows, const float *b2, float *pre2)
+{
+    const unsigned tiles = nb(rows, kTcM), parts = kTcN / kTcSplit;
+    if (tiles * parts <= m->nsm)
+        k_mlp_hidden_tc<kTcSplit><<<tiles * parts, kTcThreads, kTcSplitSmem, m->st>>>(m->h1, rows, m->w2img, b2, pre2,
+                                                                                      m->h2);
+    else
+        k_mlp_hidden_tc<kTcN><<<tiles < m->nsm ? tiles : m->nsm, kTcThreads, kTcSmem, m->st>>>(m->h1, rows, m->w2img,
+                                                                                               b2, pre2, m->h2);
+}
+
+// One batch of the 8 -> 256 -> 256 -> 4 network in five kernels: rows idx[0..
+// rows) (null: 0, 1, ...) of x and t.  ad.m null: the gradient into m->grad;
+// else the Adam step.
+bool batch_is_fused(const boids_mlp *m) { return m->w2img && m->in == kFIn && m->out == kFOut; }
+
+void fused_batch(boids_mlp *m, const float *x, const float *t, const int *idx, int rows, const AdamArgs &ad)
+{
+    const __nv_bfloat16 *W1 = m->p16 + m->off[0], *W2 = m->p16 + m->off[2], *W3 = m->p16 + m->off[4];
+    const float *b1 = m->p + m->off[1], *b2 = m->p + m->off[3], *b3 = m->p + m->off[5];
+    const unsigned row_ctas = nb(rows, 16);
+    k_mlp_first<<<row_ctas + kTcN * kTcK / 8 / kFThreads, kFThreads, 0, m->st>>>(
+        x, idx, rows, W1, b1, W2, m->w2img, m->x16, m->pre1, m->h1, (int)row_ctas);
+    hidden_tc(m, rows, b2, m->pre2);
+    k_mlp_out<<<row_ctas, kFThreads, 0, m->st>>>(m->h2, m->pre2, t, idx, rows, W3, b3, 1.f / (float)(rows * kFOut),
+                                                m->dy, m->dy16, m->d2, m->d2_16, m->loss);
+    k_mlp_back2<<<32 + 8 + 4 * row_ctas + 32 + 1, kFThreads, kBackSmem, m->st>>>(
+        m->h1, m->h2, m->pre1, m->dy, m->dy16, m->d2, m->d2_16, rows, W2, m->grad + m->off[2], m->grad + m->off[3],
+        m->grad + m->off[4], m->grad + m->off[5], m->d1, m->d1_16);
+    const unsigned rest = ad.m ? nb(m->np - kFIn * kFH - kFH, 4 * kFThreads) : 0;
+    k_mlp_back1<<<16 + 32 + rest, kFThreads, 0, m->st>>>(m->x16, m->d1, m->d1_16, rows, m->p, m->p16, m->grad, m->np,
+                                                         ad);
+}
+
 // Forward pass of `rows` rows already in m->x16; output in m->y.  A hidden
 // width of 256 puts the hidden-to-hidden product on the tensor cores.
 void forward(boids_mlp *m, int rows, bool need_pre = true)
@@ -641,9 +1095,7 @@ void forward(boids_mlp *m, int rows, bool need_pre = true)
     gemm(m, rowmajor(m->x16, rows, m->in), rowmajor(W1, m->in, m->h), m->pre1, m->h, m->h1, m->h, b1, nullptr, 0, 1);
     if (m->w2img) {
         k_mlp_tile_w<<<nb(kTcN * kTcK / 8, 256), 256, 0, m->st>>>(W2, m->w2img);
-        const unsigned tiles = nb(rows, kTcM);
-        k_mlp_hidden_tc<<<tiles < m->nsm ? tiles : m->nsm, kTcThreads, kTcSmem, m->st>>>(
-            m->h1, rows, m->w2img, b2, need_pre ? m->pre2 : nullptr, m->h2);
+        hidden_tc(m, rows, b2, need_pre ? m->pre2 : nullptr);
     } else {
         gemm(m, rowmajor(m->h1, rows, m->h), rowmajor(W2, m->h, m->h), m->pre2, m->h, m->h2, m->h, b2, nullptr, 0,
              1);
@@ -754,7 +1206,11 @@ int boids_mlp_create(int32_t n_in, int32_t n_hidden, int32_t n_out, uint64_t see
         m->nsm = (unsigned)nsm;
     if (ok && n_hidden == kTcN) {  // the hidden product on the tensor cores
         ok = cudaMalloc(&m->w2img, kTcBBytes) == cudaSuccess &&
-             cudaFuncSetAttribute(k_mlp_hidden_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem) ==
+             cudaFuncSetAttribute(k_mlp_hidden_tc<kTcN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem) ==
+                 cudaSuccess &&
+             cudaFuncSetAttribute(k_mlp_hidden_tc<kTcSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kTcSplitSmem) == cudaSuccess &&
+             cudaFuncSetAttribute(k_mlp_back2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBackSmem) ==
                  cudaSuccess &&
              cudaFuncSetAttribute(k_mlp_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kTcFwdSmem) == cudaSuccess;
@@ -835,10 +1291,16 @@ int boids_mlp_gradient(boids_mlp *m, const float *x, const float *t, int32_t row
     if (!m || !x || !t || !grad || rows <= 0) return fail(BOIDS_EINVAL, "boids_mlp_gradient: bad argument");
     cudaSetDevice(m->device);
     if (int rc = ensure_rows(m, rows)) return rc;
-    if (int rc = upload_rows(m, x, t, rows)) return rc;
     MCK(cudaMemsetAsync(m->loss, 0, 8, m->st));
-    forward(m, rows);
-    backward(m, rows);
+    if (batch_is_fused(m)) {
+        MCK(cudaMemcpyAsync(m->x, x, sizeof(float) * (size_t)rows * m->in, cudaMemcpyHostToDevice, m->st));
+        MCK(cudaMemcpyAsync(m->t, t, sizeof(float) * (size_t)rows * m->out, cudaMemcpyHostToDevice, m->st));
+        fused_batch(m, m->x, m->t, nullptr, rows, AdamArgs{});
+    } else {
+        if (int rc = upload_rows(m, x, t, rows)) return rc;
+        forward(m, rows);
+        backward(m, rows);
+    }
     MCK(cudaGetLastError());
     MCK(cudaMemcpyAsync(grad, m->grad, 4 * m->np, cudaMemcpyDeviceToHost, m->st));
     double l = 0;
@@ -877,6 +1339,7 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
     double epoch_loss = 0.0;
     int rc = 0;
     float *keep_x = m->x, *keep_t = m->t;
+    const bool fused = batch_is_fused(m);
     for (int ep = 0; ep < epochs && !rc; ++ep) {
         for (int i = rows - 1; i > 0; --i) {  // Fisher-Yates
             s += 0x9e3779b97f4a7c15ULL;
@@ -895,6 +1358,12 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
         int nbatch = 0;
         for (int b0 = 0; b0 < rows; b0 += batch, ++nbatch) {
             const int r = std::min(batch, rows - b0);
+            ++m->step;
+            const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
+            if (fused) {
+                fused_batch(m, X, T, d_idx + b0, r, AdamArgs{m->m, m->v, lr, b1, b2, c1, c2, eps});
+                continue;
+            }
             k_gather_rows<<<nb((long long)r * m->in, 256), 256, 0, m->st>>>(keep_x, d_idx + b0, r, m->in, bx);
             k_gather_rows<<<nb((long long)r * m->out, 256), 256, 0, m->st>>>(keep_t, d_idx + b0, r, m->out, bt);
             // the forward/backward buffers read x/t from m->x/m->t: point them at the batch
@@ -905,11 +1374,10 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
             backward(m, r);
             m->x = keep_x;
             m->t = keep_t;
-            ++m->step;
-            const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
             k_mlp_adam<<<nb(m->np, 256), 256, 0, m->st>>>(m->p, m->grad, m->m, m->v, m->p16, m->np, lr, b1, b2, c1,
                                                          c2, eps);
         }
+        if (ep + 1 < epochs) continue;  // the next epoch's indices follow on the stream
         double l = 0;
         if (cudaMemcpyAsync(&l, m->loss, 8, cudaMemcpyDeviceToHost, m->st) != cudaSuccess ||
             cudaStreamSynchronize(m->st) != cudaSuccess) {
