@@ -182,6 +182,10 @@ inline size_t dense_list_capacity(size_t ncell, size_t n)
 // 49 152 uniform 75 / 71, gathered 124 / 251; 65 537 uniform 95 / 73.  The
 // line lies where a uniform flock takes the same time with both.
 constexpr uint32_t kWarpBoids = 40960;
+// Up to this many boids and cells (padded) the allocation-free step's counting
+// sort is one kernel (k_grid_bin): on the eight SMs of its cluster the scatter
+// of more takes longer than the launches it saves.
+constexpr uint32_t kBinBoids = 16384, kBinCells = 65536;
 constexpr int kDenseCap = 512;        // candidates of a dense cell held in shared memory
 constexpr int kDenseCtasPerSm = 8;   // resident CTAs of the dense-cell kernel per SM (its launch bounds)
 constexpr int kApCap = 256;           // all-pairs engine: neighbours kept per boid (more: an O(N) scan)
@@ -224,10 +228,16 @@ cudaError_t launch_grid_classify(const StepConst &k, const DevBuffers &b, cudaSt
 cudaError_t launch_grid_scatter(const StepConst &k, const DevBuffers &b, int from, bool zero_counts,
                                 cudaStream_t s, uint64_t *launches, const FlockTable *ft = nullptr);
 // Rules + integration over the sorted state b.pos[from]; writes the new state
-// to b.pos[1-from] (diag == false) or neighbour-set fingerprints (diag == true).
+// to b.pos[1-from], or with pos3/vel3 in id order to those (diag == false), or
+// neighbour-set fingerprints (diag == true).
 cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from, bool diag,
                               bool record_forces, cudaStream_t s, uint64_t *launches,
-                              const FlockTable *ft = nullptr);
+                              const FlockTable *ft = nullptr, float *pos3 = nullptr, float *vel3 = nullptr);
+// Whether a flock's counting sort from an id-ordered state is one kernel, and
+// that kernel: pos3/vel3 sorted into b.pos[1], b.vel[1].
+bool grid_bin_small(const StepConst &k, const DevBuffers &b);
+cudaError_t launch_grid_bin(const StepConst &k, const DevBuffers &b, const float *pos3, const float *vel3,
+                            cudaStream_t s, uint64_t *launches);
 cudaError_t launch_allpairs(const StepConst &k, const DevBuffers &b, int from, bool diag,
                             bool record_forces, cudaStream_t s, uint64_t *launches);
 cudaError_t launch_ref_cells(const StepConst &k, const float4 *pos, int32_t *cells8, cudaStream_t s,

@@ -291,6 +291,7 @@ __device__ __forceinline__ void load_flock(StepConst &dst, const FlockTable &ft,
 // Where a rule kernel writes one boid's result.
 struct GridOut {
     float4 *pos_out, *vel_out;
+    float *pos3_out, *vel3_out;  // the caller's id-ordered arrays instead (null: the records above)
     uint32_t *key_out, *rank_out, *count;  // null for the all-pairs engine
     float *forces;
     int32_t *dcnt;
@@ -320,8 +321,14 @@ __device__ __forceinline__ void finish_boid(const Acc &a, float4 p4, float3 vi, 
     acc_finish(a, pi, vi, k, fc, fs, fa);
     float3 x = pi, v = vi;
     integrate(x, v, fc, fs, fa, k);
-    o.pos_out[s] = make_float4(x.x, x.y, x.z, p4.w);
-    o.vel_out[s] = make_float4(v.x, v.y, v.z, 0.f);
+    if (o.pos3_out) {
+        float *po = o.pos3_out + (size_t)3 * id, *vo = o.vel3_out + (size_t)3 * id;
+        po[0] = x.x; po[1] = x.y; po[2] = x.z;
+        vo[0] = v.x; vo[1] = v.y; vo[2] = v.z;
+    } else {
+        o.pos_out[s] = make_float4(x.x, x.y, x.z, p4.w);
+        o.vel_out[s] = make_float4(v.x, v.y, v.z, 0.f);
+    }
     if (o.key_out) {  // binning for the next step
         const uint32_t c = k.cell_base + cell_key(x, k);
         o.key_out[s] = c;
@@ -532,6 +539,75 @@ __global__ void k_grid_scatter(const float4 *__restrict__ pin, const float4 *__r
     vout[d] = vin[s];
     if (slot_of) slot_of[first + __float_as_uint(p.w)] = d;
     if (count_to_zero) count_to_zero[c] = 0;  // every binned cell, for the next step's keys
+}
+
+// The allocation-free step's counting sort of a small flock in one kernel,
+// from the caller's id-ordered arrays: a cluster of kBinCtas CTAs clears the
+// counts, keys and counts the boids, scans the counts (a contiguous part each,
+// the parts' totals exchanged through distributed shared memory) and scatters
+// the boids.  The cell starts in lstart are final (bsum is zero).
+//
+// Bound by the chain of its phases (about 10 us), which replaces a clear and
+// three kernels: the step of 1000 boids of test.ini takes 33 us where it took
+// 47 with those and an unpacking after the rules, of 16 384 gathered boids 62
+// (75).  It pays only from unsorted input: without the first phases it takes
+// as long as k_grid_scan and k_grid_scatter (a handle's step of 1000 boids
+// 29.3 against 28.0 us, of 16 384 57 against 55).
+constexpr int kBinCtas = 8, kBinThreads = 1024;
+
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(kBinCtas, 1, 1) __launch_bounds__(kBinThreads)
+k_grid_bin(const float *__restrict__ pos3, const float *__restrict__ vel3, uint32_t *key, uint32_t *rank,
+           uint32_t *count, uint32_t *lstart, uint32_t *__restrict__ bsum, uint32_t ncell_pad, uint32_t tiles,
+           float4 *__restrict__ pout, float4 *__restrict__ vout, uint32_t *slot_of, StepConst k)
+{
+    __shared__ uint32_t warp_tot[kBinThreads / 32], totals[kBinCtas];
+    const uint32_t cta = blockIdx.x, t = threadIdx.x, at = cta * kBinThreads + t;
+    constexpr uint32_t kAll = kBinCtas * kBinThreads;
+    for (uint32_t c = 4 * at; c < ncell_pad; c += 4 * kAll)
+        *reinterpret_cast<uint4 *>(count + c) = make_uint4(0, 0, 0, 0);
+    cluster_sync();
+    for (uint32_t i = at; i < k.n; i += kAll) {
+        const uint32_t c = cell_key(make_float3(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2]), k);
+        key[i] = c;
+        rank[i] = atomicAdd(count + c, 1u);
+    }
+    cluster_sync();
+    // this thread's cells, in groups of four: a contiguous part of the CTA's
+    const uint32_t groups = ncell_pad / 4, per = (groups + kAll - 1) / kAll;
+    const uint32_t g0 = min(groups, at * per), g1 = min(groups, g0 + per);
+    uint32_t sum = 0;
+    for (uint32_t g = g0; g < g1; ++g) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(count) + g);
+        sum += v.x + v.y + v.z + v.w;
+    }
+    uint32_t total;
+    uint32_t run = block_excl_scan<kBinThreads>(sum, warp_tot, total);
+    if (t < kBinCtas) {  // the CTA's total to every CTA of the cluster
+        const uint32_t mine = (uint32_t)__cvta_generic_to_shared(totals + cta);
+        uint32_t there;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(mine), "r"(t));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(there), "r"(total) : "memory");
+    }
+    for (uint32_t b = at; b < tiles; b += kAll) bsum[b] = 0;
+    cluster_sync();
+    for (uint32_t c = 0; c < cta; ++c) run += totals[c];
+    for (uint32_t g = g0; g < g1; ++g) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(count) + g);
+        reinterpret_cast<uint4 *>(lstart)[g] = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+        run += v.x + v.y + v.z + v.w;
+    }
+    cluster_sync();  // (the counts are dead: slot_of may take their place)
+    for (uint32_t i = at; i < k.n; i += kAll) {
+        const uint32_t d = __ldcg(lstart + __ldcg(key + i)) + __ldcg(rank + i);
+        pout[d] = make_float4(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2], __uint_as_float(i));
+        vout[d] = make_float4(vel3[3 * i], vel3[3 * i + 1], vel3[3 * i + 2], 0.f);
+        slot_of[i] = d;
+    }
 }
 
 // ------------------------------------------------------------------ neighbourhood segments
@@ -1376,7 +1452,12 @@ __device__ __forceinline__ void warp_finish(WarpSums &a, float4 p4, float3 vi, u
     else if (n > 0.0f && n < k.vmin_up) v = __fmul_rn(__fdiv_rn(v, n), k.vmin_f);
     const float x = lane < 3 ? wrap1(__fadd_rn(pc, v), k) : p4.w;
     const float x0 = __shfl_sync(kAll, x, 0), x1 = __shfl_sync(kAll, x, 1), x2 = __shfl_sync(kAll, x, 2);
-    if (lane < 4) {
+    if (o.pos3_out) {
+        if (lane < 3) {
+            o.pos3_out[(size_t)3 * out + lane] = x;
+            o.vel3_out[(size_t)3 * out + lane] = v;
+        }
+    } else if (lane < 4) {
         reinterpret_cast<float *>(o.pos_out + s)[lane] = x;
         reinterpret_cast<float *>(o.vel_out + s)[lane] = lane < 3 ? v : 0.f;
     }
@@ -2607,6 +2688,20 @@ cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream
     return cudaGetLastError();
 }
 
+bool grid_bin_small(const StepConst &k, const DevBuffers &b)
+{
+    return grid_by_warp(k, b, nullptr) && k.n > 0 && k.n <= kBinBoids && b.ncell_pad <= kBinCells;
+}
+
+cudaError_t launch_grid_bin(const StepConst &k, const DevBuffers &b, const float *pos3, const float *vel3,
+                            cudaStream_t st, uint64_t *launches)
+{
+    k_grid_bin<<<kBinCtas, kBinThreads, 0, st>>>(pos3, vel3, b.key, b.rank, b.count, b.lstart, b.bsum, b.ncell_pad,
+                                                 b.nscan_blocks, b.pos[1], b.vel[1], b.slot_of, k);
+    *launches += 1;
+    return cudaGetLastError();
+}
+
 cudaError_t launch_grid_classify(const StepConst &k, const DevBuffers &b, cudaStream_t st, uint64_t *launches,
                                  const FlockTable *ft)
 {
@@ -2703,7 +2798,7 @@ cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, co
 }  // namespace
 
 cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from, bool diag, bool record_forces,
-                              cudaStream_t st, uint64_t *launches, const FlockTable *ft)
+                              cudaStream_t st, uint64_t *launches, const FlockTable *ft, float *pos3, float *vel3)
 {
     const uint32_t n = ft ? ft->nslots : k.n;
     if (n == 0) return cudaSuccess;
@@ -2726,6 +2821,8 @@ cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from,
     } else {
         o.pos_out = b.pos[1 - from];
         o.vel_out = b.vel[1 - from];
+        o.pos3_out = pos3;
+        o.vel3_out = vel3;
         o.key_out = b.key;
         o.rank_out = b.rank;
         o.count = b.count;

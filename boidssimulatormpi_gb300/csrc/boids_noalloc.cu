@@ -159,10 +159,10 @@ size_t layout(const boidsgpu::StepConst &k, unsigned char *base, boidsgpu::DevBu
     b->key = reinterpret_cast<uint32_t *>(keys);
     b->rank = keys ? b->key + n : nullptr;
     b->dense_list = b->key;
-    b->count = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad));
+    b->count = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad + 4));  // and the scan's ticket behind them
+    b->ticket = b->count ? b->count + b->ncell_pad : nullptr;
     b->lstart = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad));
     b->bsum = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->nscan_blocks));
-    b->ticket = reinterpret_cast<uint32_t *>(take(4));
     b->dense_n = reinterpret_cast<uint32_t *>(take(12));
     b->dflag = take(b->ncell / 4);
     // the counts are dead after the scan: the id -> slot table of a small
@@ -211,21 +211,22 @@ extern "C" int boids_step_noalloc(const boids_params *params, const float *pos3n
     uint64_t launches = 0;
     boidsgpu::DevBuffers rules = b;  // the rule kernels bin nothing for a next step
     rules.key = rules.rank = nullptr;
-    // the array keeps the previous call's contents: clear what must start at zero
-    if ((e = cudaMemsetAsync(b.count, 0, 4 * (size_t)b.ncell_pad, st)) == cudaSuccess &&
-        (e = cudaMemsetAsync(b.ticket, 0, 4, st)) == cudaSuccess &&
-        (e = boidsgpu::launch_pack(pos3n_in, vel3n_in, b.pos[0], b.vel[0], 0, n, nullptr, 0.f, &k, b.key, b.rank,
-                                   b.count, st, &launches)) == cudaSuccess &&
-        (e = boidsgpu::launch_grid_scan(k, b, st, &launches)) == cudaSuccess &&
-        (e = boidsgpu::launch_grid_scatter(k, b, 0, false, st, &launches)) == cudaSuccess &&
-        (e = boidsgpu::launch_grid_classify(k, b, st, &launches)) == cudaSuccess &&
-        (e = boidsgpu::launch_grid_force(k, rules, 1, false, false, st, &launches)) == cudaSuccess &&
-        // the sorted copy in b.pos[1] is dead once the rules have run: it
-        // holds the id -> slot table of the unpacking
-        (e = boidsgpu::launch_unpack(b.pos[0], b.vel[0], reinterpret_cast<uint32_t *>(b.pos[1]), pos3n_out,
-                                     vel3n_out, n, st, &launches)) == cudaSuccess) {
-        return BOIDS_OK;
+    // the rules write the caller's arrays in id order
+    if (boidsgpu::grid_bin_small(k, b)) {
+        e = boidsgpu::launch_grid_bin(k, b, pos3n_in, vel3n_in, st, &launches);
+    } else {
+        // the array keeps the previous call's contents: clear the counts and the ticket
+        if ((e = cudaMemsetAsync(b.count, 0, 4 * (size_t)b.ncell_pad + 4, st)) == cudaSuccess &&
+            (e = boidsgpu::launch_pack(pos3n_in, vel3n_in, b.pos[0], b.vel[0], 0, n, nullptr, 0.f, &k, b.key, b.rank,
+                                       b.count, st, &launches)) == cudaSuccess &&
+            (e = boidsgpu::launch_grid_scan(k, b, st, &launches)) == cudaSuccess &&
+            (e = boidsgpu::launch_grid_scatter(k, b, 0, false, st, &launches)) == cudaSuccess)
+            e = boidsgpu::launch_grid_classify(k, b, st, &launches);
     }
+    if (e == cudaSuccess &&
+        (e = boidsgpu::launch_grid_force(k, rules, 1, false, false, st, &launches, nullptr, pos3n_out, vel3n_out)) ==
+            cudaSuccess)
+        return BOIDS_OK;
     char msg[160];
     std::snprintf(msg, sizeof msg, "boids_step_noalloc: %s", cudaGetErrorString(e));
     return boidsgpu::set_last_error(BOIDS_ECUDA, msg);

@@ -112,3 +112,30 @@ def test_all_pairs_at_tile_edges(boids_lib, oracle_mod, n, field):
     assert_bits_equal(gv, ov, "velocities")
     assert_bits_equal(sim.forces(), of, "forces")
     sim.close()
+
+
+@pytest.mark.parametrize("n,field", [(1, 0.7), (1023, 0.7), (8191, 0.7), (8193, 0.7), (16384, 0.7), (16385, 0.7),
+                                     (3000, 1.33), (3000, 1.4), (40960, 0.7), (40961, 0.7)])
+def test_allocation_free_step_at_its_kernels_limits(boids_lib, oracle_mod, n, field):
+    """The allocation-free step on both sides of the lines between its
+    one-kernel sort (16384 boids, 65536 cells), the warp-per-boid rules (40960
+    boids) and the general path, twice in a row on the same scratch."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    B, O, prm = boids_lib, oracle_mod, oracle_mod.MARUN2019
+    p = make_params(O, n, field, prm)
+    op, ov = O.init_state(p, "random_uniform", True, 7)
+    op, ov = op.reshape(-1).copy(), ov.reshape(-1).copy()
+    prms = B.flock_params(n, field, prm["sep"], prm["ali"], prm["coh"], prm["vmax"], prm["vmin"])
+    a = [torch.from_numpy(x.copy()).cuda() for x in (op, ov)]
+    b = [torch.empty_like(x) for x in a]
+    port = O.GridPort(p, op)
+    for call in range(2):
+        rc = B.lib().boids_step_noalloc(C.byref(prms), a[0].data_ptr(), a[1].data_ptr(), b[0].data_ptr(),
+                                        b[1].data_ptr(), None)
+        assert rc == 0, B.lib().boids_last_error().decode()
+        torch.cuda.synchronize()
+        port.step(op, ov, 1)
+        assert_bits_equal(b[0].cpu().numpy(), op, "positions, call %d" % call)
+        assert_bits_equal(b[1].cpu().numpy(), ov, "velocities, call %d" % call)
+        a, b = b, a
