@@ -425,6 +425,15 @@ __global__ void k_frame(const float4 *__restrict__ pos4, const float4 *__restric
 
 // ------------------------------------------------------------------ counting-sort binning
 
+// Programmatic dependent launch, in the chains of a small flock's steps: the
+// next kernel's CTAs are set up while this one's last ones run, and wait here
+// for its end (and its writes) before they touch anything.  A kernel launched
+// without the attribute passes straight through.
+__device__ __forceinline__ void chain_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
+}
+
 template <bool MULTI>
 __global__ void k_grid_keys(const float4 *__restrict__ pos, uint32_t *__restrict__ key,
                             uint32_t *__restrict__ rank, uint32_t *__restrict__ count, StepConst kp, FlockTable ft)
@@ -479,6 +488,7 @@ k_grid_scan(const uint32_t *__restrict__ count, uint32_t *__restrict__ lstart, u
 {
     __shared__ uint32_t warp_tot[kScanThreads / 32];
     __shared__ bool is_last;
+    chain_wait();
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     const uint4 a = *reinterpret_cast<const uint4 *>(count + base);
     const uint4 b = *reinterpret_cast<const uint4 *>(count + base + 4);
@@ -521,6 +531,7 @@ __global__ void k_grid_scatter(const float4 *__restrict__ pin, const float4 *__r
                                uint32_t *__restrict__ count_to_zero, uint32_t *__restrict__ slot_of, uint32_t n,
                                FlockTable ft)
 {
+    chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t off = 0, first = 0;  // the flock's padding and first slot
     if (MULTI) {
@@ -1477,6 +1488,7 @@ k_grid_warp(GridIn g, GridOut o, StepConst kp, FlockTable ft)
     __shared__ WarpSmem sms[kWarpWarps];
     __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
     StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
+    chain_wait();
     if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * kWarpWarps / kSlotAlign]);
     const StepConst &k = MULTI ? kf : kp;
     const uint32_t s = blockIdx.x * kWarpWarps + (threadIdx.x >> 5);
@@ -2608,6 +2620,24 @@ __global__ void k_ref_cells(const float4 *__restrict__ pos, int32_t *__restrict_
 
 static inline unsigned blocks_for(uint32_t n, unsigned t) { return (n + t - 1) / t; }
 
+// Launches a kernel that begins with chain_wait, with programmatic dependence
+// on the kernel before it when chain is set.
+template <class... P, class... A>
+static cudaError_t launch_chain(bool chain, void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st,
+                                A... args)
+{
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.stream = st;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = chain ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Whether every boid goes to k_grid_warp: flocks (or ensembles) of at most
 // kWarpBoids slots, unless the cells' split was set by hand.
 static inline bool grid_by_warp(const StepConst &k, const DevBuffers &b, const FlockTable *ft)
@@ -2683,9 +2713,9 @@ cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream
         return e;  // items, work queue, deferred
     if (by_cells && ft && b.defer_cnt && (e = cudaMemsetAsync(b.defer_cnt, 0, sizeof(uint32_t) * ft->count, st)) != cudaSuccess)
         return e;  // an ensemble's per-flock deferred counts
-    k_grid_scan<<<b.nscan_blocks, kScanThreads, 0, st>>>(b.count, b.lstart, b.bsum, b.ticket, b.nscan_blocks);
     *launches += 1;
-    return cudaGetLastError();
+    return launch_chain(!by_cells, k_grid_scan, b.nscan_blocks, kScanThreads, st, b.count, b.lstart, b.bsum, b.ticket,
+                        b.nscan_blocks);
 }
 
 bool grid_bin_small(const StepConst &k, const DevBuffers &b)
@@ -2736,15 +2766,10 @@ cudaError_t launch_grid_scatter(const StepConst &k, const DevBuffers &b, int fro
     if (n == 0) return cudaSuccess;
     uint32_t *cz = zero_counts ? b.count : nullptr;
     uint32_t *so = grid_by_warp(k, b, ft) ? b.slot_of : nullptr;
-    if (ft)
-        k_grid_scatter<true><<<blocks_for(n, 256), 256, 0, st>>>(b.pos[from], b.vel[from], b.key, b.rank, b.lstart,
-                                                                 b.bsum, b.pos[1 - from], b.vel[1 - from], cz, so, n, *ft);
-    else
-        k_grid_scatter<false><<<blocks_for(n, 256), 256, 0, st>>>(b.pos[from], b.vel[from], b.key, b.rank, b.lstart,
-                                                                  b.bsum, b.pos[1 - from], b.vel[1 - from], cz, so, n,
-                                                                  FlockTable{});
     ++*launches;
-    return cudaGetLastError();
+    return launch_chain(grid_by_warp(k, b, ft), ft ? k_grid_scatter<true> : k_grid_scatter<false>, blocks_for(n, 256),
+                        256, st, b.pos[from], b.vel[from], b.key, b.rank, b.lstart, b.bsum, b.pos[1 - from],
+                        b.vel[1 - from], cz, so, n, ft ? *ft : FlockTable{});
 }
 
 namespace {
@@ -2771,9 +2796,8 @@ cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, co
                        const FlockTable &ft, cudaStream_t st)
 {
     if (grid_by_warp(k, b, MULTI ? &ft : nullptr)) {
-        k_grid_warp<DIAG, MULTI><<<blocks_for(MULTI ? ft.nslots : k.n, kWarpWarps), kWarpWarps * 32, 0, st>>>(g, o, k,
-                                                                                                          ft);
-        return cudaGetLastError();
+        return launch_chain(true, k_grid_warp<DIAG, MULTI>, blocks_for(MULTI ? ft.nslots : k.n, kWarpWarps),
+                            kWarpWarps * 32, st, g, o, k, ft);
     }
     cudaError_t e = dense_smem_opt_in<DIAG, MULTI>();
     if (e != cudaSuccess) return e;
