@@ -307,15 +307,17 @@ k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat
 // cores run the hidden product into one of two accumulators in tensor
 // memory, and the epilogue applies bias and ReLU and folds the 256 -> 4
 // output layer in registers while the next tile's product runs in the other
-// accumulator.  Eight warps: warps w and w + 4 read the same accumulator
-// lanes, the first the columns 0..127, the second 128..255, and their partial
-// outputs meet in shared memory.  The rounding points are those of the
-// unfused pass (BF16 x, h1, h2; FP32 sums).
+// accumulator.  Sixteen warps: warps w, w + 4, w + 8 and w + 12 read the same
+// accumulator lanes, 64 columns each, and their partial outputs meet in shared
+// memory.  The rounding points are those of the unfused pass (BF16 x, h1, h2;
+// FP32 sums).  Bound by the FP32 work around the product (the first layer's
+// 8 FMA and the epilogue's 4 per activation) and its latencies.
 constexpr int kTcIn = 8, kTcOut = 4;
-constexpr int kTcFwdThreads = 256;
+constexpr int kTcFwdThreads = 512, kTcFwdParts = kTcFwdThreads / 128;  // warps w, w + 4, ...: a part of the columns each
 constexpr uint32_t kTcXBytes = kTcM * kTcIn * 4;  // a tile's inputs, 4 KB
 constexpr size_t kTcFwdSmem = kTcABytes + kTcBBytes + 1024 + 64 +
-                              sizeof(float) * (kTcN * kTcOut + kTcN + kTcOut + 2 * kTcM * kTcOut) + kTcXBytes;
+                              sizeof(float) * (kTcN * kTcOut + kTcN + kTcOut + kTcFwdParts * kTcM * kTcOut) + kTcXBytes;
+static_assert(kTcFwdSmem <= 227 * 1024, "one CTA per SM");
 
 __global__ void __launch_bounds__(kTcFwdThreads, 1)
 k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__restrict__ w1,
@@ -328,14 +330,15 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tc_smem + kTcABytes + kTcBBytes + 8);
     float *sw3 = reinterpret_cast<float *>(tc_smem + kTcABytes + kTcBBytes + 64);  // W3 as float, [k][j]
     float *sb2 = sw3 + kTcN * kTcOut, *sb3 = sb2 + kTcN;
-    float *ypart = sb3 + kTcOut;              // [2][kTcM][kTcOut]: the two column halves' outputs
-    float *sx = ypart + 2 * kTcM * kTcOut;    // the current tile's inputs, [kTcM][kTcIn]
+    float *ypart = sb3 + kTcOut;                        // [kTcFwdParts][kTcM][kTcOut]: the column parts' outputs
+    float *sx = ypart + kTcFwdParts * kTcM * kTcOut;    // the current tile's inputs, [kTcM][kTcIn]
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int ntiles = (rows + kTcM - 1) / kTcM;
     const uint32_t sa_s = (uint32_t)__cvta_generic_to_shared(sa), sb_s = (uint32_t)__cvta_generic_to_shared(sb);
     const uint32_t sx_s = (uint32_t)__cvta_generic_to_shared(sx);
     auto load_x = [&](int tile) {  // one 16-byte chunk per thread
-        static_assert(kTcXBytes / 16 == kTcFwdThreads, "a tile's inputs are one chunk per thread");
+        static_assert(kTcXBytes / 16 <= kTcFwdThreads, "a tile's inputs are at most one chunk per thread");
+        if (t >= (int)(kTcXBytes / 16)) return;
         const int m0 = tile * kTcM, r = t / 2;
         const bool in = m0 + r < rows;
         cp_async16(sx_s + 16 * t, x + (size_t)(in ? m0 + r : 0) * kTcIn + 4 * (t & 1), in ? 16u : 0u);
@@ -413,7 +416,8 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
     };
     uint32_t phase = 0, buf = 0;
     if (t == 0 && (int)blockIdx.x < ntiles) issue(0);
-    const int quarter = warp & 3, half = warp >> 2;  // accumulator lanes 32 * quarter.., columns 128 * half..
+    constexpr int kPart = kTcN / kTcFwdParts;  // columns of a warp
+    const int quarter = warp & 3, half = warp >> 2;  // accumulator lanes 32 * quarter.., columns kPart * half..
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int nxt = tile + gridDim.x;
         if (nxt < ntiles) load_x(nxt);  // sx is free: this tile's first layer is done
@@ -449,7 +453,7 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
         const uint32_t trow = tmem + buf * kTcN + ((uint32_t)(quarter * 32) << 16);
         float yo[kTcOut] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-        for (int c = half * (kTcN / 2); c < (half + 1) * (kTcN / 2); c += 32) {
+        for (int c = half * kPart; c < (half + 1) * kPart; c += 32) {
             uint32_t v[32];
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -474,12 +478,16 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
         __syncthreads();  // this accumulator is read before a later tile's product reuses it
         if (half == 0) {
             const int r = tile * kTcM + rl;
-            const float4 a0 = *reinterpret_cast<const float4 *>(ypart + rl * kTcOut);
-            const float4 a1 = *reinterpret_cast<const float4 *>(ypart + (kTcM + rl) * kTcOut);
+            float4 a = *reinterpret_cast<const float4 *>(ypart + rl * kTcOut);
+#pragma unroll
+            for (int q = 1; q < kTcFwdParts; ++q) {
+                const float4 b = *reinterpret_cast<const float4 *>(ypart + (q * kTcM + rl) * kTcOut);
+                a = make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+            }
             if (r < rows)
                 *reinterpret_cast<float4 *>(y + (size_t)r * kTcOut) =
-                    make_float4(__fadd_rn(__fadd_rn(a0.x, a1.x), sb3[0]), __fadd_rn(__fadd_rn(a0.y, a1.y), sb3[1]),
-                                __fadd_rn(__fadd_rn(a0.z, a1.z), sb3[2]), __fadd_rn(__fadd_rn(a0.w, a1.w), sb3[3]));
+                    make_float4(__fadd_rn(a.x, sb3[0]), __fadd_rn(a.y, sb3[1]), __fadd_rn(a.z, sb3[2]),
+                                __fadd_rn(a.w, sb3[3]));
         }
         buf ^= 1u;
     }
@@ -1003,6 +1011,7 @@ struct boids_mlp {
     double *loss = nullptr;
     cudaStream_t st = nullptr;
     __nv_bfloat16 *w2img = nullptr;  // the hidden weights in the tensor-core layout (hidden width 256)
+    bool img_valid = false;           // it holds the present parameters' (p16)
     unsigned nsm = 1;                 // SMs: the tensor-core kernel's persistent grid
 };
 
@@ -1095,6 +1104,7 @@ void forward(boids_mlp *m, int rows, bool need_pre = true)
     gemm(m, rowmajor(m->x16, rows, m->in), rowmajor(W1, m->in, m->h), m->pre1, m->h, m->h1, m->h, b1, nullptr, 0, 1);
     if (m->w2img) {
         k_mlp_tile_w<<<nb(kTcN * kTcK / 8, 256), 256, 0, m->st>>>(W2, m->w2img);
+        m->img_valid = false;
         hidden_tc(m, rows, b2, need_pre ? m->pre2 : nullptr);
     } else {
         gemm(m, rowmajor(m->h1, rows, m->h), rowmajor(W2, m->h, m->h), m->pre2, m->h, m->h2, m->h, b2, nullptr, 0,
@@ -1129,13 +1139,12 @@ void backward(boids_mlp *m, int rows)
     k_mlp_colsum<<<m->h, 256, 0, m->st>>>(m->d1, rows, m->h, gb1);
 }
 
-// A tensor-core tile whose wait on its accumulator gave up (the flag is
-// cleared for the next call).
-int tc_status(boids_mlp *m)
+// Waits for the call's work, and for whether a tensor-core tile's wait on its
+// accumulator gave up (the flag is cleared for the next call).
+int finish_call(boids_mlp *m)
 {
-    if (!m->w2img) return 0;
     uint32_t err = 0;
-    MCK(cudaMemcpyFromSymbolAsync(&err, g_mlp_tc_error, sizeof err, 0, cudaMemcpyDeviceToHost, m->st));
+    if (m->w2img) MCK(cudaMemcpyFromSymbolAsync(&err, g_mlp_tc_error, sizeof err, 0, cudaMemcpyDeviceToHost, m->st));
     MCK(cudaStreamSynchronize(m->st));
     if (!err) return 0;
     const uint32_t zero = 0;
@@ -1254,6 +1263,7 @@ int boids_mlp_set_params(boids_mlp *m, const float *params)
     cudaSetDevice(m->device);
     MCK(cudaMemcpyAsync(m->p, params, 4 * m->np, cudaMemcpyHostToDevice, m->st));
     k_to_bf16<<<nb(m->np, 256), 256, 0, m->st>>>(m->p, m->p16, m->np);
+    m->img_valid = false;
     MCK(cudaMemsetAsync(m->m, 0, 4 * m->np, m->st));
     MCK(cudaMemsetAsync(m->v, 0, 4 * m->np, m->st));
     m->step = 0;
@@ -1272,7 +1282,8 @@ int boids_mlp_forward(boids_mlp *m, const float *x, int32_t rows, float *y)
         MCK(cudaMemcpyAsync(m->x, x, sizeof(float) * (size_t)rows * m->in, cudaMemcpyHostToDevice, m->st));
         const __nv_bfloat16 *W1 = m->p16 + m->off[0], *W2 = m->p16 + m->off[2], *W3 = m->p16 + m->off[4];
         const float *b1 = m->p + m->off[1], *b2 = m->p + m->off[3], *b3 = m->p + m->off[5];
-        k_mlp_tile_w<<<nb(kTcN * kTcK / 8, 256), 256, 0, m->st>>>(W2, m->w2img);
+        if (!m->img_valid) k_mlp_tile_w<<<nb(kTcN * kTcK / 8, 256), 256, 0, m->st>>>(W2, m->w2img);
+        m->img_valid = true;
         const unsigned tiles = nb(rows, kTcM);
         k_mlp_forward_tc<<<tiles < m->nsm ? tiles : m->nsm, kTcFwdThreads, kTcFwdSmem, m->st>>>(
             m->x, rows, W1, b1, m->w2img, b2, W3, b3, m->y);
@@ -1282,8 +1293,7 @@ int boids_mlp_forward(boids_mlp *m, const float *x, int32_t rows, float *y)
     }
     MCK(cudaGetLastError());
     MCK(cudaMemcpyAsync(y, m->y, sizeof(float) * (size_t)rows * m->out, cudaMemcpyDeviceToHost, m->st));
-    MCK(cudaStreamSynchronize(m->st));
-    return tc_status(m);
+    return finish_call(m);
 }
 
 int boids_mlp_gradient(boids_mlp *m, const float *x, const float *t, int32_t rows, float *grad, double *loss)
@@ -1305,9 +1315,9 @@ int boids_mlp_gradient(boids_mlp *m, const float *x, const float *t, int32_t row
     MCK(cudaMemcpyAsync(grad, m->grad, 4 * m->np, cudaMemcpyDeviceToHost, m->st));
     double l = 0;
     MCK(cudaMemcpyAsync(&l, m->loss, 8, cudaMemcpyDeviceToHost, m->st));
-    MCK(cudaStreamSynchronize(m->st));
+    const int rc = finish_call(m);
     if (loss) *loss = l;
-    return tc_status(m);
+    return rc;
 }
 
 int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, int32_t epochs, int32_t batch,
@@ -1317,6 +1327,7 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
         return fail(BOIDS_EINVAL, "boids_mlp_train: bad argument");
     cudaSetDevice(m->device);
     if (batch > rows) batch = rows;
+    m->img_valid = false;  // every batch lays its own out, and ends with other parameters
     if (int rc = ensure_rows(m, rows + batch)) return rc;
     // the whole set stays resident: rows [0, rows) of x/t; batches are gathered behind it
     float *X = m->x, *T = m->t;
@@ -1387,7 +1398,7 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
         epoch_loss = l / nbatch;
     }
     if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(BOIDS_ECUDA, "boids_mlp_train: kernel launch failed");
-    if (!rc) rc = tc_status(m);
+    if (!rc) rc = finish_call(m);
     cudaFree(d_idx);
     cudaFree(bx);
     cudaFree(bt);
