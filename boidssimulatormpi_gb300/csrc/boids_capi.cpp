@@ -522,17 +522,17 @@ int boids_create(const boids_params *params, boids_sim **out)
         ALLOC(&b.count, b.ncell_pad, true);
         ALLOC(&b.lstart, b.ncell_pad);
         ALLOC(&b.bsum, b.nscan_blocks);
-        ALLOC(&b.ticket, 1, true);
+        ALLOC(&b.ticket, 2, true);
         const size_t ndense = boidsgpu::dense_list_capacity(b.ncell, n);
         ALLOC(&b.dense_list, ndense);
-        ALLOC(&b.slot_of, std::min<size_t>(n, boidsgpu::kWarpBoids));
+        if (n <= boidsgpu::kCrowdBoids) ALLOC(&b.slot_of, n);
         ALLOC(&b.dflag, b.ncell / 4);
         {
             unsigned char *carry = nullptr;
             ALLOC(&carry, (size_t)boidsgpu::kCarryBytes * n);
             b.carry = carry;
         }
-        ALLOC(&b.dense_n, 3, true);
+        ALLOC(&b.dense_n, 4, true);
         ALLOC(&b.defer, 2 * n);
         // the deferred boids' overflow rows (196 B per boid) speed the
         // further passes up and are optional: without them those passes

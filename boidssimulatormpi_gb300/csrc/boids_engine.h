@@ -105,7 +105,7 @@ struct DevBuffers {
     uint32_t *count;           // per cell (padded): boids binned so far
     uint32_t *lstart;          // per cell (padded): exclusive scan inside a tile
     uint32_t *bsum;            // per scan tile: offset of the tile
-    uint32_t *ticket;          // scan completion counter (1 word)
+    uint32_t *ticket;          // scan completion counter, and its sum of pairs (2 words, zero between scans)
     uint32_t *ap_cnt, *ap_list;  // all-pairs: per boid neighbour count and list
     uint4 *ap_emb;             // all-pairs: per boid filter vector
     float *forces;             // 9 per boid (id order), optional
@@ -114,7 +114,8 @@ struct DevBuffers {
     int32_t *dcnt;             // 3 per boid (id order)
     uint64_t *dhash;           // 3 per boid (id order)
     uint32_t *dense_list;      // dense kernel work items (cell, first boid), this step (dense_list_capacity words)
-    uint32_t *dense_n;         // dense items, the dense kernel's work queue, deferred sparse boids (3 words)
+    uint32_t *dense_n;         // dense items, the step's work queue, deferred sparse boids, pairs of boids that
+                               // share an x cell (4 words)
     uint32_t *defer;           // sparse boids deferred to further passes: (slot, lo_id), 2 words per slot (null: none);
                                // a flock's entries start at its slot_base
     uint32_t *defer_cnt;       // deferred boids per flock (a single flock: dense_n + 2)
@@ -177,11 +178,35 @@ inline size_t dense_list_capacity(size_t ncell, size_t n)
     return 2 * (items < n ? items : n);
 }
 // Flocks of up to this many boids (all flocks of an ensemble together) are
-// updated a warp per boid (k_grid_warp), the others by the cells' split.  A
+// always updated a warp per boid (k_grid_warp).  A
 // step with either, us: 32 768 boids uniform 58 / 74, gathered 90 / 215;
 // 49 152 uniform 75 / 71, gathered 124 / 251; 65 537 uniform 95 / 73.  The
 // line lies where a uniform flock takes the same time with both.
 constexpr uint32_t kWarpBoids = 40960;
+// Larger ones, up to kCrowdBoids boids (an ensemble's kCrowdSlots), are sent
+// there or by the split step for step, on the device, by the pairs of boids
+// that share an x cell (counted by the scan): a warp per boid from
+// n (kCrowdBase + kCrowdSlope n) pairs up to n (kCrowdTop - kCrowdTopSlope n),
+// above which boids accept more neighbours than k_grid_warp's list holds.
+// Without id windows in the split (the allocation-free step) there is no upper
+// line.  The split of an ensemble and of the
+// allocation-free step has no side stream and no deferral, so their line
+// starts lower, at kCrowdBare, and an ensemble's stays there.  A uniform flock
+// at the reference's density has 0.29 n pairs, a gathered one 1 to 3.2 n.  A
+// step, us, by the split / a warp per boid: 65 537 boids at 0.53 n 106 / 111,
+// at 0.72 n 194 / 117, at 1.3 n 290 / 134, at 3.0 n 264 / 177; 131 072 at
+// 0.55 n 145 / 190, at 0.75 n 252 / 210, at 1.3 n 370 / 238; 262 143 at 0.75 n
+// 331 / 430, at 0.94 n 419 / 412, at 1.3 n 511 / 447, at 3.1 n 632 / 614;
+// 370 000 at 1.3 n 626 / 620, at 3.1 n 870 / 860.  Without id windows in the
+// split (the allocation-free step), 65 537 at 2.3 n 2990 / 163.  200 steps of a
+// sweep's ensembles: 90 000 slots 79.3 / 46.0 ms, 266 000 176 / 156, 825 000
+// 427 / 433.  Flocks collapsed into clusters, at 4, 8 and 16 n pairs: 50 000
+// boids 353 / 156, 233 / 250, 339 / 693; 262 143 599 / 653, 689 / 1170,
+// 1053 / 9348; an ensemble of 16 flocks of 8192 at 4 and 8 n 550 / 392 and
+// 465 / 517.
+constexpr uint32_t kCrowdBoids = 1u << 18, kCrowdSlots = 1u << 19;
+constexpr double kCrowdTop = 8.5, kCrowdTopSlope = 1.6e-5;
+constexpr double kCrowdBase = 0.47, kCrowdBare = 0.35, kCrowdSlope = 1.75e-6;
 // Up to this many boids and cells (padded) the allocation-free step's counting
 // sort is one kernel (k_grid_bin): on the eight SMs of its cluster the scatter
 // of more takes longer than the launches it saves.

@@ -33,6 +33,7 @@
 
 namespace boidsgpu {
 
+
 // ------------------------------------------------------------------ exact reference arithmetic
 
 // Vector3D::norm (src/vector3D.cpp:64-67): sqrt((x*x + y*y) + z*z).
@@ -434,6 +435,19 @@ __device__ __forceinline__ void chain_wait()
     asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
 }
 
+// The measure that sends a step's boids to a warp each or to the cells' split:
+// the pairs of boids that share an x cell, counted by k_grid_scan.  It lives on
+// the device, so a captured step follows the flock as it gathers.
+struct Crowd {
+    uint32_t *pairs;  // null: the route was chosen on the host
+    uint32_t min;     // a warp per boid: from this many pairs
+    uint32_t span;    // to min + span - 1
+};
+__device__ __forceinline__ bool crowded(const Crowd &c) { return c.pairs && __ldcg(c.pairs) - c.min < c.span; }
+// The most boids of a cell that count: their pairs cannot overflow a word in
+// flocks of up to 2^19 boids.
+constexpr uint32_t kCrowdCap = 4096;
+
 template <bool MULTI>
 __global__ void k_grid_keys(const float4 *__restrict__ pos, uint32_t *__restrict__ key,
                             uint32_t *__restrict__ rank, uint32_t *__restrict__ count, StepConst kp, FlockTable ft)
@@ -484,7 +498,7 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *warp_t
 
 __global__ void __launch_bounds__(kScanThreads)
 k_grid_scan(const uint32_t *__restrict__ count, uint32_t *__restrict__ lstart, uint32_t *bsum,
-            uint32_t *ticket, uint32_t nblocks)
+            uint32_t *ticket, uint32_t nblocks, uint32_t *__restrict__ work, int measure)
 {
     __shared__ uint32_t warp_tot[kScanThreads / 32];
     __shared__ bool is_last;
@@ -503,6 +517,17 @@ k_grid_scan(const uint32_t *__restrict__ count, uint32_t *__restrict__ lstart, u
     for (int i = 0; i < 8; ++i) { o[i] = run; run += v[i]; }
     *reinterpret_cast<uint4 *>(lstart + base) = make_uint4(o[0], o[1], o[2], o[3]);
     *reinterpret_cast<uint4 *>(lstart + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+    if (measure) {
+        uint32_t pairs = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t c = min(v[i], kCrowdCap);
+            if (c > 1) pairs += c * (c - 1) / 2;
+        }
+        pairs = __reduce_add_sync(0xffffffffu, pairs);
+        if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(ticket + 1, pairs);
+    }
+    if (measure) __syncthreads();  // every warp's pairs before the block's ticket
     if (threadIdx.x == 0) {
         bsum[blockIdx.x] = total;
         __threadfence();
@@ -520,16 +545,22 @@ k_grid_scan(const uint32_t *__restrict__ count, uint32_t *__restrict__ lstart, u
         if (i < nblocks) bsum[i] = carry + ex;
         carry += chunk;
     }
-    if (threadIdx.x == 0) *ticket = 0;  // ready for the next launch
+    if (threadIdx.x == 0) {
+        *ticket = 0;  // ready for the next launch
+        if (work) {   // this step's work counters
+            work[0] = work[1] = work[2] = 0;
+            if (measure) work[3] = atomicExch(ticket + 1, 0u);
+        }
+    }
 }
 
 template <bool MULTI>
 __global__ void k_grid_scatter(const float4 *__restrict__ pin, const float4 *__restrict__ vin,
-                               const uint32_t *__restrict__ key, const uint32_t *__restrict__ rank,
+                               const uint32_t *__restrict__ key, const uint32_t *rank,
                                const uint32_t *__restrict__ lstart, const uint32_t *__restrict__ bsum,
                                float4 *__restrict__ pout, float4 *__restrict__ vout,
-                               uint32_t *__restrict__ count_to_zero, uint32_t *__restrict__ slot_of, uint32_t n,
-                               FlockTable ft)
+                               uint32_t *__restrict__ count_to_zero, uint32_t *slot_of, Crowd crowd,
+                               uint32_t n, FlockTable ft)
 {
     chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -544,11 +575,12 @@ __global__ void k_grid_scatter(const float4 *__restrict__ pin, const float4 *__r
         return;
     }
     const uint32_t c = key[s];
+    const bool table = slot_of && (!crowd.pairs || crowded(crowd));
     const uint32_t d = cell_start(lstart, bsum, c) + rank[s] + off;
     const float4 p = pin[s];
     pout[d] = p;
     vout[d] = vin[s];
-    if (slot_of) slot_of[first + __float_as_uint(p.w)] = d;
+    if (table) slot_of[first + __float_as_uint(p.w)] = d;
     if (count_to_zero) count_to_zero[c] = 0;  // every binned cell, for the next step's keys
 }
 
@@ -612,12 +644,12 @@ k_grid_bin(const float *__restrict__ pos3, const float *__restrict__ vel3, uint3
         reinterpret_cast<uint4 *>(lstart)[g] = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
         run += v.x + v.y + v.z + v.w;
     }
-    cluster_sync();  // (the counts are dead: slot_of may take their place)
+    cluster_sync();
     for (uint32_t i = at; i < k.n; i += kAll) {
         const uint32_t d = __ldcg(lstart + __ldcg(key + i)) + __ldcg(rank + i);
         pout[d] = make_float4(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2], __uint_as_float(i));
         vout[d] = make_float4(vel3[3 * i], vel3[3 * i + 1], vel3[3 * i + 2], 0.f);
-        slot_of[i] = d;
+        slot_of[i] = d;  // (may be rank[i])
     }
 }
 
@@ -671,10 +703,15 @@ template <bool MULTI>
 __global__ void k_grid_classify(const uint32_t *__restrict__ lstart,
                                 const uint32_t *__restrict__ bsum, uint8_t *__restrict__ dflag,
                                 uint32_t *__restrict__ dense_list, uint32_t *__restrict__ dense_n, uint32_t nfull,
-                                int windows, StepConst kp, FlockTable ft)
+                                int windows, Crowd crowd, StepConst kp, FlockTable ft)
 {
+    chain_wait();
     const uint32_t cg = blockIdx.x * blockDim.x + threadIdx.x;
     if (cg >= nfull) return;
+    if (crowded(crowd)) {  // no items, and no boids for k_grid_sparse
+        dflag[cg] = 1;
+        return;
+    }
     // boids of the cell from the scan (the counts may be zeroed meanwhile by
     // the scatter, which runs beside this kernel)
     const uint32_t b = cell_start(lstart, bsum, 4 * cg + 4) - cell_start(lstart, bsum, 4 * cg);
@@ -746,6 +783,8 @@ struct GridIn {
     const uint32_t *__restrict__ bsum;
     const uint8_t *__restrict__ dflag;  // per full-size cell: taken by k_grid_dense
     const uint32_t *__restrict__ slot_of;  // k_grid_warp: slot of each id, from its flock's slot_base
+    Crowd crowd;
+    int chain;  // k_grid_sparse and k_grid_dense were launched in a chain
 };
 
 struct SparseSmem {
@@ -1030,6 +1069,7 @@ k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
     // the flock's constants (an ensemble's CTA serves one flock); one word otherwise
     __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
     StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
+    if (g.chain) chain_wait();
     if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x]);
     const StepConst &k = MULTI ? kf : kp;
     const int G = k.G;
@@ -1045,8 +1085,8 @@ k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
     __shared__ uint32_t wcount[kRT / 32];
     const uint32_t s0 = blockIdx.x * kRT + t;
     bool mine = s0 - k.slot_base < k.n;
+    const float4 q = mine ? g.pos[s0] : make_float4(0.f, 0.f, 0.f, 0.f);
     if (mine) {
-        const float4 q = g.pos[s0];
         const uint32_t fc = k.cell_base / 4 +
                             (uint32_t)((cell1(q.z, k) * G + cell1(q.y, k)) * G + cell1(q.x, k));
         mine = !__ldg(g.dflag + fc);
@@ -1354,8 +1394,10 @@ __device__ __forceinline__ void warp_add(WarpSmem &sm, int lane, int f, float3 t
 // found through the id -> slot table take the exact tests and are added up,
 // 32 at a time.  Out of line: it is rare.
 template <bool DIAG>
-__device__ __noinline__ void warp_many(WarpSmem *smp, const GridIn &g, const StepConst &k, uint32_t s, float3 pi,
-                                       const Sight &si, float dot_lim, int nr, bool shifted, WarpSums &a)
+__device__ __noinline__ WarpSums warp_many(WarpSmem *smp, const float4 *__restrict__ gpos,
+                                           const float4 *__restrict__ gvel, const uint32_t *__restrict__ slot_of,
+                                           const StepConst &k, uint32_t s, float3 pi, Sight si, float dot_lim, int nr,
+                                           bool shifted)
 {
     constexpr unsigned kAll = 0xffffffffu;
     WarpSmem &sm = *smp;
@@ -1365,7 +1407,7 @@ __device__ __noinline__ void warp_many(WarpSmem *smp, const GridIn &g, const Ste
     constexpr int kGroup = 16;                                // map words expanded at a time
     static_assert(kWarpIds == 32 * kWarpList, "the map takes the list's ids");
     static_assert(2 * (32 * kGroup + 32) <= sizeof(sm.lsl) + sizeof(sm.ord), "a group's hits fit");
-    a = WarpSums{};
+    WarpSums a{};
     for (uint32_t w0 = 0; w0 < k.n; w0 += kWarpIds) {
         for (int i = lane; i < kWarpList; i += 32) map[i] = 0;
         __syncwarp();
@@ -1375,7 +1417,7 @@ __device__ __noinline__ void warp_many(WarpSmem *smp, const GridIn &g, const Ste
             const float3 q = make_float3(pi.x - sh.x, pi.y - sh.y, pi.z - sh.z);
             for (uint32_t off = lane; off < rn.y; off += 32) {
                 const uint32_t slot = (rn.x & 0x7fffffffu) + off;
-                const float4 pj = __ldg(g.pos + slot);
+                const float4 pj = __ldg(gpos + slot);
                 const float dx = pj.x - q.x, dy = pj.y - q.y, dz = pj.z - q.z;
                 const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
                 const float dv = __fmaf_rn(si.v.z, dz, __fmaf_rn(si.v.y, dy, __fmul_rn(si.v.x, dx)));
@@ -1410,11 +1452,11 @@ __device__ __noinline__ void warp_many(WarpSmem *smp, const GridIn &g, const Ste
                 float4 vj = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < nh) {
                     id = w0 + hits[h0 + lane];
-                    const uint32_t slot = __ldg(g.slot_of + k.slot_base + id);
-                    const float4 pj = __ldg(g.pos + slot);
+                    const uint32_t slot = __ldg(slot_of + k.slot_base + id);
+                    const float4 pj = __ldg(gpos + slot);
                     t = shifted ? image3(xyz(pj), pi, k) : xyz(pj);
                     f = pair_flags(pi, si, t, k);
-                    if (f) vj = __ldg(g.vel + slot);
+                    if (f) vj = __ldg(gvel + slot);
                 }
                 warp_add<DIAG>(sm, lane, f, t, vj, id, pi, a);
                 const int done = min(nh, 32);
@@ -1428,6 +1470,7 @@ __device__ __noinline__ void warp_many(WarpSmem *smp, const GridIn &g, const Ste
             __syncwarp();
         }
     }
+    return a;
 }
 
 // finish_boid by the lanes of a warp.
@@ -1481,21 +1524,12 @@ __device__ __forceinline__ void warp_finish(WarpSums &a, float4 p4, float3 vi, u
         o.forces[(size_t)9 * out + lane] = f;
 }
 
-template <bool DIAG, bool MULTI>
-__global__ void __launch_bounds__(kWarpWarps * 32, kWarpCtas)
-k_grid_warp(GridIn g, GridOut o, StepConst kp, FlockTable ft)
+// The update of the boid in slot s, by the 32 lanes of a warp.
+template <bool DIAG>
+__device__ __forceinline__ void warp_boid(WarpSmem &sm, const GridIn &g, const GridOut &o, const StepConst &k, uint32_t s,
+                                          int lane)
 {
-    __shared__ WarpSmem sms[kWarpWarps];
-    __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
-    StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
-    chain_wait();
-    if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * kWarpWarps / kSlotAlign]);
-    const StepConst &k = MULTI ? kf : kp;
-    const uint32_t s = blockIdx.x * kWarpWarps + (threadIdx.x >> 5);
-    if (s - k.slot_base >= k.n) return;
-    WarpSmem &sm = sms[threadIdx.x >> 5];
     constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 p4 = __ldg(g.pos + s);
@@ -1620,7 +1654,7 @@ k_grid_warp(GridIn g, GridOut o, StepConst kp, FlockTable ft)
     }
     __syncwarp();
     if (nl > kWarpList) {
-        warp_many<DIAG>(&sm, g, k, s, pi, si, dot_lim, nr, shifted, a);
+        a = warp_many<DIAG>(&sm, g.pos, g.vel, g.slot_of, k, s, pi, si, dot_lim, nr, shifted);
     } else if (nl > 0) {
         // the accepted neighbours in id order, the next 32 neighbours' loads in
         // flight under each 32's sums
@@ -1646,6 +1680,59 @@ k_grid_warp(GridIn g, GridOut o, StepConst kp, FlockTable ft)
         }
     }
     warp_finish<DIAG>(a, p4, si.v, s, lane, o, k);
+}
+
+template <bool DIAG, bool MULTI>
+__global__ void __launch_bounds__(kWarpWarps * 32, kWarpCtas)
+k_grid_warp(GridIn g, GridOut o, StepConst kp, FlockTable ft)
+{
+    __shared__ WarpSmem sms[kWarpWarps];
+    __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
+    StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
+    chain_wait();
+    if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * kWarpWarps / kSlotAlign]);
+    const StepConst &k = MULTI ? kf : kp;
+    const uint32_t s = blockIdx.x * kWarpWarps + (threadIdx.x >> 5);
+    if (s - k.slot_base >= k.n) return;
+    warp_boid<DIAG>(sms[threadIdx.x >> 5], g, o, k, s, threadIdx.x & 31);
+}
+
+// The same where the scan's measure decides whether the boids come here: a
+// grid that fills the GPU once, whose CTAs take kWarpWarps consecutive boids at
+// a time from a queue, so that a step that does not come here costs one short
+// launch (2 us; a CTA per four boids, most of them to end at once, took 24 us
+// at 65 537 boids and 100 at 262 143).  Bound as k_grid_warp.  Consecutive
+// boids share their candidates in L1: a queue of single boids per warp took
+// 149 us a step for 134 (65 537 boids, 1.3 n pairs), four boids in turn per
+// warp 173.
+template <bool DIAG, bool MULTI>
+__global__ void __launch_bounds__(kWarpWarps * 32, kWarpCtas)
+k_grid_warp_queue(GridIn g, GridOut o, uint32_t *__restrict__ taken, StepConst kp, FlockTable ft)
+{
+    chain_wait();
+    if (!crowded(g.crowd)) return;
+    static_assert(kSlotAlign % kWarpWarps == 0, "the boids taken together are of one flock");
+    __shared__ WarpSmem sms[kWarpWarps];
+    __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
+    __shared__ uint32_t at;
+    StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
+    if (MULTI && threadIdx.x == 0) kf.flock = ~0u;
+    for (;;) {
+        if (threadIdx.x == 0) at = kWarpWarps * atomicAdd(taken, 1u);
+        __syncthreads();
+        const uint32_t s = at + (threadIdx.x >> 5);
+        if (at >= (MULTI ? ft.nslots : kp.n)) return;
+        if (MULTI) {
+            const uint32_t f = ft.blk_flock[at / kSlotAlign];
+            if (f != kf.flock) {
+                __syncthreads();
+                load_flock(kf, ft, f);
+            }
+        }
+        const StepConst &k = MULTI ? kf : kp;
+        if (s - k.slot_base < k.n) warp_boid<DIAG>(sms[threadIdx.x >> 5], g, o, k, s, threadIdx.x & 31);
+        __syncthreads();
+    }
 }
 
 // ------------------------------------------------------------------ dense cells: CTA per cell
@@ -2001,6 +2088,7 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
     extern __shared__ __align__(16) unsigned char dense_smem_raw[];
     DenseSmem &sm = *reinterpret_cast<DenseSmem *>(dense_smem_raw);
     const int t = threadIdx.x;
+    if (g.chain) chain_wait();
     for (;;) {
         if (t == 0) sm.work = atomicAdd(dense_n + 1, 1u);
         __syncthreads();
@@ -2623,12 +2711,13 @@ static inline unsigned blocks_for(uint32_t n, unsigned t) { return (n + t - 1) /
 // Launches a kernel that begins with chain_wait, with programmatic dependence
 // on the kernel before it when chain is set.
 template <class... P, class... A>
-static cudaError_t launch_chain(bool chain, void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st,
-                                A... args)
+static cudaError_t launch_chain(bool chain, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                                cudaStream_t st, A... args)
 {
     cudaLaunchConfig_t c{};
     c.gridDim = dim3(grid);
     c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
     c.stream = st;
     cudaLaunchAttribute a{};
     a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -2643,6 +2732,18 @@ static cudaError_t launch_chain(bool chain, void (*kernel)(P...), unsigned grid,
 static inline bool grid_by_warp(const StepConst &k, const DevBuffers &b, const FlockTable *ft)
 {
     return b.slot_of && !k.tuned && (ft ? ft->nslots : k.n) <= kWarpBoids;
+}
+
+// Larger flocks that have the table of slots are sent there or by the cells'
+// split in each step, on the device.
+static inline Crowd crowd_route(const StepConst &k, const DevBuffers &b, const FlockTable *ft)
+{
+    if (!b.slot_of || k.tuned || grid_by_warp(k, b, ft)) return Crowd{nullptr, 0, 0};
+    const double n = ft ? ft->nslots : k.n;
+    const double line = (ft || !b.carry ? kCrowdBare : kCrowdBase) + (ft ? 0. : kCrowdSlope * n);
+    const double top = !b.carry ? 1e9 : kCrowdTop - kCrowdTopSlope * n;
+    const uint32_t min = (uint32_t)(n * line);
+    return Crowd{b.dense_n + 3, min, (uint32_t)fmax(0., fmin(4e9, n * top) - min)};
 }
 
 cudaError_t launch_pack(const float *pos3, const float *vel3, float4 *pos4, float4 *vel4, uint32_t i0, uint32_t i1,
@@ -2709,13 +2810,11 @@ cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream
 {
     cudaError_t e = cudaSuccess;
     const bool by_cells = !grid_by_warp(k, b, ft);
-    if (by_cells && (e = cudaMemsetAsync(b.dense_n, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess)
-        return e;  // items, work queue, deferred
     if (by_cells && ft && b.defer_cnt && (e = cudaMemsetAsync(b.defer_cnt, 0, sizeof(uint32_t) * ft->count, st)) != cudaSuccess)
         return e;  // an ensemble's per-flock deferred counts
     *launches += 1;
-    return launch_chain(!by_cells, k_grid_scan, b.nscan_blocks, kScanThreads, st, b.count, b.lstart, b.bsum, b.ticket,
-                        b.nscan_blocks);
+    return launch_chain(!by_cells, k_grid_scan, b.nscan_blocks, kScanThreads, 0, st, b.count, b.lstart, b.bsum, b.ticket,
+                        b.nscan_blocks, by_cells ? b.dense_n : nullptr, crowd_route(k, b, ft).pairs != nullptr);
 }
 
 bool grid_bin_small(const StepConst &k, const DevBuffers &b)
@@ -2739,24 +2838,23 @@ cudaError_t launch_grid_classify(const StepConst &k, const DevBuffers &b, cudaSt
     cudaError_t e;
     const uint32_t nfull = b.ncell / 4;
     const int windows = b.carry != nullptr;
+    const Crowd crowd = crowd_route(k, b, ft);
     // with a side stream the classification runs beside what the caller
     // queues next (the scatter); launch_grid_force waits for it
     cudaStream_t cs = st;
-    if (b.aux) {
+    const bool side = b.aux != nullptr, chain = !side && !ft;
+    if (side) {
         if ((e = cudaEventRecord(b.fork, st)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(b.aux, b.fork, 0)) != cudaSuccess) return e;
         cs = b.aux;
     }
-    if (ft)
-        k_grid_classify<true><<<blocks_for(nfull, 256), 256, 0, cs>>>(b.lstart, b.bsum, b.dflag,
-                                                                       b.dense_list, b.dense_n, nfull, windows, k, *ft);
-    else
-        k_grid_classify<false><<<blocks_for(nfull, 256), 256, 0, cs>>>(b.lstart, b.bsum, b.dflag,
-                                                                        b.dense_list, b.dense_n, nfull, windows, k,
-                                                                        FlockTable{});
-    if (b.aux && (e = cudaEventRecord(b.cjoin, b.aux)) != cudaSuccess) return e;
+    e = launch_chain(chain, ft ? k_grid_classify<true> : k_grid_classify<false>, blocks_for(nfull, 256), 256, 0, cs,
+                     b.lstart, b.bsum, b.dflag, b.dense_list, b.dense_n, nfull, windows, crowd, k,
+                     ft ? *ft : FlockTable{});
+    if (e != cudaSuccess) return e;
+    if (side && (e = cudaEventRecord(b.cjoin, b.aux)) != cudaSuccess) return e;
     *launches += 1;
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 cudaError_t launch_grid_scatter(const StepConst &k, const DevBuffers &b, int from, bool zero_counts,
@@ -2765,11 +2863,12 @@ cudaError_t launch_grid_scatter(const StepConst &k, const DevBuffers &b, int fro
     const uint32_t n = ft ? ft->nslots : k.n;
     if (n == 0) return cudaSuccess;
     uint32_t *cz = zero_counts ? b.count : nullptr;
-    uint32_t *so = grid_by_warp(k, b, ft) ? b.slot_of : nullptr;
+    const Crowd crowd = crowd_route(k, b, ft);
+    uint32_t *so = grid_by_warp(k, b, ft) || crowd.pairs ? b.slot_of : nullptr;
     ++*launches;
-    return launch_chain(grid_by_warp(k, b, ft), ft ? k_grid_scatter<true> : k_grid_scatter<false>, blocks_for(n, 256),
-                        256, st, b.pos[from], b.vel[from], b.key, b.rank, b.lstart, b.bsum, b.pos[1 - from],
-                        b.vel[1 - from], cz, so, n, ft ? *ft : FlockTable{});
+    return launch_chain(grid_by_warp(k, b, ft) || (!ft && !b.aux), ft ? k_grid_scatter<true> : k_grid_scatter<false>, blocks_for(n, 256),
+                        256, 0, st, b.pos[from], b.vel[from], b.key, b.rank, b.lstart, b.bsum, b.pos[1 - from],
+                        b.vel[1 - from], cz, so, crowd, n, ft ? *ft : FlockTable{});
 }
 
 namespace {
@@ -2797,12 +2896,16 @@ cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, co
 {
     if (grid_by_warp(k, b, MULTI ? &ft : nullptr)) {
         return launch_chain(true, k_grid_warp<DIAG, MULTI>, blocks_for(MULTI ? ft.nslots : k.n, kWarpWarps),
-                            kWarpWarps * 32, st, g, o, k, ft);
+                            kWarpWarps * 32, 0, st, g, o, k, ft);
     }
     cudaError_t e = dense_smem_opt_in<DIAG, MULTI>();
     if (e != cudaSuccess) return e;
+    if (g.crowd.pairs) {
+        e = launch_chain(!MULTI, k_grid_warp_queue<DIAG, MULTI>, b.dense_grid, kWarpWarps * 32, 0, st, g, o, b.dense_n + 1, k, ft);
+        if (e != cudaSuccess) return e;
+    }
     if (b.aux && (e = cudaStreamWaitEvent(st, b.cjoin, 0)) != cudaSuccess) return e;  // the classification
-    k_grid_sparse<DIAG, MULTI><<<nsp, kRT, 0, st>>>(g, o, k, ft);
+    if ((e = launch_chain(g.chain, k_grid_sparse<DIAG, MULTI>, nsp, kRT, 0, st, g, o, k, ft)) != cudaSuccess) return e;
     const unsigned nmore = MULTI ? nsp : min(nsp, 2 * b.dense_grid);
     if (o.defer && b.aux) {
         // the deferred boids and the dense cells are disjoint: run them side by side
@@ -2815,8 +2918,8 @@ cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, co
         return cudaGetLastError();
     }
     if (o.defer) k_grid_sparse_more<DIAG, MULTI><<<nmore, kRT, 0, st>>>(g, o, k, ft);
-    k_grid_dense<DIAG, MULTI><<<b.dense_grid, kDT, sizeof(DenseSmem), st>>>(g, o, b.dense_list, b.dense_n, k, ft);
-    return cudaGetLastError();
+    return launch_chain(g.chain && !o.defer, k_grid_dense<DIAG, MULTI>, b.dense_grid, kDT, sizeof(DenseSmem), st, g, o,
+                        b.dense_list, b.dense_n, k, ft);
 }
 
 }  // namespace
@@ -2826,7 +2929,7 @@ cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from,
 {
     const uint32_t n = ft ? ft->nslots : k.n;
     if (n == 0) return cudaSuccess;
-    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, b.dflag, b.slot_of};
+    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, b.dflag, b.slot_of, crowd_route(k, b, ft), !b.aux && !ft};
     GridOut o{};
     o.carry = static_cast<Acc *>(b.carry);
     o.wscratch = b.carry ? b.wscratch : nullptr;
@@ -2857,7 +2960,7 @@ cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from,
     cudaError_t e;
     if (ft) e = diag ? grid_force<true, true>(k, g, o, b, nsp, *ft, st) : grid_force<false, true>(k, g, o, b, nsp, *ft, st);
     else e = diag ? grid_force<true, false>(k, g, o, b, nsp, none, st) : grid_force<false, false>(k, g, o, b, nsp, none, st);
-    if (e == cudaSuccess) *launches += grid_by_warp(k, b, ft) ? 1 : (o.defer ? 3 : 2);
+    if (e == cudaSuccess) *launches += grid_by_warp(k, b, ft) ? 1 : 2 + (o.defer ? 1 : 0) + (g.crowd.pairs ? 1 : 0);
     return e;
 }
 

@@ -159,17 +159,19 @@ size_t layout(const boidsgpu::StepConst &k, unsigned char *base, boidsgpu::DevBu
     b->key = reinterpret_cast<uint32_t *>(keys);
     b->rank = keys ? b->key + n : nullptr;
     b->dense_list = b->key;
-    b->count = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad + 4));  // and the scan's ticket behind them
+    b->count = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad + 8));  // and the scan's ticket behind them
     b->ticket = b->count ? b->count + b->ncell_pad : nullptr;
     b->lstart = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->ncell_pad));
     b->bsum = reinterpret_cast<uint32_t *>(take(4 * (size_t)b->nscan_blocks));
-    b->dense_n = reinterpret_cast<uint32_t *>(take(12));
+    b->dense_n = reinterpret_cast<uint32_t *>(take(16));
     b->dflag = take(b->ncell / 4);
-    // the counts are dead after the scan: the id -> slot table of a small
-    // flock takes their place where it fits, so that it costs no scratch there
-    if (k.n <= boidsgpu::kWarpBoids)
-        b->slot_of = n <= b->ncell_pad ? b->count : reinterpret_cast<uint32_t *>(take(4 * n));
-    b->carry = nullptr;  // no id windows: cells over the dense list's capacity stay per-boid
+    // the id -> slot table takes the ranks' place: the state comes in id order,
+    // so the thread that scatters boid i is the one that read its rank (and
+    // where the table is used, the work list is not)
+    b->slot_of = b->rank;
+    // no id windows: cells over the dense list's capacity stay per-boid where the
+    // flock goes by the cells' split (a gathered one goes a warp per boid)
+    b->carry = nullptr;
     b->defer = nullptr;  // and the thread-per-boid kernel takes all of its boids' passes
     return off;
 }
@@ -216,7 +218,7 @@ extern "C" int boids_step_noalloc(const boids_params *params, const float *pos3n
         e = boidsgpu::launch_grid_bin(k, b, pos3n_in, vel3n_in, st, &launches);
     } else {
         // the array keeps the previous call's contents: clear the counts and the ticket
-        if ((e = cudaMemsetAsync(b.count, 0, 4 * (size_t)b.ncell_pad + 4, st)) == cudaSuccess &&
+        if ((e = cudaMemsetAsync(b.count, 0, 4 * (size_t)b.ncell_pad + 8, st)) == cudaSuccess &&
             (e = boidsgpu::launch_pack(pos3n_in, vel3n_in, b.pos[0], b.vel[0], 0, n, nullptr, 0.f, &k, b.key, b.rank,
                                        b.count, st, &launches)) == cudaSuccess &&
             (e = boidsgpu::launch_grid_scan(k, b, st, &launches)) == cudaSuccess &&

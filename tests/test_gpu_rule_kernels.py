@@ -139,3 +139,86 @@ def test_allocation_free_step_at_its_kernels_limits(boids_lib, oracle_mod, n, fi
         assert_bits_equal(b[0].cpu().numpy(), op, "positions, call %d" % call)
         assert_bits_equal(b[1].cpu().numpy(), ov, "velocities, call %d" % call)
         a, b = b, a
+
+
+def gathered(n, field, share, seed, cluster=64):
+    """A state of n boids, that share of them in clusters of about so many, the others uniform."""
+    rng = np.random.default_rng(seed)
+    m = int(n * share)
+    centre = rng.uniform(0, field, (m // cluster + 1, 3))
+    pos = np.concatenate([np.mod(centre[rng.integers(0, len(centre), m)] + rng.normal(0, 0.012, (m, 3)), field),
+                          rng.uniform(0, field, (n - m, 3))])
+    v = rng.normal(size=pos.shape)
+    v *= rng.uniform(0.001, 0.005, (n, 1)) / np.linalg.norm(v, axis=1, keepdims=True)
+    perm = rng.permutation(n)
+    return pos[perm].astype(np.float32).reshape(-1), v[perm].astype(np.float32).reshape(-1)
+
+
+# pairs sharing an x cell: below, about and over the lower line, over the upper one
+@pytest.mark.parametrize("share,cluster", [(0.0, 64), (0.06, 64), (0.12, 64), (1.0, 64), (0.5, 1000)])
+@pytest.mark.parametrize("n", [40961, 65537, 262144, 262145])
+def test_route_by_crowding(boids_lib, n, share, cluster):
+    """Flocks over 40960 boids, whose steps go a warp per boid or by the cells'
+    split as the scan's measure has it (up to 262144 boids), against the split
+    alone: state, forces and neighbour sets, over updates that cross the line,
+    and the allocation-free step."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    B = boids_lib
+    prm = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008), vmax=0.005, vmin=0.001)
+    field = (n / 16384) ** (1 / 3)
+    pos, vel = gathered(n, field, share, n, cluster)
+    a, b = make_sim(B, "grid", n, field, prm), make_sim(B, "grid", n, field, prm)
+    b.set_tuning(*b.tuning())
+    for s in (a, b):
+        s.set_state(pos, vel)
+    for x, y in zip(a.neighbor_sets(), b.neighbor_sets()):
+        assert np.array_equal(x, y)
+    for steps in (1, 33):
+        for s in (a, b):
+            s.update(steps)
+        for x, y in zip(a.state(), b.state()):
+            assert_bits_equal(x, y, "state")
+        assert_bits_equal(a.forces(), b.forces(), "forces")
+    q = [torch.from_numpy(np.ascontiguousarray(x).reshape(-1).copy()).cuda() for x in a.state()]
+    r = [torch.empty_like(x) for x in q]
+    prms = B.flock_params(n, field, prm["sep"], prm["ali"], prm["coh"], prm["vmax"], prm["vmin"])
+    rc = B.lib().boids_step_noalloc(C.byref(prms), q[0].data_ptr(), q[1].data_ptr(), r[0].data_ptr(), r[1].data_ptr(),
+                                    None)
+    assert rc == 0, B.lib().boids_last_error().decode()
+    torch.cuda.synchronize()
+    b.update(1)
+    for x, y in zip(r, b.state()):
+        assert_bits_equal(x.cpu().numpy(), np.asarray(y).reshape(-1), "allocation-free step")
+    a.close()
+    b.close()
+
+
+def test_ensemble_route_by_crowding(boids_lib):
+    """An ensemble over 40960 slots whose uniform and gathered flocks (one of a
+    single boid, one of an odd size) go a warp per boid, against the split."""
+    B = boids_lib
+    m = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008))
+    sizes = (30001, 1, 129, 16384, 5000)
+    flocks = [(B.flock_params(n, max(0.7, (n / 16384) ** (1 / 3)), m["sep"], m["ali"], m["coh"], 0.005, 0.001),
+               B.INIT_RANDOM_UNIFORM, n) for n in sizes]
+    a, b = B.Ensemble(flocks), B.Ensemble(flocks)
+    b.set_tuning(*b.tuning())
+    for e in (a, b):
+        e.init()
+        for f in (0, 4):
+            e.set_state(f, *gathered(sizes[f], flocks[f][0].field_size, 1.0, f))
+    for steps in (1, 17, 40):
+        for e in (a, b):
+            e.step(steps)
+        for f in range(len(sizes)):
+            for x, y in zip(a.state(f), b.state(f)):
+                assert_bits_equal(x, y, "flock %d" % f)
+    for e in (a, b):
+        e.stats()  # bins the state; the step goes on from there
+        e.step(1)
+    for f in range(len(sizes)):
+        for x, y in zip(a.state(f), b.state(f)):
+            assert_bits_equal(x, y, "flock %d" % f)
+    a.close()
+    b.close()
