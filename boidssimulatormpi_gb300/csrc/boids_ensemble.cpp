@@ -17,9 +17,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 using boidsgpu::DevBuffers;
@@ -160,6 +164,55 @@ int bin_now(boids_ensemble *e)
     e->binned = true;
     e->binned_tuned = e->tuned;
     return 0;
+}
+
+// A flock's 3 n drawn floats, at out + n, spread to n records (x, y, z, w).
+// Record i ends before the floats of boid i + 1 begin, so in place.
+void spread(float *out, uint32_t n, bool ids)
+{
+    const float *in = out + n;
+    for (uint32_t i = 0; i < n; ++i) {
+        const float x = in[3 * (size_t)i], y = in[3 * (size_t)i + 1], z = in[3 * (size_t)i + 2];
+        float *r = out + 4 * (size_t)i;
+        r[0] = x;
+        r[1] = y;
+        r[2] = z;
+        if (ids) std::memcpy(r + 3, &i, 4);
+        else r[3] = 0.f;
+    }
+}
+
+// Every flock's initial state as packed records, the padding zero.  A flock's
+// sequence of random numbers is its own, so threads draw flocks side by side
+// (a sweep's 48 flocks, 318 000 boids: 2.0 ms with 16 threads, 13.9 with one).
+void draw_flocks(const boids_ensemble *e, float4 *hp, float4 *hv)
+{
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+        for (size_t f; (f = next.fetch_add(1)) < e->desc.size();) {
+            const boids_flock_desc &d = e->desc[f];
+            const StepConst &k = e->ks[f];
+            float *p = reinterpret_cast<float *>(hp + k.slot_base), *v = reinterpret_cast<float *>(hv + k.slot_base);
+            boidsgpu::draw_initial_state(&d.params, d.init_kind == BOIDS_INIT_TEST, d.rand_seed, p + k.n, v + k.n);
+            spread(p, k.n, true);
+            spread(v, k.n, false);
+            const size_t end = f + 1 < e->ks.size() ? e->ks[f + 1].slot_base : e->nslots;
+            const size_t pad = 4 * (end - k.slot_base - k.n);
+            std::fill_n(p + 4 * (size_t)k.n, pad, 0.f);
+            std::fill_n(v + 4 * (size_t)k.n, pad, 0.f);
+        }
+    };
+    // a thread per 8192 boids at most: starting one takes as long as drawing 500
+    const size_t most = std::min<size_t>({std::thread::hardware_concurrency(), e->desc.size(), 16,
+                                          (size_t)e->total_boids / 8192 + 1});
+    std::vector<std::thread> helpers;
+    try {
+        helpers.reserve(most);
+        while (helpers.size() + 1 < most) helpers.emplace_back(work);
+    } catch (...) {  // no more threads to be had: those there are do it
+    }
+    work();
+    for (auto &t : helpers) t.join();
 }
 
 // Put the state back into buffer 0, where the captured graph expects it.
@@ -355,28 +408,20 @@ int boids_ensemble_init(boids_ensemble *e)
     if (!e) return fail(BOIDS_EINVAL, "boids_ensemble_init: null handle");
     int rc = use_device(e);
     if (rc) return rc;
-    std::vector<float4> hp(e->nslots, make_float4(0.f, 0.f, 0.f, 0.f)), hv(e->nslots, make_float4(0.f, 0.f, 0.f, 0.f));
-    std::vector<float> pos, vel;
-    for (size_t f = 0; f < e->desc.size(); ++f) {
-        const boids_flock_desc &d = e->desc[f];
-        const uint32_t n = e->ks[f].n;
-        pos.assign((size_t)3 * n, 0.f);
-        vel.assign((size_t)3 * n, 0.f);
-        boidsgpu::draw_initial_state(&d.params, d.init_kind == BOIDS_INIT_TEST, d.rand_seed, pos.data(), vel.data());
-        const uint32_t base = e->ks[f].slot_base;
-        for (uint32_t i = 0; i < n; ++i) {
-            float w;
-            std::memcpy(&w, &i, 4);
-            hp[base + i] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], w);
-            hv[base + i] = make_float4(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2], 0.f);
-        }
-    }
-    CK(cudaMemcpyAsync(e->b.pos[0], hp.data(), sizeof(float4) * e->nslots, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(e->b.vel[0], hv.data(), sizeof(float4) * e->nslots, cudaMemcpyHostToDevice, e->stream));
+    const size_t ns = std::max<size_t>(e->nslots, 1);
+    struct Free {
+        void operator()(float4 *p) const { std::free(p); }
+    };
+    std::unique_ptr<float4[], Free> hp(static_cast<float4 *>(std::malloc(sizeof(float4) * ns)));
+    std::unique_ptr<float4[], Free> hv(static_cast<float4 *>(std::malloc(sizeof(float4) * ns)));
+    if (!hp || !hv) return fail(BOIDS_ENOMEM, "boids_ensemble_init: out of host memory");
+    draw_flocks(e, hp.get(), hv.get());
+    CK(cudaMemcpyAsync(e->b.pos[0], hp.get(), sizeof(float4) * e->nslots, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemcpyAsync(e->b.vel[0], hv.get(), sizeof(float4) * e->nslots, cudaMemcpyHostToDevice, e->stream));
     e->cur = 0;
     if ((rc = bin_fresh(e))) return rc;
     e->has_state = true;
-    CK(cudaStreamSynchronize(e->stream));  // the host vectors die here
+    CK(cudaStreamSynchronize(e->stream));  // the host arrays die here
     return BOIDS_OK;
 }
 

@@ -222,3 +222,21 @@ def test_ensemble_route_by_crowding(boids_lib):
             assert_bits_equal(x, y, "flock %d" % f)
     a.close()
     b.close()
+
+
+def test_ensemble_initial_states(boids_lib, oracle_mod):
+    """Flocks drawn side by side (more than 8192 boids in all), of both
+    placements and odd sizes, against the oracle's sequence for each alone."""
+    B, O, prm = boids_lib, oracle_mod, oracle_mod.MARUN2019
+    sizes = (16385, 1, 127, 129, 8000, 30000)
+    flocks = [(B.flock_params(n, 1.3, prm["sep"], prm["ali"], prm["coh"], prm["vmax"], prm["vmin"]),
+               B.INIT_TEST if f % 2 else B.INIT_RANDOM_UNIFORM, 11 * f + 3) for f, n in enumerate(sizes)]
+    e = B.Ensemble(flocks)
+    for _ in range(2):
+        e.init()
+        for f, n in enumerate(sizes):
+            op, ov = O.init_state(make_params(O, n, 1.3, prm), "test" if f % 2 else "random_uniform", True, 11 * f + 3)
+            p, v = e.state(f)
+            assert_bits_equal(p.reshape(-1), op.reshape(-1), "positions of flock %d" % f)
+            assert_bits_equal(v.reshape(-1), ov.reshape(-1), "velocities of flock %d" % f)
+    e.close()
