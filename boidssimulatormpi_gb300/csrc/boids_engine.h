@@ -207,6 +207,9 @@ constexpr uint32_t kWarpBoids = 40960;
 constexpr uint32_t kCrowdBoids = 1u << 18, kCrowdSlots = 1u << 19;
 constexpr double kCrowdTop = 8.5, kCrowdTopSlope = 1.6e-5;
 constexpr double kCrowdBase = 0.47, kCrowdBare = 0.35, kCrowdSlope = 1.75e-6;
+// Up to this many boids and cells (padded) a flock's counting sort is one
+// CTA's work (k_grid_sort, k_grid_bin_one).
+constexpr uint32_t kSortBoids = 1024, kSortCells = 4096;
 // Up to this many boids and cells (padded) the allocation-free step's counting
 // sort is one kernel (k_grid_bin): on the eight SMs of its cluster the scatter
 // of more takes longer than the launches it saves.

@@ -429,10 +429,12 @@ __global__ void k_frame(const float4 *__restrict__ pos4, const float4 *__restric
 // Programmatic dependent launch, in the chains of a small flock's steps: the
 // next kernel's CTAs are set up while this one's last ones run, and wait here
 // for its end (and its writes) before they touch anything.  A kernel launched
-// without the attribute passes straight through.
+// without the attribute passes straight through.  (The next kernel is let in
+// after this one's own wait: letting it in before took 1 to 5 % longer from
+// 1000 to 5000 boids.)
 __device__ __forceinline__ void chain_wait()
 {
-    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // The measure that sends a step's boids to a warp each or to the cells' split:
@@ -584,6 +586,91 @@ __global__ void k_grid_scatter(const float4 *__restrict__ pin, const float4 *__r
     if (count_to_zero) count_to_zero[c] = 0;  // every binned cell, for the next step's keys
 }
 
+// Scan and scatter of a flock of at most kSortBoids boids and kSortCells cells
+// in one CTA: the boids' records are loaded beside the counts, and the scanned
+// starts are read back from shared memory.  The starts in lstart are final
+// (bsum is zero).  Bound by one load, one block scan and one store, where
+// k_grid_scan and k_grid_scatter are six dependent trips to L2 and a launch: a
+// step of 1000 boids of test.ini 20.9 us, 22.7 with those, of 100 boids 13.2
+// (15.9), of 1024 of marun2019.ini 15.9 (17.4).  With two boids a thread and
+// twice the cells 2048 boids gained nothing, with four 4096 lost 20 %.
+constexpr int kSortThreads = kSortBoids;
+static_assert(kSortCells == 4 * kSortThreads, "a thread takes one boid and one vector of counts");
+
+__global__ void __launch_bounds__(kSortThreads)
+k_grid_sort(const float4 *__restrict__ pin, const float4 *__restrict__ vin, const uint32_t *__restrict__ key,
+            const uint32_t *__restrict__ rank, uint32_t *count, uint32_t *__restrict__ lstart,
+            uint32_t *__restrict__ bsum, uint32_t ncell_pad, uint32_t tiles, float4 *__restrict__ pout,
+            float4 *__restrict__ vout, int zero_counts, uint32_t *__restrict__ slot_of, uint32_t n)
+{
+    __shared__ uint32_t warp_tot[kSortThreads / 32];
+    __shared__ __align__(16) uint32_t start[kSortCells];
+    const uint32_t t = threadIdx.x, c0 = 4 * t;
+    chain_wait();
+    uint4 a = make_uint4(0, 0, 0, 0);
+    if (c0 < ncell_pad) a = *reinterpret_cast<const uint4 *>(count + c0);
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), v = p;
+    uint32_t c = 0, r = 0, total;
+    if (t < n) {
+        c = key[t];
+        r = rank[t];
+        p = pin[t];
+        v = vin[t];
+    }
+    const uint32_t run = block_excl_scan<kSortThreads>(a.x + a.y + a.z + a.w, warp_tot, total);
+    if (c0 < ncell_pad) {
+        const uint4 x = make_uint4(run, run + a.x, run + a.x + a.y, run + a.x + a.y + a.z);
+        *reinterpret_cast<uint4 *>(start + c0) = x;
+        *reinterpret_cast<uint4 *>(lstart + c0) = x;
+        if (zero_counts) *reinterpret_cast<uint4 *>(count + c0) = make_uint4(0, 0, 0, 0);  // for the next step's keys
+    }
+    if (t < tiles) bsum[t] = 0;
+    __syncthreads();
+    if (t >= n) return;
+    const uint32_t d = start[c] + r;
+    pout[d] = p;
+    vout[d] = v;
+    slot_of[__float_as_uint(p.w)] = d;
+}
+
+// The allocation-free step's counting sort of as small a flock, from the
+// caller's id-ordered arrays: the counts and ranks never leave shared memory
+// (a step of 1000 boids of test.ini 24 us, 31.5 with k_grid_bin).
+__global__ void __launch_bounds__(kSortThreads)
+k_grid_bin_one(const float *__restrict__ pos3, const float *__restrict__ vel3, uint32_t *__restrict__ lstart,
+               uint32_t *__restrict__ bsum, uint32_t ncell_pad, uint32_t tiles, float4 *__restrict__ pout,
+               float4 *__restrict__ vout, uint32_t *__restrict__ slot_of, StepConst k)
+{
+    __shared__ uint32_t warp_tot[kSortThreads / 32];
+    __shared__ __align__(16) uint32_t start[kSortCells];  // the counts, then the starts
+    const uint32_t t = threadIdx.x, c0 = 4 * t;
+    chain_wait();
+    uint4 &mine = *reinterpret_cast<uint4 *>(start + c0);
+    mine = make_uint4(0, 0, 0, 0);
+    float3 p = make_float3(0.f, 0.f, 0.f), v = p;
+    uint32_t c = 0, r = 0, total;
+    if (t < k.n) {
+        p = make_float3(pos3[3 * t], pos3[3 * t + 1], pos3[3 * t + 2]);
+        v = make_float3(vel3[3 * t], vel3[3 * t + 1], vel3[3 * t + 2]);
+        c = cell_key(p, k);
+    }
+    __syncthreads();
+    if (t < k.n) r = atomicAdd(start + c, 1u);
+    __syncthreads();
+    const uint4 a = mine;
+    const uint32_t run = block_excl_scan<kSortThreads>(a.x + a.y + a.z + a.w, warp_tot, total);
+    const uint4 x = make_uint4(run, run + a.x, run + a.x + a.y, run + a.x + a.y + a.z);
+    mine = x;
+    if (c0 < ncell_pad) *reinterpret_cast<uint4 *>(lstart + c0) = x;
+    if (t < tiles) bsum[t] = 0;
+    __syncthreads();
+    if (t >= k.n) return;
+    const uint32_t d = start[c] + r;
+    pout[d] = make_float4(p.x, p.y, p.z, __uint_as_float(t));
+    vout[d] = make_float4(v.x, v.y, v.z, 0.f);
+    slot_of[t] = d;
+}
+
 // The allocation-free step's counting sort of a small flock in one kernel,
 // from the caller's id-ordered arrays: a cluster of kBinCtas CTAs clears the
 // counts, keys and counts the boids, scans the counts (a contiguous part each,
@@ -591,9 +678,8 @@ __global__ void k_grid_scatter(const float4 *__restrict__ pin, const float4 *__r
 // the boids.  The cell starts in lstart are final (bsum is zero).
 //
 // Bound by the chain of its phases (about 10 us), which replaces a clear and
-// three kernels: the step of 1000 boids of test.ini takes 33 us where it took
-// 47 with those and an unpacking after the rules, of 16 384 gathered boids 62
-// (75).  It pays only from unsorted input: without the first phases it takes
+// three kernels: the step of 16 384 gathered boids takes 59 us where it took
+// 75 with those and an unpacking after the rules.  It pays only from unsorted input: without the first phases it takes
 // as long as k_grid_scan and k_grid_scatter (a handle's step of 1000 boids
 // 29.3 against 28.0 us, of 16 384 57 against 55).
 constexpr int kBinCtas = 8, kBinThreads = 1024;
@@ -610,6 +696,7 @@ k_grid_bin(const float *__restrict__ pos3, const float *__restrict__ vel3, uint3
 {
     __shared__ uint32_t warp_tot[kBinThreads / 32], totals[kBinCtas];
     const uint32_t cta = blockIdx.x, t = threadIdx.x, at = cta * kBinThreads + t;
+    chain_wait();
     constexpr uint32_t kAll = kBinCtas * kBinThreads;
     for (uint32_t c = 4 * at; c < ncell_pad; c += 4 * kAll)
         *reinterpret_cast<uint4 *>(count + c) = make_uint4(0, 0, 0, 0);
@@ -2805,9 +2892,16 @@ cudaError_t launch_grid_keys(const StepConst &k, const float4 *pos, uint32_t *ke
     return cudaGetLastError();
 }
 
+// Whether launch_grid_scatter does the scan's work, too.
+static inline bool grid_sort_small(const StepConst &k, const DevBuffers &b, const FlockTable *ft)
+{
+    return !ft && grid_by_warp(k, b, ft) && k.n <= kSortBoids && b.ncell_pad <= kSortCells;
+}
+
 cudaError_t launch_grid_scan(const StepConst &k, const DevBuffers &b, cudaStream_t st, uint64_t *launches,
                              const FlockTable *ft)
 {
+    if (grid_sort_small(k, b, ft) && k.n) return cudaSuccess;
     cudaError_t e = cudaSuccess;
     const bool by_cells = !grid_by_warp(k, b, ft);
     if (by_cells && ft && b.defer_cnt && (e = cudaMemsetAsync(b.defer_cnt, 0, sizeof(uint32_t) * ft->count, st)) != cudaSuccess)
@@ -2825,7 +2919,10 @@ bool grid_bin_small(const StepConst &k, const DevBuffers &b)
 cudaError_t launch_grid_bin(const StepConst &k, const DevBuffers &b, const float *pos3, const float *vel3,
                             cudaStream_t st, uint64_t *launches)
 {
-    k_grid_bin<<<kBinCtas, kBinThreads, 0, st>>>(pos3, vel3, b.key, b.rank, b.count, b.lstart, b.bsum, b.ncell_pad,
+    if (grid_sort_small(k, b, nullptr))
+        k_grid_bin_one<<<1, kSortThreads, 0, st>>>(pos3, vel3, b.lstart, b.bsum, b.ncell_pad, b.nscan_blocks, b.pos[1],
+                                                   b.vel[1], b.slot_of, k);
+    else k_grid_bin<<<kBinCtas, kBinThreads, 0, st>>>(pos3, vel3, b.key, b.rank, b.count, b.lstart, b.bsum, b.ncell_pad,
                                                  b.nscan_blocks, b.pos[1], b.vel[1], b.slot_of, k);
     *launches += 1;
     return cudaGetLastError();
@@ -2862,6 +2959,12 @@ cudaError_t launch_grid_scatter(const StepConst &k, const DevBuffers &b, int fro
 {
     const uint32_t n = ft ? ft->nslots : k.n;
     if (n == 0) return cudaSuccess;
+    if (grid_sort_small(k, b, ft)) {
+        ++*launches;
+        return launch_chain(true, k_grid_sort, 1, kSortThreads, 0, st, b.pos[from], b.vel[from], b.key, b.rank, b.count,
+                            b.lstart, b.bsum, b.ncell_pad, b.nscan_blocks, b.pos[1 - from], b.vel[1 - from],
+                            (int)zero_counts, b.slot_of, k.n);
+    }
     uint32_t *cz = zero_counts ? b.count : nullptr;
     const Crowd crowd = crowd_route(k, b, ft);
     uint32_t *so = grid_by_warp(k, b, ft) || crowd.pairs ? b.slot_of : nullptr;

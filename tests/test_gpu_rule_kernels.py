@@ -240,3 +240,36 @@ def test_ensemble_initial_states(boids_lib, oracle_mod):
             assert_bits_equal(p.reshape(-1), op.reshape(-1), "positions of flock %d" % f)
             assert_bits_equal(v.reshape(-1), ov.reshape(-1), "velocities of flock %d" % f)
     e.close()
+
+
+@pytest.mark.parametrize("field", [0.21, 0.52, 0.57])  # 4, 10 and 11 cells per axis: 256, 4000 and 5324 in all
+@pytest.mark.parametrize("n", [1, 2, 1023, 1024, 1025])
+def test_one_block_sort_at_its_limits(boids_lib, oracle_mod, n, field):
+    """Flocks on both sides of the one-block counting sort's 1024 boids and
+    4096 cells: a handle's updates and the allocation-free step, twice."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    B, O, prm = boids_lib, oracle_mod, oracle_mod.MARUN2019
+    p = make_params(O, n, field, prm)
+    op, ov = (x.reshape(-1).copy() for x in O.init_state(p, "random_uniform", True, 3))
+    sim = make_sim(B, "grid", n, field, prm)
+    sim.set_state(op, ov)
+    c, h = sim.neighbor_sets()
+    oc, oh = O.neighbor_sets(p, op, ov)
+    assert np.array_equal(c, oc) and np.array_equal(h, oh)
+    prms = B.flock_params(n, field, prm["sep"], prm["ali"], prm["coh"], prm["vmax"], prm["vmin"])
+    a = [torch.from_numpy(x.copy()).cuda() for x in (op, ov)]
+    b = [torch.empty_like(x) for x in a]
+    port = O.GridPort(p, op)
+    for call in range(2):
+        rc = B.lib().boids_step_noalloc(C.byref(prms), a[0].data_ptr(), a[1].data_ptr(), b[0].data_ptr(),
+                                        b[1].data_ptr(), None)
+        assert rc == 0, B.lib().boids_last_error().decode()
+        torch.cuda.synchronize()
+        sim.update(1)
+        port.step(op, ov, 1)
+        for got in ([x.cpu().numpy() for x in b], [np.asarray(x).reshape(-1) for x in sim.state()]):
+            assert_bits_equal(got[0], op, "positions, call %d" % call)
+            assert_bits_equal(got[1], ov, "velocities, call %d" % call)
+        a, b = b, a
+    sim.close()
