@@ -2599,8 +2599,10 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
 // Bound by instruction issue (62 % of the slots, the tensor pipe 57 % active):
 // 1024 pairs take 67 warp instructions, half of them in the 40 % of the steps
 // in which some pair passes, where a box filter on the FP32 offsets took 15.7
-// per pair and thread.  N = 65 536, F = 1.6: 0.39 ms a launch (1.79 before),
-// 1.1e13 pairs/s.  One code path tests the queue: inlined at each of the 32
+// per pair and thread.  N = 65 536, F = 1.6: an update takes 0.415 ms (1.87
+// with that filter), 1.0e13 pairs/s.  Only the j tile of a step in which some
+// pair passed is looked through: 0.427 ms with both, and 0.613 against 0.648
+// at F = 0.9.  One code path tests the queue: inlined at each of the 32
 // results it cost 0.1 ms in instruction fetches.  mma.sync serves better than
 // tcgen05 here: the product is eight deep and every one of its N^2 results has
 // to come back through registers to be compared, so the tensor rate is not
@@ -2686,7 +2688,7 @@ k_ap_pairs(const float4 *__restrict__ pos, const float4 *__restrict__ vel, const
     const uint32_t *bw = reinterpret_cast<const uint32_t *>(sj) + 4 * g + t;
     for (uint32_t jt = 0; jt < jpad; jt += 16) {  // two tiles of 8 j
         float d[2][kApTilesM][4];
-        int all = -1;  // sign set: no pair passed
+        int all[2] = {-1, -1};  // sign set: no pair of the j tile passed
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t b = bw[4 * (jt + 8 * h)];
@@ -2704,17 +2706,22 @@ k_ap_pairs(const float4 *__restrict__ pos, const float4 *__restrict__ vel, const
 #pragma unroll
             for (int m = 0; m < kApTilesM; ++m)
 #pragma unroll
-                for (int r = 0; r < 4; ++r) all &= __float_as_int(d[h][m][r]);
-        if (!__any_sync(kAll, all >= 0)) continue;
+                for (int r = 0; r < 4; ++r) all[h] &= __float_as_int(d[h][m][r]);
+        if (!__any_sync(kAll, (all[0] & all[1]) >= 0)) continue;
         // a bit per result, the first one highest: 0 for a pair that passed
-        uint32_t miss = 0;
+        uint32_t miss = 0xffffffffu;
         static_assert(2 * kApTilesM * 4 == 32, "a lane's results fill a word");
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h) {
+            if (!__any_sync(kAll, all[h] >= 0)) {
+                miss = (miss << 16) | 0xffffu;
+                continue;
+            }
 #pragma unroll
             for (int m = 0; m < kApTilesM; ++m)
 #pragma unroll
                 for (int r = 0; r < 4; ++r) miss = __funnelshift_l(__float_as_uint(d[h][m][r]), miss, 1);
+        }
         for (;;) {  // each lane's next passing pair
             const unsigned hm = __ballot_sync(kAll, ~miss != 0);
             if (!hm) break;
