@@ -132,7 +132,6 @@ constexpr size_t kTcSmem = kTcABytes + kTcBBytes + 1024 + 64;
 constexpr size_t kTcSplitSmem = kTcABytes + 64 * kTcK * 2 + 1024 + 64;  // 64 of the columns
 constexpr uint32_t kTcSpinLimit = 1u << 22;      // bounded wait on the accumulator
 
-__device__ uint32_t g_mlp_tc_error;  // set when a tile's wait gave up (the host reports it)
 
 __host__ __device__ constexpr uint32_t core_off(uint32_t r, uint32_t k)
 {
@@ -178,7 +177,8 @@ static_assert(kTcSplitSmem == kTcABytes + kTcSplit * kTcK * 2 + 1024 + 64, "kTcS
 template <int kN>
 __global__ void __launch_bounds__(kTcThreads, 1)
 k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat16 *__restrict__ wimg,
-                const float *__restrict__ bias, float *__restrict__ pre, __nv_bfloat16 *__restrict__ h)
+                const float *__restrict__ bias, float *__restrict__ pre, __nv_bfloat16 *__restrict__ h,
+                uint32_t *err)
 {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     constexpr uint32_t kB = kN * kTcK * 2;  // its part of the weight image
@@ -252,7 +252,7 @@ k_mlp_hidden_tc(const __nv_bfloat16 *__restrict__ a, int rows, const __nv_bfloat
         done = __syncthreads_and(done);  // one decision for the whole CTA
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (!done) {
-            atomicExch(&g_mlp_tc_error, 1u);
+            *reinterpret_cast<volatile uint32_t *>(err) = 1u;
             ok = false;
             break;
         }
@@ -332,7 +332,7 @@ static_assert(kTcFwdSmem <= 227 * 1024, "one CTA per SM");
 __global__ void __launch_bounds__(kTcFwdThreads, 1)
 k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__restrict__ w1,
                  const float *__restrict__ b1, const __nv_bfloat16 *__restrict__ wimg, const float *__restrict__ b2,
-                 const __nv_bfloat16 *__restrict__ w3, const float *__restrict__ b3, float *__restrict__ y)
+                 const __nv_bfloat16 *__restrict__ w3, const float *__restrict__ b3, float *__restrict__ y, uint32_t *err)
 {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     unsigned char *sa = tc_smem, *sb = tc_smem + kTcABytes;
@@ -444,7 +444,7 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
         done = __syncthreads_and(done);  // one decision for the CTA; the next inputs are in place
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (!done) {
-            atomicExch(&g_mlp_tc_error, 1u);
+            *reinterpret_cast<volatile uint32_t *>(err) = 1u;
             break;
         }
         // the next tile's first layer into the freed buffer, and its product
@@ -1023,6 +1023,7 @@ struct boids_mlp {
           *d2 = nullptr, *d1 = nullptr;
     __nv_bfloat16 *x16 = nullptr, *h1 = nullptr, *h2 = nullptr, *dy16 = nullptr, *d2_16 = nullptr, *d1_16 = nullptr;
     double *loss = nullptr;
+    uint32_t *err = nullptr;  // pinned: set by a tile whose wait gave up
     cudaStream_t st = nullptr;
     __nv_bfloat16 *w2img = nullptr;  // the hidden weights in the tensor-core layout (hidden width 256)
     bool img_valid = false;           // it holds the present parameters' (p16)
@@ -1097,10 +1098,10 @@ void hidden_tc(boids_mlp *m, int rows, const float *b2, float *pre2)
     const unsigned tiles = nb(rows, kTcM), parts = kTcN / kTcSplit;
     if (tiles * parts <= m->nsm)
         launch_chain(m, k_mlp_hidden_tc<kTcSplit>, tiles * parts, kTcThreads, kTcSplitSmem, m->h1, rows, m->w2img, b2,
-                     pre2, m->h2);
+                     pre2, m->h2, m->err);
     else
         launch_chain(m, k_mlp_hidden_tc<kTcN>, tiles < m->nsm ? tiles : m->nsm, kTcThreads, kTcSmem, m->h1, rows,
-                     m->w2img, b2, pre2, m->h2);
+                     m->w2img, b2, pre2, m->h2, m->err);
 }
 
 // One batch of the 8 -> 256 -> 256 -> 4 network in five kernels: rows idx[0..
@@ -1170,16 +1171,14 @@ void backward(boids_mlp *m, int rows)
     k_mlp_colsum<<<m->h, 256, 0, m->st>>>(m->d1, rows, m->h, gb1);
 }
 
-// Waits for the call's work, and for whether a tensor-core tile's wait on its
-// accumulator gave up (the flag is cleared for the next call).
+// Waits for the call's work, and says whether a tensor-core tile's wait on its
+// accumulator gave up (the word is cleared for the next call).  The word lies
+// in pinned host memory, so that looking at it takes no copy (8 us of a call).
 int finish_call(boids_mlp *m)
 {
-    uint32_t err = 0;
-    if (m->w2img) MCK(cudaMemcpyFromSymbolAsync(&err, g_mlp_tc_error, sizeof err, 0, cudaMemcpyDeviceToHost, m->st));
     MCK(cudaStreamSynchronize(m->st));
-    if (!err) return 0;
-    const uint32_t zero = 0;
-    MCK(cudaMemcpyToSymbolAsync(g_mlp_tc_error, &zero, sizeof zero, 0, cudaMemcpyHostToDevice, m->st));
+    if (!m->err || !*reinterpret_cast<volatile uint32_t *>(m->err)) return 0;
+    *m->err = 0;
     return fail(BOIDS_ECUDA, "boids_mlp: a tensor-core tile's wait for its accumulator gave up");
 }
 
@@ -1246,6 +1245,7 @@ int boids_mlp_create(int32_t n_in, int32_t n_hidden, int32_t n_out, uint64_t see
         m->nsm = (unsigned)nsm;
     if (ok && n_hidden == kTcN) {  // the hidden product on the tensor cores
         ok = cudaMalloc(&m->w2img, kTcBBytes) == cudaSuccess &&
+             cudaHostAlloc(&m->err, sizeof *m->err, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess &&
              cudaFuncSetAttribute(k_mlp_hidden_tc<kTcN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem) ==
                  cudaSuccess &&
              cudaFuncSetAttribute(k_mlp_hidden_tc<kTcSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1255,6 +1255,7 @@ int boids_mlp_create(int32_t n_in, int32_t n_hidden, int32_t n_out, uint64_t see
              cudaFuncSetAttribute(k_mlp_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kTcFwdSmem) == cudaSuccess;
     }
+    if (m->err) *m->err = 0;
     if (!ok) {
         cudaGetLastError();
         boids_mlp_destroy(m);
@@ -1273,6 +1274,7 @@ void boids_mlp_destroy(boids_mlp *m)
     void *q[] = {m->p, m->grad, m->m, m->v, m->p16, m->loss, m->w2img};
     for (void *p : q)
         if (p) cudaFree(p);
+    if (m->err) cudaFreeHost(m->err);
     if (m->st) cudaStreamDestroy(m->st);
     delete m;
 }
@@ -1317,7 +1319,7 @@ int boids_mlp_forward(boids_mlp *m, const float *x, int32_t rows, float *y)
         m->img_valid = true;
         const unsigned tiles = nb(rows, kTcM);
         k_mlp_forward_tc<<<tiles < m->nsm ? tiles : m->nsm, kTcFwdThreads, kTcFwdSmem, m->st>>>(
-            m->x, rows, W1, b1, m->w2img, b2, W3, b3, m->y);
+            m->x, rows, W1, b1, m->w2img, b2, W3, b3, m->y, m->err);
     } else {
         if (int rc = upload_rows(m, x, nullptr, rows)) return rc;
         forward(m, rows, false);  // inference: the backward pass's pre-activations are not needed
