@@ -28,7 +28,7 @@ timed state against the CPU baseline's, bit for bit), `trajectory` (the
 workload's whole 1000-update run from its seeded initial state, timed as one
 region, with default thresholds and with one retune), `late_regime` (steps
 after that run, when the flock has gathered), `allpairs` (the all-pairs
-engine's N^2 kernels at N=65536, F=1.6, against the FP32 lane-issue peak),
+engine's N^2 kernels at N=65536, F=1.6),
 `ensemble` (the 256-flock batched sweep) and `surrogate_sweep` (the recorded
 plain vs screened sweep at 16 384 boids and 2000 updates, not timed here).
 
@@ -336,18 +336,20 @@ def cpu_baseline_sample(a, pos, vel, gpu_after=None):
     return out
 
 
-def fp32_lane_peak(sm_mhz, sms):
-    """FP32 lane-instructions per second the SMs can issue: 128 lanes per SM
-    per clock."""
-    return sms * 128 * sm_mhz * 1e6
+def measured_peaks():
+    """The card's measured copy and matrix-product rates ({} where they were not measured)."""
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            return json.load(f)
+    except (OSError, ValueError):
+        return {}
 
 
 def run_allpairs(a, B, local, stream, torch):
     """The all-pairs engine on its own N^2 kernels at N=65536, F=1.6 (the
     same density), the reference's src/boid_simulation.cpp configuration:
-    device time per update, and the pair filter's FP32 rate against the
-    lane-issue peak at the sampled SM clock (10 FP32 operations per ordered
-    pair)."""
+    device time per update, and the rate of the pair filter's matrix product
+    (eight multiply-adds per ordered pair) against the measured BF16 peak."""
     n, field = 65536, 1.6
     m = MARUN2019
     sim = B.BoidSimulation("allpairs", device=local, allpairs_kernels=True)
@@ -368,18 +370,16 @@ def run_allpairs(a, B, local, stream, torch):
     ms = e0.elapsed_time(e1) / steps
     sim.close()
     c = clk.summary()
-    props = torch.cuda.get_device_properties(local)
-    mhz = c["sm_mhz"] or 2070.0
     pairs = float(n) * n
-    achieved = 10 * pairs / (ms / 1e3)
-    peak = fp32_lane_peak(mhz, props.multi_processor_count)
+    achieved = 16 * pairs / (ms / 1e3)
+    measured = measured_peaks().get("bf16_tflops")
+    peak = (measured or 1900.0) * 1e12
     return {"n": n, "field_size": field, "kernels": "all pairs (N^2): k_ap_pairs + k_ap_accumulate",
             "steps": steps, "ms_per_step": ms, "value": n / (ms / 1e3), "unit": UNIT,
-            "roofline": {"bound": "fp32_issue", "achieved": achieved / 1e12, "peak": peak / 1e12,
-                         "unit": "TFLOP/s (FP32 lane operations)", "frac": achieved / peak,
-                         "ops_per_pair": 10, "pairs_per_step": pairs,
-                         "peak_is": "%d SMs x 128 FP32 lanes x %.0f MHz (sampled)"
-                                    % (props.multi_processor_count, mhz)},
+            "roofline": {"bound": "issue (ALU and mma.sync)", "achieved": achieved / 1e12, "peak": peak / 1e12,
+                         "unit": "TFLOP/s (the filter's 8-deep product)", "frac": achieved / peak,
+                         "ops_per_pair": 16, "pairs_per_step": pairs, "pairs_per_s": pairs / (ms / 1e3),
+                         "peak_source": "measured" if measured else "fallback"},
             "clocks": c}
 
 
@@ -546,12 +546,7 @@ def run_ours(a):
     ens = run_ensemble(a, B, rank, dist) if a.ensemble_flocks > 0 else None
     if rank != 0:
         return
-    peaks = {}
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            peaks = json.load(f)
-    except (OSError, ValueError):
-        pass
+    peaks = measured_peaks()
     peak = peaks.get("hbm_gbs")
     peak_src = "measured" if peak else "fallback"
     peak = peak or 6800.0

@@ -11,19 +11,21 @@
 // (src/boid_simulation.cpp:161, src/boid_simulation_grid.cpp:191), so the
 // results are bit-identical to the reference's, not merely close.
 //
-// Grid step = scan of cell counts -> the scatter into cell order, beside the
-// classification of every full-size cell -> rule kernels that split the
-// boids by the occupancy of their cell:
+// Grid step = scan of cell counts -> the scatter into cell order -> the rules.
+// A flock of up to kWarpBoids boids, and a larger one while it is gathered
+// (kCrowdBoids), is updated by k_grid_warp or k_grid_warp_queue, a warp per
+// boid.  Else every full-size cell is classified (beside the scatter) and the
+// boids are split by the occupancy of their cell:
 //   k_grid_sparse  one thread per boid; candidates of the 27 cells around it
 //                  are filtered, exactly tested (the warp's hits dealt to all
 //                  its lanes), and kept sorted by id; boids that need more
 //                  than one pass are queued, with the neighbours their list
 //                  could not keep, for
 //   k_grid_sparse_more, which runs their further passes in full warps beside
-//   k_grid_dense   one CTA per crowded cell; the 27-cell candidates are
-//                  sorted by id once in shared memory, the exact tests mark
-//                  rule masks, and ordered sums walk the masks in id order.
-// Both integrate, write the new state in place of the sorted slot and bin it
+//   k_grid_dense   one CTA per 32 boids of a crowded cell; the 27-cell
+//                  candidates are sorted by id once in shared memory, and a
+//                  warp per boid filters, tests and adds them up in id order.
+// All integrate, write the new state in place of the sorted slot and bin it
 // for the next step (cell key + rank from an atomic count).
 #include "boids_engine.h"
 

@@ -15,9 +15,11 @@
 // memory, and the epilogue reads it back with tcgen05.ld, adds the bias and
 // writes the FP32 pre-activation and the BF16 ReLU.  The other products --
 // the thin input and output layers (K or N of 8 and 4) and the backward
-// pass -- are one strided GEMM kernel on mma.sync m16n8k16 (BF16 operands,
-// FP32 accumulators): small, latency-bound products where a warp-level MMA
-// with operands read straight from L2 is the simplest fast form.
+// pass -- run on mma.sync m16n8k16 (BF16 operands, FP32 accumulators), small,
+// latency-bound products: a training batch of the 8 -> 256 -> 256 -> 4 network
+// is five fused kernels (k_mlp_first, the hidden product, k_mlp_out,
+// k_mlp_back2, k_mlp_back1), another shape's goes through one strided GEMM
+// kernel.
 #include "boids.h"
 
 #include <cuda_bf16.h>

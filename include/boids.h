@@ -189,8 +189,9 @@ int boids_profile_read(boids_sim *sim, boids_profile_t *out, int32_t reset);
  * tune[2] cand_defer  candidates in the cell's 27-cell neighbourhood,
  * tune[3] lone_cand   ... or any boid with over this many candidates.
  * Defaults 16, 4, 192, 96; until they are set (or chosen by boids_autotune),
- * flocks of up to 40960 boids are updated a warp per boid instead, without a
- * split.  No counterpart in the reference. */
+ * flocks of up to 40960 boids, and those of up to 262144 while they are
+ * gathered, are updated a warp per boid instead, without a split.  No
+ * counterpart in the reference. */
 int boids_set_tuning(boids_sim *sim, const int32_t *tune4);
 int boids_get_tuning(boids_sim *sim, int32_t *tune4);
 
