@@ -171,7 +171,7 @@ struct boids_sim {
     };
     StepGraph graphs[2];
     bool graph_off = false;     // capture failed once on this handle
-    // set_state/get_state move the state in kXferChunks pieces of ids; with
+    // set_state/get_state move the state in up to kXferChunks pieces of ids; with
     // the side stream, one piece is packed (or copied out) while the next is
     // copied (or unpacked): one event per piece
     static constexpr int kXferChunks = 4;
@@ -607,10 +607,17 @@ void boids_destroy(boids_sim *s)
 
 namespace {
 
-// First id of transfer piece c (of kXferChunks), on a 1024-id boundary.
-static uint32_t xfer_start(uint32_t n, int c)
+// Pieces of n boids' transfers.  A piece more hides part of the packing under
+// the copies and costs two more copies and an event each way, about 5 us: a
+// set_state, an update and a get_state take, with 1, 2 and 4 pieces, 134, 142
+// and 163 us at 65 537 boids, 413, 419 and 431 at 2^19, 758, 747 and 757 at
+// 2^20, 2895, 2825 and 2808 at 2^22.
+static int xfer_pieces(uint32_t n) { return n <= 3u << 18 ? 1 : (n <= 1u << 21 ? 2 : boids_sim::kXferChunks); }
+
+// First id of transfer piece c (of so many), on a 1024-id boundary.
+static uint32_t xfer_start(uint32_t n, int c, int pieces)
 {
-    const uint64_t b = ((uint64_t)n * (uint32_t)c / boids_sim::kXferChunks + 1023) & ~(uint64_t)1023;
+    const uint64_t b = ((uint64_t)n * (uint32_t)c / (uint32_t)pieces + 1023) & ~(uint64_t)1023;
     return (uint32_t)std::min<uint64_t>(b, n);
 }
 
@@ -618,7 +625,7 @@ static uint32_t xfer_start(uint32_t n, int c)
 // pieces' events exist (made on first use; without them, one piece).
 static bool xfer_pipelined(boids_sim *s)
 {
-    if (!s->b.aux) return false;
+    if (!s->b.aux || xfer_pieces(s->k.n) == 1) return false;
     for (cudaEvent_t &ev : s->xfer_ev)
         if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
             ev = nullptr;
@@ -658,9 +665,9 @@ static int set_state_n(boids_sim *s, const float *pos3n, const float *vel3n)
         // grid, so a state that fails the range check only wastes it) on
         // the side stream while the next piece is copied
         cudaStream_t ps = pipe ? s->b.aux : s->stream;
-        const int pieces = pipe ? boids_sim::kXferChunks : 1;
+        const int pieces = pipe ? xfer_pieces(n) : 1;
         for (int c = 0; c < pieces; ++c) {
-            const uint32_t i0 = pipe ? xfer_start(n, c) : 0, i1 = pipe ? xfer_start(n, c + 1) : n;
+            const uint32_t i0 = xfer_start(n, c, pieces), i1 = xfer_start(n, c + 1, pieces);
             if (i1 <= i0) continue;
             const size_t off = (size_t)3 * i0, bytes = sizeof(float) * 3 * (size_t)(i1 - i0);
             CK(cudaMemcpyAsync(dpos + off, pos3n + off, bytes, cudaMemcpyHostToDevice, s->stream));
@@ -883,9 +890,9 @@ int boids_get_state(boids_sim *s, float *pos3n, float *vel3n)
         // each piece is unpacked on the engine's stream and copied out on
         // the side stream while the next piece is unpacked
         cudaStream_t cs = pipe ? s->b.aux : s->stream;
-        const int pieces = pipe ? boids_sim::kXferChunks : 1;
+        const int pieces = pipe ? xfer_pieces(n) : 1;
         for (int c = 0; c < pieces; ++c) {
-            const uint32_t i0 = pipe ? xfer_start(n, c) : 0, i1 = pipe ? xfer_start(n, c + 1) : n;
+            const uint32_t i0 = xfer_start(n, c, pieces), i1 = xfer_start(n, c + 1, pieces);
             if (i1 <= i0) continue;
             const size_t off = (size_t)3 * i0, bytes = sizeof(float) * 3 * (size_t)(i1 - i0);
             CK(boidsgpu::launch_unpack_gather(p4, v4, slot_of, dpos, dvel, i0, i1, n, s->stream, &s->launches));

@@ -273,3 +273,26 @@ def test_one_block_sort_at_its_limits(boids_lib, oracle_mod, n, field):
             assert_bits_equal(got[1], ov, "velocities, call %d" % call)
         a, b = b, a
     sim.close()
+
+
+@pytest.mark.parametrize("n", [1, 1025, 786432, 786433, (1 << 21) + 1])
+def test_state_round_trip_in_pieces(boids_lib, n):
+    """set_state and get_state on both sides of the sizes at which they move
+    the state in one, two and four pieces, the bad coordinate in the last
+    piece included."""
+    B = boids_lib
+    prm = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008), vmax=0.005, vmin=0.001)
+    field = max(0.3, (n / 16384) ** (1 / 3))
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(0, field * 0.999, 3 * n).astype(np.float32)
+    vel = rng.uniform(-0.003, 0.003, 3 * n).astype(np.float32)
+    sim = make_sim(B, "grid", n, field, prm, record_forces=False)
+    sim.set_state(pos, vel)
+    p, v = sim.state()
+    assert_bits_equal(np.asarray(p).reshape(-1), pos, "positions")
+    assert_bits_equal(np.asarray(v).reshape(-1), vel, "velocities")
+    bad = pos.copy()
+    bad[-1] = field * 1.5
+    with pytest.raises(B.BoidsError):
+        sim.set_state(bad, vel)
+    sim.close()
