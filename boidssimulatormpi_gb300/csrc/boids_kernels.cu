@@ -855,13 +855,12 @@ __global__ void k_grid_classify(const uint32_t *__restrict__ lstart,
 // warps.  The per-boid tables (segments, hit buffer, sorted list) live in
 // shared memory, one column per thread: as local memory they overflow L1 and
 // every access goes to L2.
-constexpr int kBufA = 13;
+constexpr int kBufA = 16;     // (13 flushed more often: 170 us a step of 262 143 boids for 167; 18 costs two CTAs an SM)
 constexpr int kListA = kListCap;
-constexpr int kRT = 128;      // threads of k_grid_sparse
+constexpr int kRT = 128;      // threads of k_grid_sparse_more
 constexpr int kSegA = 18;     // at most 9 rows x 2 runs (a run split where x wraps)
 // Candidates loaded together in the filter loop: 3 keeps the kernel within
-// 80 registers (6 CTAs per SM, as the shared tables allow) and is 1-2 %
-// faster than 2; 4 takes 96 registers, 5 CTAs per SM, and is 6 % slower.
+// 80 registers; with 2 a step was 1-2 % slower, with 4 (96 registers) 4 %.
 constexpr int kCandStep = 3;
 static_assert(kBufA > kCandStep, "the hit buffer holds an iteration's hits");
 
@@ -876,15 +875,15 @@ struct GridIn {
     int chain;  // k_grid_sparse and k_grid_dense were launched in a chain
 };
 
-struct SparseSmem {
-    uint32_t seg0[kSegA][kRT];   // first slot | x shift << 29 | (z shift < 0) << 31
-    uint32_t seg1[kSegA][kRT];   // end slot   | y shift << 29 | (z shift > 0) << 31
-    uint32_t buf[kBufA][kRT];    // filter hits: slot | shifted << 31
-    uint64_t lst[kListA][kRT];   // accepted neighbours, sorted: id << 32 | slot | flags << 29
+struct SparseSmem {              // of one warp, a column per lane
+    uint32_t seg0[kSegA][32];    // first slot | x shift << 29 | (z shift < 0) << 31
+    uint32_t seg1[kSegA][32];    // end slot   | y shift << 29 | (z shift > 0) << 31
+    uint32_t buf[kBufA][32];     // filter hits: slot | shifted << 31
+    uint64_t lst[kListA][32];    // accepted neighbours, sorted: id << 32 | slot | flags << 29
 };
 
 // The segments of the boid at pi, whose full-size cell is (cy, cz) along y
-// and z, into the thread's columns of sm.seg0/seg1: in each neighbour row,
+// and z, into the lane's columns of sm.seg0/seg1: in each neighbour row,
 // the x cells that a sphere of radius sqrt(trim_r2) around it reaches.
 // Empty runs are not stored.  Returns the number of candidates.
 __device__ __forceinline__ uint32_t sparse_segments(SparseSmem &sm, int t, float3 pi, int cy, int cz,
@@ -1021,7 +1020,7 @@ __device__ __forceinline__ uint32_t sparse_segments_ahead(SparseSmem &sm, int t,
     return ncand;
 }
 
-// The m neighbours of the thread's column of sm.lst (sorted by id) added to
+// The m neighbours of the lane's column of sm.lst (sorted by id) added to
 // a in that order, each entry's loads issued one entry ahead.
 template <bool DIAG>
 __device__ __forceinline__ void list_accumulate(const SparseSmem &sm, int t, int m, float3 pi, Acc &a,
@@ -1051,7 +1050,7 @@ __device__ __forceinline__ void list_accumulate(const SparseSmem &sm, int t, int
 // One pass of a warp (all lanes call it together) over the candidates of its
 // lanes that still need one: the filter, the exact tests of the buffered
 // hits, and the accepted neighbours with ids above lo_id kept sorted in the
-// thread's column of sm.lst, at most kListA.  Those lanes then accumulate
+// lane's column of sm.lst, at most kListA.  Those lanes then accumulate
 // their list; a lane that accepted more than the list held keeps need and
 // moves lo_id up to the last id it accumulated.  With ovf (this lane's row),
 // every accepted neighbour that leaves the list or never enters it is
@@ -1123,7 +1122,7 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
             // for as many rounds; each verdict goes back into the finder's
             // buffer (slot | rules << 29, rules 0: not accepted), and each
             // lane then files its own accepted hits in its sorted list.
-            const int lane = t & 31, wbase = t & ~31;
+            const int lane = t;
             int incl = nb;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1152,7 +1151,7 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
                 so.inv_nv = __shfl_sync(0xffffffffu, sight.inv_nv, L);
                 const int olo = __shfl_sync(0xffffffffu, lo32, L);
                 if (i < total) {
-                    const uint32_t wb = sm.buf[q][wbase + L];
+                    const uint32_t wb = sm.buf[q][L];
                     const uint32_t jb = wb & 0x7fffffffu;
                     const float4 pj = __ldg(g.pos + jb);
                     int f = 0;
@@ -1162,7 +1161,7 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
                         const float3 tt = (wb >> 31) ? image3(xyz(pj), po, k) : xyz(pj);
                         f = pair_flags(po, so, tt, k);
                     }
-                    sm.buf[q][wbase + L] = jb | ((uint32_t)f << 29);
+                    sm.buf[q][L] = jb | ((uint32_t)f << 29);
                 }
             }
             __syncwarp();  // the verdicts are written
@@ -1202,7 +1201,7 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
 
 // A deferred boid's further passes from its overflow row (on <= kOvfCap
 // entries, every accepted neighbour with an id above lo_id): the next
-// kListA ids sorted in the thread's column of sm.lst and accumulated, until
+// kListA ids sorted in the lane's column of sm.lst and accumulated, until
 // none is left.  Per lane; no candidate is walked again.
 template <bool DIAG>
 __device__ __forceinline__ void ovf_passes(SparseSmem &sm, int t, const uint64_t *__restrict__ row, uint32_t on,
@@ -1228,55 +1227,36 @@ __device__ __forceinline__ void ovf_passes(SparseSmem &sm, int t, const uint64_t
     }
 }
 
+// One warp a CTA, so that a warp's tables are free for the next as soon as it
+// is done (and those whose boids all lie in dense cells are gone at once):
+// against CTAs of four warps, which packed the boids outside dense cells into
+// full warps, a step of 262 143 boids takes 167 us (172, uniform), of 2^20 420
+// (415, uniform), 711 (737) 20 updates later, 1593 (1701) after 100 and 2068
+// (2178) after 400.  With the system's 1 KB per CTA 21 warps fit an SM (24).
 template <bool DIAG, bool MULTI>
-__global__ void __launch_bounds__(kRT)
+__global__ void __launch_bounds__(32)
 k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
 {
-    static_assert(kRT == kSlotAlign, "a CTA serves one flock");
+    static_assert(kSlotAlign % 32 == 0, "a CTA serves one flock");
     __shared__ SparseSmem sm;
     // the flock's constants (an ensemble's CTA serves one flock); one word otherwise
     __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
     StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
     if (g.chain) chain_wait();
-    if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x]);
+    if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * 32 / kSlotAlign]);
     const StepConst &k = MULTI ? kf : kp;
-    const int G = k.G;
-    const int t = threadIdx.x;
-    const int lane = t & 31, wid = t >> 5;
+    const int lane = threadIdx.x;
     const unsigned below = (1u << lane) - 1u;
-    // This CTA's boids outside dense cells (the others are k_grid_dense's),
-    // compacted onto its first threads so that warps run full and the
-    // warps left over exit at once.
-    // (cslot[t] is read only by thread t before it first writes its own
-    // buffer column, which cslot shares)
-    uint32_t *cslot = sm.buf[0];
-    __shared__ uint32_t wcount[kRT / 32];
-    const uint32_t s0 = blockIdx.x * kRT + t;
-    bool mine = s0 - k.slot_base < k.n;
-    const float4 q = mine ? g.pos[s0] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (mine) {
-        const uint32_t fc = k.cell_base / 4 +
-                            (uint32_t)((cell1(q.z, k) * G + cell1(q.y, k)) * G + cell1(q.x, k));
-        mine = !__ldg(g.dflag + fc);
-    }
-    const unsigned bal = __ballot_sync(0xffffffffu, mine);
-    if (lane == 0) wcount[wid] = __popc(bal);
-    __syncthreads();
-    uint32_t before = 0, total = 0;
-#pragma unroll
-    for (int i = 0; i < kRT / 32; ++i) {
-        if (i < wid) before += wcount[i];
-        total += wcount[i];
-    }
-    if (mine) cslot[before + __popc(bal & below)] = s0;
-    __syncthreads();
-    if ((uint32_t)(wid * 32) >= total) return;  // the whole warp is idle
-    const bool act = (uint32_t)t < total;
-    const uint32_t s = act ? cslot[t] : s0;
+    // this warp's boids outside dense cells (the others are k_grid_dense's)
+    const uint32_t s = blockIdx.x * 32 + lane;
+    bool act = s - k.slot_base < k.n;
     const float4 p4 = act ? g.pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 v4 = act ? g.vel[s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float3 pi = xyz(p4);
-    const uint32_t nc = act ? sparse_segments(sm, t, pi, cell1(pi.y, k), cell1(pi.z, k), g, k) : 0;
+    const int cy = cell1(pi.y, k), cz = cell1(pi.z, k);
+    if (act) act = !__ldg(g.dflag + (k.cell_base / 4 + (uint32_t)((cz * k.G + cy) * k.G + cell1(pi.x, k))));
+    if (!__any_sync(0xffffffffu, act)) return;
+    const uint32_t nc = act ? sparse_segments(sm, lane, pi, cy, cz, g, k) : 0;
     const Sight sight = make_sight(xyz(v4));
     const float dot_lim = k.cone_pre ? -(sight.nv * k.dot_eps) : -INFINITY;  // cone pre-test
     Acc a;
@@ -1284,7 +1264,7 @@ k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
     int64_t lo_id = -1;  // ids <= lo_id were accumulated by earlier passes
     bool need = act;
     uint32_t ovf_n = 0;
-    sparse_pass<DIAG>(sm, t, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k,
+    sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k,
                       o.ovf && act ? o.ovf + (size_t)s * kOvfCap : nullptr, ovf_n);
     if (o.defer) {
         // Boids with more accepted neighbours than one list holds go to
@@ -1307,7 +1287,7 @@ k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
         return;
     }
     while (__any_sync(0xffffffffu, need))
-        sparse_pass<DIAG>(sm, t, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n);
+        sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n);
     if (act) finish_boid<DIAG>(a, p4, sight.v, s, o, k);
 }
 
@@ -1320,10 +1300,11 @@ template <bool DIAG, bool MULTI>
 __global__ void __launch_bounds__(kRT)
 k_grid_sparse_more(GridIn g, GridOut o, StepConst kp, FlockTable ft)
 {
-    __shared__ SparseSmem sm;
+    __shared__ SparseSmem wsm[kRT / 32];
     __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
     StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31;
+    SparseSmem &sm = wsm[t >> 5];
     uint32_t first = 0, count, stride;  // entries [first + base, first + count), base += stride
     uint32_t base = blockIdx.x * kRT;
     if (MULTI) {
@@ -1357,14 +1338,14 @@ k_grid_sparse_more(GridIn g, GridOut o, StepConst kp, FlockTable ft)
         // candidates again
         const uint32_t on = act && o.ovf ? o.ovf_n[s] : (uint32_t)kOvfCap + 1;
         const bool from_row = on <= (uint32_t)kOvfCap;
-        if (from_row) ovf_passes<DIAG>(sm, t, o.ovf + (size_t)s * kOvfCap, on, lo_id, pi, a, g, k);
+        if (from_row) ovf_passes<DIAG>(sm, lane, o.ovf + (size_t)s * kOvfCap, on, lo_id, pi, a, g, k);
         bool need = act && !from_row;
-        const uint32_t nc = need ? sparse_segments_ahead(sm, t, pi, cell1(pi.y, k), cell1(pi.z, k), g, k) : 0;
+        const uint32_t nc = need ? sparse_segments_ahead(sm, lane, pi, cell1(pi.y, k), cell1(pi.z, k), g, k) : 0;
         const Sight sight = make_sight(xyz(v4));
         const float dot_lim = k.cone_pre ? -(sight.nv * k.dot_eps) : -INFINITY;
         uint32_t ovf_n = 0;
         while (__any_sync(0xffffffffu, need))
-            sparse_pass<DIAG>(sm, t, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n);
+            sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n);
         if (act) finish_boid<DIAG>(a, p4, sight.v, s, o, k);
     }
 }
@@ -3096,7 +3077,7 @@ cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, co
         if (e != cudaSuccess) return e;
     }
     if (b.aux && (e = cudaStreamWaitEvent(st, b.cjoin, 0)) != cudaSuccess) return e;  // the classification
-    if ((e = launch_chain(g.chain, k_grid_sparse<DIAG, MULTI>, nsp, kRT, 0, st, g, o, k, ft)) != cudaSuccess) return e;
+    if ((e = launch_chain(g.chain, k_grid_sparse<DIAG, MULTI>, nsp * (kRT / 32), 32, 0, st, g, o, k, ft)) != cudaSuccess) return e;
     const unsigned nmore = MULTI ? nsp : min(nsp, 2 * b.dense_grid);
     if (o.defer && b.aux) {
         // the deferred boids and the dense cells are disjoint: run them side by side
