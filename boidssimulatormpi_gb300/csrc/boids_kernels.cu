@@ -855,7 +855,7 @@ __global__ void k_grid_classify(const uint32_t *__restrict__ lstart,
 // warps.  The per-boid tables (segments, hit buffer, sorted list) live in
 // shared memory, one column per thread: as local memory they overflow L1 and
 // every access goes to L2.
-constexpr int kBufA = 16;     // (13 flushed more often: 170 us a step of 262 143 boids for 167; 18 costs two CTAs an SM)
+constexpr int kBufA = 16;     // (13: 172 us a step of 262 143 boids for 167; 18 and more: 23 warps on an SM)
 constexpr int kListA = kListCap;
 constexpr int kRT = 128;      // threads of k_grid_sparse_more
 constexpr int kSegA = 18;     // at most 9 rows x 2 runs (a run split where x wraps)
@@ -878,7 +878,7 @@ struct GridIn {
 struct SparseSmem {              // of one warp, a column per lane
     uint32_t seg0[kSegA][32];    // first slot | x shift << 29 | (z shift < 0) << 31
     uint32_t seg1[kSegA][32];    // end slot   | y shift << 29 | (z shift > 0) << 31
-    uint32_t buf[kBufA][32];     // filter hits: slot | shifted << 31
+    uint16_t buf[kBufA][32];     // filter hits: offset in the segment | segment << 8 | rules << 13
     uint64_t lst[kListA][32];    // accepted neighbours, sorted: id << 32 | slot | flags << 29
 };
 
@@ -1058,7 +1058,8 @@ __device__ __forceinline__ void list_accumulate(const SparseSmem &sm, int t, int
 template <bool DIAG>
 __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, float3 pi, const Sight &sight,
                                             float dot_lim, uint32_t nc, bool &need, int64_t &lo_id, Acc &a,
-                                            const GridIn &g, const StepConst &k, uint64_t *ovf, uint32_t &ovf_n)
+                                            const GridIn &g, const StepConst &k, uint64_t *ovf, uint32_t &ovf_n,
+                                            bool &moved)
 {
     const float3 vi = sight.v;
     const uint32_t mine = need ? nc : 0;
@@ -1067,7 +1068,8 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
     uint32_t more = 0;  // accepted neighbours with id > lo_id in this pass
     int qs = -1;
     uint32_t j = 0, jend = 0;  // global slots [j, jend) of the current segment
-    uint32_t swrap = 0;        // 1 << 31 when the segment crosses a periodic face
+    moved = false;
+    uint32_t tag = 0;          // the segment << 8, plus the offset of slot j in it
     float qx = 0.f, qy = 0.f, qz = 0.f;
     // the next segment (none is empty): its slots and the query point
     auto advance = [&]() {
@@ -1081,19 +1083,19 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
         qx = __fmaf_rn(-__int2float_rn(vx), k.Ff, pi.x);
         qy = __fmaf_rn(-__int2float_rn(vy), k.Ff, pi.y);
         qz = __fmaf_rn(-__int2float_rn(vz), k.Ff, pi.z);
-        swrap = ((w0 | w1) & 0xe0000000u) ? 0x80000000u : 0u;
+        tag = (uint32_t)qs << 8;
     };
-    auto filter = [&](float4 pj, float3 q, uint32_t jc, uint32_t wrap) {
+    auto filter = [&](float4 pj, float3 q, uint32_t jc, uint32_t entry) {
         const float dx = pj.x - q.x, dy = pj.y - q.y, dz = pj.z - q.z;
         const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
         const float dv = __fmaf_rn(vi.z, dz, __fmaf_rn(vi.y, dy, __fmul_rn(vi.x, dx)));
-        if (d2 < k.filt_r2 && dv >= dot_lim && jc != s) sm.buf[nb++][t] = jc | wrap;
+        if (d2 < k.filt_r2 && dv >= dot_lim && jc != s) sm.buf[nb++][t] = (uint16_t)entry;
     };
     // kCandStep candidates per iteration, so that their loads are in flight
     // together; the buffers are flushed with room for the next kCandStep hits
     for (uint32_t it = 0; it < max_nc; it += kCandStep) {
         bool vc[kCandStep];
-        uint32_t cc[kCandStep], sc[kCandStep];  // candidate slots and their wrap flags
+        uint32_t cc[kCandStep], sc[kCandStep];  // candidate slots and their buffer entries
         float3 qc[kCandStep];
         float4 pc[kCandStep];
 #pragma unroll
@@ -1106,7 +1108,7 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
                 if (j == jend) advance();
                 cc[u] = j++;
                 qc[u] = make_float3(qx, qy, qz);
-                sc[u] = swrap;
+                sc[u] = tag++;
             }
         }
 #pragma unroll
@@ -1115,7 +1117,8 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
         for (int u = 0; u < kCandStep; ++u)
             if (vc[u]) filter(pc[u], qc[u], cc[u], sc[u]);
         // exact tests of the buffered hits, the whole warp together
-        if (__any_sync(0xffffffffu, nb > kBufA - kCandStep) || it + kCandStep >= max_nc) {
+        const bool far = (tag & 255u) >= 256u - kCandStep;  // the offsets are about to run out
+        if (__any_sync(0xffffffffu, nb > kBufA - kCandStep || far) || it + kCandStep >= max_nc) {
             // The warp's hits are tested 32 at a time whatever lane found
             // them (hit i of the lanes' buffers laid end to end goes to lane
             // i % 32), so that a lane with many hits does not hold the warp
@@ -1152,23 +1155,24 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
                 const int olo = __shfl_sync(0xffffffffu, lo32, L);
                 if (i < total) {
                     const uint32_t wb = sm.buf[q][L];
-                    const uint32_t jb = wb & 0x7fffffffu;
-                    const float4 pj = __ldg(g.pos + jb);
+                    const uint32_t w0 = sm.seg0[wb >> 8][L], w1 = sm.seg1[wb >> 8][L];
+                    const float4 pj = __ldg(g.pos + ((w0 & 0x1fffffffu) + (wb & 255u)));
                     int f = 0;
                     if ((int)__float_as_uint(pj.w) > olo) {
                         // a filter hit from a segment without periodic shift is
                         // nearer than F/2 on every axis: its own minimum image
-                        const float3 tt = (wb >> 31) ? image3(xyz(pj), po, k) : xyz(pj);
+                        const float3 tt = ((w0 | w1) & 0xe0000000u) ? image3(xyz(pj), po, k) : xyz(pj);
                         f = pair_flags(po, so, tt, k);
                     }
-                    sm.buf[q][L] = jb | ((uint32_t)f << 29);
+                    sm.buf[q][L] = (uint16_t)(wb | ((uint32_t)f << 13));
                 }
             }
             __syncwarp();  // the verdicts are written
             for (int q = 0; q < nb; ++q) {
-                const uint32_t en = sm.buf[q][t];
-                if (!(en >> 29)) continue;
-                const uint32_t jb = en & 0x1fffffffu;
+                const uint32_t hit = sm.buf[q][t];
+                if (!(hit >> 13)) continue;
+                const uint32_t jb = (sm.seg0[(hit >> 8) & 31u][t] & 0x1fffffffu) + (hit & 255u);
+                const uint32_t en = jb | ((hit >> 13) << 29);
                 const uint32_t idj = __float_as_uint(__ldg(&g.pos[jb].w));
                 ++more;
                 const uint64_t e = ((uint64_t)idj << 32) | (uint64_t)en;
@@ -1190,6 +1194,11 @@ __device__ __forceinline__ void sparse_pass(SparseSmem &sm, int t, uint32_t s, f
             }
             __syncwarp();  // the buffers are free for the next hits
             nb = 0;
+            if (far) {  // the segment goes on from here
+                sm.seg0[qs][t] += tag & 255u;
+                tag &= ~255u;
+                moved = true;
+            }
         }
     }
     if (need) {
@@ -1228,20 +1237,23 @@ __device__ __forceinline__ void ovf_passes(SparseSmem &sm, int t, const uint64_t
 }
 
 // One warp a CTA, so that a warp's tables are free for the next as soon as it
-// is done (and those whose boids all lie in dense cells are gone at once):
-// against CTAs of four warps, which packed the boids outside dense cells into
-// full warps, a step of 262 143 boids takes 167 us (172, uniform), of 2^20 420
-// (415, uniform), 711 (737) 20 updates later, 1593 (1701) after 100 and 2068
-// (2178) after 400.  With the system's 1 KB per CTA 21 warps fit an SM (24).
+// is done (and those whose boids all lie in dense cells are gone at once), and
+// tables small enough for 24 of them on an SM (with the system's 1 KB each):
+// a hit is an offset of 8 bits in a segment, and a segment that goes on beyond
+// 255 slots is moved on behind a flush.  Against CTAs of four warps with whole
+// slots in their buffers a step takes, us: 262 143 boids 167 (172), 2^20 one
+// update after a uniform start 377 (374), 6 after 406 (414), 20 after 803
+// (847), 100 after 1600 (1701), 400 after 2075 (2178), 2^22 4 after 1390 (1425).
+// (With whole slots in one warp's buffer, 21 on an SM: 420 after 6.)
 template <bool DIAG, bool MULTI>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(32, 24)
 k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
 {
     static_assert(kSlotAlign % 32 == 0, "a CTA serves one flock");
-    __shared__ SparseSmem sm;
-    // the flock's constants (an ensemble's CTA serves one flock); one word otherwise
-    __shared__ __align__(8) uint32_t kf_words[MULTI ? sizeof(StepConst) / 4 : 1];
-    StepConst &kf = *reinterpret_cast<StepConst *>(kf_words);
+    // the tables, and an ensemble's flock's constants
+    __shared__ __align__(16) unsigned char smem[sizeof(SparseSmem) + (MULTI ? sizeof(StepConst) : 0)];
+    SparseSmem &sm = *reinterpret_cast<SparseSmem *>(smem);
+    StepConst &kf = *reinterpret_cast<StepConst *>(smem + (MULTI ? sizeof(SparseSmem) : 0));
     if (g.chain) chain_wait();
     if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * 32 / kSlotAlign]);
     const StepConst &k = MULTI ? kf : kp;
@@ -1256,7 +1268,7 @@ k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
     const int cy = cell1(pi.y, k), cz = cell1(pi.z, k);
     if (act) act = !__ldg(g.dflag + (k.cell_base / 4 + (uint32_t)((cz * k.G + cy) * k.G + cell1(pi.x, k))));
     if (!__any_sync(0xffffffffu, act)) return;
-    const uint32_t nc = act ? sparse_segments(sm, lane, pi, cy, cz, g, k) : 0;
+    uint32_t nc = act ? sparse_segments(sm, lane, pi, cy, cz, g, k) : 0;
     const Sight sight = make_sight(xyz(v4));
     const float dot_lim = k.cone_pre ? -(sight.nv * k.dot_eps) : -INFINITY;  // cone pre-test
     Acc a;
@@ -1264,8 +1276,9 @@ k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
     int64_t lo_id = -1;  // ids <= lo_id were accumulated by earlier passes
     bool need = act;
     uint32_t ovf_n = 0;
+    bool moved;
     sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k,
-                      o.ovf && act ? o.ovf + (size_t)s * kOvfCap : nullptr, ovf_n);
+                      o.ovf && act ? o.ovf + (size_t)s * kOvfCap : nullptr, ovf_n, moved);
     if (o.defer) {
         // Boids with more accepted neighbours than one list holds go to
         // k_grid_sparse_more with their partial sums: every further pass
@@ -1286,8 +1299,10 @@ k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
         }
         return;
     }
-    while (__any_sync(0xffffffffu, need))
-        sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n);
+    while (__any_sync(0xffffffffu, need)) {
+        if (moved) nc = sparse_segments(sm, lane, pi, cy, cz, g, k);
+        sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n, moved);
+    }
     if (act) finish_boid<DIAG>(a, p4, sight.v, s, o, k);
 }
 
@@ -1340,12 +1355,15 @@ k_grid_sparse_more(GridIn g, GridOut o, StepConst kp, FlockTable ft)
         const bool from_row = on <= (uint32_t)kOvfCap;
         if (from_row) ovf_passes<DIAG>(sm, lane, o.ovf + (size_t)s * kOvfCap, on, lo_id, pi, a, g, k);
         bool need = act && !from_row;
-        const uint32_t nc = need ? sparse_segments_ahead(sm, lane, pi, cell1(pi.y, k), cell1(pi.z, k), g, k) : 0;
+        uint32_t nc = need ? sparse_segments_ahead(sm, lane, pi, cell1(pi.y, k), cell1(pi.z, k), g, k) : 0;
         const Sight sight = make_sight(xyz(v4));
         const float dot_lim = k.cone_pre ? -(sight.nv * k.dot_eps) : -INFINITY;
         uint32_t ovf_n = 0;
-        while (__any_sync(0xffffffffu, need))
-            sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n);
+        bool moved = false;
+        while (__any_sync(0xffffffffu, need)) {
+            if (moved) nc = sparse_segments_ahead(sm, lane, pi, cell1(pi.y, k), cell1(pi.z, k), g, k);
+            sparse_pass<DIAG>(sm, lane, s, pi, sight, dot_lim, nc, need, lo_id, a, g, k, nullptr, ovf_n, moved);
+        }
         if (act) finish_boid<DIAG>(a, p4, sight.v, s, o, k);
     }
 }

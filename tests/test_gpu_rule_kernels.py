@@ -296,3 +296,28 @@ def test_state_round_trip_in_pieces(boids_lib, n):
     with pytest.raises(B.BoidsError):
         sim.set_state(bad, vel)
     sim.close()
+
+
+@pytest.mark.parametrize("m", [254, 257, 600])
+def test_long_segments_thread_per_boid(boids_lib, oracle_mod, m):
+    """Runs of candidates longer than a buffer entry's offset, several passes
+    per boid, in an ensemble (whose passes follow one another in one kernel)."""
+    B, O, prm = boids_lib, oracle_mod, oracle_mod.MARUN2019
+    sizes = (m + 40, 200)
+    flocks = [(B.flock_params(n, FIELD, prm["sep"], prm["ali"], prm["coh"], prm["vmax"], prm["vmin"]),
+               B.INIT_RANDOM_UNIFORM, 1) for n in sizes]
+    e = B.Ensemble(flocks)
+    e.init()
+    e.set_tuning(*(1 << 30,) * 4)
+    want = []
+    for f, n in enumerate(sizes):
+        pos, vel = crowd_state(m if f == 0 else 100, n - (m if f == 0 else 100), 0.35, f)
+        e.set_state(f, pos, vel)
+        p = make_params(O, n, FIELD, prm)
+        O.GridPort(p, pos).step(pos, vel, 1)
+        want.append((pos, vel))
+    e.step(1)
+    for f in range(len(sizes)):
+        for x, y in zip(e.state(f), want[f]):
+            assert_bits_equal(x.reshape(-1), y, "flock %d" % f)
+    e.close()
