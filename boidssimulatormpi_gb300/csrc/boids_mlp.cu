@@ -1366,27 +1366,47 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
     if (int rc = ensure_rows(m, rows + batch)) return rc;
     // the whole set stays resident: rows [0, rows) of x/t; batches are gathered behind it
     float *X = m->x, *T = m->t;
-    MCK(cudaMemcpyAsync(X, x, sizeof(float) * (size_t)rows * m->in, cudaMemcpyHostToDevice, m->st));
-    MCK(cudaMemcpyAsync(T, t, sizeof(float) * (size_t)rows * m->out, cudaMemcpyHostToDevice, m->st));
     int *d_idx = nullptr;
     float *bx = nullptr, *bt = nullptr;
+    // An epoch's order lies in one of two host arrays, and its copy may read the
+    // array as late as the stream comes to it: `sent` says when it has, and the
+    // array is rewritten after that.  With two, an epoch's order is drawn and
+    // queued while the last one's is still waiting to be sent.
+    std::vector<int> order[2] = {std::vector<int>(rows), std::vector<int>(rows)};
+    cudaEvent_t sent[2] = {nullptr, nullptr};
+    auto release = [&]() {
+        for (cudaEvent_t ev : sent)
+            if (ev) cudaEventDestroy(ev);
+        cudaFree(d_idx);
+        cudaFree(bx);
+        cudaFree(bt);
+    };
     if (cudaMalloc(&d_idx, sizeof(int) * rows) != cudaSuccess ||
         cudaMalloc(&bx, sizeof(float) * (size_t)batch * m->in) != cudaSuccess ||
         cudaMalloc(&bt, sizeof(float) * (size_t)batch * m->out) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(d_idx);
-        cudaFree(bx);
+        release();
         return fail(BOIDS_ENOMEM, "boids_mlp_train: cudaMalloc failed");
     }
-    std::vector<int> idx(rows);
-    for (int i = 0; i < rows; ++i) idx[i] = i;
+    for (int i = 0; i < rows; ++i) order[1][i] = i;
     uint64_t s = shuffle_seed;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     double epoch_loss = 0.0;
     int rc = 0;
     float *keep_x = m->x, *keep_t = m->t;
     const bool fused = batch_is_fused(m);
+    if (cudaEventCreateWithFlags(&sent[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&sent[1], cudaEventDisableTiming) != cudaSuccess ||
+        cudaMemcpyAsync(X, x, sizeof(float) * (size_t)rows * m->in, cudaMemcpyHostToDevice, m->st) != cudaSuccess ||
+        cudaMemcpyAsync(T, t, sizeof(float) * (size_t)rows * m->out, cudaMemcpyHostToDevice, m->st) != cudaSuccess)
+        rc = fail(BOIDS_ECUDA, "boids_mlp_train: copy failed");
     for (int ep = 0; ep < epochs && !rc; ++ep) {
+        std::vector<int> &idx = order[ep & 1];
+        if (ep >= 2 && cudaEventSynchronize(sent[ep & 1]) != cudaSuccess) {
+            rc = fail(BOIDS_ECUDA, std::string("boids_mlp_train: ") + cudaGetErrorString(cudaGetLastError()));
+            break;
+        }
+        idx = order[(ep + 1) & 1];  // the last epoch's order, shuffled on
         for (int i = rows - 1; i > 0; --i) {  // Fisher-Yates
             s += 0x9e3779b97f4a7c15ULL;
             uint64_t z = s;
@@ -1397,6 +1417,7 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
             std::swap(idx[i], idx[j]);
         }
         if (cudaMemcpyAsync(d_idx, idx.data(), sizeof(int) * rows, cudaMemcpyHostToDevice, m->st) != cudaSuccess ||
+            cudaEventRecord(sent[ep & 1], m->st) != cudaSuccess ||
             cudaMemsetAsync(m->loss, 0, 8, m->st) != cudaSuccess) {
             rc = fail(BOIDS_ECUDA, "boids_mlp_train: copy failed");
             break;
@@ -1434,9 +1455,8 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
     }
     if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(BOIDS_ECUDA, "boids_mlp_train: kernel launch failed");
     if (!rc) rc = finish_call(m);
-    cudaFree(d_idx);
-    cudaFree(bx);
-    cudaFree(bt);
+    else cudaStreamSynchronize(m->st);  // no copy reads the caller's rows or the orders after the call
+    release();
     if (last_epoch_loss) *last_epoch_loss = epoch_loss;
     return rc;
 }
