@@ -1317,8 +1317,11 @@ int boids_mlp_forward(boids_mlp *m, const float *x, int32_t rows, float *y)
         MCK(cudaMemcpyAsync(m->x, x, sizeof(float) * (size_t)rows * m->in, cudaMemcpyHostToDevice, m->st));
         const __nv_bfloat16 *W1 = m->p16 + m->off[0], *W2 = m->p16 + m->off[2], *W3 = m->p16 + m->off[4];
         const float *b1 = m->p + m->off[1], *b2 = m->p + m->off[3], *b3 = m->p + m->off[5];
-        if (!m->img_valid) k_mlp_tile_w<<<nb(kTcN * kTcK / 8, 256), 256, 0, m->st>>>(W2, m->w2img);
-        m->img_valid = true;
+        if (!m->img_valid) {
+            k_mlp_tile_w<<<nb(kTcN * kTcK / 8, 256), 256, 0, m->st>>>(W2, m->w2img);
+            MCK(cudaGetLastError());
+            m->img_valid = true;
+        }
         const unsigned tiles = nb(rows, kTcM);
         k_mlp_forward_tc<<<tiles < m->nsm ? tiles : m->nsm, kTcFwdThreads, kTcFwdSmem, m->st>>>(
             m->x, rows, W1, b1, m->w2img, b2, W3, b3, m->y, m->err);

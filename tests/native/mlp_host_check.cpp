@@ -7,6 +7,10 @@
 //   mlp_host_check train HIDDEN ROWS BATCH EPOCHS [FAIL_AT]
 //       one training call; with FAIL_AT the so-many-th queued operation after
 //       its start fails.  Prints "rc copies late pending orders distinct".
+//   mlp_host_check image FAIL_AT
+//       two forward calls, the first with its so-many-th operation failing (0:
+//       none).  Prints "rc rc images", images: how often the second call laid
+//       the weight image out.
 #include <cuda_runtime_api.h>
 
 #include <algorithm>
@@ -52,7 +56,18 @@ cudaError_t put(Op op)
     queue_.push_back(std::move(op));
     return cudaSuccess;
 }
-cudaError_t launched() { return put(Op{[] {}, nullptr}); }
+std::map<const void *, std::string> &names()   // kernels, by their host stubs (registered before main)
+{
+    static std::map<const void *, std::string> n;
+    return n;
+}
+std::map<std::string, int> launches_;          // those launched
+cudaError_t launched(const void *f)
+{
+    const cudaError_t e = put(Op{[] {}, nullptr});
+    if (e == cudaSuccess) ++launches_[names()[f]];
+    return e;
+}
 
 }  // namespace
 
@@ -69,7 +84,10 @@ extern "C" {
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
 void __cudaRegisterFatBinaryEnd(void **) {}
 void __cudaUnregisterFatBinary(void **) {}
-void __cudaRegisterFunction(void **, const char *, char *, const char *, int, void *, void *, void *, void *, int *) {}
+void __cudaRegisterFunction(void **, const char *f, char *, const char *name, int, void *, void *, void *, void *, int *)
+{
+    names()[f] = name;
+}
 cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f)
 {
     *k = (cudaKernel_t)f;
@@ -77,8 +95,8 @@ cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f)
 }
 unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void *) { return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3 *, dim3 *, size_t *, void *) { return cudaSuccess; }
-cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void **, size_t, cudaStream_t) { return launched(); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *, void **) { return launched(); }
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **, size_t, cudaStream_t) { return launched(k); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *f, void **) { return launched(f); }
 
 cudaError_t cudaMalloc(void **p, size_t n) { *p = std::calloc(n, 1); return cudaSuccess; }
 cudaError_t cudaFree(void *p) { drain(); std::free(p); return cudaSuccess; }
@@ -160,10 +178,31 @@ static int train(int hidden, int rows, int batch, int epochs, int fail_at)
     return 0;
 }
 
+static int image(int fail_at)
+{
+    boids_mlp *m = nullptr;
+    if (boids_mlp_create(8, 256, 4, 1, 0, &m)) return 1;
+    std::vector<float> x(8 * 100, 0.5f), y(4 * 100);
+    queued_ = 0;
+    fail_at_ = fail_at;
+    const int rc1 = boids_mlp_forward(m, x.data(), 100, y.data());
+    fail_at_ = 0;
+    cudaGetLastError();
+    launches_.clear();
+    const int rc2 = boids_mlp_forward(m, x.data(), 100, y.data());
+    int images = 0;
+    for (const auto &l : launches_)
+        if (l.first.find("k_mlp_tile_w") != std::string::npos) images += l.second;
+    std::printf("%d %d %d\n", rc1, rc2, images);
+    boids_mlp_destroy(m);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     if (argc >= 6 && !std::strcmp(argv[1], "train"))
         return train(std::atoi(argv[2]), std::atoi(argv[3]), std::atoi(argv[4]), std::atoi(argv[5]),
                      argc > 6 ? std::atoi(argv[6]) : 0);
+    if (argc == 3 && !std::strcmp(argv[1], "image")) return image(std::atoi(argv[2]));
     return 2;
 }

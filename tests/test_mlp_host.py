@@ -42,3 +42,12 @@ def test_a_failed_training_call_leaves_no_copy_of_host_memory(mlp_host, fail_at)
     rc, _, late, pending, orders, _ = mlp_host("train", 256, 1000, 256, 4, fail_at)
     assert rc != 0
     assert late == 0 and pending == 0 and orders >= 0
+
+
+@pytest.mark.parametrize("fail_at,images", [(0, 0), (1, 1), (2, 1)])
+def test_weight_image_is_kept_only_when_it_was_laid_out(mlp_host, fail_at, images):
+    """A forward call whose upload or weight image failed leaves no image for
+    the next one to take for the present parameters'."""
+    rc1, rc2, laid = mlp_host("image", fail_at)
+    assert (rc1 != 0) == (fail_at != 0) and rc2 == 0
+    assert laid == images
