@@ -2763,6 +2763,7 @@ k_ap_accumulate(const float4 *__restrict__ pos, const float4 *__restrict__ vel, 
     if (i >= k.n) return;
     float4 p4 = __ldg(pos + i), v4 = __ldg(vel + i);
     uint32_t m = cnt[i], e0 = list[(size_t)i * cap + lane];  // (entries past the count are not used)
+    __syncwarp();  // every lane has its count before lane 0 clears it
     for (;;) {
         const uint32_t nx = i + step;
         float4 p_next = zero4, v_next = zero4;

@@ -114,6 +114,26 @@ def test_all_pairs_at_tile_edges(boids_lib, oracle_mod, n, field):
     sim.close()
 
 
+@pytest.mark.parametrize("n", [4863, 4864, 4865, 9729])
+def test_all_pairs_with_one_boid_a_warp_and_more(boids_lib, n):
+    """The N^2 kernels where their last one's 4864 warps have one boid each,
+    or go on to another: the neighbour counts that it clears are those it has
+    read, update after update (against the same engine on device cells)."""
+    prm = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008), vmax=0.005, vmin=0.001)
+    field = (n / 16384) ** (1 / 3)
+    pos, vel = gathered(n, field, 0.5, n)
+    a, b = make_sim(boids_lib, "pairs", n, field, prm), make_sim(boids_lib, "allpairs", n, field, prm)
+    for s in (a, b):
+        s.set_state(pos, vel)
+    for _ in range(3):
+        for s in (a, b):
+            s.update(1)
+        for x, y in zip(a.state(), b.state()):
+            assert_bits_equal(x, y, "state")
+    a.close()
+    b.close()
+
+
 @pytest.mark.parametrize("n,field", [(1, 0.7), (1023, 0.7), (8191, 0.7), (8193, 0.7), (16384, 0.7), (16385, 0.7),
                                      (3000, 1.33), (3000, 1.4), (40960, 0.7), (40961, 0.7)])
 def test_allocation_free_step_at_its_kernels_limits(boids_lib, oracle_mod, n, field):
