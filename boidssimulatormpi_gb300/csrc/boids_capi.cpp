@@ -21,6 +21,8 @@
 using boidsgpu::DevBuffers;
 using boidsgpu::RuleConst;
 using boidsgpu::StepConst;
+using boidsgpu::f_dn;
+using boidsgpu::f_up;
 
 namespace {
 
@@ -44,20 +46,6 @@ int cuda_fail(cudaError_t e, const char *where)
     } while (0)
 
 // ------------------------------------------------------------------ exact float thresholds
-
-float f_dn(double d)  // largest float <= d
-{
-    float f = (float)d;
-    if ((double)f > d) f = std::nextafter(f, -INFINITY);
-    return f;
-}
-
-float f_up(double d)  // smallest float >= d
-{
-    float f = (float)d;
-    if ((double)f < d) f = std::nextafter(f, INFINITY);
-    return f;
-}
 
 int64_t ordinal(float x)
 {
@@ -377,25 +365,12 @@ int make_constants(const boids_params &p, StepConst &k, bool *ref_ok)
         const float rup = f_up(radii[r]);
         if (rup > rmax) rmax = rup;
     }
-    // Conservative filter radius: the exact distance test can only accept a
-    // pair whose approximate distance is below this (rounding of the image
-    // shift and of the filter's own arithmetic is far below the margin).
-    const double ulpF = std::nextafter(std::fmax(k.Ff, 1.0f), INFINITY) - std::fmax(k.Ff, 1.0f);
-    const double rf = (double)rmax * (1.0 + 1e-4) + 8.0 * ulpF;
+    const double ulpF = boidsgpu::filter_ulp(k.Ff), rf = boidsgpu::filter_radius(rmax, k.Ff);
     k.filt_r2 = (float)(rf * rf);
     k.box_lim = (float)(p.field_size / 2 - rf * (1.0 + 1e-4) - 8.0 * ulpF);
-    {
-        // The all-pairs product filter sums cos(2 pi dx / F) over the axes, for
-        // a pair within rf at least 3 - (2 pi rf / F)^2 / 2 (cos a >= 1 - a^2 / 2).
-        // Rounding cosines and sines (at most 1) to half precision moves each
-        // by at most 2^-12, an axis's sum by 2 sqrt(2) 2^-12 + 2^-23: 2.08e-3
-        // over the axes; the angles of coordinates up to 4 F (2^-23 relative),
-        // sincospif, the FP32 sum of eight products and ap_min's own split into
-        // two half-precision terms add less than 1e-4.
-        const double r = 2.0 * M_PI * (rf * (1.0 + 1e-4) + 8.0 * ulpF) / p.field_size;
-        k.ap_turn = (float)(2.0 / p.field_size);
-        k.ap_min = f_dn(3.0 - r * r / 2.0 - 2.3e-3);
-    }
+    const boidsgpu::ApFilter apf = boidsgpu::ap_filter(rf, p.field_size);
+    k.ap_turn = apf.turn;
+    k.ap_min = apf.min;
     // The filters' relative vector differs from the exact imaged one by a
     // few ulps of the coordinates (at most 2F in magnitude), each dot
     // product by those times |v|_1 <= sqrt(3)|v| plus three roundings of

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include "boids_softfp.h"
 
 namespace boidsgpu {
@@ -19,6 +21,46 @@ namespace boidsgpu {
 // whose correctly rounded square root reaches r; the view-cone test
 // acos(c) <= pi*a (src/boid.cpp:34-35) becomes cstar <= c <= 1, with cstar
 // found on the host with the same acosf the reference calls.
+inline float f_dn(double d)  // largest float <= d
+{
+    float f = (float)d;
+    if ((double)f > d) f = std::nextafter(f, -INFINITY);
+    return f;
+}
+
+inline float f_up(double d)  // smallest float >= d
+{
+    float f = (float)d;
+    if ((double)f < d) f = std::nextafter(f, INFINITY);
+    return f;
+}
+
+// Conservative filter radius: the exact distance test can only accept a
+// pair whose approximate distance is below this (rounding of the image
+// shift and of the filter's own arithmetic is far below the margin).
+inline double filter_ulp(float F) { return std::nextafter(std::fmax(F, 1.0f), INFINITY) - std::fmax(F, 1.0f); }
+inline double filter_radius(float rmax, float F) { return (double)rmax * (1.0 + 1e-4) + 8.0 * filter_ulp(F); }
+
+// The all-pairs product filter's angle scale and least sum.  It sums
+// cos(2 pi dx / F) over the axes, for a pair within rf at least
+// 3 - (2 pi rf / F)^2 / 2 (cos a >= 1 - a^2 / 2).  Rounding cosines and sines
+// (at most 1) to half precision moves each by at most 2^-12, an axis's sum by
+// 2 sqrt(2) 2^-12 + 2^-23: 2.08e-3 over the axes; the angles of coordinates up
+// to 4 F (2^-23 relative), sincospif, the FP32 sum of eight products and min's
+// own split into two half-precision terms add less than 1e-4.
+// Three cosines never sum to less than -3: -4 passes every pair, whatever the
+// radius, and its terms stay within half precision.  A field so small that the
+// scale overflows gets angles of zero, which pass every pair, too.
+struct ApFilter {
+    float turn, min;
+};
+inline ApFilter ap_filter(double rf, double F)
+{
+    const double r = 2.0 * 3.141592653589793 * (rf * (1.0 + 1e-4) + 8.0 * filter_ulp((float)F)) / F;
+    const float turn = (float)(2.0 / F);
+    return ApFilter{std::isfinite(turn) ? turn : 0.f, f_dn(std::fmax(-4.0, 3.0 - r * r / 2.0 - 2.3e-3))};
+}
+
 struct RuleConst {
     float d2_lim;     // radius test: d2 < d2_lim
     float cstar;      // smallest c with (double)acosf(c) <= M_PI*sight_angle

@@ -114,6 +114,25 @@ def test_all_pairs_at_tile_edges(boids_lib, oracle_mod, n, field):
     sim.close()
 
 
+@pytest.mark.parametrize("field", [0.02, 0.0008, 1e-6])
+def test_all_pairs_with_sight_of_many_fields(boids_lib, oracle_mod, field):
+    """Radii of 2.5, 62 and 50 000 fields: every pair is in reach of the N^2 kernels' filter."""
+    O, prm, n = oracle_mod, dict(oracle_mod.MARUN2019), 300
+    prm["vmax"], prm["vmin"] = field / 10, field / 50
+    rng = np.random.default_rng(3)
+    pos = rng.uniform(0, field, 3 * n).astype(np.float32)
+    vel = (rng.normal(size=3 * n) * field / 50).astype(np.float32)
+    op, ov = pos.copy(), vel.copy()
+    O.step_allpairs(make_params(O, n, field, prm), op, ov, 2)
+    sim = make_sim(boids_lib, "pairs", n, field, prm)
+    sim.set_state(pos, vel)
+    sim.update(2)
+    gp, gv = sim.state()
+    assert_bits_equal(gp, op, "positions")
+    assert_bits_equal(gv, ov, "velocities")
+    sim.close()
+
+
 @pytest.mark.parametrize("n", [4863, 4864, 4865, 9729])
 def test_all_pairs_with_one_boid_a_warp_and_more(boids_lib, n):
     """The N^2 kernels where their last one's 4864 warps have one boid each,
