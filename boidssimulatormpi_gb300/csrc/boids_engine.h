@@ -51,6 +51,12 @@ inline double filter_radius(float rmax, float F) { return (double)rmax * (1.0 + 
 // Three cosines never sum to less than -3: -4 passes every pair, whatever the
 // radius, and its terms stay within half precision.  A field so small that the
 // scale overflows gets angles of zero, which pass every pair, too.
+// The terms of a boid are w = -min (at most 4) and u, what w's rounding left
+// of it; a boid too far outside the field for its angles adds kApPass to both.
+// Rows and columns past the last boid have kApPad in their place: no angles
+// and -16, which rejects them with every boid (w + kApPass + u < 16).
+constexpr float kApPass = 8.f;
+constexpr uint32_t kApPad = 0xcc00u;  // -16 in half precision
 struct ApFilter {
     float turn, min;
 };

@@ -2632,7 +2632,7 @@ __global__ void k_ap_embed(const float4 *__restrict__ pos, uint4 *__restrict__ e
     }
     // (a NaN coordinate, which no rule accepts, leaves its cosine and sine zero)
     const __half w = __float2half_rn(-k.ap_min);
-    const float pass = far > 4.f * k.Ff ? 8.f : 0.f, u = -k.ap_min - __half2float(w);
+    const float pass = far > 4.f * k.Ff ? kApPass : 0.f, u = -k.ap_min - __half2float(w);
     h[3] = __floats2half2_rn(__half2float(w) + pass, u + pass);
     emb[i] = *reinterpret_cast<const uint4 *>(h);
 }
@@ -2650,7 +2650,7 @@ k_ap_pairs(const float4 *__restrict__ pos, const float4 *__restrict__ vel, const
     const uint32_t j0 = blockIdx.y * tile_j, jn = min(tile_j, n - j0), jpad = (jn + 15) & ~15u;
     const uint32_t i0 = blockIdx.x * kApTileI + wid * kApWarpI;
     for (uint32_t q = threadIdx.x; q < jpad; q += kApThreads) {
-        uint4 e = make_uint4(0, 0, 0, 0xc8000000u);  // past the end: no angles, u = -8
+        uint4 e = make_uint4(0, 0, 0, kApPad << 16);  // past the end: no angles, and a u that rejects every pair
         if (q < jn) e = emb[j0 + q];
         e.w = (e.w & 0xffff0000u) | 0x3c00u;
         sj[q] = e;
@@ -2662,7 +2662,7 @@ k_ap_pairs(const float4 *__restrict__ pos, const float4 *__restrict__ vel, const
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint32_t i = i0 + 16 * m + 8 * r + g;
-            a[m][r] = i < n ? ew[4 * (size_t)i + t] : 0u;
+            a[m][r] = i < n ? ew[4 * (size_t)i + t] : (t == 3 ? kApPad : 0u);  // past the end: the same by its w
             if (t == 3) a[m][r] = (a[m][r] & 0xffffu) | 0x3c000000u;  // (w, 1)
         }
     __syncthreads();

@@ -38,7 +38,7 @@ def embed(x, field, turn):
                                           (0.05, 0.02), (1.0, 0.05), (1.0, 0.0172), (1.0, 0.01), (1.0, 1e-6),
                                           (1e30, 1.0), (float("inf"), 1.0), (1.0, 1e-39)])
 def test_shipped_filter_keeps_every_pair_in_reach(constants, radius, field):
-    rf, turn, least = constants(radius, field)
+    rf, turn, least, _, _ = constants(radius, field)
     assert np.isfinite(turn) and -4.0 <= least < 3.0
     w = f16(f32(-least))
     u = f16(f32(-least) - f32(w))
@@ -59,3 +59,19 @@ def test_shipped_filter_keeps_every_pair_in_reach(constants, radius, field):
     s = s + f32(w) + f32(u)
     assert inside.sum() > 50
     assert not np.signbit(s[inside]).any()
+
+
+@pytest.mark.parametrize("radius,field", [(0.05, 1.6), (0.05, (777 / 16384) ** (1 / 3)), (0.05, (65537 / 16384) ** (1 / 3)),
+                                          (0.05, 0.16), (1.0, 0.05), (float("inf"), 1.0)])
+def test_rows_and_columns_past_the_end_are_rejected(constants, radius, field):
+    """A row or column of padding makes a negative product with every boid's
+    vector, one too far outside for its angles included: none of its pairs is
+    queued for the exact tests."""
+    _, _, least, far, pad = constants(radius, field)
+    pad = np.uint16(int(pad)).view(f16)
+    w = f32(f16(f32(-least)))
+    u = f32(-least) - w
+    for extra in (0.0, far):  # a boid's (w, u); the other side's terms are 1, a padding's angles 0
+        bw, bu = f32(f16(w + f32(extra))), f32(f16(u + f32(extra)))
+        assert f32(pad) + bu < 0 and bw + f32(pad) < 0
+    assert f32(pad) + f32(pad) < 0
