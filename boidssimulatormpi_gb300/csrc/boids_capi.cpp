@@ -948,35 +948,30 @@ int boids_autotune(boids_sim *s, int32_t steps_per_trial)
         cudaEventCreate(&t0) != cudaSuccess || cudaEventCreate(&t1) != cudaSuccess)
         rc = cuda_fail(cudaGetLastError(), "boids_autotune");
     const StepConst keep = s->k;
-    float best = INFINITY;
-    int best_i = -1;
-    for (int c = 0; !rc && c < boidsgpu::kTuneCount; ++c) {
+    auto use = [&](int c, bool split) {
         s->k.dense_min = boidsgpu::kTuneCand[c][0];
         s->k.defer_min = boidsgpu::kTuneCand[c][1];
         s->k.cand_defer = boidsgpu::kTuneCand[c][2];
         s->k.lone_cand = boidsgpu::kTuneCand[c][3];
-        s->k.tuned = c > 0;  // the first is the default, with the default's choice of kernels
-        if ((rc = restore()) || (rc = boids_step(s, 1))) break;  // one warm-up update
-        float ms = 0.f;
-        if (cudaEventRecord(t0, s->stream) != cudaSuccess || (rc = boids_step(s, steps_per_trial)) ||
+        s->k.tuned = split;
+    };
+    auto trial = [&](int c, bool split, float *ms) -> int {
+        use(c, split);
+        int r = restore();
+        if (r || (r = boids_step(s, 1))) return r;  // one warm-up update
+        if (cudaEventRecord(t0, s->stream) != cudaSuccess || (r = boids_step(s, steps_per_trial)) ||
             cudaEventRecord(t1, s->stream) != cudaSuccess || cudaEventSynchronize(t1) != cudaSuccess ||
-            cudaEventElapsedTime(&ms, t0, t1) != cudaSuccess) {
-            if (!rc) rc = cuda_fail(cudaGetLastError(), "boids_autotune timing");
-            break;
-        }
-        if (ms < best) {
-            best = ms;
-            best_i = c;
-        }
-    }
+            cudaEventElapsedTime(ms, t0, t1) != cudaSuccess)
+            return r ? r : cuda_fail(cudaGetLastError(), "boids_autotune timing");
+        return 0;
+    };
+    const bool routed = s->b.slot_of != nullptr;
+    float ms[boidsgpu::kTuneCount] = {}, choice_ms = INFINITY;
+    for (int c = 0; !rc && c < boidsgpu::kTuneCount; ++c) rc = trial(c, c > 0, &ms[c]);
+    const int best = rc ? 0 : boidsgpu::tune_choice(ms, routed);
+    if (!rc && best > 0 && routed) rc = trial(best, false, &choice_ms);
     s->k = keep;
-    if (!rc && best_i >= 0) {
-        s->k.dense_min = boidsgpu::kTuneCand[best_i][0];
-        s->k.defer_min = boidsgpu::kTuneCand[best_i][1];
-        s->k.cand_defer = boidsgpu::kTuneCand[best_i][2];
-        s->k.lone_cand = boidsgpu::kTuneCand[best_i][3];
-        s->k.tuned = best_i > 0;
-    }
+    if (!rc) use(best, best > 0 && boidsgpu::tune_splits(ms[best], choice_ms));
     int rc2 = restore();
     if (!rc2 && cudaStreamSynchronize(s->stream) != cudaSuccess) rc2 = cuda_fail(cudaGetLastError(), "boids_autotune");
     s->steps_done = steps_done;

@@ -131,7 +131,8 @@ struct StepConst {
     // defer_min or more whose 27-cell neighbourhood holds over cand_defer
     // boids, and any non-empty cell whose neighbourhood holds over lone_cand.
     uint32_t dense_min, defer_min, cand_defer, lone_cand;
-    uint32_t tuned;  // those were set (boids_set_tuning, an autotuner): the split applies whatever the size
+    uint32_t tuned;  // the split applies whatever the size: those were set by boids_set_tuning, or an autotuner
+                     // found the split with them faster than the choice between it and a warp per boid
 };
 
 // A batched ensemble's flock table, in device memory.  Every block of
@@ -255,6 +256,26 @@ constexpr uint32_t kWarpBoids = 40960;
 constexpr uint32_t kCrowdBoids = 1u << 18, kCrowdSlots = 1u << 19;
 constexpr double kCrowdTop = 8.5, kCrowdTopSlope = 1.6e-5;
 constexpr double kCrowdBase = 0.47, kCrowdBare = 0.35, kCrowdSlope = 1.75e-6;
+// The autotuners time the default set with the choice above (or the split, if
+// the flock has no other: routed == false), the others with the split.  What a
+// flock gains now it can lose many times over once its state has changed: on a
+// uniform flock the set without dense cells is the fastest by 1 to 5 % (65 537
+// boids 67 us a step for 69, 262 143 143 for 148), and with it the same flock
+// took 1222 and 2270 us once it had gathered, where the choice takes 146 and
+// 522.  So a routed flock leaves the default for a set faster by kTuneMargin
+// only, and the choice only where the split with that set beats the choice with
+// it by as much (262 143 boids in small clusters 446 us for 680).
+constexpr float kTuneMargin = 1.1f;
+// The set to keep, from every set's time.
+inline int tune_choice(const float *ms, bool routed)
+{
+    int best = 0;
+    for (int c = 1; c < kTuneCount; ++c)
+        if (ms[c] < ms[best]) best = c;
+    return routed && !(ms[best] * kTuneMargin < ms[0]) ? 0 : best;
+}
+// Whether that set comes with the split alone, from its times with it and with the choice.
+inline bool tune_splits(float split_ms, float choice_ms) { return split_ms * kTuneMargin < choice_ms; }
 // Up to this many boids and cells (padded) a flock's counting sort is one
 // CTA's work (k_grid_sort, k_grid_bin_one).
 constexpr uint32_t kSortBoids = 1024, kSortCells = 4096;

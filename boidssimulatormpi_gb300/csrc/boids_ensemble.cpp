@@ -79,7 +79,7 @@ struct boids_ensemble {
     cudaGraphExec_t graph = nullptr;
     uint64_t graph_launches = 0;  // kernel launches per replay
     uint64_t launches = 0;
-    bool tuned = false;       // tune was set or chosen by the autotuner
+    bool tuned = false;       // the split whatever the size (StepConst::tuned)
     uint32_t tune[4] = {boidsgpu::kDenseMin, boidsgpu::kDeferMin, boidsgpu::kCandDefer, boidsgpu::kLoneCand};
 };
 
@@ -562,8 +562,6 @@ int boids_ensemble_autotune(boids_ensemble *e, int32_t steps_per_trial)
         return bin_fresh(e);
     };
     cudaEvent_t t0 = nullptr, t1 = nullptr;
-    float best = INFINITY;
-    int best_i = 0;
     rc = 0;
     if (cudaMemcpyAsync(sp, e->b.pos[0], bytes, cudaMemcpyDeviceToDevice, e->stream) != cudaSuccess ||
         cudaMemcpyAsync(sv, e->b.vel[0], bytes, cudaMemcpyDeviceToDevice, e->stream) != cudaSuccess ||
@@ -572,27 +570,26 @@ int boids_ensemble_autotune(boids_ensemble *e, int32_t steps_per_trial)
     uint32_t keep[4];
     std::memcpy(keep, e->tune, sizeof keep);
     const bool keep_tuned = e->tuned;
-    for (int c = 0; !rc && c < boidsgpu::kTuneCount; ++c) {
+    auto trial = [&](int c, bool split, float *ms) -> int {
         std::memcpy(e->tune, boidsgpu::kTuneCand[c], sizeof e->tune);
-        e->tuned = c > 0;  // the first is the default, with the default's choice of kernels
-        if ((rc = upload_table(e)) || (rc = restore()) || (rc = step_once(e))) break;  // one warm-up step
-        if (cudaEventRecord(t0, e->stream) != cudaSuccess) { rc = cuda_fail(cudaGetLastError(), "cudaEventRecord"); break; }
-        for (int t = 0; t < steps_per_trial && !rc; ++t) rc = step_once(e);
-        if (rc) break;
-        float ms = 0.f;
-        if (cudaEventRecord(t1, e->stream) != cudaSuccess || cudaEventSynchronize(t1) != cudaSuccess ||
-            cudaEventElapsedTime(&ms, t0, t1) != cudaSuccess) {
-            rc = cuda_fail(cudaGetLastError(), "autotune timing");
-            break;
-        }
-        if (ms < best) {
-            best = ms;
-            best_i = (int)c;
-        }
-    }
-    if (!rc) std::memcpy(e->tune, boidsgpu::kTuneCand[best_i], sizeof e->tune);
-    else std::memcpy(e->tune, keep, sizeof e->tune);
-    e->tuned = rc ? keep_tuned : best_i > 0;
+        e->tuned = split;
+        int r = upload_table(e);
+        if (r || (r = restore()) || (r = step_once(e))) return r;  // one warm-up step
+        CK(cudaEventRecord(t0, e->stream));
+        for (int t = 0; t < steps_per_trial; ++t)
+            if ((r = step_once(e))) return r;
+        CK(cudaEventRecord(t1, e->stream));
+        CK(cudaEventSynchronize(t1));
+        CK(cudaEventElapsedTime(ms, t0, t1));
+        return 0;
+    };
+    const bool routed = e->b.slot_of != nullptr;
+    float ms[boidsgpu::kTuneCount] = {}, choice_ms = INFINITY;
+    for (int c = 0; !rc && c < boidsgpu::kTuneCount; ++c) rc = trial(c, c > 0, &ms[c]);
+    const int best = rc ? 0 : boidsgpu::tune_choice(ms, routed);
+    if (!rc && best > 0 && routed) rc = trial(best, false, &choice_ms);
+    std::memcpy(e->tune, rc ? keep : boidsgpu::kTuneCand[best], sizeof e->tune);
+    e->tuned = rc ? keep_tuned : best > 0 && boidsgpu::tune_splits(ms[best], choice_ms);
     int rc2 = upload_table(e);
     if (!rc2) rc2 = restore();
     if (!rc2 && cudaStreamSynchronize(e->stream) != cudaSuccess) rc2 = cuda_fail(cudaGetLastError(), "autotune");

@@ -188,16 +188,17 @@ int boids_profile_read(boids_sim *sim, boids_profile_t *out, int32_t reset);
  * tune[1] defer_min   ... or this many with over
  * tune[2] cand_defer  candidates in the cell's 27-cell neighbourhood,
  * tune[3] lone_cand   ... or any boid with over this many candidates.
- * Defaults 16, 4, 192, 96; until they are set (or chosen by boids_autotune),
- * flocks of up to 40960 boids, and those of up to 262144 while they are
- * gathered, are updated a warp per boid instead, without a split.  No
- * counterpart in the reference. */
+ * Defaults 16, 4, 192, 96; until they are set here, flocks of up to 40960
+ * boids, and those of up to 262144 while they are gathered, are updated a warp
+ * per boid instead, without a split.  No counterpart in the reference. */
 int boids_set_tuning(boids_sim *sim, const int32_t *tune4);
 int boids_get_tuning(boids_sim *sim, int32_t *tune4);
 
 /* Time a few updates with each candidate threshold set on a copy of the
  * current state, keep the fastest, and put the state back (grid engine; a
- * no-op for the all-pairs engine).  Crowded flocks favour other thresholds
+ * no-op for the all-pairs engine).  Flocks of up to 262144 boids keep the
+ * defaults unless a set is faster by 10 %, and the choice between a warp per
+ * boid and the split unless the split is faster by as much.  Crowded flocks favour other thresholds
  * than uniform ones, so long runs may call it again as the flock gathers.
  * get_force values of the last update are lost.  steps_per_trial <= 0 picks
  * a default.  No counterpart in the reference. */
@@ -282,7 +283,8 @@ int boids_ensemble_get_state(boids_ensemble *ens, uint32_t flock, float *pos3n, 
 int boids_ensemble_stats(boids_ensemble *ens, double *out);
 /* Time a few steps with each candidate of the dense-cell thresholds (which
  * cells take the CTA-per-cell kernel) on a copy of the current state and
- * keep the fastest; results do not depend on the choice.  steps_per_trial
+ * keep the fastest (as boids_autotune, where at most 524288 state slots have
+ * the choice); results do not depend on the choice.  steps_per_trial
  * <= 0 picks a default.  Leaves the state as it was. */
 int boids_ensemble_autotune(boids_ensemble *ens, int32_t steps_per_trial);
 /* Chosen thresholds: dense_min, defer_min, cand_defer, lone_cand. */

@@ -263,6 +263,44 @@ def test_ensemble_route_by_crowding(boids_lib):
     b.close()
 
 
+@pytest.mark.parametrize("batch", [False, True])  # a handle, an ensemble
+@pytest.mark.parametrize("collapsed", [False, True])
+@pytest.mark.parametrize("n", [3000, 50000])
+def test_autotuned_flock_keeps_its_route(boids_lib, n, collapsed, batch):
+    """Thresholds that an autotuner chose on a uniform or a collapsed flock
+    take no route away from it: a gathered state has the kernels of an untuned
+    flock, and the same bits."""
+    B = boids_lib
+    prm = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008), vmax=0.005, vmin=0.001)
+    field = max(0.7, (n / 16384) ** (1 / 3))
+
+    def flock():
+        if not batch:
+            s = make_sim(B, "grid", n, field, prm, record_forces=False)
+            return s, s.set_state, s.update, s.state
+        p = B.flock_params(n, field, prm["sep"], prm["ali"], prm["coh"], prm["vmax"], prm["vmin"])
+        e = B.Ensemble([(p, B.INIT_RANDOM_UNIFORM, 1)])
+        e.init()
+        return e, lambda *s: e.set_state(0, *s), e.step, lambda: e.state(0)
+
+    crowd, loose = gathered(n, field, float(collapsed), 1, 1000), gathered(n, field, 1.0, 2, 64)
+    seen = []
+    for tune in (True, False):
+        h, put, step, get = flock()
+        put(*crowd)
+        if tune:
+            h.autotune(2)
+        put(*loose)
+        step(1)
+        before = h.kernel_launches()
+        step(1)
+        seen.append((h.kernel_launches() - before, *get()))
+        h.close()
+    assert seen[0][0] == seen[1][0]
+    for x, y in zip(seen[0][1:], seen[1][1:]):
+        assert_bits_equal(x, y, "state")
+
+
 def test_ensemble_initial_states(boids_lib, oracle_mod):
     """Flocks drawn side by side (more than 8192 boids in all), of both
     placements and odd sizes, against the oracle's sequence for each alone."""
