@@ -2073,7 +2073,7 @@ struct DenseSmem {
     float seg_s[18][3];
     uint32_t work, flock;
     uint32_t nw, cut;              // huge cells: window size, histogram cut
-    uint32_t wcut[kMaxCuts], nwcut, wbin;  // huge cells: planned window ends (in bins of wbin ids)
+    uint32_t wcut[kMaxCuts], nwcut, wlast;  // huge cells: planned window ends (ids), and the bins they take
     uint32_t woff[kMaxCuts + 1];           // and, when bucketed, each planned window's first scratch entry
     uint32_t wbucketed;
     uint32_t wtot[kDT / 32];       // block scan scratch
@@ -2148,34 +2148,38 @@ __device__ uint32_t dense_window(DenseSmem &sm, const GridIn &g, int ns, uint32_
     }
 }
 
-// The id windows of a huge cell planned from one histogram of its
-// candidates' ids over [0, nid) (kWinBins bins of wbin ids): window ends are
-// cut greedily where the running count would pass kDenseCap, at most
-// kMaxCuts of them.  Windows beyond the plan, or past a single bin that alone
-// overflows the list, are cut by dense_window instead.  One histogram pass
+// The next id windows of a huge cell, from id lo, planned from one histogram of
+// its candidates' ids (kWinBins bins, so narrow that one holds a quarter of the
+// list where ids are spread evenly): window ends are cut greedily where the
+// running count would pass kDenseCap, at most kMaxCuts of them; when they are
+// done, the next are planned.  A window that begins with a bin that alone
+// overflows the list is cut by dense_window instead.  One histogram pass
 // for all windows, where dense_window needs one per window.  With a scratch
 // of cap entries (this CTA's) that holds the planned windows, a second pass
 // files the candidates by bin, and each planned window is then read from
 // the scratch instead of scanning the whole neighbourhood again; an entry is
 // id << 34 | segment << 29 | slot.
-
-__device__ void dense_window_plan(DenseSmem &sm, const GridIn &g, int ns, uint32_t nid, uint64_t *scratch,
-                                  uint32_t cap)
+__device__ void dense_window_plan(DenseSmem &sm, const GridIn &g, int ns, uint32_t lo, uint32_t nid,
+                                  uint64_t *scratch, uint32_t cap)
 {
     static_assert((kWinBins + 1) * 4 <= sizeof(sm.u), "the prefix counts live in the sort buffers");
     static_assert(kWinBins % kDT == 0, "bins per thread");
     constexpr int kPer = kWinBins / kDT;
     uint32_t *hist = reinterpret_cast<uint32_t *>(&sm.u);
     const int t = threadIdx.x;
-    const uint32_t w = (nid + kWinBins - 1) / kWinBins;
+    const uint32_t even = (uint32_t)((uint64_t)nid * (kDenseCap / 4) / sm.seg_k0[ns]);
+    const uint32_t w = max(1u, min((nid - lo + kWinBins - 1) / kWinBins, even));  // ids of a bin
     for (int i = t; i <= kWinBins; i += kDT) hist[i] = 0;
     __syncthreads();
     for (int sgi = 0; sgi < ns; ++sgi) {
         const uint32_t j0 = sm.seg_j0[sgi], len = sm.seg_k0[sgi + 1] - sm.seg_k0[sgi];
-        for (uint32_t q = t; q < len; q += kDT) atomicAdd(&hist[__float_as_uint(__ldg(&g.pos[j0 + q].w)) / w], 1u);
+        for (uint32_t q = t; q < len; q += kDT) {
+            const uint32_t id = __float_as_uint(__ldg(&g.pos[j0 + q].w)), bin = (id - lo) / w;
+            if (id >= lo && bin < (uint32_t)kWinBins) atomicAdd(&hist[bin], 1u);
+        }
     }
     __syncthreads();
-    // exclusive prefix: hist[b] = candidates in bins below b, hist[kWinBins] = all
+    // exclusive prefix: hist[b] = candidates in bins below b, hist[kWinBins] in all bins
     uint32_t loc[kPer], sum = 0;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) { loc[i] = hist[t * kPer + i]; sum += loc[i]; }
@@ -2196,13 +2200,13 @@ __device__ void dense_window_plan(DenseSmem &sm, const GridIn &g, int ns, uint32
                 if (hist[mid] <= target) lo_b = mid; else hi_b = mid;
             }
             if (lo_b == start) break;  // bin `start` alone holds more than the list
-            sm.wcut[nc++] = lo_b;
+            sm.wcut[nc++] = min(nid, lo + lo_b * w);
+            sm.woff[nc] = hist[lo_b];
             start = lo_b;
         }
         sm.nwcut = nc;
-        sm.wbin = w;
+        sm.wlast = start;
         sm.woff[0] = 0;
-        for (uint32_t c = 0; c < nc; ++c) sm.woff[c + 1] = hist[sm.wcut[c]];
         // bucket the planned windows' candidates when the scratch holds them
         sm.wbucketed = nc > 0 && scratch != nullptr && sm.woff[nc] <= cap;
     }
@@ -2211,14 +2215,14 @@ __device__ void dense_window_plan(DenseSmem &sm, const GridIn &g, int ns, uint32
     // File every candidate of the planned windows at its bin's next entry
     // (the prefix counts become running ends): a window is then the
     // contiguous run woff[c] .. woff[c + 1] of the scratch, in bin order.
-    const uint32_t last_bin = sm.wcut[sm.nwcut - 1];
+    const uint32_t last_bin = sm.wlast;
     for (int sgi = 0; sgi < ns; ++sgi) {
         const uint32_t j0 = sm.seg_j0[sgi], len = sm.seg_k0[sgi + 1] - sm.seg_k0[sgi];
         for (uint32_t q = t; q < len; q += kDT) {
             const uint32_t slot = j0 + q;
             const uint32_t id = __float_as_uint(__ldg(&g.pos[slot].w));
-            const uint32_t bin = id / w;
-            if (bin < last_bin)
+            const uint32_t bin = (id - lo) / w;
+            if (id >= lo && bin < last_bin)
                 scratch[atomicAdd(&hist[bin], 1u)] = ((uint64_t)id << 34) | ((uint64_t)sgi << 29) | slot;
         }
     }
@@ -2308,16 +2312,16 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
             continue;
         }
 
-        if (huge)
-            dense_window_plan(sm, g, ns, k.n, o.wscratch ? o.wscratch + (size_t)blockIdx.x * o.wcap : nullptr,
-                              o.wcap);
         uint32_t lo = 0;  // this window's ids: [lo, hi)
-        uint32_t wi = 0;  // windows done
+        uint32_t wi = 0;  // windows of the present plan that are done (0: one is due)
         for (;;) {
             uint32_t hi = k.n, nw = ncand;
             if (huge) {
+                if (wi == 0)
+                    dense_window_plan(sm, g, ns, lo, k.n,
+                                      o.wscratch ? o.wscratch + (size_t)blockIdx.x * o.wcap : nullptr, o.wcap);
                 const bool planned = wi < sm.nwcut;
-                hi = planned ? min(k.n, sm.wcut[wi] * sm.wbin) : dense_window(sm, g, ns, lo, k.n);
+                hi = planned ? sm.wcut[wi] : dense_window(sm, g, ns, lo, k.n);
                 // gather the window's (id, segment, gather index) keys
                 if (planned && sm.wbucketed) {  // its run of the scratch
                     const uint64_t *run = o.wscratch + (size_t)blockIdx.x * o.wcap + sm.woff[wi];
@@ -2344,7 +2348,7 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
                         }
                     }
                 }
-                ++wi;
+                wi = wi + 1 < sm.nwcut ? wi + 1 : 0;
                 __syncthreads();
                 nw = sm.nw;
             } else {

@@ -64,6 +64,43 @@ def test_crowds_over_the_list_across_id_windows(boids_lib, oracle_mod, others):
     assert c.max() > 256
 
 
+@pytest.mark.parametrize("spread", [True, False])  # the crowd's ids over all, or the lowest
+@pytest.mark.parametrize("m", [16000, 17000, 36000])
+def test_crowds_over_one_plan_of_id_windows(boids_lib, m, spread):
+    """More candidates than the 32 id windows that the dense-cell kernel plans
+    at once: the next ones planned behind them, in a handle (files candidates
+    by window) and in an ensemble, against a warp per boid."""
+    B = boids_lib
+    prm = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008), vmax=0.005, vmin=0.001)
+    pos, vel = crowd_state(m, 2000, 0.0, m)
+    n = len(pos) // 3
+    if not spread:
+        far = np.abs(np.mod(pos.reshape(n, 3) + FIELD / 2, FIELD) - FIELD / 2).max(1) > 0.02
+        order = np.argsort(far, kind="stable")
+        pos, vel = (np.ascontiguousarray(x.reshape(n, 3)[order]).reshape(-1) for x in (pos, vel))
+    a, b = make_sim(B, "grid", n, FIELD, prm), make_sim(B, "grid", n, FIELD, prm)
+    b.set_tuning(*b.tuning())
+    for s in (a, b):
+        s.set_state(pos, vel)
+    for x, y in zip(a.neighbor_sets(), b.neighbor_sets()):
+        assert np.array_equal(x, y)
+    for s in (a, b):
+        s.update(2)
+    for x, y in zip(a.state(), b.state()):
+        assert_bits_equal(x, y, "state")
+    assert_bits_equal(a.forces(), b.forces(), "forces")
+    p = B.flock_params(n, FIELD, prm["sep"], prm["ali"], prm["coh"], prm["vmax"], prm["vmin"])
+    e = B.Ensemble([(p, B.INIT_RANDOM_UNIFORM, 1)])
+    e.init()
+    e.set_tuning(*e.tuning())
+    e.set_state(0, pos, vel)
+    e.step(2)
+    for x, y in zip(a.state(), e.state(0)):
+        assert_bits_equal(x, y, "ensemble")
+    for s in (a, b, e):
+        s.close()
+
+
 def test_ensemble_tuned_between_statistics_and_step(boids_lib):
     """Thresholds set while the statistics' binning waits for its step: that
     step runs on what was classified, the later ones by the thresholds."""
