@@ -202,7 +202,7 @@ constexpr int kDeferMin = 4;          // default defer_min
 constexpr int kCandDefer = 192;       // default cand_defer
 constexpr int kLoneCand = 96;         // default lone_cand
 constexpr int kCarryBytes = 72;       // partial sums of one boid between id windows
-constexpr uint32_t kWinScratch = 32768;  // most candidates a CTA files by window (32 windows of 1024)
+constexpr uint32_t kWinScratch = 32768;  // most candidates a CTA files by window (twice what 32 windows hold)
 
 // Dense-cell threshold sets the autotuners try, {dense_min, defer_min,
 // cand_defer, lone_cand}; the first is the default.  Crowded (clustered)
@@ -215,15 +215,30 @@ constexpr uint32_t kTuneCand[][4] = {
 constexpr int kTuneCount = sizeof(kTuneCand) / sizeof(kTuneCand[0]);
 
 // The dense kernel's work items are (full-size cell, first boid) pairs, one
-// per kDenseRound boids of a dense cell, so that the boids of one crowded
-// cell spread over several CTAs.  Words the work list can need in one step:
-// at most one item per non-empty cell plus one per kDenseRound boids, and
-// never more than one per boid, two words per item.
-constexpr int kDenseRound = 32;
+// per kDenseItem boids of a dense cell, so that the boids of one crowded
+// cell spread over several CTAs.  Every item gathers and sorts its cell's
+// neighbourhood.  Where that takes id windows (over kDenseCap candidates), a
+// remainder of up to half an item is shared among the cell's other items
+// (dense_per_item), and while a CTA has many items to come it takes up to
+// kDenseTake at once and does a cell's in a row together: without either,
+// uniform flocks of 16 to 48 times the reference's density took 5 to 13 % longer
+// than with items of 128 boids (2^20 boids at 32 times, us a step: 7110, now
+// 6405, 6265 with those; at 16 times 3670, 3245, 3465), which in turn cost
+// gathered flocks 10 to 30 % up to 2^19 boids (262 143 400 updates after a
+// uniform start 777, now 655; 2^20 2350 and 2030).  Sharing remainders in all
+// cells, or taking several items at once until fewer are left (kDenseLeft 1, 2),
+// cost those 2 to 10 %.
+constexpr int kDenseItem = 32;
+constexpr uint32_t kDenseTake = 4;  // most items taken at once ...
+constexpr uint32_t kDenseLeft = 3;  // ... which is those left over, for every CTA so many times
+constexpr int kDenseRound = 64;     // boids whose results a CTA holds in shared memory, over an item's most
+// Words the work list can need in one step: at most one item per non-empty
+// cell plus one per kDenseItem boids, and never more than one per boid, two
+// words per item.
 inline size_t dense_list_capacity(size_t ncell, size_t n)
 {
     const size_t by_cells = ncell / 4;
-    const size_t items = (by_cells < n ? by_cells : n) + n / kDenseRound + 1;
+    const size_t items = (by_cells < n ? by_cells : n) + n / kDenseItem + 1;
     return 2 * (items < n ? items : n);
 }
 // Flocks of up to this many boids (all flocks of an ensemble together) are
@@ -284,6 +299,14 @@ constexpr uint32_t kSortBoids = 1024, kSortCells = 4096;
 // of more takes longer than the launches it saves.
 constexpr uint32_t kBinBoids = 16384, kBinCells = 65536;
 constexpr int kDenseCap = 512;        // candidates of a dense cell held in shared memory
+// Boids per item of a dense cell of b boids with ncand candidates.
+__host__ __device__ inline uint32_t dense_per_item(uint32_t b, uint32_t ncand)
+{
+    if (ncand <= (uint32_t)kDenseCap || b <= kDenseItem) return kDenseItem;
+    const uint32_t items = (b + kDenseItem / 2) / kDenseItem;
+    return (b + items - 1) / items;
+}
+static_assert(kDenseItem + kDenseItem / 2 <= kDenseRound, "an item is one round");
 constexpr int kDenseCtasPerSm = 8;   // resident CTAs of the dense-cell kernel per SM (its launch bounds)
 constexpr int kApCap = 256;           // all-pairs engine: neighbours kept per boid (more: an O(N) scan)
 constexpr uint32_t kMaxBoids = 1u << 29;  // slot index packs into 29 bits

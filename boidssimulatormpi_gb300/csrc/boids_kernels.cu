@@ -826,11 +826,11 @@ __global__ void k_grid_classify(const uint32_t *__restrict__ lstart,
         }
         if (dense_rule(b, ncand, k, windows)) {
             flag = 1;
-            const uint32_t items = (b + kDenseRound - 1) / kDenseRound;
+            const uint32_t per = dense_per_item(b, ncand), items = (b + per - 1) / per;
             const uint32_t at = atomicAdd(dense_n, items);
             for (uint32_t r = 0; r < items; ++r) {
                 dense_list[2 * (at + r)] = cg;
-                dense_list[2 * (at + r) + 1] = r * kDenseRound;
+                dense_list[2 * (at + r) + 1] = r * per;
             }
         }
     }
@@ -2068,10 +2068,12 @@ struct DenseSmem {
         __align__(16) float st[kDT / 32][9][kSumCols];  // per warp: a round's summands, by component
     } v;
     uint16_t hits[kDT / 32][kHitRing];     // per warp: filter hits (candidates), a ring
-    uint32_t res[12][kDenseRound + 1];     // the item's sums and counts, by boid
+    uint32_t res[12][kDenseRound + 1];     // a round's sums and counts, by boid
     uint32_t seg_j0[18], seg_k0[19];
     float seg_s[18][3];
-    uint32_t work, flock;
+    // the next item, the end of those taken from the queue, all items, how many to take next
+    uint32_t work, wend, wall, wtake;
+    uint32_t flock;
     uint32_t nw, cut;              // huge cells: window size, histogram cut
     uint32_t wcut[kMaxCuts], nwcut, wlast;  // huge cells: planned window ends (ids), and the bins they take
     uint32_t woff[kMaxCuts + 1];           // and, when bucketed, each planned window's first scratch entry
@@ -2229,11 +2231,11 @@ __device__ void dense_window_plan(DenseSmem &sm, const GridIn &g, int ns, uint32
     __syncthreads();
 }
 
-// One CTA takes one work item at a time (dynamic queue): a crowded cell and
-// up to kDenseRound of its boids (a cell with more boids is several items,
-// taken by several CTAs).  The cell's 27-cell candidates are sorted by id once
-// per item.  Then each warp takes a boid at a time: its lanes filter the list
-// in half precision, 64 candidates an iteration, the hits are compacted into
+// One CTA takes a work item or a few at a time (dynamic queue): a crowded cell
+// and about kDenseItem of its boids (a cell with more boids is several items,
+// taken by several CTAs, or done together by one).  The cell's 27-cell
+// candidates are sorted by id, once for the items done together.  Then each
+// warp takes a boid at a time: its lanes filter the list in half precision, 64 candidates an iteration, the hits are compacted into
 // the warp's queue, 32 of them at a time take the exact tests, and the
 // accepted, compacted again, are added up by nine lanes, one component of the
 // three rules' sums each.  The list is in id order and every compaction keeps
@@ -2260,13 +2262,30 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
     DenseSmem &sm = *reinterpret_cast<DenseSmem *>(dense_smem_raw);
     const int t = threadIdx.x;
     if (g.chain) chain_wait();
+    // how many items to take next, from those that are left: several while the
+    // CTAs have many to come, one by one towards the end
+    auto take_of = [&](uint32_t left) { return min(max(left / (kDenseLeft * gridDim.x), 1u), kDenseTake); };
+    if (t == 0) {
+        sm.work = sm.wend = 0;
+        sm.wall = dense_n[0];
+        sm.wtake = take_of(sm.wall);
+    }
     for (;;) {
-        if (t == 0) sm.work = atomicAdd(dense_n + 1, 1u);
+        if (t == 0 && sm.work >= sm.wend) {  // the next items from the queue
+            const uint32_t take = sm.wtake, first = atomicAdd(dense_n + 1, take), all = sm.wall;
+            sm.work = first;
+            sm.wend = min(all, first + take);
+            sm.wtake = take_of(all - min(all, first + take * gridDim.x));  // when the other CTAs have taken as many
+        }
         __syncthreads();
-        const uint32_t w = sm.work;
-        if (w >= dense_n[0]) break;
+        const uint32_t w = sm.work, wend = sm.wend;
+        if (w >= wend) break;
         const uint32_t cg = dense_list[2 * w];        // global full-size cell
-        const uint32_t rbeg = dense_list[2 * w + 1];  // the item's first boid of the cell
+        const uint32_t rbeg = dense_list[2 * w + 1];  // the items' first boid of the cell
+        uint32_t run = 1;                             // items of that cell, done together
+#pragma unroll
+        for (uint32_t q = 1; q < kDenseTake; ++q)
+            if (w + q < wend && dense_list[2 * (w + q)] == cg) run = q + 1;
         if (MULTI) {
             if (t == 0) {  // the flock: last with cell4 <= cg
                 uint32_t lo = 0, hi = ft.count;
@@ -2309,6 +2328,7 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
         const bool huge = ncand > (uint32_t)kDenseCap;
         if (huge && !o.carry) {  // not listed so by k_grid_classify; kept for safety
             __syncthreads();
+            if (t == 0) sm.work = w + run;
             continue;
         }
 
@@ -2414,171 +2434,177 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
 
             // A warp per boid of the item.  The candidates are in id order, so the
             // filter's hits, the accepted among them and their summands are too.
-            const uint32_t rend = min(b, rbeg + (uint32_t)kDenseRound);
             const uint32_t npairs = (nw + 1) / 2;
             const int lane = t & 31, wid = t >> 5;
             const unsigned below = (1u << lane) - 1u;
             uint16_t *hits = sm.hits[wid];
             float(&st)[9][kSumCols] = sm.v.st[wid];
-            for (uint32_t i = rbeg + wid; i < rend; i += kDT / 32) {
-                const uint32_t s = own0 + i;
-                const float3 pi = xyz(__ldg(g.pos + s));
-                const Sight si = make_sight(xyz(__ldg(g.vel + s)));
-                // lane c < 9: component c of (cohesion, separation, alignment)
-                float acc = 0.f;
-                int ncoh = 0, nsep = 0, nali = 0;
-                uint64_t h0 = 0, h1 = 0, h2 = 0;
-                if (!first) {  // the earlier id windows' sums
-                    const Acc *cin = o.carry + s;
-                    if (lane < 9) acc = reinterpret_cast<const float *>(cin)[lane];
-                    ncoh = cin->ncoh;
-                    nsep = cin->nsep;
-                    nali = cin->nali;
-                }
-                // The filter in half precision, two candidates per instruction:
-                // it keeps every pair within the filter radius and drops only
-                // pairs whose exact v . r is negative (the bounds are in hfilt,
-                // hdot0 and hdot1); the exact tests decide the rest.
-                const __half2 bx = __float2half2_rn((pi.x - cen.x) * k.hsc);
-                const __half2 by = __float2half2_rn((pi.y - cen.y) * k.hsc);
-                const __half2 bz = __float2half2_rn((pi.z - cen.z) * k.hsc);
-                const float vt = si.nv * k.hvsc;
-                const bool pre = k.cone_pre && vt <= 1.0f;
-                const __half2 hvx = __float2half2_rn(pre ? si.v.x * k.hvsc : 0.f);
-                const __half2 hvy = __float2half2_rn(pre ? si.v.y * k.hvsc : 0.f);
-                const __half2 hvz = __float2half2_rn(pre ? si.v.z * k.hvsc : 0.f);
-                const __half2 hf2 = __half2half2(__float2half_ru(k.hfilt));
-                const __half2 hd2 = __half2half2(pre ? __float2half_rd(-(k.hdot0 + k.hdot1 * vt))
-                                                     : __ushort_as_half((unsigned short)0xfc00u));  // -inf
-                uint32_t qh = 0, nq = 0;  // the ring's head and length, the same in every lane
-                for (uint32_t p0 = 0; p0 < npairs; p0 += 32) {
-                    const uint32_t pp = p0 + lane;
-                    unsigned keep = 0;
-                    if (pp < npairs) {
-                        const __half2 dx = __hsub2(sm.hx[pp], bx), dy = __hsub2(sm.hy[pp], by),
-                                      dz = __hsub2(sm.hz[pp], bz);
-                        const __half2 d2 = __hfma2(dz, dz, __hfma2(dy, dy, __hmul2(dx, dx)));
-                        const __half2 dv = __hfma2(hvz, dz, __hfma2(hvy, dy, __hmul2(hvx, dx)));
-                        keep = __hlt2_mask(d2, hf2) & __hge2_mask(dv, hd2);
+            const uint32_t iend = min(b, rbeg + run * dense_per_item(b, ncand));
+            for (uint32_t r0 = rbeg; r0 < iend; r0 += kDenseRound) {  // a round's results at a time
+                const uint32_t rend = min(iend, r0 + (uint32_t)kDenseRound);
+                for (uint32_t i = r0 + wid; i < rend; i += kDT / 32) {
+                    const uint32_t s = own0 + i;
+                    const float3 pi = xyz(__ldg(g.pos + s));
+                    const Sight si = make_sight(xyz(__ldg(g.vel + s)));
+                    // lane c < 9: component c of (cohesion, separation, alignment)
+                    float acc = 0.f;
+                    int ncoh = 0, nsep = 0, nali = 0;
+                    uint64_t h0 = 0, h1 = 0, h2 = 0;
+                    if (!first) {  // the earlier id windows' sums
+                        const Acc *cin = o.carry + s;
+                        if (lane < 9) acc = reinterpret_cast<const float *>(cin)[lane];
+                        ncoh = cin->ncoh;
+                        nsep = cin->nsep;
+                        nali = cin->nali;
                     }
-                    const bool e0 = keep & 1u, e1 = keep >> 16;
-                    const unsigned m0 = __ballot_sync(0xffffffffu, e0), m1 = __ballot_sync(0xffffffffu, e1);
-                    uint32_t at = qh + nq + __popc(m0 & below) + __popc(m1 & below);
-                    if (e0) hits[at++ & (kHitRing - 1)] = (uint16_t)(2 * pp);
-                    if (e1) hits[at & (kHitRing - 1)] = (uint16_t)(2 * pp + 1);
-                    nq += __popc(m0) + __popc(m1);
-                    // exact tests of 32 hits at a time, and the sums of those accepted;
-                    // the last pairs' hits whatever their number
-                    const uint32_t enough = p0 + 32 < npairs ? 32u : 1u;
-                    while (nq >= enough) {
-                        __syncwarp();
-                        int f = 0;
-                        float4 cq = make_float4(0.f, 0.f, 0.f, 0.f);
-                        uint32_t q = 0;
-                        if ((uint32_t)lane < nq) {
-                            q = hits[(qh + lane) & (kHitRing - 1)];
-                            cq = sm.u.spos[q];
-                            if (__float_as_uint(cq.w) != s) f = pair_flags(pi, si, xyz(cq), k);
+                    // The filter in half precision, two candidates per instruction:
+                    // it keeps every pair within the filter radius and drops only
+                    // pairs whose exact v . r is negative (the bounds are in hfilt,
+                    // hdot0 and hdot1); the exact tests decide the rest.
+                    const __half2 bx = __float2half2_rn((pi.x - cen.x) * k.hsc);
+                    const __half2 by = __float2half2_rn((pi.y - cen.y) * k.hsc);
+                    const __half2 bz = __float2half2_rn((pi.z - cen.z) * k.hsc);
+                    const float vt = si.nv * k.hvsc;
+                    const bool pre = k.cone_pre && vt <= 1.0f;
+                    const __half2 hvx = __float2half2_rn(pre ? si.v.x * k.hvsc : 0.f);
+                    const __half2 hvy = __float2half2_rn(pre ? si.v.y * k.hvsc : 0.f);
+                    const __half2 hvz = __float2half2_rn(pre ? si.v.z * k.hvsc : 0.f);
+                    const __half2 hf2 = __half2half2(__float2half_ru(k.hfilt));
+                    const __half2 hd2 = __half2half2(pre ? __float2half_rd(-(k.hdot0 + k.hdot1 * vt))
+                                                         : __ushort_as_half((unsigned short)0xfc00u));  // -inf
+                    uint32_t qh = 0, nq = 0;  // the ring's head and length, the same in every lane
+                    for (uint32_t p0 = 0; p0 < npairs; p0 += 32) {
+                        const uint32_t pp = p0 + lane;
+                        unsigned keep = 0;
+                        if (pp < npairs) {
+                            const __half2 dx = __hsub2(sm.hx[pp], bx), dy = __hsub2(sm.hy[pp], by),
+                                          dz = __hsub2(sm.hz[pp], bz);
+                            const __half2 d2 = __hfma2(dz, dz, __hfma2(dy, dy, __hmul2(dx, dx)));
+                            const __half2 dv = __hfma2(hvz, dz, __hfma2(hvy, dy, __hmul2(hvx, dx)));
+                            keep = __hlt2_mask(d2, hf2) & __hge2_mask(dv, hd2);
                         }
-                        const uint32_t done = min(nq, 32u);
-                        qh += done;
-                        nq -= done;
-                        const unsigned am = __ballot_sync(0xffffffffu, f != 0);
-                        if (!am) continue;
-                        const int m = __popc(am);
-                        const bool co = f & 1, se = f & 2, al = f & 4;
-                        const unsigned cm = __ballot_sync(0xffffffffu, co), em = __ballot_sync(0xffffffffu, se),
-                                       lm = __ballot_sync(0xffffffffu, al);
-                        ncoh += __popc(cm);
-                        nsep += __popc(em);
-                        nali += __popc(lm);
-                        // Column by column, lanes 0-8 add the accepted up, a component
-                        // each.  A rule that did not accept a neighbour adds +0, which
-                        // leaves a float sum that started at +0 unchanged (it is never
-                        // -0): every sum is the reference's sequence of additions.
-                        if (f) {
-                            const int c = __popc(am & below);
-                            st[0][c] = co ? cq.x : 0.f;
-                            st[1][c] = co ? cq.y : 0.f;
-                            st[2][c] = co ? cq.z : 0.f;
-                            st[6][c] = al ? sm.svx[q] : 0.f;
-                            st[7][c] = al ? sm.svy[q] : 0.f;
-                            st[8][c] = al ? sm.svz[q] : 0.f;
-                            if (em) {
-                                float3 u = make_float3(0.f, 0.f, 0.f);
-                                if (se) {  // Vector3D::normalized of pi - t
-                                    const float dx = __fsub_rn(pi.x, cq.x), dy = __fsub_rn(pi.y, cq.y),
-                                                dz = __fsub_rn(pi.z, cq.z);
-                                    const float n = nrm3(dx, dy, dz);
-                                    u = make_float3(__fdiv_rn(dx, n), __fdiv_rn(dy, n), __fdiv_rn(dz, n));
+                        const bool e0 = keep & 1u, e1 = keep >> 16;
+                        const unsigned m0 = __ballot_sync(0xffffffffu, e0), m1 = __ballot_sync(0xffffffffu, e1);
+                        uint32_t at = qh + nq + __popc(m0 & below) + __popc(m1 & below);
+                        if (e0) hits[at++ & (kHitRing - 1)] = (uint16_t)(2 * pp);
+                        if (e1) hits[at & (kHitRing - 1)] = (uint16_t)(2 * pp + 1);
+                        nq += __popc(m0) + __popc(m1);
+                        // exact tests of 32 hits at a time, and the sums of those accepted;
+                        // the last pairs' hits whatever their number
+                        const uint32_t enough = p0 + 32 < npairs ? 32u : 1u;
+                        while (nq >= enough) {
+                            __syncwarp();
+                            int f = 0;
+                            float4 cq = make_float4(0.f, 0.f, 0.f, 0.f);
+                            uint32_t q = 0;
+                            if ((uint32_t)lane < nq) {
+                                q = hits[(qh + lane) & (kHitRing - 1)];
+                                cq = sm.u.spos[q];
+                                if (__float_as_uint(cq.w) != s) f = pair_flags(pi, si, xyz(cq), k);
+                            }
+                            const uint32_t done = min(nq, 32u);
+                            qh += done;
+                            nq -= done;
+                            const unsigned am = __ballot_sync(0xffffffffu, f != 0);
+                            if (!am) continue;
+                            const int m = __popc(am);
+                            const bool co = f & 1, se = f & 2, al = f & 4;
+                            const unsigned cm = __ballot_sync(0xffffffffu, co), em = __ballot_sync(0xffffffffu, se),
+                                           lm = __ballot_sync(0xffffffffu, al);
+                            ncoh += __popc(cm);
+                            nsep += __popc(em);
+                            nali += __popc(lm);
+                            // Column by column, lanes 0-8 add the accepted up, a component
+                            // each.  A rule that did not accept a neighbour adds +0, which
+                            // leaves a float sum that started at +0 unchanged (it is never
+                            // -0): every sum is the reference's sequence of additions.
+                            if (f) {
+                                const int c = __popc(am & below);
+                                st[0][c] = co ? cq.x : 0.f;
+                                st[1][c] = co ? cq.y : 0.f;
+                                st[2][c] = co ? cq.z : 0.f;
+                                st[6][c] = al ? sm.svx[q] : 0.f;
+                                st[7][c] = al ? sm.svy[q] : 0.f;
+                                st[8][c] = al ? sm.svz[q] : 0.f;
+                                if (em) {
+                                    float3 u = make_float3(0.f, 0.f, 0.f);
+                                    if (se) {  // Vector3D::normalized of pi - t
+                                        const float dx = __fsub_rn(pi.x, cq.x), dy = __fsub_rn(pi.y, cq.y),
+                                                    dz = __fsub_rn(pi.z, cq.z);
+                                        const float n = nrm3(dx, dy, dz);
+                                        u = make_float3(__fdiv_rn(dx, n), __fdiv_rn(dy, n), __fdiv_rn(dz, n));
+                                    }
+                                    st[3][c] = u.x;
+                                    st[4][c] = u.y;
+                                    st[5][c] = u.z;
                                 }
-                                st[3][c] = u.x;
-                                st[4][c] = u.y;
-                                st[5][c] = u.z;
+                                if (DIAG) {
+                                    const uint64_t h = id_hash(__float_as_uint(__ldg(&g.pos[__float_as_uint(cq.w)].w)));
+                                    if (co) h0 += h;
+                                    if (se) h1 += h;
+                                    if (al) h2 += h;
+                                }
                             }
-                            if (DIAG) {
-                                const uint64_t h = id_hash(__float_as_uint(__ldg(&g.pos[__float_as_uint(cq.w)].w)));
-                                if (co) h0 += h;
-                                if (se) h1 += h;
-                                if (al) h2 += h;
+                            // columns m .. up to a multiple of four: +0
+                            const int pad = (4 - m) & 3;
+                            if (lane < 9 * 4 && (lane & 3) < pad) st[lane >> 2][m + (lane & 3)] = 0.f;
+                            if (lane < pad) st[8][m + lane] = 0.f;
+                            __syncwarp();
+                            if (lane < 9 && (em || lane < 3 || lane >= 6)) {
+                                const float *row = st[lane];
+                                for (int c = 0; c < m; c += 4) {
+                                    const float4 x = *reinterpret_cast<const float4 *>(row + c);
+                                    acc = __fadd_rn(acc, x.x);
+                                    acc = __fadd_rn(acc, x.y);
+                                    acc = __fadd_rn(acc, x.z);
+                                    acc = __fadd_rn(acc, x.w);
+                                }
                             }
+                            __syncwarp();
                         }
-                        // columns m .. up to a multiple of four: +0
-                        const int pad = (4 - m) & 3;
-                        if (lane < 9 * 4 && (lane & 3) < pad) st[lane >> 2][m + (lane & 3)] = 0.f;
-                        if (lane < pad) st[8][m + lane] = 0.f;
-                        __syncwarp();
-                        if (lane < 9 && (em || lane < 3 || lane >= 6)) {
-                            const float *row = st[lane];
-                            for (int c = 0; c < m; c += 4) {
-                                const float4 x = *reinterpret_cast<const float4 *>(row + c);
-                                acc = __fadd_rn(acc, x.x);
-                                acc = __fadd_rn(acc, x.y);
-                                acc = __fadd_rn(acc, x.z);
-                                acc = __fadd_rn(acc, x.w);
-                            }
+                    }
+                    const uint32_t word = lane < 9 ? __float_as_uint(acc)
+                                                   : (uint32_t)(lane == 9 ? ncoh : (lane == 10 ? nsep : nali));
+                    if (DIAG) {
+#pragma unroll
+                        for (int q = 16; q > 0; q >>= 1) {
+                            h0 += __shfl_xor_sync(0xffffffffu, h0, q);
+                            h1 += __shfl_xor_sync(0xffffffffu, h1, q);
+                            h2 += __shfl_xor_sync(0xffffffffu, h2, q);
                         }
-                        __syncwarp();
+                        if (lane == 0) {
+                            uint64_t *hs =
+                                last ? o.dhash + 3 * (size_t)(__float_as_uint(g.pos[s].w) + (k.slot_base - k.slot_off))
+                                     : o.carry[s].h;
+                            const uint64_t *hc = first ? nullptr : o.carry[s].h;
+                            hs[0] = h0 + (hc ? hc[0] : 0);
+                            hs[1] = h1 + (hc ? hc[1] : 0);
+                            hs[2] = h2 + (hc ? hc[2] : 0);
+                        }
+                        if (last && lane >= 9 && lane < 12)
+                            o.dcnt[3 * (size_t)(__float_as_uint(g.pos[s].w) + (k.slot_base - k.slot_off)) + lane - 9] =
+                                (int)word;
+                    }
+                    if (lane < 12) {
+                        if (!last) reinterpret_cast<uint32_t *>(o.carry + s)[lane] = word;
+                        else if (!DIAG) sm.res[lane][i - r0] = word;
                     }
                 }
-                const uint32_t word = lane < 9 ? __float_as_uint(acc)
-                                               : (uint32_t)(lane == 9 ? ncoh : (lane == 10 ? nsep : nali));
-                if (DIAG) {
+                __syncthreads();  // the list is free, the results are written
+                if (!DIAG && last && (uint32_t)t < rend - r0) {
+                    const uint32_t s = own0 + r0 + t;
+                    Acc a;
+                    uint32_t *aw = reinterpret_cast<uint32_t *>(&a);
 #pragma unroll
-                    for (int q = 16; q > 0; q >>= 1) {
-                        h0 += __shfl_xor_sync(0xffffffffu, h0, q);
-                        h1 += __shfl_xor_sync(0xffffffffu, h1, q);
-                        h2 += __shfl_xor_sync(0xffffffffu, h2, q);
-                    }
-                    if (lane == 0) {
-                        uint64_t *hs = last ? o.dhash + 3 * (size_t)(__float_as_uint(g.pos[s].w) + (k.slot_base - k.slot_off))
-                                            : o.carry[s].h;
-                        const uint64_t *hc = first ? nullptr : o.carry[s].h;
-                        hs[0] = h0 + (hc ? hc[0] : 0);
-                        hs[1] = h1 + (hc ? hc[1] : 0);
-                        hs[2] = h2 + (hc ? hc[2] : 0);
-                    }
-                    if (last && lane >= 9 && lane < 12)
-                        o.dcnt[3 * (size_t)(__float_as_uint(g.pos[s].w) + (k.slot_base - k.slot_off)) + lane - 9] =
-                            (int)word;
+                    for (int c = 0; c < 12; ++c) aw[c] = sm.res[c][t];
+                    finish_boid<DIAG>(a, g.pos[s], xyz(g.vel[s]), s, o, k);
                 }
-                if (lane < 12) {
-                    if (!last) reinterpret_cast<uint32_t *>(o.carry + s)[lane] = word;
-                    else if (!DIAG) sm.res[lane][i - rbeg] = word;
-                }
-            }
-            __syncthreads();  // the list is free, the results are written
-            if (!DIAG && last && (uint32_t)t < rend - rbeg) {
-                const uint32_t s = own0 + rbeg + t;
-                Acc a;
-                uint32_t *aw = reinterpret_cast<uint32_t *>(&a);
-#pragma unroll
-                for (int c = 0; c < 12; ++c) aw[c] = sm.res[c][t];
-                finish_boid<DIAG>(a, g.pos[s], xyz(g.vel[s]), s, o, k);
+                if (last && rend < iend) __syncthreads();  // the results are read
             }
             if (last) break;
             lo = hi;
         }
+        if (t == 0) sm.work = w + run;
     }
 }
 
@@ -3399,7 +3425,7 @@ cudaError_t launch_ensemble_stats(const DevBuffers &b, int from, const FlockTabl
     if ((e = cudaMemsetAsync(err, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
     k_stat_moments<<<nb, kStatThreads, 0, st>>>(b.pos[from], b.vel[from], ft, acc, parent);
     k_stat_com<<<blocks_for(ft.count, 128), 128, 0, st>>>(acc, ft.ks, ft.count, com);
-    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, nullptr, nullptr};  // k_stat_pairs reads only cells
+    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum};  // k_stat_pairs reads only cells
     k_stat_pairs<<<nb, kStatThreads, 0, st>>>(g, ft, com, link, acc, parent, err);
     k_stat_roots<<<blocks_for(ft.nslots, 256), 256, 0, st>>>(ft, parent, size, err);
     k_stat_largest<<<blocks_for(ft.nslots, 256), 256, 0, st>>>(ft, parent, size, largest);

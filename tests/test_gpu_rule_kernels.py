@@ -64,6 +64,31 @@ def test_crowds_over_the_list_across_id_windows(boids_lib, oracle_mod, others):
     assert c.max() > 256
 
 
+@pytest.mark.parametrize("density,share", [(16, 0.0), (22, 0.0), (44, 0.0), (6, 1.0)])
+def test_items_done_together(boids_lib, density, share):
+    """So many dense-cell items that a CTA takes several at once, of cells with
+    a remainder to share among their items (34, 47 and 94 boids a cell) and of
+    clusters, against the thread-per-boid kernel alone."""
+    B = boids_lib
+    prm = dict(sep=(0.01, 0.5, 0.002), ali=(0.05, 1 / 3, 0.06), coh=(0.05, 0.5, 0.008), vmax=0.005, vmin=0.001)
+    n = 300001
+    field = (n / (16384 * density)) ** (1 / 3)
+    pos, vel = gathered(n, field, share, density, 90)
+    a, b = make_sim(B, "grid", n, field, prm), make_sim(B, "grid", n, field, prm)
+    b.set_tuning(*(1 << 30,) * 4)
+    for s in (a, b):
+        s.set_state(pos, vel)
+    for x, y in zip(a.neighbor_sets(), b.neighbor_sets()):
+        assert np.array_equal(x, y)
+    for s in (a, b):
+        s.update(1)
+    for x, y in zip(a.state(), b.state()):
+        assert_bits_equal(x, y, "state")
+    assert_bits_equal(a.forces(), b.forces(), "forces")
+    for s in (a, b):
+        s.close()
+
+
 @pytest.mark.parametrize("spread", [True, False])  # the crowd's ids over all, or the lowest
 @pytest.mark.parametrize("m", [16000, 17000, 36000])
 def test_crowds_over_one_plan_of_id_windows(boids_lib, m, spread):
