@@ -1244,23 +1244,28 @@ __device__ __forceinline__ void ovf_passes(SparseSmem &sm, int t, const uint64_t
 // slots in their buffers a step takes, us: 262 143 boids 167 (172), 2^20 one
 // update after a uniform start 377 (374), 6 after 406 (414), 20 after 803
 // (847), 100 after 1600 (1701), 400 after 2075 (2178), 2^22 4 after 1390 (1425).
-// (With whole slots in one warp's buffer, 21 on an SM: 420 after 6.)
+// (With whole slots in one warp's buffer, 21 on an SM: 420 after 6.)  An
+// ensemble's CTAs have four warps, for one copy of the flock's constants: with
+// one a step of 16 uniform flocks of 16 384 took 188 us for 165, 15 updates
+// after 290 for 260; gathered 812 for 825.
+__host__ __device__ constexpr int sparse_warps(bool ensemble) { return ensemble ? 4 : 1; }
 template <bool DIAG, bool MULTI>
-__global__ void __launch_bounds__(32, 24)
+__global__ void __launch_bounds__(32 * sparse_warps(MULTI), 24 / sparse_warps(MULTI))
 k_grid_sparse(GridIn g, GridOut o, StepConst kp, FlockTable ft)
 {
-    static_assert(kSlotAlign % 32 == 0, "a CTA serves one flock");
+    constexpr int kW = sparse_warps(MULTI);
+    static_assert(kSlotAlign % (32 * kW) == 0, "a CTA serves one flock");
     // the tables, and an ensemble's flock's constants
-    __shared__ __align__(16) unsigned char smem[sizeof(SparseSmem) + (MULTI ? sizeof(StepConst) : 0)];
-    SparseSmem &sm = *reinterpret_cast<SparseSmem *>(smem);
-    StepConst &kf = *reinterpret_cast<StepConst *>(smem + (MULTI ? sizeof(SparseSmem) : 0));
+    __shared__ __align__(16) unsigned char smem[kW * sizeof(SparseSmem) + (MULTI ? sizeof(StepConst) : 0)];
+    SparseSmem &sm = reinterpret_cast<SparseSmem *>(smem)[kW > 1 ? threadIdx.x >> 5 : 0];
+    StepConst &kf = *reinterpret_cast<StepConst *>(smem + (MULTI ? kW * sizeof(SparseSmem) : 0));
     if (g.chain) chain_wait();
-    if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * 32 / kSlotAlign]);
+    if (MULTI) load_flock(kf, ft, ft.blk_flock[blockIdx.x * 32 * kW / kSlotAlign]);
     const StepConst &k = MULTI ? kf : kp;
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     // this warp's boids outside dense cells (the others are k_grid_dense's)
-    const uint32_t s = blockIdx.x * 32 + lane;
+    const uint32_t s = blockIdx.x * 32 * kW + threadIdx.x;
     bool act = s - k.slot_base < k.n;
     const float4 p4 = act ? g.pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 v4 = act ? g.vel[s] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -3126,7 +3131,9 @@ cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, co
         if (e != cudaSuccess) return e;
     }
     if (b.aux && (e = cudaStreamWaitEvent(st, b.cjoin, 0)) != cudaSuccess) return e;  // the classification
-    if ((e = launch_chain(g.chain, k_grid_sparse<DIAG, MULTI>, nsp * (kRT / 32), 32, 0, st, g, o, k, ft)) != cudaSuccess) return e;
+    e = launch_chain(g.chain, k_grid_sparse<DIAG, MULTI>, nsp * (kRT / 32 / sparse_warps(MULTI)),
+                     32 * sparse_warps(MULTI), 0, st, g, o, k, ft);
+    if (e != cudaSuccess) return e;
     const unsigned nmore = MULTI ? nsp : min(nsp, 2 * b.dense_grid);
     if (o.defer && b.aux) {
         // the deferred boids and the dense cells are disjoint: run them side by side
