@@ -181,6 +181,7 @@ struct DevBuffers {
                                // k_grid_warp takes every boid (null: it never does)
     uint8_t *dflag;            // per full-size cell: 1 when the dense kernel takes it
     void *carry;               // per slot, kCarryBytes: partial sums between id windows (null: no windows)
+    double crowd_min, crowd_max;  // an ensemble: the pairs from which, and up to which, its boids go a warp each
     uint32_t *flag;            // set_state range check (1 word)
     uint32_t ncell, ncell_pad, nscan_blocks;
     uint32_t dense_grid;       // CTAs of the dense-cell kernel
@@ -250,27 +251,59 @@ constexpr uint32_t kWarpBoids = 40960;
 // Larger ones, up to kCrowdBoids boids (an ensemble's kCrowdSlots), are sent
 // there or by the split step for step, on the device, by the pairs of boids
 // that share an x cell (counted by the scan): a warp per boid from
-// n (kCrowdBase + kCrowdSlope n) pairs up to n (kCrowdTop - kCrowdTopSlope n),
-// above which boids accept more neighbours than k_grid_warp's list holds.
-// Without id windows in the split (the allocation-free step) there is no upper
-// line.  The split of an ensemble and of the
-// allocation-free step has no side stream and no deferral, so their line
-// starts lower, at kCrowdBare, and an ensemble's stays there.  A uniform flock
+// crowd_line pairs a boid up to crowd_top, above which boids
+// accept more neighbours than k_grid_warp's list holds.  Without id windows in
+// the split (the allocation-free step) there is no upper line.  A uniform flock
 // at the reference's density has 0.29 n pairs, a gathered one 1 to 3.2 n.  A
 // step, us, by the split / a warp per boid: 65 537 boids at 0.53 n 106 / 111,
 // at 0.72 n 194 / 117, at 1.3 n 290 / 134, at 3.0 n 264 / 177; 131 072 at
 // 0.55 n 145 / 190, at 0.75 n 252 / 210, at 1.3 n 370 / 238; 262 143 at 0.75 n
 // 331 / 430, at 0.94 n 419 / 412, at 1.3 n 511 / 447, at 3.1 n 632 / 614;
 // 370 000 at 1.3 n 626 / 620, at 3.1 n 870 / 860.  Without id windows in the
-// split (the allocation-free step), 65 537 at 2.3 n 2990 / 163.  200 steps of a
-// sweep's ensembles: 90 000 slots 79.3 / 46.0 ms, 266 000 176 / 156, 825 000
-// 427 / 433.  Flocks collapsed into clusters, at 4, 8 and 16 n pairs: 50 000
+// split (the allocation-free step), 65 537 at 2.3 n 2990 / 163.  Ensembles of
+// flocks that gather together, whose split has no side stream and no
+// deferral: 65 536 slots at 0.38 n 116 / 133, at 0.46 n 141 / 135; 131 072 at
+// 0.68 n 225 / 239, at 0.79 n 269 / 243; 262 144 at 0.68 n 359 / 431, at 0.79 n
+// 429 / 440, at 1.0 n 533 / 462; 491 520 at 0.79 n 725 / 792, at 1.0 n 891 / 826.
+// Flocks collapsed into clusters, at 4, 8 and 16 n pairs: 50 000
 // boids 353 / 156, 233 / 250, 339 / 693; 262 143 599 / 653, 689 / 1170,
 // 1053 / 9348; an ensemble of 16 flocks of 8192 at 4 and 8 n 550 / 392 and
-// 465 / 517.
+// 465 / 517.  Flocks of up to kWarpBoids, which know no such line, take longer
+// than by the split only where they have collapsed, from 24 576 boids on (at most
+// 2.1 times, 40 960 in clusters of 4000: 2242 / 1180).
 constexpr uint32_t kCrowdBoids = 1u << 18, kCrowdSlots = 1u << 19;
-constexpr double kCrowdTop = 8.5, kCrowdTopSlope = 1.6e-5;
-constexpr double kCrowdBase = 0.47, kCrowdBare = 0.35, kCrowdSlope = 1.75e-6;
+constexpr double kCrowdTop = 8.5, kCrowdTopSlope = 1.6e-5, kCrowdTopEnsemble = 6.0;
+enum CrowdKind { CROWD_HANDLE, CROWD_BARE, CROWD_ENSEMBLE };  // the split's form: a handle's, the allocation-free step's, ...
+// The pairs a boid from which a flock goes a warp per boid: even is what the
+// flock would have spread evenly over its cells, n the boids (slots) of the step.
+inline double crowd_line(double even, double n, CrowdKind kind)
+{
+    const bool many = kind == CROWD_ENSEMBLE;
+    const double line = many ? std::fmin(0.2 + 3.8e-6 * n, 0.78 + 2.5e-7 * n)
+                             : (kind == CROWD_HANDLE ? 0.47 : 0.35) + 1.75e-6 * n;
+    // From 3.3 times the reference's density on a flock that is still even
+    // makes full items of all its cells, the split's best state, until so many
+    // cells have more candidates than the shared list (or, in small flocks, too few
+    // items): at 6 times the density 262 143 boids 445 / 554 us a step, 65 537
+    // 144 / 164, the allocation-free step of 262 143 520 / 553, 48 flocks of 8192
+    // 733 / 988; at 8 times 65 537 216 / 201; at 12 times 131 072 429 / 416.
+    if (even >= 0.95) {
+        const double most = many ? 1.2 + 2.3e-11 * n * n : (kind == CROWD_HANDLE ? 1.6 + 1e-5 * n : (n < 150000 ? 0. : 2.));
+        return std::fmax(line, std::fmin(1.5 * even, most));
+    }
+    // From 1.45 times on its cells of a few boids have too many candidates for a
+    // thread each: an ensemble's split is at its worst (16 flocks of 16 384 at twice
+    // the density 658 / 457).
+    return many && even >= 0.42 ? even - 0.45 : line;
+}
+// And up to which: beyond what an even flock has, as long as its boids' lists hold that
+// (at 24 times the density 65 537 boids 487 / 351, 262 143 1331 / 1207).  The line
+// falls with the ids that a boid's search has to pass over, which are an ensemble's
+// flock's own, however many flocks there are.
+inline double crowd_top(double even, double n, CrowdKind kind)
+{
+    return (kind == CROWD_ENSEMBLE ? kCrowdTopEnsemble : kCrowdTop - kCrowdTopSlope * n) + (even <= 14. ? even : 0.);
+}
 // The autotuners time the default set with the choice above (or the split, if
 // the flock has no other: routed == false), the others with the split.  What a
 // flock gains now it can lose many times over once its state has changed: on a

@@ -141,7 +141,7 @@ int step_once(boids_ensemble *e)
 {
     if (!e->binned) {
         CK(boidsgpu::launch_grid_scan(e->ks[0], e->b, e->stream, &e->launches, &e->ft));
-    CK(boidsgpu::launch_grid_classify(e->ks[0], e->b, e->stream, &e->launches, &e->ft));
+        CK(boidsgpu::launch_grid_classify(e->ks[0], e->b, e->stream, &e->launches, &e->ft));
         CK(boidsgpu::launch_grid_scatter(e->ks[0], e->b, e->cur, true, e->stream, &e->launches, &e->ft));
         e->cur = 1 - e->cur;
     }
@@ -339,6 +339,12 @@ int boids_ensemble_create(const boids_flock_desc *flocks, uint32_t count, boids_
     ALLOC(&b.dense_list, boidsgpu::dense_list_capacity(b.ncell, e->total_boids));
     ALLOC(&b.dense_n, 4);
     if (ns <= boidsgpu::kCrowdSlots) ALLOC(&b.slot_of, ns);
+    for (const StepConst &k : e->ks) {
+        const double even = k.n / (8.0 * k.G * k.G * k.G);
+        b.crowd_min += k.n * boidsgpu::crowd_line(even, (double)ns, boidsgpu::CROWD_ENSEMBLE);
+        b.crowd_max += k.n * boidsgpu::crowd_top(even, (double)ns, boidsgpu::CROWD_ENSEMBLE);
+    }
+    b.crowd_min = std::max(b.crowd_min, 0.0);
     ALLOC(&b.dflag, b.ncell / 4);
     {
         unsigned char *carry = nullptr;

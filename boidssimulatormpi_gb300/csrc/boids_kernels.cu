@@ -2950,10 +2950,11 @@ static inline Crowd crowd_route(const StepConst &k, const DevBuffers &b, const F
 {
     if (!b.slot_of || k.tuned || grid_by_warp(k, b, ft)) return Crowd{nullptr, 0, 0};
     const double n = ft ? ft->nslots : k.n;
-    const double line = (ft || !b.carry ? kCrowdBare : kCrowdBase) + (ft ? 0. : kCrowdSlope * n);
-    const double top = !b.carry ? 1e9 : kCrowdTop - kCrowdTopSlope * n;
-    const uint32_t min = (uint32_t)(n * line);
-    return Crowd{b.dense_n + 3, min, (uint32_t)fmax(0., fmin(4e9, n * top) - min)};
+    const double even = n / (2. * b.ncell);
+    const double from = ft ? b.crowd_min : n * crowd_line(even, n, b.carry ? CROWD_HANDLE : CROWD_BARE);
+    const double to = !b.carry ? 4e9 : (ft ? b.crowd_max : n * crowd_top(even, n, CROWD_HANDLE));
+    const uint32_t min = (uint32_t)fmin(4e9, from);
+    return Crowd{b.dense_n + 3, min, (uint32_t)fmax(0., fmin(4e9, to) - min)};
 }
 
 cudaError_t launch_pack(const float *pos3, const float *vel3, float4 *pos4, float4 *vel4, uint32_t i0, uint32_t i1,
