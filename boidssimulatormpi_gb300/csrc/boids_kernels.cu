@@ -504,8 +504,9 @@ __global__ void __launch_bounds__(kScanThreads)
 k_grid_scan(const uint32_t *__restrict__ count, uint32_t *__restrict__ lstart, uint32_t *bsum,
             uint32_t *ticket, uint32_t nblocks, uint32_t *__restrict__ work, int measure)
 {
-    __shared__ uint32_t warp_tot[kScanThreads / 32];
+    __shared__ uint32_t warp_tot[kScanThreads / 32], block_pairs;
     __shared__ bool is_last;
+    if (threadIdx.x == 0) block_pairs = 0;
     chain_wait();
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     const uint4 a = *reinterpret_cast<const uint4 *>(count + base);
@@ -529,10 +530,11 @@ k_grid_scan(const uint32_t *__restrict__ count, uint32_t *__restrict__ lstart, u
             if (c > 1) pairs += c * (c - 1) / 2;
         }
         pairs = __reduce_add_sync(0xffffffffu, pairs);
-        if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(ticket + 1, pairs);
+        if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&block_pairs, pairs);
+        __syncthreads();  // every warp's pairs before the block's ticket
     }
-    if (measure) __syncthreads();  // every warp's pairs before the block's ticket
     if (threadIdx.x == 0) {
+        if (measure && block_pairs) atomicAdd(ticket + 1, block_pairs);
         bsum[blockIdx.x] = total;
         __threadfence();
         is_last = atomicAdd(ticket, 1u) == nblocks - 1;
@@ -3128,7 +3130,8 @@ cudaError_t grid_force(const StepConst &k, const GridIn &g, const GridOut &o, co
     cudaError_t e = dense_smem_opt_in<DIAG, MULTI>();
     if (e != cudaSuccess) return e;
     if (g.crowd.pairs) {
-        e = launch_chain(!MULTI, k_grid_warp_queue<DIAG, MULTI>, b.dense_grid, kWarpWarps * 32, 0, st, g, o, b.dense_n + 1, k, ft);
+        e = launch_chain(true, k_grid_warp_queue<DIAG, MULTI>, b.dense_grid, kWarpWarps * 32, 0, st, g, o,
+                         b.dense_n + 1, k, ft);
         if (e != cudaSuccess) return e;
     }
     if (b.aux && (e = cudaStreamWaitEvent(st, b.cjoin, 0)) != cudaSuccess) return e;  // the classification
