@@ -488,6 +488,9 @@ int boids_create(const boids_params *params, boids_sim **out)
     ALLOC(&b.vel[1], n);
     ALLOC(&b.stage, 6 * n);
     ALLOC(&b.flag, 1, true);
+    int nsm = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p.device);
+    b.sms = (uint32_t)std::max(1, nsm);
     if (G) {
         b.ncell = (uint32_t)(4 * G) * G * G;
         b.ncell_pad = (b.ncell + 1 + boidsgpu::kScanTile - 1) / boidsgpu::kScanTile * boidsgpu::kScanTile;
@@ -535,9 +538,7 @@ int boids_create(const boids_params *params, boids_sim **out)
             delete s;
             return cuda_fail(ce, "cudaStreamCreate (side stream)");
         }
-        int nsm = 0;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p.device);
-        b.dense_grid = (uint32_t)std::max(1, nsm) * boidsgpu::kDenseCtasPerSm;
+        b.dense_grid = b.sms * boidsgpu::kDenseCtasPerSm;
         b.wcap = (uint32_t)std::min<size_t>(boidsgpu::kWinScratch, std::max<size_t>(n, 1));
         ALLOC(&b.wscratch, (size_t)b.wcap * b.dense_grid);
     }

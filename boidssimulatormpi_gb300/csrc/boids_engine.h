@@ -177,13 +177,14 @@ struct DevBuffers {
     // forked from and joined back to the engine's stream (null: in order).
     cudaStream_t aux;
     cudaEvent_t fork, join, cjoin;  // cjoin: the classification's end (it runs beside the scatter)
-    uint32_t *slot_of;         // slot of each id after the scatter (from its flock's slot_base), kept where
-                               // k_grid_warp takes every boid (null: it never does)
+    uint32_t *slot_of;         // slot of each id after the scatter (from its flock's slot_base), for steps that
+                               // go a warp per boid (null: none does)
     uint8_t *dflag;            // per full-size cell: 1 when the dense kernel takes it
     void *carry;               // per slot, kCarryBytes: partial sums between id windows (null: no windows)
     double crowd_min, crowd_max;  // an ensemble: the pairs from which, and up to which, its boids go a warp each
     uint32_t *flag;            // set_state range check (1 word)
     uint32_t ncell, ncell_pad, nscan_blocks;
+    uint32_t sms;              // SMs of the device (a handle's)
     uint32_t dense_grid;       // CTAs of the dense-cell kernel
     uint32_t ap_cap;
 };
@@ -360,8 +361,6 @@ cudaError_t launch_unpack_index(const float4 *pos4, uint32_t *slot_of, uint32_t 
 cudaError_t launch_unpack_gather(const float4 *pos4, const float4 *vel4, const uint32_t *slot_of, float *pos3,
                                  float *vel3, uint32_t i0, uint32_t i1, uint32_t n, cudaStream_t s,
                                  uint64_t *launches);
-cudaError_t launch_unpack(const float4 *pos4, const float4 *vel4, uint32_t *slot_of, float *pos3, float *vel3,
-                          uint32_t n, cudaStream_t s, uint64_t *launches);
 // One .ptcl frame in id order: pframe gets 3 floats per boid, or 12 with
 // forces (xyz + the nine get_force floats; zeros when force9 is null);
 // vframe (nullable) gets vx,vy,vz.

@@ -2990,14 +2990,6 @@ cudaError_t launch_unpack_gather(const float4 *pos4, const float4 *vel4, const u
     return cudaGetLastError();
 }
 
-cudaError_t launch_unpack(const float4 *pos4, const float4 *vel4, uint32_t *slot_of, float *pos3, float *vel3,
-                          uint32_t n, cudaStream_t st, uint64_t *launches)
-{
-    cudaError_t e = launch_unpack_index(pos4, slot_of, n, st, launches);
-    if (e != cudaSuccess) return e;
-    return launch_unpack_gather(pos4, vel4, slot_of, pos3, vel3, 0, n, n, st, launches);
-}
-
 cudaError_t launch_frame(const float4 *pos4, const float4 *vel4, const float *force9, float *pframe,
                          float *vframe, int with_forces, uint32_t n, cudaStream_t st, uint64_t *launches)
 {
@@ -3204,7 +3196,7 @@ cudaError_t launch_allpairs(const StepConst &k, const DevBuffers &b, int from, b
     // the j tiles shrink until the GPU has a few CTAs per SM: where every pair
     // passes the filter (a small field), the exact tests are the work
     uint32_t tile_j = kApTileJ;
-    while (tile_j > 16 && (uint64_t)blocks_for(k.n, kApTileI) * blocks_for(k.n, tile_j) < 4 * 152) tile_j /= 2;
+    while (tile_j > 16 && (uint64_t)blocks_for(k.n, kApTileI) * blocks_for(k.n, tile_j) < 4 * b.sms) tile_j /= 2;
     dim3 grid(blocks_for(k.n, kApTileI), blocks_for(k.n, tile_j));
     k_ap_pairs<<<grid, kApThreads, 0, st>>>(b.pos[from], b.vel[from], b.ap_emb, b.ap_cnt, b.ap_list, b.ap_cap, tile_j,
                                             k);
@@ -3221,7 +3213,7 @@ cudaError_t launch_allpairs(const StepConst &k, const DevBuffers &b, int from, b
         o.vel_out = b.vel[1 - from];
         o.forces = record_forces ? b.forces : nullptr;
     }
-    const unsigned nb = min(blocks_for(k.n, kWarpWarps), 152u * kWarpCtas), nt = kWarpWarps * 32;
+    const unsigned nb = min(blocks_for(k.n, kWarpWarps), b.sms * kWarpCtas), nt = kWarpWarps * 32;
     if (diag) {
         k_ap_accumulate<true><<<nb, nt, 0, st>>>(b.pos[from], b.vel[from], b.ap_cnt, b.ap_list, b.ap_cap, o, k);
     } else {

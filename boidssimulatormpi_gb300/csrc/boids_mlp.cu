@@ -370,7 +370,7 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
 #pragma unroll
     for (int e = 0; e < 8; ++e) b1r[e] = b1[k0 + e];
     // the first layer of a tile (its inputs in sx) into shared memory: warp w
-    // takes rows w, w + 8, ..., lane its 8 columns; rows past the end are zero
+    // takes rows w, w + 16, ..., lane its 8 columns; rows past the end are zero
     auto layer1 = [&](int tile) {
         const int m0 = tile * kTcM;
         for (int r = warp; r < kTcM; r += kTcFwdThreads / 32) {
@@ -429,7 +429,7 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
     uint32_t phase = 0, buf = 0;
     if (t == 0 && (int)blockIdx.x < ntiles) issue(0);
     constexpr int kPart = kTcN / kTcFwdParts;  // columns of a warp
-    const int quarter = warp & 3, half = warp >> 2;  // accumulator lanes 32 * quarter.., columns kPart * half..
+    const int quarter = warp & 3, part = warp >> 2;  // accumulator lanes 32 * quarter.., columns kPart * part..
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int nxt = tile + gridDim.x;
         if (nxt < ntiles) load_x(nxt);  // sx is free: this tile's first layer is done
@@ -460,12 +460,12 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
                 issue((buf ^ 1u) * kTcN);
             }
         }
-        // epilogue: bias, ReLU, BF16 and the output layer over this warp's half of the columns
+        // epilogue: bias, ReLU, BF16 and the output layer over this warp's part of the columns
         const int rl = quarter * 32 + lane;  // row within the tile
         const uint32_t trow = tmem + buf * kTcN + ((uint32_t)(quarter * 32) << 16);
         float yo[kTcOut] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-        for (int c = half * kPart; c < (half + 1) * kPart; c += 32) {
+        for (int c = part * kPart; c < (part + 1) * kPart; c += 32) {
             uint32_t v[32];
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -485,10 +485,10 @@ k_mlp_forward_tc(const float *__restrict__ x, int rows, const __nv_bfloat16 *__r
                 for (int j = 0; j < kTcOut; ++j) yo[j] = __fmaf_rn(hv, sw3[(c + e) * kTcOut + j], yo[j]);
             }
         }
-        *reinterpret_cast<float4 *>(ypart + (half * kTcM + rl) * kTcOut) = make_float4(yo[0], yo[1], yo[2], yo[3]);
+        *reinterpret_cast<float4 *>(ypart + (part * kTcM + rl) * kTcOut) = make_float4(yo[0], yo[1], yo[2], yo[3]);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();  // this accumulator is read before a later tile's product reuses it
-        if (half == 0) {
+        if (part == 0) {
             const int r = tile * kTcM + rl;
             float4 a = *reinterpret_cast<const float4 *>(ypart + rl * kTcOut);
 #pragma unroll
@@ -1367,10 +1367,11 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
     if (batch > rows) batch = rows;
     m->img_valid = false;  // every batch lays its own out, and ends with other parameters
     if (int rc = ensure_rows(m, rows + batch)) return rc;
-    // the whole set stays resident: rows [0, rows) of x/t; batches are gathered behind it
+    // the whole set stays resident: rows [0, rows) of x/t
     float *X = m->x, *T = m->t;
+    const bool fused = batch_is_fused(m);
     int *d_idx = nullptr;
-    float *bx = nullptr, *bt = nullptr;
+    float *bx = nullptr, *bt = nullptr;  // a gathered batch (the fused one gathers for itself)
     // An epoch's order lies in one of two host arrays, and its copy may read the
     // array as late as the stream comes to it: `sent` says when it has, and the
     // array is rewritten after that.  With two, an epoch's order is drawn and
@@ -1385,8 +1386,8 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
         cudaFree(bt);
     };
     if (cudaMalloc(&d_idx, sizeof(int) * rows) != cudaSuccess ||
-        cudaMalloc(&bx, sizeof(float) * (size_t)batch * m->in) != cudaSuccess ||
-        cudaMalloc(&bt, sizeof(float) * (size_t)batch * m->out) != cudaSuccess) {
+        (!fused && (cudaMalloc(&bx, sizeof(float) * (size_t)batch * m->in) != cudaSuccess ||
+                    cudaMalloc(&bt, sizeof(float) * (size_t)batch * m->out) != cudaSuccess))) {
         cudaGetLastError();
         release();
         return fail(BOIDS_ENOMEM, "boids_mlp_train: cudaMalloc failed");
@@ -1397,7 +1398,6 @@ int boids_mlp_train(boids_mlp *m, const float *x, const float *t, int32_t rows, 
     double epoch_loss = 0.0;
     int rc = 0;
     float *keep_x = m->x, *keep_t = m->t;
-    const bool fused = batch_is_fused(m);
     if (cudaEventCreateWithFlags(&sent[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&sent[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaMemcpyAsync(X, x, sizeof(float) * (size_t)rows * m->in, cudaMemcpyHostToDevice, m->st) != cudaSuccess ||
