@@ -35,6 +35,9 @@ def lines(tmp_path_factory):
     (0.29, 0.37, 262144, ENSEMBLE, False), (0.29, 0.68, 262144, ENSEMBLE, False), (0.29, 1.0, 262144, ENSEMBLE, True),
     (0.29, 0.79, 491520, ENSEMBLE, False), (0.29, 1.34, 491520, ENSEMBLE, True), (0.29, 3.1, 491520, ENSEMBLE, True),
     (0.29, 3.7, 393216, ENSEMBLE, True),
+    # a quarter of it
+    (0.07, 0.27, 100000, ENSEMBLE, False), (0.07, 0.50, 100000, ENSEMBLE, True),
+    (0.07, 0.62, 256000, ENSEMBLE, False), (0.07, 1.15, 256000, ENSEMBLE, True),
     # uniform at twice, 6, 12 and 24 times that, and the same gathered
     (0.58, 0.58, 262144, ENSEMBLE, True), (0.58, 0.58, 393216, ENSEMBLE, True),
     (1.74, 1.74, 65537, HANDLE, False), (1.74, 1.74, 262143, HANDLE, False), (1.74, 3.0, 65537, HANDLE, True),
