@@ -376,8 +376,10 @@ def run_allpairs(a, B, local, stream, torch):
     peak = (measured or 1900.0) * 1e12
     return {"n": n, "field_size": field, "kernels": "all pairs (N^2): k_ap_pairs + k_ap_accumulate",
             "steps": steps, "ms_per_step": ms, "value": n / (ms / 1e3), "unit": UNIT,
-            "roofline": {"bound": "issue (ALU and mma.sync)", "achieved": achieved / 1e12, "peak": peak / 1e12,
+            "roofline": {"bound": "bf16 matrix product", "achieved": achieved / 1e12, "peak": peak / 1e12,
                          "unit": "TFLOP/s (the filter's 8-deep product)", "frac": achieved / peak,
+                         "limited_by": "mma.sync's rate and the ALU work on its results (profiles/"
+                                       "ncu_rule_kernels_warp_per_boid.md)",
                          "ops_per_pair": 16, "pairs_per_step": pairs, "pairs_per_s": pairs / (ms / 1e3),
                          "peak_source": "measured" if measured else "fallback"},
             "clocks": c}

@@ -849,8 +849,9 @@ __global__ void k_grid_classify(const uint32_t *__restrict__ lstart,
 // max-over-warp length).  Candidates passing the squared-distance filter are
 // buffered, and whenever one buffer is nearly full the warp runs the exact
 // tests of all its lanes' hits, dealt to its lanes 32 at a time whichever
-// lane found them, so the expensive test runs with nearly every lane busy.  The filter drops candidates behind the boid (the view-cone
-// pre-test, StepConst::dot_eps).  Accepted neighbours are kept sorted by id,
+// lane found them, so the expensive test runs with nearly every lane busy.  The
+// filter drops candidates behind the boid (the view-cone pre-test,
+// StepConst::dot_eps).  Accepted neighbours are kept sorted by id,
 // at most kListA per pass; a boid with more takes further passes, each
 // keeping the next kListA ids, so accumulation is always in ascending id --
 // for a single flock in k_grid_sparse_more, so that those passes run in full
@@ -1401,13 +1402,13 @@ k_grid_sparse_more(GridIn g, GridOut o, StepConst kp, FlockTable ft)
 // which needs no sort: the filter's hits are marked in a bit map over ids.
 //
 // Bound by instruction issue once every SM has its 32 warps, by the length of
-// one boid's chain of loads, tests and sums below that (about 15 us).  A step
-// of 1000 boids of test.ini takes 28 us where the split of cells over
-// k_grid_sparse and k_grid_dense took 109 (their few CTAs leave most SMs
-// idle), gathered flocks of 16 384 boids 54 us (188), of 32 768 boids 90 us
-// (215), uniform ones 36 us (65) and 58 us (74), all with the counting sort.
-// Per-boid work is about five times k_grid_sparse's on a uniform flock
-// (1240 warp instructions against 190 a boid), hence kWarpBoids.
+// one boid's chain of loads, tests and sums below that (about 14 us).  A step
+// of 1000 boids of test.ini takes 21 us (28 before its counting sort was one
+// kernel) where the split of cells over k_grid_sparse and k_grid_dense took 109
+// (their few CTAs leave most SMs idle), gathered flocks of 16 384 boids 54 us
+// (188), of 32 768 boids 90 us (215), uniform ones 35 us (63) and 56 us (74), all
+// with the counting sort.  Per-boid work is about five times k_grid_sparse's on a
+// uniform flock (1240 warp instructions against 206 a boid), hence kWarpBoids.
 constexpr int kWarpWarps = 4;    // warps of a CTA
 constexpr int kWarpCtas = 8;     // CTAs per SM
 constexpr int kWarpList = 256;   // accepted neighbours kept
@@ -2251,8 +2252,8 @@ __device__ void dense_window_plan(DenseSmem &sm, const GridIn &g, int ns, uint32
 // each fit the list; the sums are carried from window to window through
 // o.carry.
 //
-// Bound by instruction issue (74 % of the slots at 8 CTAs per SM, N = 2^20
-// after 1000 updates).  A warp per boid replaced a lane per (boid, chunk of
+// Bound by instruction issue (76 % of the slots at 8 CTAs per SM, N = 2^20
+// after 1000 updates: 2.20 ms).  A warp per boid replaced a lane per (boid, chunk of
 // candidates) with rule masks and a lane per sum: that form needed a round of
 // up to 72 boids to fill its lanes, so items held up to 128 boids and a small
 // flock's few items left most SMs idle.  Items of 32 boids and no barrier
@@ -2630,17 +2631,17 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
 // not exact enough.
 //
 // 64 boids a warp against 8 at a time: four mma.m16n8k8, and an AND over their
-// 16 results a lane, whose sign says whether any pair passed.  Survivors are queued per warp and take the exact
-// tests 32 at a time; accepted neighbours are appended to the boid's list
-// (unordered).
+// 16 results a lane, whose sign says whether any pair passed.  Survivors are
+// queued per warp and take the exact tests 32 at a time; accepted neighbours are
+// appended to the boid's list (unordered).
 //
-// Bound by instruction issue (62 % of the slots, the tensor pipe 57 % active):
-// 1024 pairs take 67 warp instructions, half of them in the 40 % of the steps
-// in which some pair passes, where a box filter on the FP32 offsets took 15.7
-// per pair and thread.  N = 65 536, F = 1.6: an update takes 0.415 ms (1.87
-// with that filter), 1.0e13 pairs/s.  Only the j tile of a step in which some
-// pair passed is looked through: 0.427 ms with both, and 0.613 against 0.648
-// at F = 0.9.  One code path tests the queue: inlined at each of the 32
+// Bound by the tensor pipe and the work on its results (68 % and, on the ALU,
+// 65 % busy, 62 % of the issue slots): 1024 pairs take 58 warp instructions,
+// where a box filter on the FP32 offsets took 15.7 per pair and thread.
+// N = 65 536, F = 1.6: an update takes 0.411 ms from a uniform start (1.82 with
+// that filter), 1.0e13 pairs/s, and 0.452 over the next 60; 65 537 boids 0.412 (0.674 with a last tile's missing rows not
+// rejected by the product).  Only the j tile of a step in which some pair passed
+// is looked through: 0.427 ms with both before the last change, 0.415 with it.  One code path tests the queue: inlined at each of the 32
 // results it cost 0.1 ms in instruction fetches.  mma.sync serves better than
 // tcgen05 here: the product is eight deep and every one of its N^2 results has
 // to come back through registers to be compared, so the tensor rate is not
