@@ -22,7 +22,7 @@
 //                  than one pass are queued, with the neighbours their list
 //                  could not keep, for
 //   k_grid_sparse_more, which runs their further passes in full warps beside
-//   k_grid_dense   one CTA per 32 boids of a crowded cell; the 27-cell
+//   k_grid_dense   one CTA per about 32 boids of a crowded cell; the 27-cell
 //                  candidates are sorted by id once in shared memory, and a
 //                  warp per boid filters, tests and adds them up in id order.
 // All integrate, write the new state in place of the sorted slot and bin it
