@@ -300,13 +300,27 @@ inline double crowd_line(double even, double n, CrowdKind kind)
     // the density 658 / 457).
     return many && even >= 0.42 ? even - 0.45 : line;
 }
-// And up to which: beyond what an even flock has, as long as its boids' lists hold that
-// (at 24 times the density 65 537 boids 487 / 351, 262 143 1331 / 1207).  The line
+// And up to which: beyond what an even flock has, as long as k_grid_warp's lists
+// hold the neighbours that its boids accept on average (at 24 times the density, 103
+// of them, 65 537 boids 487 / 351 us, 262 143 1331 / 1207; at 48 times, 206, 632 /
+// 883 and 2310 / 2763; at 56 times, 240, 1413 / 929 and 11 900 / 2865).  The line
 // falls with the ids that a boid's search has to pass over, which are an ensemble's
 // flock's own, however many flocks there are.
-inline double crowd_top(double even, double n, CrowdKind kind)
+constexpr double kCrowdSeen = 207.;  // 3.5 deviations below the lists' 256
+inline double crowd_top(double even, double seen, double n, CrowdKind kind)
 {
-    return (kind == CROWD_ENSEMBLE ? kCrowdTopEnsemble : kCrowdTop - kCrowdTopSlope * n) + (even <= 14. ? even : 0.);
+    return (kind == CROWD_ENSEMBLE ? kCrowdTopEnsemble : kCrowdTop - kCrowdTopSlope * n) +
+           (seen <= kCrowdSeen ? even : 0.);
+}
+// The neighbours that a boid of an even flock accepts: the most of its rules' view cones hold.
+inline double crowd_seen(const StepConst &k)
+{
+    double most = 0.;
+    for (const RuleConst &q : k.rule) {
+        const double r = std::sqrt((double)q.d2_lim) / k.F;
+        most = std::fmax(most, k.n * 4.18879 * r * r * r * (q.all_round ? 1. : (1. - (double)q.cstar) / 2.));
+    }
+    return most;
 }
 // The autotuners time the default set with the choice above (or the split, if
 // the flock has no other: routed == false), the others with the split.  What a

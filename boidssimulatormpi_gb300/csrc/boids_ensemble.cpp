@@ -354,7 +354,7 @@ int boids_ensemble_create(const boids_flock_desc *flocks, uint32_t count, boids_
     for (const StepConst &k : e->ks) {
         const double even = k.n / (8.0 * k.G * k.G * k.G);
         b.crowd_min += k.n * boidsgpu::crowd_line(even, (double)ns, boidsgpu::CROWD_ENSEMBLE);
-        b.crowd_max += k.n * boidsgpu::crowd_top(even, (double)ns, boidsgpu::CROWD_ENSEMBLE);
+        b.crowd_max += k.n * boidsgpu::crowd_top(even, boidsgpu::crowd_seen(k), (double)ns, boidsgpu::CROWD_ENSEMBLE);
     }
     b.crowd_min = std::max(b.crowd_min, 0.0);
     ALLOC(&b.dflag, b.ncell / 4);

@@ -2955,7 +2955,7 @@ static inline Crowd crowd_route(const StepConst &k, const DevBuffers &b, const F
     const double n = ft ? ft->nslots : k.n;
     const double even = n / (2. * b.ncell);
     const double from = ft ? b.crowd_min : n * crowd_line(even, n, b.carry ? CROWD_HANDLE : CROWD_BARE);
-    const double to = !b.carry ? 4e9 : (ft ? b.crowd_max : n * crowd_top(even, n, CROWD_HANDLE));
+    const double to = !b.carry ? 4e9 : (ft ? b.crowd_max : n * crowd_top(even, crowd_seen(k), n, CROWD_HANDLE));
     const uint32_t min = (uint32_t)fmin(4e9, from);
     return Crowd{b.dense_n + 3, min, (uint32_t)fmax(0., fmin(4e9, to) - min)};
 }

@@ -19,7 +19,8 @@ def lines(tmp_path_factory):
                     os.path.join(ROOT, "tests", "native", "crowd_lines.cpp"), "-o", exe], check=True)
 
     def get(even, n, kind):
-        r = subprocess.run([exe], input="%r %r %d\n" % (even, n, kind), capture_output=True, text=True, check=True)
+        seen = 14.8 * even  # marun2019's cones: half of the ball
+        r = subprocess.run([exe], input="%r %r %r %d\n" % (even, seen, n, kind), capture_output=True, text=True, check=True)
         return tuple(float(x) for x in r.stdout.split())
 
     return get
@@ -43,7 +44,8 @@ def lines(tmp_path_factory):
     (1.74, 1.74, 65537, HANDLE, False), (1.74, 1.74, 262143, HANDLE, False), (1.74, 3.0, 65537, HANDLE, True),
     (1.74, 1.74, 262143, BARE, False), (2.32, 2.32, 262143, BARE, True),
     (1.74, 1.74, 262144, ENSEMBLE, False), (1.74, 1.74, 65536, ENSEMBLE, True),
-    (3.48, 3.48, 131072, HANDLE, True), (4.64, 4.64, 393216, ENSEMBLE, False), (6.96, 6.96, 262143, HANDLE, True),
+    (3.48, 3.48, 131072, HANDLE, True), (4.64, 4.64, 393216, ENSEMBLE, False), (6.96, 6.96, 262143, HANDLE, True), (13.9, 13.9, 41000, HANDLE, True),
+    (16.4, 16.4, 131072, HANDLE, False),
     # collapsed
     (0.29, 16.0, 262143, HANDLE, False), (0.29, 8.0, 131072, ENSEMBLE, False), (43.0, 43.0, 65537, HANDLE, False),
 ])
