@@ -229,8 +229,10 @@ constexpr int kTuneCount = sizeof(kTuneCand) / sizeof(kTuneCand[0]);
 // gathered flocks 10 to 30 % up to 2^19 boids (262 143 400 updates after a
 // uniform start 777, now 655; 2^20 2350 and 2030).  Sharing remainders in all
 // cells, or taking several items at once until fewer are left (kDenseLeft 1, 2),
-// cost those 2 to 10 %.
+// cost those 2 to 10 %; in flocks of 41 000 to 65 537 boids, whose items are few,
+// sharing any cost 2 to 4 % (at 56 times the density 837 and 860).
 constexpr int kDenseItem = 32;
+constexpr uint32_t kDenseShare = 100000;  // boids from which remainders are shared
 constexpr uint32_t kDenseTake = 4;  // most items taken at once ...
 constexpr uint32_t kDenseLeft = 3;  // ... which is those left over, for every CTA so many times
 constexpr int kDenseRound = 64;     // boids whose results a CTA holds in shared memory, over an item's most
@@ -350,10 +352,11 @@ constexpr uint32_t kSortBoids = 1024, kSortCells = 4096;
 // of more takes longer than the launches it saves.
 constexpr uint32_t kBinBoids = 16384, kBinCells = 65536;
 constexpr int kDenseCap = 512;        // candidates of a dense cell held in shared memory
-// Boids per item of a dense cell of b boids with ncand candidates.
-__host__ __device__ inline uint32_t dense_per_item(uint32_t b, uint32_t ncand)
+// Boids per item of a dense cell of b boids with ncand candidates (share: the
+// step has kDenseShare boids or more).
+__host__ __device__ inline uint32_t dense_per_item(uint32_t b, uint32_t ncand, bool share)
 {
-    if (ncand <= (uint32_t)kDenseCap || b <= kDenseItem) return kDenseItem;
+    if (!share || ncand <= (uint32_t)kDenseCap || b <= kDenseItem) return kDenseItem;
     const uint32_t items = (b + kDenseItem / 2) / kDenseItem;
     return (b + items - 1) / items;
 }

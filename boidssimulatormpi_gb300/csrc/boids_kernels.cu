@@ -794,7 +794,7 @@ template <bool MULTI>
 __global__ void k_grid_classify(const uint32_t *__restrict__ lstart,
                                 const uint32_t *__restrict__ bsum, uint8_t *__restrict__ dflag,
                                 uint32_t *__restrict__ dense_list, uint32_t *__restrict__ dense_n, uint32_t nfull,
-                                int windows, Crowd crowd, StepConst kp, FlockTable ft)
+                                int windows, bool share, Crowd crowd, StepConst kp, FlockTable ft)
 {
     chain_wait();
     const uint32_t cg = blockIdx.x * blockDim.x + threadIdx.x;
@@ -828,7 +828,7 @@ __global__ void k_grid_classify(const uint32_t *__restrict__ lstart,
         }
         if (dense_rule(b, ncand, k, windows)) {
             flag = 1;
-            const uint32_t per = dense_per_item(b, ncand), items = (b + per - 1) / per;
+            const uint32_t per = dense_per_item(b, ncand, share), items = (b + per - 1) / per;
             const uint32_t at = atomicAdd(dense_n, items);
             for (uint32_t r = 0; r < items; ++r) {
                 dense_list[2 * (at + r)] = cg;
@@ -876,6 +876,7 @@ struct GridIn {
     const uint32_t *__restrict__ slot_of;  // k_grid_warp: slot of each id, from its flock's slot_base
     Crowd crowd;
     int chain;  // k_grid_sparse and k_grid_dense were launched in a chain
+    bool share;  // dense_per_item
 };
 
 struct SparseSmem {              // of one warp, a column per lane
@@ -2447,7 +2448,7 @@ k_grid_dense(GridIn g, GridOut o, const uint32_t *__restrict__ dense_list, uint3
             const unsigned below = (1u << lane) - 1u;
             uint16_t *hits = sm.hits[wid];
             float(&st)[9][kSumCols] = sm.v.st[wid];
-            const uint32_t iend = min(b, rbeg + run * dense_per_item(b, ncand));
+            const uint32_t iend = min(b, rbeg + run * dense_per_item(b, ncand, g.share));
             for (uint32_t r0 = rbeg; r0 < iend; r0 += kDenseRound) {  // a round's results at a time
                 const uint32_t rend = min(iend, r0 + (uint32_t)kDenseRound);
                 for (uint32_t i = r0 + wid; i < rend; i += kDT / 32) {
@@ -3065,7 +3066,7 @@ cudaError_t launch_grid_classify(const StepConst &k, const DevBuffers &b, cudaSt
         cs = b.aux;
     }
     e = launch_chain(chain, ft ? k_grid_classify<true> : k_grid_classify<false>, blocks_for(nfull, 256), 256, 0, cs,
-                     b.lstart, b.bsum, b.dflag, b.dense_list, b.dense_n, nfull, windows, crowd, k,
+                     b.lstart, b.bsum, b.dflag, b.dense_list, b.dense_n, nfull, windows, (ft ? ft->nslots : k.n) >= kDenseShare, crowd, k,
                      ft ? *ft : FlockTable{});
     if (e != cudaSuccess) return e;
     if (side && (e = cudaEventRecord(b.cjoin, b.aux)) != cudaSuccess) return e;
@@ -3154,7 +3155,7 @@ cudaError_t launch_grid_force(const StepConst &k, const DevBuffers &b, int from,
 {
     const uint32_t n = ft ? ft->nslots : k.n;
     if (n == 0) return cudaSuccess;
-    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, b.dflag, b.slot_of, crowd_route(k, b, ft), !b.aux && !ft};
+    GridIn g{b.pos[from], b.vel[from], b.lstart, b.bsum, b.dflag, b.slot_of, crowd_route(k, b, ft), !b.aux && !ft, n >= kDenseShare};
     GridOut o{};
     o.carry = static_cast<Acc *>(b.carry);
     o.wscratch = b.carry ? b.wscratch : nullptr;
